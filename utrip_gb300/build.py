@@ -73,8 +73,9 @@ def build(verbose: bool = False, extra: list[str] | None = None) -> Path:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
         os.replace(tmp, lib)
     probe = LIBDIR / PROBELIB
-    if not probe.exists() or probe.stat().st_mtime < PROBE.stat().st_mtime:
-        cmd = [nvcc(), ARCH, "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-shared",
+    deps = [PROBE, CSRC / "fd64.cuh"]
+    if not probe.exists() or any(probe.stat().st_mtime < d.stat().st_mtime for d in deps):
+        cmd = [nvcc(), ARCH, "-O3", "-std=c++17", "-Xcompiler", "-fPIC", f"-I{CSRC}", "-shared",
                str(PROBE), "-o", str(probe)]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:

@@ -5,6 +5,7 @@
 #pragma once
 #include "cans_common.cuh"
 #include "cans_internal.h"
+#include "fd64.cuh"
 
 namespace cans {
 
@@ -25,6 +26,14 @@ __device__ __forceinline__ double cfl3_cell(const double *__restrict__ S,
   const FT vx(S[P3::VX * n + g]), vy(S[P3::VY * n + g]), vz(S[P3::VZ * n + g]);
   const FT bx(S[P3::BX * n + g]), by(S[P3::BY * n + g]), bz(S[P3::BZ * n + g]);
   const FT b2 = bx * bx + by * by + bz * bz;
+  if constexpr (!E) {
+    // the same with one reciprocal and one reciprocal root: 16 FP64
+    // instructions in place of 42 (three divisions and a root)
+    const double v2 = fma(vx.v, vx.v, fma(vy.v, vy.v, vz.v * vz.v));
+    const double s = fma(fma(ph.gm, pr.v, b2.v * ph.pi4i_cfl), fd::rcp(ro.v), v2);
+    const double dm = fd::minp(fd::minp(ax.d[i], ay.d[j]), az.d[k]);
+    return safety * dm * fd::rsqrt_(s);
+  }
   const FT ca2 = b2 * FT(ph.pi4i_cfl) / ro;
   const FT cs2 = FT(ph.gm) * pr / ro;
   const FT v2 = vx * vx + vy * vy + vz * vz;

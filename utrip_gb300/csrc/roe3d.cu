@@ -149,7 +149,7 @@ __device__ __forceinline__ void roe_flux(const RoeK &K, const double *L,
 // to the sign of a zero result; the sign test runs on the integer pipe.
 __device__ __forceinline__ double minmod(double a, double b) {
   const long long x = __double_as_longlong(a) ^ __double_as_longlong(b);
-  return x >= 0 ? copysign(fmin(fabs(a), fabs(b)), a) : 0.0;
+  return x >= 0 ? fd::mul_sign(fd::minp(fd::abs_(a), fd::abs_(b)), a) : 0.0;
 }
 
 // Conserved variables of a primitive state (roe_m.f:42-47).
@@ -184,7 +184,7 @@ __device__ __forceinline__ void to_primitive(const RoeK &K, const F<E> *u,
     vy = u[U_RX + 1] / ro;
     vz = u[U_RX + 2] / ro;
   } else {
-    const T roi = T(1.0) / ro;
+    const T roi(fd::rcp(ro.v));
     vx = u[U_RX] * roi;
     vy = u[U_RX + 1] * roi;
     vz = u[U_RX + 2] * roi;
@@ -211,12 +211,13 @@ __device__ __forceinline__ void add_divergence(F<E> *u, const double *__restrict
   using T = F<E>;
   const double *Fa = Fl + (size_t)a * 8 * g.n;
   const size_t st = stride(g, a);
+  const T w = T(fac) * T(di);
 #pragma unroll
   for (int v = 0; v < 8; v++) {
     if (v == U_BX + a) continue;
     const T fm(__ldg(Fa + v * g.n + c - st)), f0(__ldg(Fa + v * g.n + c));
     if constexpr (E) u[v] = u[v] + T(fac) * ((fm - f0) / T(d));
-    else u[v] = u[v] + T(fac) * ((fm - f0) * T(di));
+    else u[v] = u[v] + w * (fm - f0);
   }
 }
 
@@ -352,6 +353,10 @@ __device__ __forceinline__ double cfl2_cell(const double *__restrict__ S, size_t
   const FT bx(S[P3::BX * n + g]), by(S[P3::BY * n + g]), bz(S[P3::BZ * n + g]);
   const FT b2 = bx * bx + by * by + bz * bz;
   const FT v2 = vx * vx + vy * vy + vz * vz;
+  if constexpr (!E) {  // one reciprocal and one reciprocal root (see cfl3_cell)
+    const double q = fma(fma(ph.gm, pr.v, b2.v * ph.pi4i), fd::rcp(ro.v), v2.v);
+    return safety * fd::minp(ax.d[i], ay.d[j]) * fd::rsqrt_(q);
+  }
   const FT ca2 = b2 * FT(ph.pi4i) / ro;
   const FT cs2 = FT(ph.gm) * pr / ro;
   const FT dtcfl = fmin_(FT(ax.d[i]), FT(ay.d[j])) / fsqrt(v2 + cs2 + ca2);
@@ -455,6 +460,7 @@ static RoeK make_roek(double gm) {
   k.ggm1 = gm / (gm - 1.0);
   k.sq4pi = std::sqrt(k.pi4);
   k.sq4pii = std::sqrt(k.pi4i);
+  k.gm218 = k.gm21 * k.pi8i;
   return k;
 }
 

@@ -1,8 +1,11 @@
 // Arithmetic peaks of the device for the benchmark's rooflines: the FP64
 // and FP32 fused-multiply-add throughput.  Built into its own library,
 // libcansprobe.so, beside libcansgpu.so: it is measurement tooling for
-// bench.py, not part of the C ABI of the solver.
+// bench.py, not part of the C ABI of the solver.  It also evaluates the FP64
+// functions of fd64.cuh on arrays, for their accuracy test.
 #include <cuda_runtime.h>
+
+#include "fd64.cuh"
 
 namespace {
 
@@ -61,4 +64,41 @@ extern "C" int cans_probe_fp64_tflops(double *tflops) {
 }
 extern "C" int cans_probe_fp32_tflops(double *tflops) {
   return measure<float>(tflops, 65536, 0.999999f, 1e-7f);
+}
+
+namespace {
+// op 0 rcp, 1 sqrt, 2 rsqrt, 3 and 4 the two results of sqrt_rsqrt, 5 lt(x, w),
+// 6 max(x, w), 7 the positive part
+__global__ void k_fd64(int op, const double *x, const double *w, double *y, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double a = x[i], b = w[i];
+  double s = 0.0, r = 0.0;
+  switch (op) {
+    case 0: r = cans::fd::rcp(a); break;
+    case 1: r = cans::fd::sqrt_(a); break;
+    case 2: r = cans::fd::rsqrt_(a); break;
+    case 3: cans::fd::sqrt_rsqrt(a, r, s); break;
+    case 4: cans::fd::sqrt_rsqrt(a, s, r); break;
+    case 5: r = cans::fd::lt(a, b) ? 1.0 : 0.0; break;
+    case 6: r = cans::fd::max_(a, b); break;
+    default: r = cans::fd::pos_part(a); break;
+  }
+  y[i] = r;
+}
+}  // namespace
+
+// y[i] = the function `op` of fd64.cuh of x[i] (and w[i]); host arrays.
+// Synchronous; 0 on success.
+extern "C" int cans_probe_fd64(int op, const double *x, const double *w, double *y, int n) {
+  if (n < 1 || !x || !w || !y || op < 0 || op > 7) return 1;
+  double *d = nullptr;
+  const size_t b = sizeof(double) * (size_t)n;
+  if (cudaMalloc(&d, 3 * b) != cudaSuccess) return 2;
+  cudaMemcpy(d, x, b, cudaMemcpyHostToDevice);
+  cudaMemcpy(d + n, w, b, cudaMemcpyHostToDevice);
+  k_fd64<<<(n + 255) / 256, 256>>>(op, d, d + n, d + 2 * (size_t)n, n);
+  const cudaError_t e = cudaMemcpy(y, d + 2 * (size_t)n, b, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e == cudaSuccess ? 0 : 2;
 }
