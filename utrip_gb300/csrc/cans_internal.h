@@ -131,6 +131,13 @@ cudaError_t launch_mlw3d(bool exact, int tile, const double *A, double *B,
                          int ix, int jx, int kx, const Axis &ax,
                          const Axis &ay, const Axis &az, const Phys &ph,
                          double dt, Ctl *ctl, Box3 box, cudaStream_t s);
+// The z chunk (at most kmax planes) that fills the GPU best (mlw3d.cu).
+int balance_kchunk(long long bxy, int nz, int kmax, int slots);
+// The fast policy's step of the three (mlw3d_fast.cu): grav, res or neither.
+cudaError_t launch_mlw3d_fast(int tile, const double *A, double *B, int ix, int jx, int kx,
+                              const Axis &ax, const Axis &ay, const Axis &az, const Phys &ph,
+                              double dt, Ctl *ctl, Box3 box, cudaStream_t s, const double *grav,
+                              const double *res);
 // 3-D mlw_m_g (mlw3d.cu): grav = gx, gxm, gy, gym, gz, gzm (n each)
 int mlw3d_g_tile_count();
 cudaError_t launch_mlw3d_g(bool exact, int tile, const double *A, double *B, int ix,

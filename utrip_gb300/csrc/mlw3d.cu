@@ -1,4 +1,5 @@
-// Fused 3-D modified Lax-Wendroff step (sm_103a, FP64).
+// Fused 3-D modified Lax-Wendroff step, exact policy (sm_103a, FP64), and the
+// 3-D CFL and frame kernels.  The fast policy's step is in mlw3d_fast.cu.
 //
 // Replaces the body of cans3d/hdmlw/mlw_m.f:2-453 with its primitives
 // mlwhalf (cans3d/hdmlw/mlwhalf.f:38-65), mlwfull (mlwfull.f:34-52) and
@@ -105,26 +106,20 @@ __device__ __forceinline__ void corner_flux_src(int v, int dir, int &f, bool &ne
 
 // Cell stage: primitives of one cell -> conserved variables, E and the
 // cell fluxes of cans3d/hdmlw/mlw_m.f:74-202, into one ring slot.
-template <bool E, bool R = false>
+template <bool R = false>
 __device__ __forceinline__ void cell_stage(const double *__restrict__ A,
                                            size_t n, size_t g, double *sl,
                                            int NC, int c, const Phys &ph,
                                            const double *__restrict__ res = nullptr) {
-  using FT = F<E>;
+  using FT = F<true>;
   const FT gm(ph.gm), gm1(ph.gm1), pi8i(ph.pi8i), pi4i(ph.pi4i);
   const FT ro(A[P3::RO * n + g]), pr(A[P3::PR * n + g]);
   const FT vx(A[P3::VX * n + g]), vy(A[P3::VY * n + g]), vz(A[P3::VZ * n + g]);
   const FT bx(A[P3::BX * n + g]), by(A[P3::BY * n + g]), bz(A[P3::BZ * n + g]);
   const FT vv = vx * vx + vy * vy + vz * vz;
   const FT bb = bx * bx + by * by + bz * bz;
-  FT ee, ep;
-  if constexpr (E) {
-    ee = pr / gm1 + 0.5 * ro * vv + pi8i * bb;
-    ep = pr * gm / gm1 + 0.5 * ro * vv;
-  } else {
-    ee = pr * ph.gm1i + 0.5 * ro * vv + pi8i * bb;
-    ep = pr * ph.ggm1 + 0.5 * ro * vv;
-  }
+  const FT ee = pr / gm1 + 0.5 * ro * vv + pi8i * bb;
+  const FT ep = pr * gm / gm1 + 0.5 * ro * vv;
   FT ex = -vy * bz + vz * by;
   FT ey = -vz * bx + vx * bz;
   FT ez = -vx * by + vy * bx;
@@ -156,7 +151,7 @@ __device__ __forceinline__ void cell_stage(const double *__restrict__ A,
 
 }  // namespace
 
-template <bool E, int TX, int TY, bool G = false, bool R = false>
+template <int TX, int TY, bool G = false, bool R = false>
 __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, 1)
     k_mlw3d(const double *__restrict__ A, double *__restrict__ B, int ix,
             int jx, int kx, Axis ax, Axis ay, Axis az, Phys ph, double dt_arg,
@@ -164,7 +159,7 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, 1)
             const double *__restrict__ grav = nullptr,
             const double *__restrict__ res = nullptr) {
   using T = Tile3<TX, TY, G>;
-  using FT = F<E>;
+  using FT = F<true>;
   extern __shared__ double smem[];
   double *scell = smem;                                   // [2][C3::N][NC]
   double *scorn = scell + 2 * (size_t)C3::N * T::NC;      // [2][K3::N][NK]
@@ -204,7 +199,7 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, 1)
     double *sl = cslot(k);
     if (in_arr) {
       const size_t g = (size_t)gi + (size_t)gj * ix + (size_t)k * plane;
-      cell_stage<E, R>(A, n, g, sl, T::NC, tid, ph, res);
+      cell_stage<R>(A, n, g, sl, T::NC, tid, ph, res);
       if constexpr (G) {  // mlw_m_g.f:135-136, 154, 172, 190
         const FT ro(sl[(size_t)C3::RO * T::NC + tid]);
         const FT vx(sl[(size_t)C3::VX * T::NC + tid]), vy(sl[(size_t)C3::VY * T::NC + tid]);
@@ -261,40 +256,6 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, 1)
     }
     const FT dxim(ax.dim[a]), dyim(ay.dim[b]), dzim(az.dim[k]);
     FT un[8];
-    if constexpr (!E) {  // same predictor, fewer rounded operations
-      const double cxk = dt.v * dxim.v * 0.25, cyk = dt.v * dyim.v * 0.25,
-                   czk = dt.v * dzim.v * 0.25;
-#pragma unroll
-      for (int v = 0; v < 8; v++) {
-        const double *Lv = L + (size_t)v * T::NC, *Uv = U + (size_t)v * T::NC;
-        double r = 0.125 * (((Lv[p10] + Lv[p00]) + (Lv[p11] + Lv[p01])) +
-                            ((Uv[p10] + Uv[p00]) + (Uv[p11] + Uv[p01])));
-        int f;
-        bool ng;
-        cell_flux_src(v, 0, f, ng);
-        if (f != NOF) {
-          const double *a = L + (size_t)f * T::NC, *b = U + (size_t)f * T::NC;
-          const double s = ((a[p10] - a[p00]) + (a[p11] - a[p01])) +
-                           ((b[p10] - b[p00]) + (b[p11] - b[p01]));
-          r = fma(ng ? cxk : -cxk, s, r);
-        }
-        cell_flux_src(v, 1, f, ng);
-        if (f != NOF) {
-          const double *a = L + (size_t)f * T::NC, *b = U + (size_t)f * T::NC;
-          const double s = ((a[p01] - a[p00]) + (a[p11] - a[p10])) +
-                           ((b[p01] - b[p00]) + (b[p11] - b[p10]));
-          r = fma(ng ? cyk : -cyk, s, r);
-        }
-        cell_flux_src(v, 2, f, ng);
-        if (f != NOF) {
-          const double *a = L + (size_t)f * T::NC, *b = U + (size_t)f * T::NC;
-          const double s = ((b[p00] - a[p00]) + (b[p10] - a[p10])) +
-                           ((b[p01] - a[p01]) + (b[p11] - a[p11]));
-          r = fma(ng ? czk : -czk, s, r);
-        }
-        un[v] = FT(r);
-      }
-    } else {
 #pragma unroll
     for (int v = 0; v < 8; v++) {
       const int su = v;  // conserved fields are 0..7
@@ -331,7 +292,6 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, 1)
       }
       un[v] = r;
     }
-    }
     if constexpr (G) {
       // mlwsrch part 2 (mlwsrch.f:41-47): un += dt * (average of the eight
       // cell sources around the corner), energy and the three momenta
@@ -339,30 +299,14 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, 1)
 #pragma unroll
       for (int q = 0; q < 4; q++) {
         const double *l = gL + q * T::NC, *u = gU + q * T::NC;
-        if constexpr (E) {
-          const FT sh = (FT(l[p10]) + FT(l[p00]) + FT(l[p11]) + FT(l[p01]) + FT(u[p10]) +
-                         FT(u[p00]) + FT(u[p11]) + FT(u[p01])) * 0.125;
-          un[1 + q] = un[1 + q] + dt * sh;
-        } else {
-          const double sh = ((l[p10] + l[p00]) + (l[p11] + l[p01])) +
-                            ((u[p10] + u[p00]) + (u[p11] + u[p01]));
-          un[1 + q] = FT(fma(dt.v * 0.125, sh, un[1 + q].v));
-        }
+        const FT sh = (FT(l[p10]) + FT(l[p00]) + FT(l[p11]) + FT(l[p01]) + FT(u[p10]) +
+                       FT(u[p00]) + FT(u[p11]) + FT(u[p01])) * 0.125;
+        un[1 + q] = un[1 + q] + dt * sh;
       }
     }
     const FT roh = un[0], eeh = un[1], rxh = un[2], ryh = un[3], rzh = un[4];
     const FT bxh = un[5], byh = un[6], bzh = un[7];
-    FT vxh, vyh, vzh;
-    if constexpr (E) {
-      vxh = rxh / roh;
-      vyh = ryh / roh;
-      vzh = rzh / roh;
-    } else {
-      const FT rinv(1.0 / roh.v);
-      vxh = rxh * rinv;
-      vyh = ryh * rinv;
-      vzh = rzh * rinv;
-    }
+    const FT vxh = rxh / roh, vyh = ryh / roh, vzh = rzh / roh;
     const FT vv = vxh * vxh + vyh * vyh + vzh * vzh;
     const FT bb = bxh * bxh + byh * byh + bzh * bzh;
     const FT prh = gm1 * (eeh - 0.5 * roh * vv - pi8i * bb);
@@ -374,9 +318,7 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, 1)
       eyh = eyh + FT(rq[1]);
       ezh = ezh + FT(rq[2]);
     }
-    FT ep;
-    if constexpr (E) ep = prh * gm / gm1 + 0.5 * roh * vv;
-    else ep = prh * ph.ggm1 + 0.5 * roh * vv;
+    const FT ep = prh * gm / gm1 + 0.5 * roh * vv;
     KS(K3::XRO) = (roh * vxh).v;
     KS(K3::YRO) = (roh * vyh).v;
     KS(K3::ZRO) = (roh * vzh).v;
@@ -490,87 +432,6 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, 1)
       const FT qzd = qav * FT(az.dm[k - 1]) * max0(fabs_(vz0 - FT(pvz)) - CANS_AV_EPS) *
                      FT(az.dim[k - 1]);
       FT unew[8];
-      if constexpr (!E) {
-        // Fast policy: each new conserved value is a linear combination of
-        // 37 stencil values with per-cell coefficients, one chain of FMAs.
-        const double h = hdt.v;
-        const double fcx = h * hdx.v, fcy = h * hdy.v, fcz = h * hdz.v;
-        const double hx_ = h * dxi.v, hy_ = h * dyi.v, hz_ = h * dzi.v;
-        const double wxL0 = hx_ * uz0.v * uy0.v, wxL1 = hx_ * uz0.v * uy1.v;
-        const double wxU0 = hx_ * uz1.v * uy0.v, wxU1 = hx_ * uz1.v * uy1.v;
-        const double wyL0 = hy_ * ux0.v * uz0.v, wyU0 = hy_ * ux0.v * uz1.v;
-        const double wyL1 = hy_ * ux1.v * uz0.v, wyU1 = hy_ * ux1.v * uz1.v;
-        const double wzSW = hz_ * uy0.v * ux0.v, wzSE = hz_ * uy0.v * ux1.v;
-        const double wzNW = hz_ * uy1.v * ux0.v, wzNE = hz_ * uy1.v * ux1.v;
-        const double ae = dt.v * dxi.v * qxe.v, aw = dt.v * dxi.v * qxw.v;
-        const double an = dt.v * dyi.v * qyn.v, as = dt.v * dyi.v * qys.v;
-        const double au = dt.v * dzi.v * qzu.v, ad = dt.v * dzi.v * qzd.v;
-        const double a1 = 1.0 - (((ae + aw) + (an + as)) + (au + ad));
-#pragma unroll
-        for (int v = 0; v < 8; v++) {
-          const double *Sv = S0 + (size_t)v * T::NC;
-          double r = a1 * Sv[c];
-          r = fma(ae, Sv[cE], r);
-          r = fma(aw, Sv[cW], r);
-          r = fma(an, Sv[cN], r);
-          r = fma(as, Sv[cS], r);
-          r = fma(au, S1[(size_t)v * T::NC + c], r);
-          r = fma(ad, pu[v], r);
-          int f;
-          bool ng;
-          cell_flux_src(v, 0, f, ng);
-          if (f != NOF)
-            r = fma(ng ? fcx : -fcx, S0[(size_t)f * T::NC + cE] - S0[(size_t)f * T::NC + cW], r);
-          cell_flux_src(v, 1, f, ng);
-          if (f != NOF)
-            r = fma(ng ? fcy : -fcy, S0[(size_t)f * T::NC + cN] - S0[(size_t)f * T::NC + cS], r);
-          cell_flux_src(v, 2, f, ng);
-          if (f != NOF) {
-            const double up = ng ? -S1[(size_t)f * T::NC + c] : S1[(size_t)f * T::NC + c];
-            r = fma(-fcz, up - pfz[v], r);
-          }
-          corner_flux_src(v, 0, f, ng);
-          if (f != NOF) {
-            const double *L = KL + (size_t)f * T::NK, *U = KU + (size_t)f * T::NK;
-            const double sg = ng ? 1.0 : -1.0;
-            r = fma(sg * wxL0, L[kSE] - L[kSW], r);
-            r = fma(sg * wxL1, L[kNE] - L[kNW], r);
-            r = fma(sg * wxU0, U[kSE] - U[kSW], r);
-            r = fma(sg * wxU1, U[kNE] - U[kNW], r);
-          }
-          corner_flux_src(v, 1, f, ng);
-          if (f != NOF) {
-            const double *L = KL + (size_t)f * T::NK, *U = KU + (size_t)f * T::NK;
-            const double sg = ng ? 1.0 : -1.0;
-            r = fma(sg * wyL0, L[kNW] - L[kSW], r);
-            r = fma(sg * wyU0, U[kNW] - U[kSW], r);
-            r = fma(sg * wyL1, L[kNE] - L[kSE], r);
-            r = fma(sg * wyU1, U[kNE] - U[kSE], r);
-          }
-          corner_flux_src(v, 2, f, ng);
-          if (f != NOF) {
-            const double *L = KL + (size_t)f * T::NK, *U = KU + (size_t)f * T::NK;
-            const double sg = ng ? 1.0 : -1.0;
-            r = fma(sg * wzSW, U[kSW] - L[kSW], r);
-            r = fma(sg * wzSE, U[kSE] - L[kSE], r);
-            r = fma(sg * wzNW, U[kNW] - L[kNW], r);
-            r = fma(sg * wzNE, U[kNE] - L[kNE], r);
-          }
-          if constexpr (G) {
-            if (v >= 1 && v <= 4) {  // mlwsrch part 1 and mlwsrcf
-              const int q = v - 1;
-              r = fma(h, gcslot(k)[q * T::NC + c], r);
-              const double *gl = gkslot(k - 1) + q * T::NK, *gu = gkslot(k) + q * T::NK;
-              const double sl_ = fma(uy0.v, fma(ux0.v, gl[kSW], ux1.v * gl[kSE]),
-                                     uy1.v * fma(ux0.v, gl[kNW], ux1.v * gl[kNE]));
-              const double su_ = fma(uy0.v, fma(ux0.v, gu[kSW], ux1.v * gu[kSE]),
-                                     uy1.v * fma(ux0.v, gu[kNW], ux1.v * gu[kNE]));
-              r = fma(h, fma(uz0.v, sl_, uz1.v * su_), r);
-            }
-          }
-          unew[v] = FT(r);
-        }
-      } else {
 #pragma unroll
       for (int v = 0; v < 8; v++) {
         FT du(0.0);
@@ -640,20 +501,9 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, 1)
              dt * (dzi * (qzu * (FT(S1[(size_t)v * T::NC + c]) - u) - qzd * (u - FT(pu[v]))));
         unew[v] = u + du;
       }
-      }
       const FT ro = unew[0], ee = unew[1], rx = unew[2], ry = unew[3], rz = unew[4];
       const FT bx = unew[5], by = unew[6], bz = unew[7];
-      FT vx, vy, vz;
-      if constexpr (E) {
-        vx = rx / ro;
-        vy = ry / ro;
-        vz = rz / ro;
-      } else {
-        const FT rinv(1.0 / ro.v);
-        vx = rx * rinv;
-        vy = ry * rinv;
-        vz = rz * rinv;
-      }
+      const FT vx = rx / ro, vy = ry / ro, vz = rz / ro;
       const FT vv = vx * vx + vy * vy + vz * vz;
       const FT bb = bx * bx + by * by + bz * bz;
       const FT pr = gm1 * (ee - 0.5 * ro * vv - pi8i * bb);
@@ -671,22 +521,12 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, 1)
         // cans3d/common/cfl_m.f:52-59 (pi in single precision)
         const FT b2 = bx * bx + by * by + bz * bz;
         const FT v2 = vx * vx + vy * vy + vz * vz;
-        if constexpr (E) {
-          const FT ca2 = b2 * FT(ph.pi4i_cfl) / ro;
-          const FT cs2 = gm * pr / ro;
-          const FT dmn = fmin_(fmin_(FT(ax.d[gi]), FT(ay.d[gj])), FT(az.d[k]));
-          const double dtq = (FT(ctl->safety) * (dmn / fsqrt(v2 + cs2 + ca2))).v;
-          if (dtq < dmin) dmin = dtq;
-          bad |= bad_cell(ro.v, pr.v, dtq);
-        } else {
-          // largest S*max(1/dx^2,1/dy^2,1/dz^2) gives the smallest dt; dmin
-          // holds minus that key (see the block reduction below)
-          const double rinv = 1.0 / ro.v;
-          const double s = v2.v + fma(gm.v, pr.v, ph.pi4i_cfl * b2.v) * rinv;
-          const double kk = s * fmax(fmax(dxi.v * dxi.v, dyi.v * dyi.v), dzi.v * dzi.v);
-          if (-kk < dmin) dmin = -kk;
-          bad |= bad_cell(ro.v, pr.v, kk);
-        }
+        const FT ca2 = b2 * FT(ph.pi4i_cfl) / ro;
+        const FT cs2 = gm * pr / ro;
+        const FT dmn = fmin_(fmin_(FT(ax.d[gi]), FT(ay.d[gj])), FT(az.d[k]));
+        const double dtq = (FT(ctl->safety) * (dmn / fsqrt(v2 + cs2 + ca2))).v;
+        if (dtq < dmin) dmin = dtq;
+        bad |= bad_cell(ro.v, pr.v, dtq);
       }
       save_prev(k);
     }
@@ -712,16 +552,10 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, 1)
   }
   if (ctl != nullptr) {
     count_bad_block(bad, &ctl->nonfinite, tid);
-    if constexpr (E) {
-      block_min_to(&ctl->cfl_bits, dmin, sred, tid, T::NT);
-    } else {
-      const double m = block_min(dmin, sred, tid, T::NT);  // -(largest key)
-      if (tid == 0 && m < 0.0) atomic_min_pos(&ctl->cfl_bits, ctl->safety / sqrt(-m));
-    }
+    block_min_to(&ctl->cfl_bits, dmin, sred, tid, T::NT);
   }
 }
 
-namespace {
 // The z chunk (at most kmax planes) that fills the GPU best: a launch of b
 // blocks with `slots` resident at a time takes ceil(b / slots) waves, and a
 // block of kc planes costs about kc + 1 plane steps (its prologue loads two
@@ -744,9 +578,10 @@ int balance_kchunk(long long bxy, int nz, int kmax, int slots) {
   return best;
 }
 
+namespace {
 constexpr int kMaxDevices3 = 64;
 
-template <bool E, int TX, int TY, bool G = false, bool R = false>
+template <int TX, int TY, bool G = false, bool R = false>
 cudaError_t launch3(const double *A, double *B, int ix, int jx, int kx,
                     const Axis &ax, const Axis &ay, const Axis &az,
                     const Phys &ph, double dt, Ctl *ctl, Box3 box, int kchunk,
@@ -765,14 +600,14 @@ cudaError_t launch3(const double *A, double *B, int ix, int jx, int kx,
   {
     std::lock_guard<std::mutex> lk(mu);
     if (!slots_of[dev]) {
-      e = cudaFuncSetAttribute(k_mlw3d<E, TX, TY, G, R>,
+      e = cudaFuncSetAttribute(k_mlw3d<TX, TY, G, R>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem_bytes);
       if (e != cudaSuccess) return e;
       int sms = 0, per_sm = 0;
       if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
         return e;
       if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-               &per_sm, k_mlw3d<E, TX, TY, G, R>, T::NT, T::smem_bytes)) != cudaSuccess)
+               &per_sm, k_mlw3d<TX, TY, G, R>, T::NT, T::smem_bytes)) != cudaSuccess)
         return e;
       slots_of[dev] = sms * (per_sm > 0 ? per_sm : 1);
     }
@@ -782,7 +617,7 @@ cudaError_t launch3(const double *A, double *B, int ix, int jx, int kx,
   kchunk = balance_kchunk((long long)bx * by, kx - 2, kchunk, slots);
   dim3 grid(bx, by, (kx - 2 + kchunk - 1) / kchunk);
   dim3 block(T::NT);
-  k_mlw3d<E, TX, TY, G, R><<<grid, block, T::smem_bytes, s>>>(
+  k_mlw3d<TX, TY, G, R><<<grid, block, T::smem_bytes, s>>>(
       A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box, kchunk, grav, res);
   count_launch();
   return cudaGetLastError();
@@ -800,21 +635,18 @@ cudaError_t launch_mlw3d_g(bool exact, int tile, const double *A, double *B, int
                            const Phys &ph, const double *grav, double dt, Ctl *ctl,
                            Box3 box, cudaStream_t s) {
   if (ix < 3 || jx < 3 || kx < 3 || grav == nullptr) return cudaErrorInvalidValue;
+  if (!exact)
+    return launch_mlw3d_fast(tile, A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box, s, grav,
+                             nullptr);
   const int kchunk = (tile == 1 || tile == 3) ? 32 : 64;
   if (tile == 3)
-    return exact ? launch3<true, 24, 8, true>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box,
-                                              kchunk, s, grav)
-                 : launch3<false, 24, 8, true>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl,
-                                               box, kchunk, s, grav);
+    return launch3<24, 8, true>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box,
+                                              kchunk, s, grav);
   if (tile == 2)
-    return exact ? launch3<true, 16, 12, true>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box,
-                                               kchunk, s, grav)
-                 : launch3<false, 16, 12, true>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl,
-                                                box, kchunk, s, grav);
-  return exact ? launch3<true, 16, 8, true>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box,
-                                            kchunk, s, grav)
-               : launch3<false, 16, 8, true>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box,
-                                             kchunk, s, grav);
+    return launch3<16, 12, true>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box,
+                                               kchunk, s, grav);
+  return launch3<16, 8, true>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box,
+                                            kchunk, s, grav);
 }
 
 int mlw3d_tile_count() { return 3; }
@@ -825,16 +657,15 @@ cudaError_t launch_mlw3d_res(bool exact, int tile, const double *A, double *B, i
                              int jx, int kx, const Axis &ax, const Axis &ay, const Axis &az,
                              const Phys &ph, const double *res, double dt, Ctl *ctl,
                              Box3 box, cudaStream_t s) {
+  if (!exact)
+    return launch_mlw3d_fast(tile, A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box, s, nullptr,
+                             res);
   const int kchunk = (tile == 1) ? 32 : 64;
   if (tile == 2)
-    return exact ? launch3<true, 16, 8, false, true>(A, B, ix, jx, kx, ax, ay, az, ph, dt,
-                                                     ctl, box, kchunk, s, nullptr, res)
-                 : launch3<false, 16, 8, false, true>(A, B, ix, jx, kx, ax, ay, az, ph, dt,
-                                                      ctl, box, kchunk, s, nullptr, res);
-  return exact ? launch3<true, 16, 16, false, true>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl,
-                                                    box, kchunk, s, nullptr, res)
-               : launch3<false, 16, 16, false, true>(A, B, ix, jx, kx, ax, ay, az, ph, dt,
+    return launch3<16, 8, false, true>(A, B, ix, jx, kx, ax, ay, az, ph, dt,
                                                      ctl, box, kchunk, s, nullptr, res);
+  return launch3<16, 16, false, true>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl,
+                                                    box, kchunk, s, nullptr, res);
 }
 
 cudaError_t launch_mlw3d(bool exact, int tile, const double *A, double *B,
@@ -842,14 +673,15 @@ cudaError_t launch_mlw3d(bool exact, int tile, const double *A, double *B,
                          const Axis &ay, const Axis &az, const Phys &ph,
                          double dt, Ctl *ctl, Box3 box, cudaStream_t s) {
   if (ix < 3 || jx < 3 || kx < 3) return cudaErrorInvalidValue;
+  if (!exact)
+    return launch_mlw3d_fast(tile, A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box, s, nullptr,
+                             nullptr);
   // tile: 0 = 16x16 tiles, z chunks of 64; 1 = 16x16, chunks of 32;
   //       2 = 16x8 tiles, chunks of 64
   const int kchunk = (tile == 1) ? 32 : 64;
   if (tile == 2)
-    return exact ? launch3<true, 16, 8>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box, kchunk, s)
-                 : launch3<false, 16, 8>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box, kchunk, s);
-  return exact ? launch3<true, 16, 16>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box, kchunk, s)
-               : launch3<false, 16, 16>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box, kchunk, s);
+    return launch3<16, 8>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box, kchunk, s);
+  return launch3<16, 16>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box, kchunk, s);
 }
 
 // ---------------------------------------------------------------------------
