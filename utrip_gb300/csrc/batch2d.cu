@@ -4,16 +4,15 @@
 // layer of cans2d/md_mhdkh/hdmlw/model.f) for many grid sizes and plasma
 // betas.  Run one at a time, a small grid fills a fraction of the 152 SMs and
 // every step pays the launch latency of its kernels.  Here one loop iteration
-// of every run is four launches in total:
+// of every run is two launches in total:
 //   1. a persistent step kernel: one block per resident slot; each block pulls
-//      (run, tile) work items from a device work queue and applies the same
-//      fused tile step as the single-run kernel (mlw2d_tile.cuh), with the
+//      (run, tile) work items from a device work queue and applies the single
+//      run's block (mlw2d_march.cuh; exact policy: mlw2d_tile.cuh) with the
 //      run's own arrays, metrics, dt and CFL accumulator;
-//   2.-3. the boundary programs of all runs, x faces then y faces;
-//   4. the frame CFL of each run (one block per run), the loop bookkeeping of
-//      each run (finish_iteration), and the reset of the work queue.
+//   2. the boundary programs, frame CFLs and loop ends of all runs
+//      (bcframe2d.cuh), and the reset of the work queue.
 // Each run keeps its own dt, t, ns and termination exactly as if it ran
-// alone, so the results equal single-run results bit for bit.  The four
+// alone, so the exact policy's results equal single-run results bit for bit.  The
 // launches are captured in a CUDA graph; the tile shape and the cells per
 // thread are picked by timing (cans_batch_autotune).
 #include <cuda_runtime.h>
@@ -23,10 +22,11 @@
 #include <string>
 #include <vector>
 
-#include "bc_line.cuh"
+#include "bcframe2d.cuh"
 #include "cans_common.cuh"
 #include "cans_gpu.h"
 #include "cans_internal.h"
+#include "mlw2d_march.cuh"
 #include "mlw2d_tile.cuh"
 
 namespace cans {
@@ -42,120 +42,88 @@ struct BatchGrid {
   int tile0;      // first work item of this run
 };
 
-// Step of every run: persistent blocks pull work items until the queue is
-// exhausted.
-template <bool E, bool M3, int TX, int TY, int RPT>
+// The next work item of a persistent block, or -1: the run it belongs to in *run,
+// its tile in *tile.
+__device__ __forceinline__ int next_item(const BatchGrid *__restrict__ grids, int ngrids,
+                                         int nitems, unsigned int *queue, int *run, int *tile) {
+  __shared__ int s_item;
+  if (threadIdx.x == 0) s_item = (int)atomicAdd(queue, 1u);
+  __syncthreads();
+  const int item = s_item;
+  __syncthreads();  // every thread has read s_item before it is rewritten
+  if (item >= nitems) return -1;
+  int lo = 0, hi = ngrids - 1;  // last run whose first item <= item
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (grids[mid].tile0 <= item) lo = mid;
+    else hi = mid - 1;
+  }
+  *run = lo;
+  *tile = item - grids[lo].tile0;
+  return item;
+}
+
+// Step of every run in the exact policy: persistent blocks pull work items until
+// the queue is exhausted.
+template <bool M3, int TX, int TY, int RPT>
 __global__ void __launch_bounds__(TX *TY / RPT, 1)
     k_mlw2d_batch(const BatchGrid *__restrict__ grids, int ngrids, int nitems,
                   unsigned int *queue) {
   extern __shared__ double smem[];
-  __shared__ int s_item;
-  for (;;) {
-    if (threadIdx.x == 0) s_item = (int)atomicAdd(queue, 1u);
-    __syncthreads();
-    const int item = s_item;
-    __syncthreads();  // every thread has read s_item before it is rewritten
-    if (item >= nitems) break;
-    int lo = 0, hi = ngrids - 1;  // last run whose first item <= item
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (grids[mid].tile0 <= item) lo = mid;
-      else hi = mid - 1;
-    }
-    const BatchGrid &G = grids[lo];
+  int run, t;
+  while (next_item(grids, ngrids, nitems, queue, &run, &t) >= 0) {
+    const BatchGrid &G = grids[run];
     Ctl *ctl = G.ctl;
     if (ctl->done | ctl->pause) continue;
-    const int t = item - G.tile0;
-    tile_step<E, M3, TX, TY, RPT>(ctl->buf[ctl->cur], ctl->buf[ctl->cur ^ 1], G.ix,
-                                  G.jx, G.ax, G.ay, G.ph, ctl->dt, ctl->safety,
-                                  &ctl->cfl_bits, G.box, t % G.ntx, t / G.ntx,
-                                  G.ntx, G.nty, smem, nullptr, nullptr, &ctl->nonfinite);
+    tile_step<M3, TX, TY, RPT>(ctl->buf[ctl->cur], ctl->buf[ctl->cur ^ 1], G.ix,
+                               G.jx, G.ax, G.ay, G.ph, ctl->dt, ctl->safety,
+                               &ctl->cfl_bits, G.box, t % G.ntx, t / G.ntx,
+                               G.ntx, G.nty, smem, nullptr, nullptr, &ctl->nonfinite);
   }
 }
 
-// Boundary program of one axis for every run: blockIdx.y is the run.
-__global__ void k_bc_batch(const BatchGrid *__restrict__ grids,
-                           const BcTable *__restrict__ tables, int nvar,
-                           int axis) {
-  const BatchGrid &G = grids[blockIdx.y];
-  const Ctl *ctl = G.ctl;
-  if (ctl->done | ctl->pause) return;
-  double *S = ctl->buf[ctl->cur ^ 1];
-  const BcTable &bc = tables[blockIdx.y];
-  const int n0 = G.ix, n1 = G.jx;
-  const int n = axis == 0 ? n0 : n1;
-  const size_t stride = axis == 0 ? 1 : (size_t)n0;
-  const long long nlines = (long long)n0 * n1 / n;
-  const size_t nall = (size_t)n0 * n1;
-  const double *dxm = axis == 0 ? G.ax.dm : G.ay.dm;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-       t < nlines * nvar; t += (long long)gridDim.x * blockDim.x) {
-    const int v = (int)(t / nlines);
-    const long long line = t % nlines;
-    double *q = S + (size_t)v * nall + line_base(axis, line, n0, n1);
-    const int klo = bc.kind[v][2 * axis], khi = bc.kind[v][2 * axis + 1];
-    if (klo >= 0) bd_line(klo, 0, bc.margin, bc.margin, q, n, stride, bc.q0[v][2 * axis], dxm);
-    if (khi >= 0)
-      bd_line(khi, 1, bc.margin, bc.margin, q, n, stride, bc.q0[v][2 * axis + 1], dxm);
+// The same in the fast policy: an item is a segment of `seg` rows of a strip of
+// 32 columns, stepped by the single run's marching block (mlw2d_march.cuh), so
+// that a batch runs its zones at the rate of a step that fills the GPU.
+constexpr int kBatchCH = 8;
+template <bool M3>
+__global__ void __launch_bounds__(March<kBatchCH, M3, false>::NT, 2)
+    k_mlw2d_batch_fast(const BatchGrid *__restrict__ grids, int ngrids, int nitems, int seg,
+                       unsigned int *queue) {
+  extern __shared__ double smem_march[];
+  int run, t;
+  while (next_item(grids, ngrids, nitems, queue, &run, &t) >= 0) {
+    const BatchGrid &G = grids[run];
+    Ctl *ctl = G.ctl;
+    if (ctl->done | ctl->pause) continue;
+    MarchArgs m{};
+    m.A = ctl->buf[ctl->cur];
+    m.B = ctl->buf[ctl->cur ^ 1];
+    m.ix = G.ix;
+    m.jx = G.jx;
+    m.dt = ctl->dt;
+    m.safety = ctl->safety;
+    m.cfl = &ctl->cfl_bits;
+    m.bad = &ctl->nonfinite;
+    m.box = G.box;
+    const int jb = 1 + (t / G.ntx) * seg;
+    march_block<F64N, kBatchCH, M3, false, false, 0>(m, G.ax, G.ay, G.ph, t % G.ntx, G.ntx, jb,
+                                                     min(G.jx - 2, jb + seg - 1), smem_march);
   }
 }
 
-// Frame CFL and loop bookkeeping of every run (one block per run), then the
-// reset of the work queue for the next step.
+// Boundary program, frame CFL and loop end of every run (blockIdx.y) as a single
+// run's k_bcframe2d does them, and the reset of the work queue for the next
+// step.  One launch for what were three; the frame CFL of a run, on one SM
+// before, spreads over the blocks of its row of the grid.
 template <bool E, bool M3>
-__global__ void k_frame_batch(const BatchGrid *__restrict__ grids, int margin,
-                              unsigned int *queue) {
-  using FT = F<E>;
-  using P = Prim<M3>;
-  __shared__ double red[32];
-  if (blockIdx.x == 0 && threadIdx.x == 0) *queue = 0u;
-  const BatchGrid &G = grids[blockIdx.x];
-  Ctl *ctl = G.ctl;
-  if (ctl->done | ctl->pause) return;
-  const double *S = ctl->buf[ctl->cur ^ 1];
-  const int ix = G.ix, jx = G.jx, w = margin + 1;
-  const size_t n = (size_t)ix * jx;
-  const long long nrow = 2LL * w * ix;
-  const long long total = nrow + (jx - 2LL * w) * 2LL * w;
-  const FT gm(G.ph.gm), pi4i(G.ph.pi4i), safety(ctl->safety);
-  double dmin = __longlong_as_double(0x7ff0000000000000LL);
-  bool bad = false;
-  for (long long f = threadIdx.x; f < total; f += blockDim.x) {
-    int i, j;
-    if (f < nrow) {
-      const long long r = f / ix;
-      i = (int)(f % ix);
-      j = (r < w) ? (int)r : (int)(jx - 2 * w + r);
-    } else {
-      const long long q = f - nrow;
-      j = (int)(w + q / (2 * w));
-      const int c = (int)(q % (2 * w));
-      i = (c < w) ? c : (ix - 2 * w + c);
-    }
-    const size_t g = (size_t)i + (size_t)j * ix;
-    const FT ro(S[P::RO * n + g]), pr(S[P::PR * n + g]);
-    const FT vx(S[P::VX * n + g]), vy(S[P::VY * n + g]);
-    const FT bx(S[P::BX * n + g]), by(S[P::BY * n + g]);
-    FT b2, v2;
-    if constexpr (M3) {
-      const FT vz(S[P::VZ * n + g]), bz(S[P::BZ * n + g]);
-      b2 = bx * bx + by * by + bz * bz;
-      v2 = vx * vx + vy * vy + vz * vz;
-    } else {
-      b2 = bx * bx + by * by;
-      v2 = vx * vx + vy * vy;
-    }
-    const FT ca2 = b2 * pi4i / ro;
-    const FT cs2 = gm * pr / ro;
-    const FT dtcfl = fmin_(FT(G.ax.d[i]), FT(G.ay.d[j])) / fsqrt(v2 + cs2 + ca2);
-    const double dtq = (safety * dtcfl).v;
-    if (dtq < dmin) dmin = dtq;
-    bad |= bad_cell(ro.v, pr.v, dtq);
-  }
-  count_bad_block(bad, &ctl->nonfinite, threadIdx.x);
-  block_min_to(&ctl->cfl_bits, dmin, red, threadIdx.x, blockDim.x);
-  __syncthreads();
-  if (threadIdx.x == 0) finish_iteration(ctl);
+__global__ void __launch_bounds__(32 * Prim<M3>::N)
+    k_bcframe_batch(const BatchGrid *__restrict__ grids, const BcTable *__restrict__ tables,
+                    unsigned int *queue) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *queue = 0u;
+  const BatchGrid &G = grids[blockIdx.y];
+  bcframe2d<E, M3>(G.ix, G.jx, G.ax, G.ay, G.ph, tables[blockIdx.y], G.ctl, blockIdx.x,
+                   gridDim.x);
 }
 
 // Start of every run (the first CFL is reduced into cfl_bits beforehand).
@@ -168,48 +136,68 @@ __global__ void k_prepare_batch(const BatchGrid *__restrict__ grids, int ngrids)
 }
 
 // ---------------------------------------------------------------------------
-// Configurations the autotuner chooses from: tile shape and cells per thread.
+// Configurations the autotuner chooses from: tile shape and cells per thread of
+// the exact policy; rows of a work item of the fast one (strips of 32 columns):
+// long segments recompute fewer halo rows, short ones fill the last wave.
 struct BatchConfig {
   int tx, ty, rpt;
 };
 static const BatchConfig kConfigs[] = {
     {32, 8, 2}, {32, 8, 1}, {32, 16, 2}, {16, 16, 2}, {32, 16, 4}, {64, 8, 2}};
+static const BatchConfig kFastConfigs[] = {
+    {32, 32, 0}, {32, 16, 0}, {32, 24, 0}, {32, 48, 0}, {32, 64, 0}, {32, 40, 0}};
 constexpr int kNumConfigs = sizeof(kConfigs) / sizeof(kConfigs[0]);
+static_assert(sizeof(kFastConfigs) == sizeof(kConfigs), "one index serves both policies");
 
-template <bool E, bool M3, int TX, int TY, int RPT>
-static cudaError_t launch_batch_cfg(const BatchGrid *grids, int ngrids, int nitems,
-                                    unsigned int *queue, cudaStream_t s) {
-  using T = Tile<TX, TY, M3, RPT>;
-  static int resident = 0;  // per template instance
-  auto kern = k_mlw2d_batch<E, M3, TX, TY, RPT>;
+// Persistent blocks: as many as the device holds at once.
+template <class Kern, class... Args>
+static cudaError_t launch_persistent(Kern kern, int &resident, int nt, size_t smem, int nitems,
+                                     cudaStream_t s, Args... args) {
   if (resident == 0) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)T::smem_bytes);
+                                         (int)smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0, dev = 0, sms = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, T::NT, T::smem_bytes);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nt, smem);
     if (e != cudaSuccess) return e;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     resident = (per_sm > 0 ? per_sm : 1) * sms;
   }
   const int blocks = resident < nitems ? resident : nitems;
-  kern<<<blocks > 0 ? blocks : 1, T::NT, T::smem_bytes, s>>>(grids, ngrids, nitems, queue);
+  kern<<<blocks > 0 ? blocks : 1, nt, smem, s>>>(args...);
   count_launch();
   return cudaGetLastError();
 }
 
-template <bool E, bool M3>
+template <bool M3, int TX, int TY, int RPT>
+static cudaError_t launch_batch_cfg(const BatchGrid *grids, int ngrids, int nitems,
+                                    unsigned int *queue, cudaStream_t s) {
+  using T = Tile<TX, TY, M3, RPT>;
+  static int resident = 0;  // per template instance
+  return launch_persistent(k_mlw2d_batch<M3, TX, TY, RPT>, resident, T::NT, T::smem_bytes, nitems,
+                           s, grids, ngrids, nitems, queue);
+}
+
+template <bool M3>
 static cudaError_t launch_batch(int cfg, const BatchGrid *grids, int ngrids,
                                 int nitems, unsigned int *queue, cudaStream_t s) {
   switch (cfg) {
-    case 1: return launch_batch_cfg<E, M3, 32, 8, 1>(grids, ngrids, nitems, queue, s);
-    case 2: return launch_batch_cfg<E, M3, 32, 16, 2>(grids, ngrids, nitems, queue, s);
-    case 3: return launch_batch_cfg<E, M3, 16, 16, 2>(grids, ngrids, nitems, queue, s);
-    case 4: return launch_batch_cfg<E, M3, 32, 16, 4>(grids, ngrids, nitems, queue, s);
-    case 5: return launch_batch_cfg<E, M3, 64, 8, 2>(grids, ngrids, nitems, queue, s);
-    default: return launch_batch_cfg<E, M3, 32, 8, 2>(grids, ngrids, nitems, queue, s);
+    case 1: return launch_batch_cfg<M3, 32, 8, 1>(grids, ngrids, nitems, queue, s);
+    case 2: return launch_batch_cfg<M3, 32, 16, 2>(grids, ngrids, nitems, queue, s);
+    case 3: return launch_batch_cfg<M3, 16, 16, 2>(grids, ngrids, nitems, queue, s);
+    case 4: return launch_batch_cfg<M3, 32, 16, 4>(grids, ngrids, nitems, queue, s);
+    case 5: return launch_batch_cfg<M3, 64, 8, 2>(grids, ngrids, nitems, queue, s);
+    default: return launch_batch_cfg<M3, 32, 8, 2>(grids, ngrids, nitems, queue, s);
   }
+}
+template <bool M3>
+static cudaError_t launch_batch_fast(int cfg, const BatchGrid *grids, int ngrids, int nitems,
+                                     unsigned int *queue, cudaStream_t s) {
+  using T = March<kBatchCH, M3, false>;
+  static int resident = 0;  // per template instance
+  return launch_persistent(k_mlw2d_batch_fast<M3>, resident, T::NT, T::smem_bytes, nitems, s,
+                           grids, ngrids, nitems, kFastConfigs[cfg].ty, queue);
 }
 
 }  // namespace cans
@@ -258,7 +246,7 @@ struct cans_batch {
   BatchGrid *d_grids = nullptr;
   BcTable *d_bc = nullptr;
   unsigned int *d_queue = nullptr;
-  int nitems = 0, max_lines = 0;
+  int nitems = 0, frame_blocks = 1;
   cudaGraphExec_t graph = nullptr;
   int graph_iters = 0, graph_nodes = 0;
 };
@@ -274,8 +262,8 @@ void drop_graph(cans_batch *b) {
 // Tiles of every run under the current configuration, uploaded with the
 // run descriptions and boundary tables.
 int sync_tables(cans_batch *b) {
-  const BatchConfig c = kConfigs[b->config];
-  int item = 0, maxl = 0;
+  const BatchConfig c = b->exact ? kConfigs[b->config] : kFastConfigs[b->config];
+  int item = 0, frame = 0;
   b->hgrids.resize(b->ngrids);
   for (int r = 0; r < b->ngrids; r++) {
     auto &G = b->g[r];
@@ -292,10 +280,10 @@ int sync_tables(cans_batch *b) {
     H.nty = (G.jx - 2 + c.ty - 1) / c.ty;
     H.tile0 = item;
     item += H.ntx * H.nty;
-    maxl = std::max(maxl, std::max(G.ix, G.jx) * b->nvar);
+    frame = std::max(frame, (int)frame_cells(G.ix, G.jx, w, 0));
   }
   b->nitems = item;
-  b->max_lines = maxl;
+  b->frame_blocks = std::min((frame + 31) / 32, 152 * 4);
   std::vector<BcTable> bcs(b->ngrids);
   for (int r = 0; r < b->ngrids; r++) bcs[r] = b->g[r].bc;
   BK(cudaMemcpyAsync(b->d_grids, b->hgrids.data(), sizeof(BatchGrid) * b->ngrids,
@@ -311,11 +299,11 @@ int step_launch(cans_batch *b, int cfg) {
   const bool m3 = b->solver == CANS_SOLVER_MLW_M3_2D;
   cudaError_t e;
   if (b->exact)
-    e = m3 ? launch_batch<true, true>(cfg, b->d_grids, b->ngrids, b->nitems, b->d_queue, b->s)
-           : launch_batch<true, false>(cfg, b->d_grids, b->ngrids, b->nitems, b->d_queue, b->s);
+    e = m3 ? launch_batch<true>(cfg, b->d_grids, b->ngrids, b->nitems, b->d_queue, b->s)
+           : launch_batch<false>(cfg, b->d_grids, b->ngrids, b->nitems, b->d_queue, b->s);
   else
-    e = m3 ? launch_batch<false, true>(cfg, b->d_grids, b->ngrids, b->nitems, b->d_queue, b->s)
-           : launch_batch<false, false>(cfg, b->d_grids, b->ngrids, b->nitems, b->d_queue, b->s);
+    e = m3 ? launch_batch_fast<true>(cfg, b->d_grids, b->ngrids, b->nitems, b->d_queue, b->s)
+           : launch_batch_fast<false>(cfg, b->d_grids, b->ngrids, b->nitems, b->d_queue, b->s);
   BK(e);
   return CANS_OK;
 }
@@ -323,19 +311,15 @@ int step_launch(cans_batch *b, int cfg) {
 int enqueue_batch_iteration(cans_batch *b) {
   int rc = step_launch(b, b->config);
   if (rc) return rc;
-  const int bx = (b->max_lines + 255) / 256;
-  for (int axis = 0; axis < 2; axis++) {
-    k_bc_batch<<<dim3(bx, b->ngrids), 256, 0, b->s>>>(b->d_grids, b->d_bc, b->nvar, axis);
-    count_launch();
-    BK(cudaGetLastError());
-  }
   const bool m3 = b->solver == CANS_SOLVER_MLW_M3_2D;
+  const dim3 grid(b->frame_blocks, b->ngrids);
+  const int nt = 32 * b->nvar;
   if (b->exact) {
-    if (m3) k_frame_batch<true, true><<<b->ngrids, 256, 0, b->s>>>(b->d_grids, b->margin, b->d_queue);
-    else k_frame_batch<true, false><<<b->ngrids, 256, 0, b->s>>>(b->d_grids, b->margin, b->d_queue);
+    if (m3) k_bcframe_batch<true, true><<<grid, nt, 0, b->s>>>(b->d_grids, b->d_bc, b->d_queue);
+    else k_bcframe_batch<true, false><<<grid, nt, 0, b->s>>>(b->d_grids, b->d_bc, b->d_queue);
   } else {
-    if (m3) k_frame_batch<false, true><<<b->ngrids, 256, 0, b->s>>>(b->d_grids, b->margin, b->d_queue);
-    else k_frame_batch<false, false><<<b->ngrids, 256, 0, b->s>>>(b->d_grids, b->margin, b->d_queue);
+    if (m3) k_bcframe_batch<false, true><<<grid, nt, 0, b->s>>>(b->d_grids, b->d_bc, b->d_queue);
+    else k_bcframe_batch<false, false><<<grid, nt, 0, b->s>>>(b->d_grids, b->d_bc, b->d_queue);
   }
   count_launch();
   BK(cudaGetLastError());

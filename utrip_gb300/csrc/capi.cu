@@ -1507,6 +1507,13 @@ int tile_count(const cans_run *h) {
   if (h->grav) return h->ndim == 3 ? mlw3d_g_tile_count() : mlw2d_g_tile_count();
   return h->ndim == 3 ? mlw3d_tile_count() : mlw2d_tile_count();
 }
+// Tiles that differ: the fast and double-float 2-D steps run the same launch under
+// several of their numbers (launch_mlw2d_fast, launch_mlw2d_df).
+int distinct_tiles(const cans_run *h) {
+  const int n = tile_count(h);
+  if (h->ndim != 2 || h->d.exact) return n;
+  return n < (h->df ? 4 : 2) ? n : (h->df ? 4 : 2);
+}
 // 1-D: the whole loop (or one fixed step) as one cluster launch, in place
 cudaError_t launch_1d(cans_run *h, int max_steps, int fixed, double dt,
                       int start) {
@@ -2244,7 +2251,7 @@ extern "C" int cans_run_autotune(cans_run *h, int trial_steps, int *tile) {
   CK(cudaEventCreate(&e1));
   float best = 1e30f;
   int best_tile = h->tile;
-  for (int t = 0; t < tile_count(h); t++) {
+  for (int t = 0; t < distinct_tiles(h); t++) {
     CK(step_kernel(h, t, h->buf[cur], h->buf[cur ^ 1], dt, nullptr, Box3{}));
     CK(cudaEventRecord(e0, h->s));
     for (int k = 0; k < trial_steps; k++)

@@ -1,9 +1,10 @@
-// Fused 2-D modified Lax-Wendroff step (sm_103a, FP64): the single-grid
-// kernel, the CFL kernels and the frame kernel.  The tile body itself
+// Fused 2-D modified Lax-Wendroff step of the exact policy (sm_103a, FP64): the
+// single-grid kernel; and the CFL kernels and the frame kernel of both policies.  The tile body itself
 // (phases 1-3, one TX x TY tile) is in mlw2d_tile.cuh.
 #include <cuda_runtime.h>
 
 #include "bc_line.cuh"
+#include "bcframe2d.cuh"
 #include "cans_common.cuh"
 #include "cans_internal.h"
 #include "mlw2d_tile.cuh"
@@ -13,7 +14,7 @@ namespace cans {
 // One tile per block.  With a control block the step takes dt and the
 // buffers from it, does nothing once the run is done or paused, and reduces
 // the CFL of the cells inside `box`.
-template <bool E, bool M3, int TX, int TY, int RPT>
+template <bool M3, int TX, int TY, int RPT>
 __global__ void __launch_bounds__(TX *TY / RPT, 1)
     k_mlw2d(const double *__restrict__ A, double *__restrict__ B, int ix,
             int jx, Axis ax, Axis ay, Phys ph, double dt_arg,
@@ -29,7 +30,7 @@ __global__ void __launch_bounds__(TX *TY / RPT, 1)
     safety = ctl->safety;
     cfl = &ctl->cfl_bits;
   }
-  tile_step<E, M3, TX, TY, RPT>(A, B, ix, jx, ax, ay, ph, dt, safety, cfl, box,
+  tile_step<M3, TX, TY, RPT>(A, B, ix, jx, ax, ay, ph, dt, safety, cfl, box,
                                 blockIdx.x, blockIdx.y, gridDim.x, gridDim.y, smem,
                                 nullptr, nullptr, ctl ? &ctl->nonfinite : nullptr);
 }
@@ -37,12 +38,12 @@ __global__ void __launch_bounds__(TX *TY / RPT, 1)
 // The mlw_m3 step with the artificial viscosity's branch recorded (AVF = 1)
 // or held at the recorded one (AVF = 2): the forward of the adjoint's
 // finite-difference check (see tile_step).  32 x 8 tiles, no control block.
-template <bool E, int AVF>
+template <int AVF>
 __global__ void __launch_bounds__(128, 1)
     k_mlw2d_av(const double *__restrict__ A, double *__restrict__ B, int ix, int jx, Axis ax,
                Axis ay, Phys ph, double dt, unsigned char *avb, unsigned long long *nflip) {
   extern __shared__ double smem[];
-  tile_step<E, true, 32, 8, 2, false, false, AVF>(
+  tile_step<true, 32, 8, 2, false, false, AVF>(
       A, B, ix, jx, ax, ay, ph, dt, 0.0, nullptr, Box3{}, blockIdx.x, blockIdx.y, gridDim.x,
       gridDim.y, smem, nullptr, nullptr, nullptr, avb, nflip);
 }
@@ -52,11 +53,10 @@ cudaError_t launch_mlw2d_av(bool exact, int mode, const double *A, double *B, in
                             unsigned char *avb, unsigned long long *nflip, cudaStream_t s) {
   if (ix < 3 || jx < 3 || (mode != 1 && mode != 2) || !avb || (mode == 2 && !nflip))
     return cudaErrorInvalidValue;
+  if (!exact)
+    return launch_mlw2d_av_fast(mode, A, B, ix, jx, ax, ay, ph, dt, avb, nflip, s);
   using T = Tile<32, 8, true, 2>;
-  void (*k)(const double *, double *, int, int, Axis, Axis, Phys, double, unsigned char *,
-            unsigned long long *) =
-      exact ? (mode == 1 ? k_mlw2d_av<true, 1> : k_mlw2d_av<true, 2>)
-            : (mode == 1 ? k_mlw2d_av<false, 1> : k_mlw2d_av<false, 2>);
+  auto k = mode == 1 ? k_mlw2d_av<1> : k_mlw2d_av<2>;
   cudaError_t e =
       cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem_bytes);
   if (e != cudaSuccess) return e;
@@ -69,7 +69,7 @@ cudaError_t launch_mlw2d_av(bool exact, int mode, const double *A, double *B, in
 // ---------------------------------------------------------------------------
 // Tile configurations offered to the autotuner: (TX, TY).
 namespace {
-template <bool E, bool M3, int TX, int TY, int RPT = 2>
+template <bool M3, int TX, int TY, int RPT = 2>
 cudaError_t launch_tile(const double *A, double *B, int ix, int jx,
                         const Axis &ax, const Axis &ay, const Phys &ph,
                         double dt, Ctl *ctl, Box3 box, cudaStream_t s) {
@@ -77,19 +77,19 @@ cudaError_t launch_tile(const double *A, double *B, int ix, int jx,
   static bool attr_set = false;  // per template instance
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(
-        k_mlw2d<E, M3, TX, TY, RPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        k_mlw2d<M3, TX, TY, RPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
         (int)T::smem_bytes);
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
   dim3 grid((ix - 2 + TX - 1) / TX, (jx - 2 + TY - 1) / TY);
-  k_mlw2d<E, M3, TX, TY, RPT><<<grid, T::NT, T::smem_bytes, s>>>(A, B, ix, jx, ax,
+  k_mlw2d<M3, TX, TY, RPT><<<grid, T::NT, T::smem_bytes, s>>>(A, B, ix, jx, ax,
                                                                 ay, ph, dt, ctl, box);
   count_launch();
   return cudaGetLastError();
 }
 
-template <bool E, bool M3>
+template <bool M3>
 cudaError_t launch_sel(int tile, const double *A, double *B, int ix, int jx,
                        const Axis &ax, const Axis &ay, const Phys &ph,
                        double dt, Ctl *ctl, Box3 box, cudaStream_t s) {
@@ -97,18 +97,18 @@ cudaError_t launch_sel(int tile, const double *A, double *B, int ix, int jx,
   // per SM on grids where 32 x 8 leaves a partly empty last wave (512^2:
   // 1024 tiles = 3.4 waves of 304 blocks, 32 x 9: 912 = 3.0 waves)
   switch (tile) {
-    case 1: return launch_tile<E, M3, 32, 8>(A, B, ix, jx, ax, ay, ph, dt, ctl, box, s);
-    case 2: return launch_tile<E, M3, 16, 16>(A, B, ix, jx, ax, ay, ph, dt, ctl, box, s);
-    case 3: return launch_tile<E, M3, 64, 8>(A, B, ix, jx, ax, ay, ph, dt, ctl, box, s);
-    case 4: return launch_tile<E, M3, 32, 9, 1>(A, B, ix, jx, ax, ay, ph, dt, ctl, box, s);
-    case 5: return launch_tile<E, M3, 32, 10>(A, B, ix, jx, ax, ay, ph, dt, ctl, box, s);
-    default: return launch_tile<E, M3, 32, 16>(A, B, ix, jx, ax, ay, ph, dt, ctl, box, s);
+    case 1: return launch_tile<M3, 32, 8>(A, B, ix, jx, ax, ay, ph, dt, ctl, box, s);
+    case 2: return launch_tile<M3, 16, 16>(A, B, ix, jx, ax, ay, ph, dt, ctl, box, s);
+    case 3: return launch_tile<M3, 64, 8>(A, B, ix, jx, ax, ay, ph, dt, ctl, box, s);
+    case 4: return launch_tile<M3, 32, 9, 1>(A, B, ix, jx, ax, ay, ph, dt, ctl, box, s);
+    case 5: return launch_tile<M3, 32, 10>(A, B, ix, jx, ax, ay, ph, dt, ctl, box, s);
+    default: return launch_tile<M3, 32, 16>(A, B, ix, jx, ax, ay, ph, dt, ctl, box, s);
   }
 }
 }  // namespace
 
-// tile 6: the y-marching kernel of the fast mlw_m3 step (mlw2d_df.cu); the
-// exact policy and mlw_m take the 32 x 9 tile in its place
+// Tiles of the exact policy (6 and 7 stand for 32 x 9); the fast policy's are the
+// marching block's (launch_mlw2d_fast).
 int mlw2d_tile_count() { return 8; }
 
 cudaError_t launch_mlw2d(int solver, bool exact, int tile, const double *A,
@@ -116,17 +116,12 @@ cudaError_t launch_mlw2d(int solver, bool exact, int tile, const double *A,
                          const Axis &ay, const Phys &ph, double dt, Ctl *ctl,
                          Box3 box, cudaStream_t s) {
   if (ix < 3 || jx < 3) return cudaErrorInvalidValue;
-  if (tile >= 6) {  // the y-marching tile (segments balanced per SM, or by waves)
-    if (solver == 1 && !exact)
-      return launch_mlw2d_march_fast(A, B, ix, jx, ax, ay, ph, dt, ctl, box, s, tile == 7);
-    tile = 4;
-  }
-  if (solver == 1) {
-    return exact ? launch_sel<true, true>(tile, A, B, ix, jx, ax, ay, ph, dt, ctl, box, s)
-                 : launch_sel<false, true>(tile, A, B, ix, jx, ax, ay, ph, dt, ctl, box, s);
-  }
-  return exact ? launch_sel<true, false>(tile, A, B, ix, jx, ax, ay, ph, dt, ctl, box, s)
-               : launch_sel<false, false>(tile, A, B, ix, jx, ax, ay, ph, dt, ctl, box, s);
+  if (!exact)
+    return launch_mlw2d_fast(solver, tile, A, B, ix, jx, ax, ay, ph, nullptr, nullptr, dt, ctl,
+                             box, s);
+  if (tile >= 6) tile = 4;
+  return solver == 1 ? launch_sel<true>(tile, A, B, ix, jx, ax, ay, ph, dt, ctl, box, s)
+                     : launch_sel<false>(tile, A, B, ix, jx, ax, ay, ph, dt, ctl, box, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -156,10 +151,16 @@ __global__ void k_cfl2d_full(const double *__restrict__ S, int ix, int jx,
       b2 = bx * bx + by * by;
       v2 = vx * vx + vy * vy;
     }
-    const FT ca2 = b2 * pi4i / ro;
-    const FT cs2 = gm * pr / ro;
-    const FT dtcfl = fmin_(FT(ax.d[i]), FT(ay.d[j])) / fsqrt(v2 + cs2 + ca2);
-    const double dtq = (FT(safety) * dtcfl).v;
+    double dtq;
+    if constexpr (!E) {  // one reciprocal and one reciprocal root (see cfl3_cell)
+      const double q = fma(fma(ph.gm, pr.v, b2.v * ph.pi4i), fd::rcp(ro.v), v2.v);
+      dtq = safety * fd::minp(ax.d[i], ay.d[j]) * fd::rsqrt_(q);
+    } else {
+      const FT ca2 = b2 * pi4i / ro;
+      const FT cs2 = gm * pr / ro;
+      const FT dtcfl = fmin_(FT(ax.d[i]), FT(ay.d[j])) / fsqrt(v2 + cs2 + ca2);
+      dtq = (FT(safety) * dtcfl).v;
+    }
     if (dtq < dmin) dmin = dtq;
   }
   block_min_to(out, dmin, red, threadIdx.x, blockDim.x);
@@ -190,61 +191,6 @@ cudaError_t launch_cfl2d_full(int solver, bool exact, const double *S, int ix,
 // With all = 1 the CFL covers every cell: a loop whose chkdav changes cells
 // after the step reduces its CFL here alone.
 
-// Cell (i, j) of frame index f: rows j < w or j >= jx-w (all i), then
-// columns i < w or i >= ix-w of the remaining rows (every cell with all).
-__device__ __forceinline__ void frame_cell(long long f, int ix, int jx, int w, int all,
-                                           int &i, int &j) {
-  const long long nrow = 2LL * w * ix;
-  if (all) {
-    i = (int)(f % ix);
-    j = (int)(f / ix);
-  } else if (f < nrow) {
-    const long long r = f / ix;
-    i = (int)(f % ix);
-    j = (r < w) ? (int)r : (int)(jx - 2 * w + r);
-  } else {
-    const long long q = f - nrow;
-    const long long r = q / (2 * w);
-    const int cidx = (int)(q % (2 * w));
-    j = (int)(w + r);
-    i = (cidx < w) ? cidx : (ix - 2 * w + cidx);
-  }
-}
-__host__ __device__ __forceinline__ long long frame_cells(int ix, int jx, int w, int all) {
-  const long long inner_rows = jx - 2LL * w;
-  return all ? (long long)ix * jx
-             : 2LL * w * ix + (inner_rows > 0 ? inner_rows * 2LL * w : 0);
-}
-
-// cfl_m3 (cfl_m for the 7-array layout) of one cell from its values q[v]:
-// safety * the cell's time-step limit; bad is set for a cell the CFL cannot
-// use.
-template <bool E, bool M3>
-__device__ __forceinline__ double cell_dtq(const double *q, int i, int j, const Axis &ax,
-                                           const Axis &ay, const Phys &ph, double safety,
-                                           bool &bad) {
-  using FT = F<E>;
-  using P = Prim<M3>;
-  const FT gm(ph.gm), pi4i(ph.pi4i);
-  const FT ro(q[P::RO]), pr(q[P::PR]);
-  const FT vx(q[P::VX]), vy(q[P::VY]);
-  const FT bx(q[P::BX]), by(q[P::BY]);
-  FT b2, v2;
-  if constexpr (M3) {
-    const FT vz(q[P::VZ]), bz(q[P::BZ]);
-    b2 = bx * bx + by * by + bz * bz;
-    v2 = vx * vx + vy * vy + vz * vz;
-  } else {
-    b2 = bx * bx + by * by;
-    v2 = vx * vx + vy * vy;
-  }
-  const FT ca2 = b2 * pi4i / ro;
-  const FT cs2 = gm * pr / ro;
-  const FT dtcfl = fmin_(FT(ax.d[i]), FT(ay.d[j])) / fsqrt(v2 + cs2 + ca2);
-  const double dtq = (FT(safety) * dtcfl).v;
-  bad |= bad_cell(ro.v, pr.v, dtq);
-  return dtq;
-}
 template <bool E, bool M3>
 __device__ __forceinline__ double frame_dtq(const double *__restrict__ S, size_t n, int i,
                                             int j, int ix, const Axis &ax, const Axis &ay,
@@ -287,88 +233,10 @@ __global__ void k_frame2d(const double *__restrict__ S, int ix, int jx,
   }
 }
 
-// The value at 1-based position l of row `row` after the x rules.  Not
-// inlined: bc_xy_value calls it from each of its rule cases.
-__device__ __noinline__ double bc_x_value(const double *row, int ix, int m, int kxl, int kxh,
-                                          double q0l, double q0h, const double *dxm, int l) {
-  return bd_value(kxl, kxh, m, ix, q0l, q0h, dxm, l, [&](int p) { return row[p - 1]; });
-}
-// The value at 1-based (i, j) of one variable's array after the x rules of
-// every row and then (cy: where they change the cell) the y rules of column i.
-__device__ __noinline__ double bc_xy_value(const double *sv, int ix, int jx, int m, int kxl,
-                                           int kxh, int kyl, int kyh, double qxl, double qxh,
-                                           double qyl, double qyh, const double *dxmx,
-                                           const double *dxmy, int i, int j, bool cy) {
-  auto xval = [&](int j1) {
-    return bc_x_value(sv + (size_t)(j1 - 1) * ix, ix, m, kxl, kxh, qxl, qxh, dxmx, i);
-  };
-  if (!cy) return xval(j);
-  return bd_value(kyl, kyh, m, jx, qyl, qyh, dxmy, j, xval);
-}
-
-// The boundary program and the frame CFL of one loop iteration in one
-// launch, for a 2-D loop without chkdav.  A thread owns one frame cell and
-// computes each variable's value there as the x rules and then the y rules
-// of the program leave it (bd_value of the y rules over a column whose values
-// are bd_value of the x rules over their rows): the same operations as
-// k_bc_axis (x), k_bc_axis (y), so the same bits, with no barrier between the
-// axes.  A thread reads only cells that no rule changes (the step's output)
-// and writes only its own cell, so the threads are independent.  It then
-// reduces the CFL over the frame as k_frame2d does, from the values in
-// registers, and the last block ends the iteration.
 template <bool E, bool M3>
 __global__ void __launch_bounds__(32 * Prim<M3>::N)
     k_bcframe2d(int ix, int jx, Axis ax, Axis ay, Phys ph, BcTable bc, Ctl *ctl) {
-  using P = Prim<M3>;
-  // a block takes 32 frame cells; thread (c, v) = (lane, warp) evaluates
-  // variable v of cell c, and the first warp reduces the CFL of the 32 cells
-  __shared__ double q[P::N][32];
-  __shared__ double red[32];
-  if (ctl->done | ctl->pause) return;
-  double *S = ctl->buf[ctl->cur ^ 1];  // the state the step just wrote
-  const size_t n = (size_t)ix * jx;
-  const int m = bc.margin, w = m + 1;
-  const long long total = frame_cells(ix, jx, w, 0);
-  const int c = threadIdx.x & 31, v = threadIdx.x >> 5;
-  double dmin = __longlong_as_double(0x7ff0000000000000LL);
-  bool bad = false;
-  for (long long f0 = blockIdx.x * 32LL; f0 < total; f0 += gridDim.x * 32LL) {
-    const long long f = f0 + c;
-    int i = 0, j = 0;
-    if (f < total) {
-      frame_cell(f, ix, jx, w, 0, i, j);
-      const double *sv = S + (size_t)v * n;
-      const int kxl = bc.kind[v][0], kxh = bc.kind[v][1];
-      const int kyl = bc.kind[v][2], kyh = bc.kind[v][3];
-      const bool cx = bd_changes(kxl, kxh, m, ix, i + 1);
-      const bool cy = bd_changes(kyl, kyh, m, jx, j + 1);
-      const double val = bc_xy_value(sv, ix, jx, m, kxl, kxh, kyl, kyh, bc.q0[v][0],
-                                     bc.q0[v][1], bc.q0[v][2], bc.q0[v][3], ax.dm, ay.dm,
-                                     i + 1, j + 1, cy);
-      if (cx || cy) S[(size_t)v * n + (size_t)i + (size_t)j * ix] = val;
-      q[v][c] = val;
-    }
-    __syncthreads();
-    if (v == 0 && f < total) {
-      double qc[P::N];
-#pragma unroll
-      for (int u = 0; u < P::N; u++) qc[u] = q[u][c];
-      const double dtq = cell_dtq<E, M3>(qc, i, j, ax, ay, ph, ctl->safety, bad);
-      if (dtq < dmin) dmin = dtq;
-    }
-    __syncthreads();
-  }
-  count_bad_block(bad, &ctl->nonfinite, threadIdx.x);
-  block_min_to(&ctl->cfl_bits, dmin, red, threadIdx.x, blockDim.x);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    const unsigned prev = atomicAdd(&ctl->frame_blocks_done, 1u);
-    if (prev == gridDim.x - 1) {
-      __threadfence();
-      finish_iteration(ctl);
-    }
-  }
+  bcframe2d<E, M3>(ix, jx, ax, ay, ph, bc, ctl, blockIdx.x, gridDim.x);
 }
 
 cudaError_t launch_bcframe2d(int solver, bool exact, int nvar, int ix, int jx, const Axis &ax,

@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(KT *KT)
 
 constexpr int ETX = 32, ETY = 8, ERPT = 2;
 
-template <bool E, bool M3, bool G>
+template <bool M3, bool G>
 __global__ void __launch_bounds__(ETX *ETY / ERPT, 1)
     k_mlw2d_e(const double *__restrict__ A, double *__restrict__ B, int ix, int jx,
               Axis ax, Axis ay, Phys ph, const double *__restrict__ grav,
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(ETX *ETY / ERPT, 1)
     safety = ctl->safety;
     cfl = &ctl->cfl_bits;
   }
-  tile_step<E, M3, ETX, ETY, ERPT, G, true>(A, B, ix, jx, ax, ay, ph, dt, safety, cfl,
+  tile_step<M3, ETX, ETY, ERPT, G, true>(A, B, ix, jx, ax, ay, ph, dt, safety, cfl,
                                             box, blockIdx.x, blockIdx.y, gridDim.x,
                                             gridDim.y, smem, grav, res,
                                             ctl ? &ctl->nonfinite : nullptr);
@@ -273,15 +273,6 @@ cudaError_t launch_e(const double *A, double *B, int ix, int jx, const Axis &ax,
                      const Axis &ay, const Phys &ph, const double *grav,
                      const double *eta, double *res, double dt, Ctl *ctl, Box3 box,
                      cudaStream_t s) {
-  using T = Tile<ETX, ETY, M3, ERPT, G>;
-  static bool attr_set = false;  // per template instance
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(k_mlw2d_e<E, M3, G>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)T::smem_bytes);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
   const size_t n = (size_t)ix * jx;
   dim3 gc((ix + 31) / 32, (jx + 7) / 8);
   k_res_cells<E, M3><<<gc, dim3(32, 8), 0, s>>>(A, ix, jx, ax, ay, eta, res, ctl);
@@ -289,11 +280,24 @@ cudaError_t launch_e(const double *A, double *B, int ix, int jx, const Axis &ax,
   dim3 gk((ix - 1 + KT - 1) / KT, (jx - 1 + KT - 1) / KT);
   k_res_corners<E, M3><<<gk, KT * KT, 0, s>>>(A, ix, jx, ax, ay, eta + n, res, dt, ctl);
   count_launch();
-  dim3 grid((ix - 2 + ETX - 1) / ETX, (jx - 2 + ETY - 1) / ETY);
-  k_mlw2d_e<E, M3, G><<<grid, T::NT, T::smem_bytes, s>>>(A, B, ix, jx, ax, ay, ph, grav,
-                                                          res, dt, ctl, box);
-  count_launch();
-  return cudaGetLastError();
+  if constexpr (!E) {
+    return launch_mlw2d_fast(M3 ? 1 : 0, 0, A, B, ix, jx, ax, ay, ph, grav, res, dt, ctl, box, s);
+  } else {
+    using T = Tile<ETX, ETY, M3, ERPT, G>;
+    static bool attr_set = false;  // per template instance
+    if (!attr_set) {
+      cudaError_t e = cudaFuncSetAttribute(k_mlw2d_e<M3, G>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)T::smem_bytes);
+      if (e != cudaSuccess) return e;
+      attr_set = true;
+    }
+    dim3 grid((ix - 2 + ETX - 1) / ETX, (jx - 2 + ETY - 1) / ETY);
+    k_mlw2d_e<M3, G><<<grid, T::NT, T::smem_bytes, s>>>(A, B, ix, jx, ax, ay, ph, grav, res, dt,
+                                                        ctl, box);
+    count_launch();
+    return cudaGetLastError();
+  }
 }
 
 template <bool E, bool M3>

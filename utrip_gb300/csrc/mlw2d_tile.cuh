@@ -1,4 +1,5 @@
-// Fused 2-D modified Lax-Wendroff step (sm_103a, FP64): the tile body.
+// Fused 2-D modified Lax-Wendroff step, exact policy (sm_103a, FP64): the tile
+// body.  The fast and double-float policies' block is in mlw2d_march.cuh.
 //
 // One kernel replaces the whole body of the reference routines
 //   mlw_m3  cans2d/hdmlw/mlw_m3.f:64-374  (ro,pr,vx,vy,vz,bx,by,bz + az)
@@ -43,8 +44,7 @@
 // between cells i and i+1, then the y faces (i, j) between rows j and j+1,
 // ix*jx bytes each.
 //
-// In the exact policy every operation is the reference's, in its order, so
-// the result equals a -ffp-contract=off CPU build of the Fortran bit for bit.
+// Every operation is the reference's, in its order, so the result equals a -ffp-contract=off CPU build of the Fortran bit for bit.
 // Terms whose flux is identically zero (fx of bx, fy of by) are skipped: the
 // reference adds dt*(+0) to them, which leaves every value unchanged.
 #pragma once
@@ -144,8 +144,7 @@ __device__ __forceinline__ unsigned char av_branch(double dv, FT a, unsigned cha
 // single-grid kernel (one tile per block) and by the batched kernel (tiles
 // of many grids pulled from a work queue by persistent blocks).  If cfl_out
 // is non-null the CFL of the written cells inside `box` is reduced into it.
-template <bool E, bool M3, int TX, int TY, int RPT, bool G = false, bool R = false,
-          int AVF = 0>
+template <bool M3, int TX, int TY, int RPT, bool G = false, bool R = false, int AVF = 0>
 __device__ __forceinline__ void tile_step(
     const double *__restrict__ A, double *__restrict__ B, int ix, int jx,
     const Axis &ax, const Axis &ay, const Phys &ph, double dtv, double safety,
@@ -158,7 +157,7 @@ __device__ __forceinline__ void tile_step(
   using C = CellSlots<M3>;
   using K = CornerSlots<M3>;
   using P = Prim<M3>;
-  using FT = F<E>;
+  using FT = F<true>;
   double *sc = smem;                            // cells   [C::N][NC]
   double *sk = sc + (size_t)C::N * T::NC;       // corners [K::N][NK]
   double *sqx = sk + (size_t)K::N * T::NK;      // q*dxim  [TY][TX+1]
@@ -202,13 +201,8 @@ __device__ __forceinline__ void tile_step(
         bb = bx * bx + by * by;
       }
       FT ee, ep;
-      if constexpr (E) {
-        ee = pr / gm1 + 0.5 * ro * vv + pi8i * bb;     // mlw_m3.f:111
-        ep = pr * gm / gm1 + 0.5 * ro * vv;            // mlw_m3.f:141
-      } else {
-        ee = pr * ph.gm1i + 0.5 * ro * vv + pi8i * bb;
-        ep = pr * ph.ggm1 + 0.5 * ro * vv;
-      }
+      ee = pr / gm1 + 0.5 * ro * vv + pi8i * bb;     // mlw_m3.f:111
+      ep = pr * gm / gm1 + 0.5 * ro * vv;            // mlw_m3.f:141
       const FT rx = ro * vx, ry = ro * vy;
       if constexpr (G) {  // mlw_m3_g.f:95, 106, 117
         const FT gxc(grav[g]), gyc(grav[2 * n + g]);
@@ -274,20 +268,8 @@ __device__ __forceinline__ void tile_step(
       const int d = a + T::CX;            // (i  ,j+1)
       const FT dxim(ax.dim[gi]), dyim(ay.dim[gj]);
       // mlwhalf part 2: un = avg4(u) - dt*dfdx - dt*dfdy   (mlwhalf.f:45-52)
-      const double cxk = dt.v * dxim.v * 0.5, cyk = dt.v * dyim.v * 0.5;
       auto pred = [&](int su, int sfx, int sfy, bool negx, bool negy) -> FT {
-        if constexpr (!E) {  // same predictor, fewer rounded operations
-          double r = 0.25 * ((SC(su, b) + SC(su, a)) + (SC(su, cc) + SC(su, d)));
-          if (sfx != NOFLUX) {
-            const double s = (SC(sfx, b) - SC(sfx, a)) + (SC(sfx, cc) - SC(sfx, d));
-            r = fma(negx ? cxk : -cxk, s, r);
-          }
-          if (sfy != NOFLUX) {
-            const double s = (SC(sfy, d) - SC(sfy, a)) + (SC(sfy, cc) - SC(sfy, b));
-            r = fma(negy ? cyk : -cyk, s, r);
-          }
-          return FT(r);
-        }
+        
         const FT uh = 0.25 * (FT(SC(su, b)) + FT(SC(su, a)) + FT(SC(su, cc)) +
                               FT(SC(su, d)));
         FT un = uh;
@@ -312,14 +294,9 @@ __device__ __forceinline__ void tile_step(
       if constexpr (G) {
         // mlwsrch part 2: un += dt * (average of the four cell sources)
         auto srch = [&](int k, FT un) -> FT {
-          if constexpr (E) {
-            const FT sh = (FT(SGC(k, b)) + FT(SGC(k, a)) + FT(SGC(k, cc)) + FT(SGC(k, d))) /
-                          FT(4.0);
-            return un + dt * sh;
-          } else {
-            return FT(fma(dt.v, 0.25 * ((SGC(k, b) + SGC(k, a)) + (SGC(k, cc) + SGC(k, d))),
-                          un.v));
-          }
+          const FT sh = (FT(SGC(k, b)) + FT(SGC(k, a)) + FT(SGC(k, cc)) + FT(SGC(k, d))) /
+                        FT(4.0);
+          return un + dt * sh;
         };
         eeh = srch(0, eeh);
         rxh = srch(1, rxh);
@@ -334,16 +311,9 @@ __device__ __forceinline__ void tile_step(
       }
       // half-step primitives (mlw_m3.f:214-230)
       FT vxh, vyh, vzh(0.0);
-      if constexpr (E) {
-        vxh = rxh / roh;
-        vyh = ryh / roh;
-        if constexpr (M3) vzh = rzh / roh;
-      } else {
-        const FT rinv(1.0 / roh.v);
-        vxh = rxh * rinv;
-        vyh = ryh * rinv;
-        if constexpr (M3) vzh = rzh * rinv;
-      }
+      vxh = rxh / roh;
+      vyh = ryh / roh;
+      if constexpr (M3) vzh = rzh / roh;
       FT vv, bb;
       if constexpr (M3) {
         vv = vxh * vxh + vyh * vyh + vzh * vzh;
@@ -354,8 +324,7 @@ __device__ __forceinline__ void tile_step(
       }
       const FT prh = gm1 * (eeh - 0.5 * roh * vv - pi8i * bb);
       FT ep;
-      if constexpr (E) ep = prh * gm / gm1 + 0.5 * roh * vv;
-      else ep = prh * ph.ggm1 + 0.5 * roh * vv;
+      ep = prh * gm / gm1 + 0.5 * roh * vv;
       if constexpr (G) {  // corner sources (mlw_m3_g.f:194, 205, 216)
         const size_t gk = (size_t)gi + (size_t)gj * ix;
         const FT gxk(grav[n + gk]), gyk(grav[3 * n + gk]);
@@ -476,7 +445,7 @@ __device__ __forceinline__ void tile_step(
     // du for one conserved variable: half-step central difference,
     // corrector and artificial viscosity, in the reference order.
     auto dstep = [&](int su, int sfx, bool negx, int sfy, bool negy, int kfx,
-                     bool nkx, int kfy, bool nky, int gs) -> FT {
+                     bool nkx, int kfy, bool nky, int gs = -1) -> FT {
       FT du(0.0);
       // mlwhalf part 1 (mlwhalf.f:36-41)
       if (sfx != NOFLUX) {
@@ -517,97 +486,35 @@ __device__ __forceinline__ void tile_step(
       return u + du;
     };
 
-    // Fast policy: the new value of each conserved variable is a linear
-    // combination of 17 stencil values with per-cell coefficients, so it is
-    // evaluated as one chain of FMAs (mathematically the same update).
-    const double fcx = (hdt * hdx).v, fcy = (hdt * hdy).v;
-    const double fx0 = (hdt * dxi * uy0).v, fx1 = (hdt * dxi * uy1).v;
-    const double fy0 = (hdt * dyi * ux0).v, fy1 = (hdt * dyi * ux1).v;
-    const double ae = (dt * dxi * qxe).v, aw = (dt * dxi * qxw).v;
-    const double an = (dt * dyi * qyn).v, as = (dt * dyi * qys).v;
-    const double a1 = 1.0 - ((ae + aw) + (an + as));
-    auto fstep = [&](int su, int sfx, bool negx, int sfy, bool negy, int kfx,
-                     bool nkx, int kfy, bool nky, int gs) -> FT {
-      double r = a1 * SC(su, c);
-      if (G && gs >= 0) {
-        r = fma(hdt.v, SGC(gs, c), r);
-        const double w0 = (hdt * uy0).v, w1 = (hdt * uy1).v;
-        r = fma(w0, fma(ux0.v, SGK(gs, kSW), ux1.v * SGK(gs, kSE)), r);
-        r = fma(w1, fma(ux0.v, SGK(gs, kNW), ux1.v * SGK(gs, kNE)), r);
-      }
-      r = fma(ae, SC(su, cE), r);
-      r = fma(aw, SC(su, cW), r);
-      r = fma(an, SC(su, cN), r);
-      r = fma(as, SC(su, cS), r);
-      if (sfx != NOFLUX) {
-        const double d = SC(sfx, cE) - SC(sfx, cW);
-        r = fma(negx ? fcx : -fcx, d, r);
-      }
-      if (sfy != NOFLUX) {
-        const double d = SC(sfy, cN) - SC(sfy, cS);
-        r = fma(negy ? fcy : -fcy, d, r);
-      }
-      if (kfx != NOFLUX) {
-        const double d0 = SK(kfx, kSE) - SK(kfx, kSW), d1 = SK(kfx, kNE) - SK(kfx, kNW);
-        r = fma(nkx ? fx0 : -fx0, d0, r);
-        r = fma(nkx ? fx1 : -fx1, d1, r);
-      }
-      if (kfy != NOFLUX) {
-        const double d0 = SK(kfy, kNW) - SK(kfy, kSW), d1 = SK(kfy, kNE) - SK(kfy, kSE);
-        r = fma(nky ? fy0 : -fy0, d0, r);
-        r = fma(nky ? fy1 : -fy1, d1, r);
-      }
-      return FT(r);
-    };
-    auto step_var = [&](int su, int sfx, bool negx, int sfy, bool negy, int kfx,
-                        bool nkx, int kfy, bool nky, int gs = -1) -> FT {
-      if constexpr (E) return dstep(su, sfx, negx, sfy, negy, kfx, nkx, kfy, nky, gs);
-      else return fstep(su, sfx, negx, sfy, negy, kfx, nkx, kfy, nky, gs);
-    };
-    const FT ro = step_var(C::RO, C::RX, false, C::RY, false, K::XRO, false, K::YRO, false);
-    const FT ee = step_var(C::EE, C::FXE, false, C::FYE, false, K::XEE, false, K::YEE, false, 0);
+    const FT ro = dstep(C::RO, C::RX, false, C::RY, false, K::XRO, false, K::YRO, false);
+    const FT ee = dstep(C::EE, C::FXE, false, C::FYE, false, K::XEE, false, K::YEE, false, 0);
     const FT rx =
-        step_var(C::RX, C::FXRX, false, C::FYRX, false, K::XRX, false, K::YRX, false, 1);
+        dstep(C::RX, C::FXRX, false, C::FYRX, false, K::XRX, false, K::YRX, false, 1);
     const FT ry =
-        step_var(C::RY, C::FXRY, false, C::FYRY, false, K::XRY, false, K::YRY, false, 2);
-    const FT bx = step_var(C::BX, NOFLUX, false, C::EZ, false, NOFLUX, false, K::EZ, false);
-    const FT by = step_var(C::BY, C::EZ, true, NOFLUX, false, K::EZ, true, NOFLUX, false);
+        dstep(C::RY, C::FXRY, false, C::FYRY, false, K::XRY, false, K::YRY, false, 2);
+    const FT bx = dstep(C::BX, NOFLUX, false, C::EZ, false, NOFLUX, false, K::EZ, false);
+    const FT by = dstep(C::BY, C::EZ, true, NOFLUX, false, K::EZ, true, NOFLUX, false);
     FT rz(0.0), bz(0.0);
     if constexpr (M3) {
-      rz = step_var(C::RZ, C::FXRZ, false, C::FYRZ, false, K::XRZ, false, K::YRZ, false);
-      bz = step_var(C::BZ, C::EY, false, C::EX, true, K::EY, false, K::EX, true);
+      rz = dstep(C::RZ, C::FXRZ, false, C::FYRZ, false, K::XRZ, false, K::YRZ, false);
+      bz = dstep(C::BZ, C::EY, false, C::EX, true, K::EY, false, K::EX, true);
     }
     // vector potential: mlwsrch part 1 + mlwsrcf with s = -ez, -ezh
     const size_t g = (size_t)gi + (size_t)gj * ix;
     FT az;
-    if constexpr (E) {
-      FT daz(0.0);
-      daz = daz + hdt * (-FT(SC(C::EZ, c)));
-      const FT ssw = -FT(SK(K::EZ, kSW)), sse = -FT(SK(K::EZ, kSE));
-      const FT snw = -FT(SK(K::EZ, kNW)), sne = -FT(SK(K::EZ, kNE));
-      const FT sh = uy0 * (ux0 * ssw + ux1 * sse) + uy1 * (ux0 * snw + ux1 * sne);
-      daz = daz + hdt * sh;
-      az = FT(A[P::AZ * n + g]) + daz;
-    } else {
-      const double w0 = (hdt * uy0).v, w1 = (hdt * uy1).v;
-      double s = fma(ux0.v, SK(K::EZ, kSW), ux1.v * SK(K::EZ, kSE)) * w0;
-      s = fma(fma(ux0.v, SK(K::EZ, kNW), ux1.v * SK(K::EZ, kNE)), w1, s);
-      s = fma(hdt.v, SC(C::EZ, c), s);
-      az = FT(A[P::AZ * n + g] - s);
-    }
+    FT daz(0.0);
+    daz = daz + hdt * (-FT(SC(C::EZ, c)));
+    const FT ssw = -FT(SK(K::EZ, kSW)), sse = -FT(SK(K::EZ, kSE));
+    const FT snw = -FT(SK(K::EZ, kNW)), sne = -FT(SK(K::EZ, kNE));
+    const FT sh = uy0 * (ux0 * ssw + ux1 * sse) + uy1 * (ux0 * snw + ux1 * sne);
+    daz = daz + hdt * sh;
+    az = FT(A[P::AZ * n + g]) + daz;
 
     // back to primitives (mlw_m3.f:365-374)
     FT vx, vy, vz(0.0);
-    if constexpr (E) {
-      vx = rx / ro;
-      vy = ry / ro;
-      if constexpr (M3) vz = rz / ro;
-    } else {
-      const FT rinv(1.0 / ro.v);
-      vx = rx * rinv;
-      vy = ry * rinv;
-      if constexpr (M3) vz = rz * rinv;
-    }
+    vx = rx / ro;
+    vy = ry / ro;
+    if constexpr (M3) vz = rz / ro;
     FT vv, bb;
     if constexpr (M3) {
       vv = vx * vx + vy * vy + vz * vz;
@@ -639,23 +546,12 @@ __device__ __forceinline__ void tile_step(
         b2 = bx * bx + by * by;
         v2 = vx * vx + vy * vy;
       }
-      if constexpr (E) {
-        const FT ca2 = b2 * pi4i / ro;
-        const FT cs2 = gm * pr / ro;
-        const FT dtcfl = fmin_(FT(ax.d[gi]), FT(ay.d[gj])) / fsqrt(v2 + cs2 + ca2);
-        const double dtq = (FT(safety) * dtcfl).v;
-        if (dtq < dmin) dmin = dtq;
-        bad |= bad_cell(ro.v, pr.v, dtq);
-      } else {
-        // min over cells of min(dx,dy)/sqrt(S) is 1/sqrt(max of
-        // S*max(1/dx^2, 1/dy^2)): no division or root per cell.  dmin holds
-        // minus the largest key; the block converts it once.
-        const double rinv = 1.0 / ro.v;  // folded with the one above
-        const double s = v2.v + fma(gm.v, pr.v, pi4i.v * b2.v) * rinv;
-        const double kk = s * fmax(dxi.v * dxi.v, dyi.v * dyi.v);
-        if (-kk < dmin) dmin = -kk;
-        bad |= bad_cell(ro.v, pr.v, kk);
-      }
+      const FT ca2 = b2 * pi4i / ro;
+      const FT cs2 = gm * pr / ro;
+      const FT dtcfl = fmin_(FT(ax.d[gi]), FT(ay.d[gj])) / fsqrt(v2 + cs2 + ca2);
+      const double dtq = (FT(safety) * dtcfl).v;
+      if (dtq < dmin) dmin = dtq;
+      bad |= bad_cell(ro.v, pr.v, dtq);
     }
   }
 
@@ -676,12 +572,7 @@ __device__ __forceinline__ void tile_step(
   }
   if (cfl_out != nullptr) {
     if (bad_out != nullptr) count_bad_block(bad, bad_out, tid);
-    if constexpr (E) {
-      block_min_to(cfl_out, dmin, sred, tid, T::NT);
-    } else {
-      const double m = block_min(dmin, sred, tid, T::NT);  // -(largest key)
-      if (tid == 0 && m < 0.0) atomic_min_pos(cfl_out, safety / sqrt(-m));
-    }
+    block_min_to(cfl_out, dmin, sred, tid, T::NT);
   }
 #undef SC
 #undef SK

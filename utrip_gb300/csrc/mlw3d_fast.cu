@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, MINB)
     const double bx = A[P3::BX * n + g], by = A[P3::BY * n + g], bz = A[P3::BZ * n + g];
     const double rx = ro * vx, ry = ro * vy, rz = ro * vz;
     const double ek = 0.5 * fma(rx, vx, fma(ry, vy, rz * vz));
-    const double pm = ph.pi8i * fma(bx, bx, fma(by, by, bz * bz));
+    const double bb = fma(bx, bx, fma(by, by, bz * bz));
     const double ep = fma(pr, ph.ggm1, ek);
     double ex = fma(vz, by, -vy * bz), ey = fma(vx, bz, -vz * bx), ez = fma(vy, bx, -vx * by);
     if constexpr (R) {
@@ -161,8 +161,9 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, MINB)
       ey += res[n + g];
       ez += res[2 * n + g];
     }
-    const double pbx = ph.pi4i * bx, pby = ph.pi4i * by, pbz = ph.pi4i * bz, pt = pr + pm;
-    S(CRO) = ro; S(CEE) = fma(pr, ph.gm1i, ek + pm);
+    const double pbx = ph.pi4i * bx, pby = ph.pi4i * by, pbz = ph.pi4i * bz;
+    const double pt = fma(ph.pi8i, bb, pr);
+    S(CRO) = ro; S(CEE) = fma(pr, ph.gm1i, fma(ph.pi8i, bb, ek));
     S(CRX) = rx; S(CRY) = ry; S(CRZ) = rz;
     S(CBX) = bx; S(CBY) = by; S(CBZ) = bz;
     S(CEX) = ex; S(CEY) = ey; S(CEZ) = ez;
@@ -307,8 +308,8 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, MINB)
     const double ri = fd::rcp(ro);
     const double vx = rx * ri, vy = ry * ri, vz = rz * ri;
     const double ek = 0.5 * fma(rx, vx, fma(ry, vy, rz * vz));
-    const double pm = k8 * fma(bx, bx, fma(by, by, bz * bz));
-    const double pr = ph.gm1 * (ee - (ek + pm));
+    const double bb = fma(bx, bx, fma(by, by, bz * bz));
+    const double pr = ph.gm1 * fma(-k8, bb, ee - ek);
     const double ep = fma(pr, ph.ggm1, ek);
     double ex = fma(vz, by, -vy * bz), ey = fma(vx, bz, -vz * bx), ez = fma(vy, bx, -vx * by);
     if constexpr (R) {
@@ -316,7 +317,8 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, MINB)
       ey = fma(8.0, rq[1], ey);
       ez = fma(8.0, rq[2], ez);
     }
-    const double pbx = k4 * bx, pby = k4 * by, pbz = k4 * bz, pt = pr + pm;
+    const double pbx = k4 * bx, pby = k4 * by, pbz = k4 * bz;
+    const double pt = fma(k8, bb, pr);
     KS(KRX) = rx; KS(KRY) = ry; KS(KRZ) = rz;
     KS(KEX) = ex; KS(KEY) = ey; KS(KEZ) = ez;
     KS(KFX) = fma(ep, vx, fma(pbz, ey, -pby * ez));
@@ -519,7 +521,7 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, MINB)
       const double vx = rx * ri, vy = ry * ri, vz = rz * ri;
       const double ek = fma(rx, vx, fma(ry, vy, rz * vz));
       const double bb = fma(bx, bx, fma(by, by, bz * bz));
-      const double pr = ph.gm1 * (ee - fma(0.5, ek, ph.pi8i * bb));
+      const double pr = ph.gm1 * fma(-ph.pi8i, bb, fma(-0.5, ek, ee));
       const size_t g = (size_t)ii + (size_t)jj * ix + (size_t)k * plane;
       B[P3::RO * n + g] = ro;
       B[P3::PR * n + g] = pr;
