@@ -1,0 +1,82 @@
+// Stencil sums of doubles on the integer pipe (sm_103a).
+//
+// GB300 executes two FP64 lanes per SM and clock: an FP64 addition takes that
+// pipe as long as 64 issue slots, while the integer pipes of a kernel bound by
+// it stand idle.  A sum of a few doubles is formed here as an integer: the
+// significands are aligned to the largest exponent of the operands, negated
+// where the sign says so, added as 64-bit integers, and the sum is normalised and
+// rounded once.  No FP64 instruction is used.
+//
+// Accuracy: the aligned operands keep G bits below the last place of the largest
+// one (8 for a sum of four, 7 for one of up to eight: what 64 bits leave), so an
+// operand up to 2^G smaller enters exactly and a smaller one is truncated below
+// 2^-(52+G) of the largest one's power of two.  A sum of four is within 2^-58 of its
+// largest operand before its one rounding (to nearest even), where the FP64
+// chain rounds each partial sum to 2^-53; sums that cancel to zero are zero.
+//
+// The operands may be zero.  Where the largest exponent is not within the range
+// of `special` (subnormals and their neighbourhood, the largest numbers,
+// infinities, NaN) the caller forms its sums in FP64 instead.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace cans {
+namespace isum {
+
+// exponent field of x, in place
+__device__ __forceinline__ unsigned expo(double x) {
+  return (unsigned)__double2hiint(x) & 0x7ff00000u;
+}
+// no sum of operands with largest exponent E (in place) may be formed here
+__device__ __forceinline__ bool special(unsigned E) {
+  return E - 0x04000000u >= 0x7b800000u && E != 0u;  // fields 1 .. 63, 2040 .. 2047
+}
+
+// the significand bits of x (written on its words: the compiler turns a test of the
+// whole against zero into an FP64 comparison)
+__device__ __forceinline__ unsigned bits(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7fffffffu) | (unsigned)__double2loint(x);
+}
+
+// x as an integer in units of 2^-(52+G) of the power of two of exponent E >=
+// expo(x): |result| < 2^(53+G)
+template <int G> __device__ __forceinline__ long long at(double x, unsigned E) {
+  const int hi = __double2hiint(x);
+  const unsigned lo = (unsigned)__double2loint(x), e = (unsigned)hi & 0x7ff00000u;
+  const unsigned h = ((unsigned)hi & 0xfffffu) | min(e, 0x100000u);  // 0: no hidden bit
+  unsigned long long m = ((unsigned long long)h << 32 | lo) << G;
+  asm("shr.u64 %0, %0, %1;" : "+l"(m) : "r"((E - e) >> 20));  // shifts beyond 63 give 0
+  const long long s = hi >> 31;
+  return ((long long)m ^ s) - s;
+}
+
+// the double nearest to s in the units of E (ties to even)
+template <int G> __device__ __forceinline__ double out(long long s, unsigned E) {
+  const int sh = (int)(s >> 32);
+  const long long sg = sh >> 31;
+  unsigned long long m = (unsigned long long)((s ^ sg) - sg);
+  const int lz = __clzll((long long)m);
+  asm("shl.b64 %0, %0, %1;" : "+l"(m) : "r"(lz));
+  const unsigned lo = (unsigned)m;
+  const unsigned up = ((lo & 0x7ffu) + 0x3ffu + ((lo >> 11) & 1u)) >> 11;
+  // a leading bit at 52 + G is the exponent E; the hidden bit adds one to the
+  // field, and so does a carry of the rounding
+  const unsigned f = m ? E + ((unsigned)(10 - G - lz) << 20) : 0u;
+  const unsigned long long b = (m >> 11) + up;
+  return __hiloint2double((int)((unsigned)(b >> 32) + f) | (sh & (int)0x80000000), (int)b);
+}
+
+// four operands aligned to their largest exponent
+struct Four {
+  long long a, b, c, d;
+  unsigned E;
+};
+__device__ __forceinline__ Four four(double a, double b, double c, double d, bool &sp) {
+  const unsigned E = max(max(expo(a), expo(b)), max(expo(c), expo(d)));
+  sp |= special(E);
+  if (E == 0u) sp |= (bits(a) | bits(b) | bits(c) | bits(d)) != 0u;  // a subnormal
+  return {at<8>(a, E), at<8>(b, E), at<8>(c, E), at<8>(d, E), E};
+}
+
+}  // namespace isum
+}  // namespace cans

@@ -38,11 +38,13 @@
 #include <cuda_runtime.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "cans_common.cuh"
 #include "cans_internal.h"
 #include "df64.cuh"
 #include "fd64.cuh"
+#include "isum.cuh"
 #include "mlw2d_tile.cuh"  // Prim, av_branch
 
 namespace cans {
@@ -241,6 +243,137 @@ __device__ __forceinline__ void march_cell(const MarchArgs &a, size_t n, size_t 
 #undef SC
 }
 
+// The predictor's four-cell sums of a field: S the sum over the cells a, b (x+1),
+// c (x+1, y+1), d (y+1), X and Y the differences along x and y.  Fields needed in
+// two forms share their partial sums.
+template <class N, class T> struct Cells4 {
+  using V = typename N::V;
+  const V *p;  // cell a of field 0
+  bool sp = false;
+  __device__ __forceinline__ void load(int f, V &a, V &b, V &c, V &d) const {
+    const V *q = p + (size_t)f * T::NC;
+    a = q[0];
+    b = q[1];
+    c = q[T::CX + 1];
+    d = q[T::CX];
+  }
+  __device__ __forceinline__ V sum(int f) {
+    V a, b, c, d;
+    load(f, a, b, c, d);
+    return N::add(N::add(b, a), N::add(c, d));
+  }
+  __device__ __forceinline__ V dx(int f) {
+    V a, b, c, d;
+    load(f, a, b, c, d);
+    return N::add(N::sub(b, a), N::sub(c, d));
+  }
+  __device__ __forceinline__ V dy(int f) {
+    V a, b, c, d;
+    load(f, a, b, c, d);
+    return N::add(N::sub(d, a), N::sub(c, b));
+  }
+  __device__ __forceinline__ void sum_dx(int f, V &s, V &x) {
+    V a, b, c, d;
+    load(f, a, b, c, d);
+    const V l = N::add(a, d), r = N::add(b, c);
+    s = N::add(l, r);
+    x = N::sub(r, l);
+  }
+  __device__ __forceinline__ void sum_dy(int f, V &s, V &y) {
+    V a, b, c, d;
+    load(f, a, b, c, d);
+    const V l = N::add(a, b), r = N::add(d, c);
+    s = N::add(l, r);
+    y = N::sub(r, l);
+  }
+  __device__ __forceinline__ void dx_dy(int f, V &x, V &y) {
+    V a, b, c, d;
+    load(f, a, b, c, d);
+    const V u = N::sub(c, a), w = N::sub(b, d);
+    x = N::add(u, w);
+    y = N::sub(u, w);
+  }
+};
+// The same for doubles on the integer pipe (isum.cuh); sp is set where a sum must
+// be formed in FP64.
+template <class T> struct ICells4 {
+  const double *p;
+  bool sp = false;
+  __device__ __forceinline__ isum::Four load(int f) {
+    const double *q = p + (size_t)f * T::NC;
+    return isum::four(q[0], q[1], q[T::CX + 1], q[T::CX], sp);
+  }
+  __device__ __forceinline__ double sum(int f) {
+    const isum::Four q = load(f);
+    return isum::out<8>((q.a + q.b) + (q.c + q.d), q.E);
+  }
+  __device__ __forceinline__ double dx(int f) {
+    const isum::Four q = load(f);
+    return isum::out<8>((q.b - q.a) + (q.c - q.d), q.E);
+  }
+  __device__ __forceinline__ double dy(int f) {
+    const isum::Four q = load(f);
+    return isum::out<8>((q.d - q.a) + (q.c - q.b), q.E);
+  }
+  __device__ __forceinline__ void sum_dx(int f, double &s, double &x) {
+    const isum::Four q = load(f);
+    const long long l = q.a + q.d, r = q.b + q.c;
+    s = isum::out<8>(l + r, q.E);
+    x = isum::out<8>(r - l, q.E);
+  }
+  __device__ __forceinline__ void sum_dy(int f, double &s, double &y) {
+    const isum::Four q = load(f);
+    const long long l = q.a + q.b, r = q.d + q.c;
+    s = isum::out<8>(l + r, q.E);
+    y = isum::out<8>(r - l, q.E);
+  }
+  __device__ __forceinline__ void dx_dy(int f, double &x, double &y) {
+    const isum::Four q = load(f);
+    const long long u = q.c - q.a, w = q.b - q.d;
+    x = isum::out<8>(u + w, q.E);
+    y = isum::out<8>(u - w, q.E);
+  }
+};
+
+// The predictor of one corner (mlwhalf part 2): four times its conserved values
+// (ro, ee, rx, ry, bx, by, rz, bz) from the cell sums `st`.
+template <class N, class T, bool M3, bool G, class St>
+__device__ __forceinline__ void march_predict(St &st, typename N::V cx4, typename N::V cy4,
+                                              typename N::V dt, typename N::V *u) {
+  using V = typename N::V;
+  const V nx = N::neg(cx4), ny = N::neg(cy4);
+  V sx, sy, x, y;
+  st.sum_dx(CRX, sx, x);
+  st.sum_dy(CRY, sy, y);
+  u[0] = N::mad(ny, y, N::mad(nx, x, st.sum(CRO)));
+  st.dx_dy(CXY, x, y);
+  u[2] = N::mad(ny, y, N::mad(nx, st.dx(CXX), sx));
+  u[3] = N::mad(ny, st.dy(CYY), N::mad(nx, x, sy));
+  u[1] = N::mad(ny, st.dy(CFY), N::mad(nx, st.dx(CFX), st.sum(CEE)));
+  st.dx_dy(CEZ, x, y);
+  u[4] = N::mad(ny, y, st.sum(CBX));
+  u[5] = N::mad(cx4, x, st.sum(CBY));
+  if constexpr (M3) {
+    u[6] = N::mad(ny, st.dy(CYZ), N::mad(nx, st.dx(CXZ), st.sum(CRZ)));
+    u[7] = N::mad(cy4, st.dy(CEX), N::mad(nx, st.dx(CEY), st.sum(CBZ)));
+  }
+  if constexpr (G) {  // mlwsrch part 2: dt times the mean of the four sources
+    u[1] = N::mad(dt, st.sum(T::GC), u[1]);
+    u[2] = N::mad(dt, st.sum(T::GC + 1), u[2]);
+    u[3] = N::mad(dt, st.sum(T::GC + 2), u[3]);
+  }
+}
+// The same with FP64 sums, into the corner's slots: where an integer sum cannot be
+// formed (isum::special).
+template <class T, bool M3, bool G>
+__device__ __noinline__ void march_predict_fp64(const double *p, double *sk, double cx4,
+                                                double cy4, double dt) {
+  Cells4<F64N, T> st{p};
+  double u[8];
+  march_predict<F64N, T, M3, G>(st, cx4, cy4, dt, u);
+  for (int v = 0; v < (M3 ? 8 : 6); v++) sk[(size_t)v * T::NK] = u[v];
+}
+
 // Half-step values of one corner k from its four cells a, b (x+1), cc (x+1, y+1),
 // d (y+1), at four times their value (phase 2).  cx4, cy4 = 2 dt / dxm, 2 dt / dym;
 // g the corner's index in the global arrays.
@@ -250,8 +383,6 @@ __device__ __forceinline__ void march_corner(const MarchArgs &m, size_t n, size_
                                              int k, typename N::V cx4, typename N::V cy4,
                                              typename N::V dt, const PhysN<N> &P) {
   using V = typename N::V;
-  const int b = a + 1, cc = a + 1 + T::CX, d = a + T::CX;
-#define SC(s, c) sc[(size_t)(s) * T::NC + (c)]
 #define SK(s) sk[(size_t)(s) * T::NK + k]
   // global operands first, so that their latency overlaps the predictor
   double gq[2] = {0.0, 0.0}, rq[3] = {0.0, 0.0, 0.0};
@@ -266,49 +397,21 @@ __device__ __forceinline__ void march_corner(const MarchArgs &m, size_t n, size_
       rq[1] = m.res[4 * n + g];
     }
   }
-  auto sum = [&](int s) {
-    return N::add(N::add(SC(s, b), SC(s, a)), N::add(SC(s, cc), SC(s, d)));
-  };
-  auto dx = [&](int s) {
-    return N::add(N::sub(SC(s, b), SC(s, a)), N::sub(SC(s, cc), SC(s, d)));
-  };
-  auto dy = [&](int s) {
-    return N::add(N::sub(SC(s, d), SC(s, a)), N::sub(SC(s, cc), SC(s, b)));
-  };
-  auto dx_dy = [&](int s, V &x, V &y) {
-    const V u = N::sub(SC(s, cc), SC(s, a)), w = N::sub(SC(s, b), SC(s, d));
-    x = N::add(u, w);
-    y = N::sub(u, w);
-  };
-  const V nx = N::neg(cx4), ny = N::neg(cy4);
-  V sx, sy, x, y;
-  {  // rx: mean and x mass flux
-    const V l = N::add(SC(CRX, a), SC(CRX, d)), r = N::add(SC(CRX, b), SC(CRX, cc));
-    sx = N::add(l, r);
-    x = N::sub(r, l);
+  V u[8];
+  if constexpr (std::is_same<N, F64N>::value) {
+    ICells4<T> st{sc + a};
+    march_predict<N, T, M3, G>(st, cx4, cy4, dt, u);
+    if (st.sp) {  // a real branch: the FP64 sums must not be predicated in
+      march_predict_fp64<T, M3, G>(sc + a, sk + k, cx4, cy4, dt);
+#pragma unroll
+      for (int v = 0; v < (M3 ? 8 : 6); v++) u[v] = SK(v);
+    }
+  } else {
+    Cells4<N, T> st{sc + a};
+    march_predict<N, T, M3, G>(st, cx4, cy4, dt, u);
   }
-  {  // ry: mean and y mass flux
-    const V l = N::add(SC(CRY, a), SC(CRY, b)), r = N::add(SC(CRY, d), SC(CRY, cc));
-    sy = N::add(l, r);
-    y = N::sub(r, l);
-  }
-  const V ro = N::mad(ny, y, N::mad(nx, x, sum(CRO)));
-  dx_dy(CXY, x, y);
-  V rx = N::mad(ny, y, N::mad(nx, dx(CXX), sx));
-  V ry = N::mad(ny, dy(CYY), N::mad(nx, x, sy));
-  V ee = N::mad(ny, dy(CFY), N::mad(nx, dx(CFX), sum(CEE)));
-  dx_dy(CEZ, x, y);
-  const V bx = N::mad(ny, y, sum(CBX)), by = N::mad(cx4, x, sum(CBY));
-  V rz = N::zero(), bz = N::zero();
-  if constexpr (M3) {
-    rz = N::mad(ny, dy(CYZ), N::mad(nx, dx(CXZ), sum(CRZ)));
-    bz = N::mad(cy4, dy(CEX), N::mad(nx, dx(CEY), sum(CBZ)));
-  }
-  if constexpr (G) {  // mlwsrch part 2: dt times the mean of the four sources
-    ee = N::mad(dt, sum(T::GC), ee);
-    rx = N::mad(dt, sum(T::GC + 1), rx);
-    ry = N::mad(dt, sum(T::GC + 2), ry);
-  }
+  const V ro = u[0], ee = u[1], rx = u[2], ry = u[3], bx = u[4], by = u[5];
+  const V rz = M3 ? u[6] : N::zero(), bz = M3 ? u[7] : N::zero();
   const V ri = N::rcp(ro), vx = N::mul(rx, ri), vy = N::mul(ry, ri);
   const V k4 = N::scale(P.pi4i, 0.25f), k8 = N::scale(P.pi8i, 0.25f);
   V vz = N::zero(), bb = N::mad(by, by, N::sqr(bx)), rv = N::mad(rx, vx, N::mul(ry, vy));
@@ -350,7 +453,6 @@ __device__ __forceinline__ void march_corner(const MarchArgs &m, size_t n, size_
     SK(T::GK + 1) = N::mul(ro, gx);
     SK(T::GK + 2) = N::mul(ro, gy);
   }
-#undef SC
 #undef SK
 }
 

@@ -2,10 +2,11 @@
 // and FP32 fused-multiply-add throughput.  Built into its own library,
 // libcansprobe.so, beside libcansgpu.so: it is measurement tooling for
 // bench.py, not part of the C ABI of the solver.  It also evaluates the FP64
-// functions of fd64.cuh on arrays, for their accuracy test.
+// functions of fd64.cuh and the sums of isum.cuh on arrays, for their tests.
 #include <cuda_runtime.h>
 
 #include "fd64.cuh"
+#include "isum.cuh"
 
 namespace {
 
@@ -99,6 +100,36 @@ extern "C" int cans_probe_fd64(int op, const double *x, const double *w, double 
   cudaMemcpy(d + n, w, b, cudaMemcpyHostToDevice);
   k_fd64<<<(n + 255) / 256, 256>>>(op, d, d + n, d + 2 * (size_t)n, n);
   const cudaError_t e = cudaMemcpy(y, d + 2 * (size_t)n, b, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e == cudaSuccess ? 0 : 2;
+}
+
+namespace {
+// y[2i] = the sum, y[2i+1] = (b - a) + (c - d) of the operands a, b, c, d =
+// x[4i .. 4i+3]; f[i] = 1 where they must be formed in FP64
+__global__ void k_isum(const double *x, double *y, int *f, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  bool sp = false;
+  const cans::isum::Four q =
+      cans::isum::four(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3], sp);
+  y[2 * i] = cans::isum::out<8>((q.a + q.b) + (q.c + q.d), q.E);
+  y[2 * i + 1] = cans::isum::out<8>((q.b - q.a) + (q.c - q.d), q.E);
+  f[i] = sp ? 1 : 0;
+}
+}  // namespace
+
+// Host arrays of 4 n, 2 n and n values.  Synchronous; 0 on success.
+extern "C" int cans_probe_isum(const double *x, double *y, int *f, int n) {
+  if (n < 1 || !x || !y || !f) return 1;
+  double *d = nullptr;
+  const size_t b = sizeof(double) * (size_t)n;
+  if (cudaMalloc(&d, 7 * b) != cudaSuccess) return 2;
+  int *df = reinterpret_cast<int *>(d + 6 * (size_t)n);
+  cudaMemcpy(d, x, 4 * b, cudaMemcpyHostToDevice);
+  k_isum<<<(n + 255) / 256, 256>>>(d, d + 4 * (size_t)n, df, n);
+  cudaMemcpy(y, d + 4 * (size_t)n, 2 * b, cudaMemcpyDeviceToHost);
+  const cudaError_t e = cudaMemcpy(f, df, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost);
   cudaFree(d);
   return e == cudaSuccess ? 0 : 2;
 }
