@@ -85,8 +85,8 @@ __global__ void __launch_bounds__(TX *TY / RPT, 1)
 // The same in the fast policy: an item is a segment of `seg` rows of a strip of
 // 32 columns, stepped by the single run's marching block (mlw2d_march.cuh), so
 // that a batch runs its zones at the rate of a step that fills the GPU.
-constexpr int kBatchCH = 8;
-template <bool M3>
+constexpr int kBatchCH = kFastCH;
+template <bool M3, bool U>
 __global__ void __launch_bounds__(March<kBatchCH, M3, false>::NT, 2)
     k_mlw2d_batch_fast(const BatchGrid *__restrict__ grids, int ngrids, int nitems, int seg,
                        unsigned int *queue) {
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(March<kBatchCH, M3, false>::NT, 2)
     m.bad = &ctl->nonfinite;
     m.box = G.box;
     const int jb = 1 + (t / G.ntx) * seg;
-    march_block<F64N, kBatchCH, M3, false, false, 0>(m, G.ax, G.ay, G.ph, t % G.ntx, G.ntx, jb,
+    march_block<F64N, kBatchCH, M3, false, false, 0, U>(m, G.ax, G.ay, G.ph, t % G.ntx, G.ntx, jb,
                                                      min(G.jx - 2, jb + seg - 1), smem_march);
   }
 }
@@ -191,12 +191,12 @@ static cudaError_t launch_batch(int cfg, const BatchGrid *grids, int ngrids,
     default: return launch_batch_cfg<M3, 32, 8, 2>(grids, ngrids, nitems, queue, s);
   }
 }
-template <bool M3>
+template <bool M3, bool U>
 static cudaError_t launch_batch_fast(int cfg, const BatchGrid *grids, int ngrids, int nitems,
                                      unsigned int *queue, cudaStream_t s) {
   using T = March<kBatchCH, M3, false>;
   static int resident = 0;  // per template instance
-  return launch_persistent(k_mlw2d_batch_fast<M3>, resident, T::NT, T::smem_bytes, nitems, s,
+  return launch_persistent(k_mlw2d_batch_fast<M3, U>, resident, T::NT, T::smem_bytes, nitems, s,
                            grids, ngrids, nitems, kFastConfigs[cfg].ty, queue);
 }
 
@@ -234,7 +234,7 @@ struct cans_batch {
     int ix = 0, jx = 0;
     size_t n = 0;
     double *buf[2] = {nullptr, nullptr};
-    double *metrics = nullptr;  // d, dm, di, dim, u0, u1 of x then of y
+    double *metrics = nullptr;  // the arrays of x, then of y
     Ctl *ctl = nullptr;
     BcTable bc{};
     Phys ph{};
@@ -247,6 +247,7 @@ struct cans_batch {
   BcTable *d_bc = nullptr;
   unsigned int *d_queue = nullptr;
   int nitems = 0, frame_blocks = 1;
+  int uniform = 1;  // every run's axes are (Axis::uniform)
   cudaGraphExec_t graph = nullptr;
   int graph_iters = 0, graph_nodes = 0;
 };
@@ -302,8 +303,9 @@ int step_launch(cans_batch *b, int cfg) {
     e = m3 ? launch_batch<true>(cfg, b->d_grids, b->ngrids, b->nitems, b->d_queue, b->s)
            : launch_batch<false>(cfg, b->d_grids, b->ngrids, b->nitems, b->d_queue, b->s);
   else
-    e = m3 ? launch_batch_fast<true>(cfg, b->d_grids, b->ngrids, b->nitems, b->d_queue, b->s)
-           : launch_batch_fast<false>(cfg, b->d_grids, b->ngrids, b->nitems, b->d_queue, b->s);
+    e = (m3 ? b->uniform ? launch_batch_fast<true, true> : launch_batch_fast<true, false>
+            : b->uniform ? launch_batch_fast<false, true> : launch_batch_fast<false, false>)(
+        cfg, b->d_grids, b->ngrids, b->nitems, b->d_queue, b->s);
   BK(e);
   return CANS_OK;
 }
@@ -406,27 +408,18 @@ extern "C" int cans_batch_create(cans_batch **out, int ngrids,
       e = cudaMemsetAsync(G.buf[k], 0, sizeof(double) * G.n * b->nvar, b->s);
       if (e != cudaSuccess) return bail(bfail(e, "cudaMemset(state)"));
     }
-    const size_t nm = 6 * (size_t)(d.ix + d.jx);
+    const size_t nmx = kAxisArrays * (size_t)d.ix, nm = nmx + kAxisArrays * (size_t)d.jx;
     e = cudaMalloc(&G.metrics, sizeof(double) * nm);
     if (e != cudaSuccess) return bail(bfail(e, "cudaMalloc(metrics)"));
     h.assign(nm, 0.0);
-    double *hx = h.data(), *hy = h.data() + 6 * (size_t)d.ix;
-    std::memcpy(hx, d.dx, sizeof(double) * d.ix);
-    std::memcpy(hx + d.ix, d.dxm, sizeof(double) * d.ix);
-    build_axis_host(d.ix, d.dx, d.dxm, hx + 2 * d.ix, hx + 3 * d.ix, hx + 4 * d.ix, hx + 5 * d.ix);
-    std::memcpy(hy, d.dy, sizeof(double) * d.jx);
-    std::memcpy(hy + d.jx, d.dym, sizeof(double) * d.jx);
-    build_axis_host(d.jx, d.dy, d.dym, hy + 2 * d.jx, hy + 3 * d.jx, hy + 4 * d.jx, hy + 5 * d.jx);
+    place_axis(G.ax, G.metrics, d.ix);
+    place_axis(G.ay, G.metrics + nmx, d.jx);
+    G.ax.uniform = build_axis_host(d.ix, d.dx, d.dxm, h.data());
+    G.ay.uniform = build_axis_host(d.jx, d.dy, d.dym, h.data() + nmx);
+    if (!G.ax.uniform || !G.ay.uniform) b->uniform = 0;
     e = cudaMemcpyAsync(G.metrics, h.data(), sizeof(double) * nm, cudaMemcpyHostToDevice, b->s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->s);
     if (e != cudaSuccess) return bail(bfail(e, "cudaMemcpy(metrics)"));
-    double *mx = G.metrics, *my = G.metrics + 6 * (size_t)d.ix;
-    G.ax.n = d.ix;
-    G.ax.d = mx; G.ax.dm = mx + d.ix; G.ax.di = mx + 2 * d.ix; G.ax.dim = mx + 3 * d.ix;
-    G.ax.u0 = mx + 4 * d.ix; G.ax.u1 = mx + 5 * d.ix;
-    G.ay.n = d.jx;
-    G.ay.d = my; G.ay.dm = my + d.jx; G.ay.di = my + 2 * d.jx; G.ay.dim = my + 3 * d.jx;
-    G.ay.u0 = my + 4 * d.jx; G.ay.u1 = my + 5 * d.jx;
     e = cudaMalloc(&G.ctl, sizeof(Ctl));
     if (e != cudaSuccess) return bail(bfail(e, "cudaMalloc(ctl)"));
     Ctl c;

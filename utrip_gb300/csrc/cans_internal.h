@@ -26,7 +26,27 @@ struct Axis {
   int n = 0;
   double *d = nullptr, *dm = nullptr, *di = nullptr, *dim = nullptr,
          *u0 = nullptr, *u1 = nullptr;
+  // 2^32 (2 u0 - 1) and 2^32 (2 u1 - 1), for the steps that take the corner weights
+  // u0, u1 as one half and a correction; only where uniform is set, the weights
+  // of every cell 1 .. n-2 within 2^-37 of one half (a mesh equally spaced up to
+  // the rounding of its positions)
+  float *e0 = nullptr, *e1 = nullptr;
+  int uniform = 0;
 };
+// doubles of one axis's arrays (e0 and e1 share the last n)
+constexpr int kAxisArrays = 7;
+// The arrays of `a` (n cells) at mem.
+inline void place_axis(Axis &a, double *mem, int n) {
+  a.n = n;
+  a.d = mem;
+  a.dm = mem + n;
+  a.di = mem + 2 * (size_t)n;
+  a.dim = mem + 3 * (size_t)n;
+  a.u0 = mem + 4 * (size_t)n;
+  a.u1 = mem + 5 * (size_t)n;
+  a.e0 = reinterpret_cast<float *>(mem + 6 * (size_t)n);
+  a.e1 = a.e0 + n;
+}
 
 // Physical constants of one run, computed on the host exactly as the
 // reference computes them.
@@ -316,8 +336,9 @@ cudaError_t launch_bd_one(int kind, int axis, int mbnd, int margin0,
 cudaError_t launch_prepare(Ctl *ctl, cudaStream_t s);
 
 // Host-side metric construction with the reference expressions.
-void build_axis_host(int n, const double *d, const double *dm, double *di,
-                     double *dim, double *u0, double *u1);
+// Fills the host copy h (kAxisArrays n doubles, laid out as place_axis does) from
+// the cell widths d and the centre distances dm; returns Axis::uniform.
+int build_axis_host(int n, const double *d, const double *dm, double *h);
 Phys make_phys(double gm, double qav);
 
 // The stream the drop-in entry points use if one exists already (set by

@@ -30,18 +30,28 @@ unsigned long long launch_count() { return g_launches.load(); }
 
 // Reference metric set-up (cans2d/hdmlw/mlw_m3.f:70-86).  Index 0 and n-1 of
 // u0/u1 are never read by the step.
-void build_axis_host(int n, const double *d, const double *dm, double *di,
-                     double *dim, double *u0, double *u1) {
+int build_axis_host(int n, const double *d, const double *dm, double *h) {
+  Axis a;
+  place_axis(a, h, n);
+  int uniform = n >= 3;
+  std::memcpy(a.d, d, sizeof(double) * n);
+  std::memcpy(a.dm, dm, sizeof(double) * n);
   for (int i = 0; i < n; i++) {
-    di[i] = 1.0 / d[i];
-    dim[i] = 1.0 / dm[i];
-    u0[i] = 0.0;
-    u1[i] = 0.0;
+    a.di[i] = 1.0 / d[i];
+    a.dim[i] = 1.0 / dm[i];
+    a.u0[i] = 0.0;
+    a.u1[i] = 0.0;
+    a.e0[i] = a.e1[i] = 0.0f;
   }
   for (int i = 1; i < n - 1; i++) {
-    u1[i] = 0.5 * dm[i - 1] / d[i];
-    u0[i] = 0.5 * dm[i] / d[i];
+    a.u1[i] = 0.5 * dm[i - 1] / d[i];
+    a.u0[i] = 0.5 * dm[i] / d[i];
+    const double e0 = 2.0 * a.u0[i] - 1.0, e1 = 2.0 * a.u1[i] - 1.0;
+    a.e0[i] = (float)(e0 * 0x1p32);
+    a.e1[i] = (float)(e1 * 0x1p32);
+    if (!(std::fabs(e0) <= 0x1p-36 && std::fabs(e1) <= 0x1p-36)) uniform = 0;
   }
+  return uniform;
 }
 
 Phys make_phys(double gm, double qav) {
@@ -98,27 +108,21 @@ int lib_stream(cudaStream_t *s) {
   return CANS_OK;
 }
 
-// Device metric arrays of one axis (six arrays in one allocation).
+// Device metric arrays of one axis (in one allocation).
 struct DevAxis {
   Axis a;
   double *mem = nullptr;
   int cap = 0;
-  std::vector<double> h;  // host staging: d, dm, di, dim, u0, u1
+  std::vector<double> h;  // host staging
   int ensure(int n) {
     if (cap < n) {
       if (mem) cudaFree(mem);
       mem = nullptr;
       cap = 0;
-      CK(cudaMalloc(&mem, sizeof(double) * 6 * (size_t)n));
+      CK(cudaMalloc(&mem, sizeof(double) * kAxisArrays * (size_t)n));
       cap = n;
     }
-    a.n = n;
-    a.d = mem;
-    a.dm = mem + n;
-    a.di = mem + 2 * n;
-    a.dim = mem + 3 * n;
-    a.u0 = mem + 4 * n;
-    a.u1 = mem + 5 * n;
+    place_axis(a, mem, n);
     return CANS_OK;
   }
   // Upload d and dm, plus the derived arrays computed on the host with the
@@ -126,12 +130,9 @@ struct DevAxis {
   int upload(int n, const double *d, const double *dm, cudaStream_t s) {
     int rc = ensure(n);
     if (rc) return rc;
-    h.assign(6 * (size_t)n, 0.0);
-    std::memcpy(h.data(), d, sizeof(double) * n);
-    std::memcpy(h.data() + n, dm, sizeof(double) * n);
-    build_axis_host(n, d, dm, h.data() + 2 * n, h.data() + 3 * n,
-                    h.data() + 4 * n, h.data() + 5 * n);
-    CK(cudaMemcpyAsync(mem, h.data(), sizeof(double) * 6 * (size_t)n,
+    h.assign(kAxisArrays * (size_t)n, 0.0);
+    a.uniform = build_axis_host(n, d, dm, h.data());
+    CK(cudaMemcpyAsync(mem, h.data(), sizeof(double) * kAxisArrays * (size_t)n,
                        cudaMemcpyHostToDevice, s));
     return CANS_OK;
   }

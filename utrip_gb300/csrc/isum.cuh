@@ -38,11 +38,11 @@ __device__ __forceinline__ unsigned bits(double x) {
   return ((unsigned)__double2hiint(x) & 0x7fffffffu) | (unsigned)__double2loint(x);
 }
 
-// x as an integer in units of 2^-(52+G) of the power of two of exponent E >=
-// expo(x): |result| < 2^(53+G)
-template <int G> __device__ __forceinline__ long long at(double x, unsigned E) {
+// x 2^(e - expo(x)) as an integer in units of 2^-(52+G) of the power of two of
+// exponent E >= e: |result| < 2^(53+G)
+template <int G> __device__ __forceinline__ long long at(double x, unsigned e, unsigned E) {
   const int hi = __double2hiint(x);
-  const unsigned lo = (unsigned)__double2loint(x), e = (unsigned)hi & 0x7ff00000u;
+  const unsigned lo = (unsigned)__double2loint(x);
   const unsigned h = ((unsigned)hi & 0xfffffu) | min(e, 0x100000u);  // 0: no hidden bit
   unsigned long long m = ((unsigned long long)h << 32 | lo) << G;
   asm("shr.u64 %0, %0, %1;" : "+l"(m) : "r"((E - e) >> 20));  // shifts beyond 63 give 0
@@ -75,7 +75,34 @@ __device__ __forceinline__ Four four(double a, double b, double c, double d, boo
   const unsigned E = max(max(expo(a), expo(b)), max(expo(c), expo(d)));
   sp |= special(E);
   if (E == 0u) sp |= (bits(a) | bits(b) | bits(c) | bits(d)) != 0u;  // a subnormal
-  return {at<8>(a, E), at<8>(b, E), at<8>(c, E), at<8>(d, E), E};
+  return {at<8>(a, expo(a), E), at<8>(b, expo(b), E), at<8>(c, expo(c), E),
+          at<8>(d, expo(d), E), E};
+}
+
+// exponent field of 4 x
+__device__ __forceinline__ unsigned expo4(double x) {
+  const unsigned e = expo(x);
+  return e + min(e, 0x200000u);
+}
+// 2^-32 m e for an integer m and a small factor e: |e| <= 2^-4, |m| < 2^61
+__device__ __forceinline__ float scaled(long long m, float e) {
+  return __fmul_rn(__int2float_rn((int)(m >> 32)), e);
+}
+// (b - a) (1 + e0 2^-32) + (d - c) (1 + e1 2^-32) + 4 (g - f), |e0|, |e1| <= 2^-4: two
+// corner differences with weights near one and a central difference.  The
+// correction is 2^-36 of the differences and is taken to 24 bits: 2^-60 of them.
+__device__ __forceinline__ double diff6(double a, double b, double c, double d, double f,
+                                        double g, float e0, float e1, bool &sp) {
+  const unsigned ea = expo(a), eb = expo(b), ec = expo(c), ed = expo(d);
+  const unsigned ef = expo4(f), eg = expo4(g);
+  const unsigned E = max(max(max(ea, eb), max(ec, ed)), max(ef, eg));
+  sp |= special(E);
+  if (E == 0u) sp |= (bits(a) | bits(b) | bits(c) | bits(d) | bits(f) | bits(g)) != 0u;
+  const long long x = at<7>(b, eb, E) - at<7>(a, ea, E);
+  const long long y = at<7>(d, ed, E) - at<7>(c, ec, E);
+  const long long z = at<7>(g, eg, E) - at<7>(f, ef, E);
+  const int k = __float2int_rn(__fadd_rn(scaled(x, e0), scaled(y, e1)));
+  return out<7>(x + y + z + (long long)k, E);
 }
 
 }  // namespace isum

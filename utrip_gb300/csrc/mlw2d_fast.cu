@@ -11,7 +11,7 @@ namespace {
 template <bool M3, bool G, bool R>
 cudaError_t pick(int tile, const MarchArgs &m, const Axis &ax, const Axis &ay, const Phys &ph,
                  Ctl *ctl, cudaStream_t s) {
-  return launch_march<F64N, 8, M3, G, R>(m, ax, ay, ph, ctl, s, (tile & 1) != 0);
+  return launch_march<F64N, kFastCH, M3, G, R>(m, ax, ay, ph, ctl, s, (tile & 1) != 0);
 }
 template <bool M3>
 cudaError_t pick_terms(int tile, const MarchArgs &m, const Axis &ax, const Axis &ay,
@@ -57,8 +57,8 @@ cudaError_t launch_mlw2d_av_fast(int mode, const double *A, double *B, int ix, i
   m.dt = dt;
   m.avb = avb;
   m.nflip = nflip;
-  return mode == 1 ? launch_march<F64N, 8, true, false, false, 1>(m, ax, ay, ph, nullptr, s)
-                   : launch_march<F64N, 8, true, false, false, 2>(m, ax, ay, ph, nullptr, s);
+  return mode == 1 ? launch_march<F64N, kFastCH, true, false, false, 1>(m, ax, ay, ph, nullptr, s)
+                   : launch_march<F64N, kFastCH, true, false, false, 2>(m, ax, ay, ph, nullptr, s);
 }
 
 }  // namespace cans

@@ -159,6 +159,11 @@ enum {
 enum { KRX, KRY, KFX, KFY, KXX, KYY, KXY, KEZ, NK2, KXZ = NK2, KYZ, KEX, KEY, NK3 };
 constexpr int NOF = -1;
 
+// Rows of a chunk of the FP64 steps: 34 x 7 cells, 33 x 7 corners and 32 x 7 updated
+// cells fill 8, 8 and 7 warps, and two blocks of 8 warps leave 128 registers a
+// thread.
+constexpr int kFastCH = 7;
+
 template <int CH, bool M3, bool G> struct March {
   static constexpr int TX = 32, CX = TX + 2, KX = TX + 1;
   static constexpr int CR = CH + 2, KR = CH + 1;  // cell rows, corner rows
@@ -456,9 +461,107 @@ __device__ __forceinline__ void march_corner(const MarchArgs &m, size_t n, size_
 #undef SK
 }
 
+// Corner field f weighted to the cell whose lower left corner is kSW.
+template <class N, class T>
+__device__ __forceinline__ typename N::V march_to_cell(const typename N::V *sk, int f, int kSW,
+                                                       typename N::V ux0, typename N::V ux1,
+                                                       typename N::V uy0, typename N::V uy1) {
+  const typename N::V *q = sk + (size_t)f * T::NK + kSW;
+  const typename N::V s = N::mad(ux1, q[1], N::mul(ux0, q[0]));
+  const typename N::V t = N::mad(ux1, q[T::KX + 1], N::mul(ux0, q[T::KX]));
+  return N::mad(uy1, t, N::mul(uy0, s));
+}
+
+// The changes of the conserved variables of cell c (ro, ee, rx, ry, bx, by, rz,
+// bz): viscosity, central differences, corrector, gravity sources.  ae .. as are dt
+// q / (dx dxm) of the four faces, dtx = dt / dx, dty = dt / dy.
+//
+// U: the weights u0, u1 are one half up to ex0 .. ey1 (Axis::e0, e1), and the two
+// corner differences and the central difference of a direction are one integer
+// sum (isum::diff6): one FP64 instruction a direction where six are needed.
+// sp is set where such a sum must be formed in FP64.
+template <class N, class T, bool M3, bool G, bool U>
+__device__ __forceinline__ void march_du(const typename N::V *sc, const typename N::V *sk, int c,
+                                         int kSW, typename N::V ae, typename N::V aw,
+                                         typename N::V an, typename N::V as, typename N::V dtx,
+                                         typename N::V dty, typename N::V dt, typename N::V ux0,
+                                         typename N::V ux1, typename N::V uy0, typename N::V uy1,
+                                         float ex0, float ex1, float ey0, float ey1,
+                                         typename N::V *du, bool &sp) {
+  using V = typename N::V;
+  const int cE = c + 1, cW = c - 1, cN = c + T::CX, cS = c - T::CX;
+  const int kSE = kSW + 1, kNW = kSW + T::KX, kNE = kNW + 1;
+#define SC(s, c) sc[(size_t)(s) * T::NC + (c)]
+#define SK(s, c) sk[(size_t)(s) * T::NK + (c)]
+  const V aa = N::neg(N::add(N::add(ae, aw), N::add(an, as)));
+  // the corner values carry 4: hdt / 4 = dt / 8, and dt / 16 with a weight of 1/2
+  const V dtx16 = N::scale(dtx, 0.0625f), dty16 = N::scale(dty, 0.0625f);
+  const V fcx = N::scale(dtx, 0.25f), fcy = N::scale(dty, 0.25f);
+  const V hx = N::scale(dtx, 0.125f), hy = N::scale(dty, 0.125f);
+  const V fx0 = N::mul(hx, uy0), fx1 = N::mul(hx, uy1);
+  const V fy0 = N::mul(hy, ux0), fy1 = N::mul(hy, ux1);
+  auto var = [&](int su, int fx, bool nx, int kfx, int fy, bool ny, int kfy, int gs = -1) -> V {
+    V d = N::visc(ae, SC(su, cE), aw, SC(su, cW), an, SC(su, cN), as, SC(su, cS), aa, SC(su, c));
+    if constexpr (U) {
+      // fx0 (SE - SW) + fx1 (NE - NW) + fcx (E - W) = dtx/16 diff6
+      if (fx != NOF) {
+        const double q = isum::diff6(SK(kfx, kSW), SK(kfx, kSE), SK(kfx, kNW), SK(kfx, kNE),
+                                     SC(fx, cW), SC(fx, cE), ey0, ey1, sp);
+        d = N::mad(nx ? dtx16 : N::neg(dtx16), q, d);
+      }
+      if (fy != NOF) {
+        const double q = isum::diff6(SK(kfy, kSW), SK(kfy, kNW), SK(kfy, kSE), SK(kfy, kNE),
+                                     SC(fy, cS), SC(fy, cN), ex0, ex1, sp);
+        d = N::mad(ny ? dty16 : N::neg(dty16), q, d);
+      }
+    } else {
+      if (fx != NOF) {
+        d = N::mad(nx ? fcx : N::neg(fcx), N::sub(SC(fx, cE), SC(fx, cW)), d);
+        d = N::mad(nx ? fx0 : N::neg(fx0), N::sub(SK(kfx, kSE), SK(kfx, kSW)), d);
+        d = N::mad(nx ? fx1 : N::neg(fx1), N::sub(SK(kfx, kNE), SK(kfx, kNW)), d);
+      }
+      if (fy != NOF) {
+        d = N::mad(ny ? fcy : N::neg(fcy), N::sub(SC(fy, cN), SC(fy, cS)), d);
+        d = N::mad(ny ? fy0 : N::neg(fy0), N::sub(SK(kfy, kNW), SK(kfy, kSW)), d);
+        d = N::mad(ny ? fy1 : N::neg(fy1), N::sub(SK(kfy, kNE), SK(kfy, kSE)), d);
+      }
+    }
+    if constexpr (G) {
+      if (gs >= 0) {  // mlwsrch part 1 and mlwsrcf
+        d = N::mad(N::scale(dt, 0.5f), SC(T::GC + gs, c), d);
+        d = N::mad(N::scale(dt, 0.125f),
+                   march_to_cell<N, T>(sk, T::GK + gs, kSW, ux0, ux1, uy0, uy1), d);
+      }
+    }
+    return d;
+  };
+  du[0] = var(CRO, CRX, false, KRX, CRY, false, KRY);
+  du[4] = var(CBX, NOF, false, NOF, CEZ, false, KEZ);
+  du[5] = var(CBY, CEZ, true, KEZ, NOF, false, NOF);
+  if constexpr (M3) du[7] = var(CBZ, CEY, false, KEY, CEX, true, KEX);
+  du[1] = var(CEE, CFX, false, KFX, CFY, false, KFY, 0);
+  du[2] = var(CRX, CXX, false, KXX, CXY, false, KXY, 1);
+  du[3] = var(CRY, CXY, false, KXY, CYY, false, KYY, 2);
+  if constexpr (M3) du[6] = var(CRZ, CXZ, false, KXZ, CYZ, false, KYZ);
+#undef SC
+#undef SK
+}
+// The same in FP64, for the cells march_du's integer sums leave.
+template <class T, bool M3, bool G>
+__device__ __noinline__ void march_du_fp64(const double *sc, const double *sk, int c, int kSW,
+                                           double ae, double aw, double an, double as, double dtx,
+                                           double dty, double dt, double ux0, double ux1,
+                                           double uy0, double uy1, double *du) {
+  bool sp = false;
+  double d[8];
+  march_du<F64N, T, M3, G, false>(sc, sk, c, kSW, ae, aw, an, as, dtx, dty, dt, ux0, ux1, uy0,
+                                  uy1, 0.0f, 0.0f, 0.0f, 0.0f, d, sp);
+  for (int v = 0; v < (M3 ? 8 : 6); v++) du[v] = d[v];
+}
+
 // Rows jb .. je of strip `strip` (of nstrips) of one grid.  Every thread of the
 // block calls it; smem holds March<CH, M3, G>::smem_bytes.
-template <class N, int CH, bool M3, bool G, bool R, int AVF>
+template <class N, int CH, bool M3, bool G, bool R, int AVF, bool U>
 __device__ __forceinline__ void march_block(const MarchArgs &m, const Axis &ax, const Axis &ay,
                                             const Phys &ph, int strip, int nstrips, int jb,
                                             int je, double *smem) {
@@ -485,7 +588,7 @@ __device__ __forceinline__ void march_block(const MarchArgs &m, const Axis &ax, 
   const bool col = gi3 <= ix - 2;
   const V dxi = N::in(col ? ax.di[gi3] : 0.0);
   const V ux0 = N::in(col ? ax.u0[gi3] : 0.0), ux1 = N::in(col ? ax.u1[gi3] : 0.0);
-  const V dtx = N::mul(dt, dxi), fcx = N::scale(dtx, 0.25f), ix2 = N::sqr(dxi);
+  const V dtx = N::mul(dt, dxi), ix2 = N::sqr(dxi);
   const int fxi = tid % T::KX, fxr = tid / T::KX;
   const bool facex = tid < T::NQX && i0 + fxi < ix;
   const V qxc = facex ? N::mul(N::mul(P.qav, N::in(ax.dm[i0 - 1 + fxi])),
@@ -573,68 +676,45 @@ __device__ __forceinline__ void march_block(const MarchArgs &m, const Axis &ax, 
       double bz0 = 0.0;
       if constexpr (M3) bz0 = A[Q::BZ * n + g];
       const int c = lx + ly * T::CX;
-      const int cE = c + 1, cW = c - 1, cN = c + T::CX, cS = c - T::CX;
-      const int kSW = (lx - 1) + (ly - 1) * T::KX, kSE = kSW + 1;
-      const int kNW = kSW + T::KX, kNE = kNW + 1;
+      const int kSW = (lx - 1) + (ly - 1) * T::KX;
       const V dyi = N::in(ay.di[gj]);
       const V uy0 = N::in(ay.u0[gj]), uy1 = N::in(ay.u1[gj]);
-      const V dty = N::mul(dt, dyi), fcy = N::scale(dty, 0.25f);
-      // the corner values carry 4: hdt / 4 = dt / 8
-      const V hx = N::scale(dtx, 0.125f), hy = N::scale(dty, 0.125f);
-      const V fx0 = N::mul(hx, uy0), fx1 = N::mul(hx, uy1);
-      const V fy0 = N::mul(hy, ux0), fy1 = N::mul(hy, ux1);
+      const V dty = N::mul(dt, dyi);
       const V ae = N::mul(dtx, sqx[lx + (ly - 1) * T::KX]);
       const V aw = N::mul(dtx, sqx[lx - 1 + (ly - 1) * T::KX]);
       const V an = N::mul(dty, sqy[(lx - 1) + ly * T::TX]);
       const V as = N::mul(dty, sqy[(lx - 1) + (ly - 1) * T::TX]);
-      const V aa = N::neg(N::add(N::add(ae, aw), N::add(an, as)));
-      auto to_cell = [&](int f) {  // corner field f weighted to the cell, times 4
-        const V s = N::mad(ux1, SK(f, kSE), N::mul(ux0, SK(f, kSW)));
-        const V t = N::mad(ux1, SK(f, kNE), N::mul(ux0, SK(f, kNW)));
-        return N::mad(uy1, t, N::mul(uy0, s));
-      };
-      auto dvar = [&](int su, int sfx, bool negx, int sfy, bool negy, int kfx, bool nkx, int kfy,
-                      bool nky, int gs = -1) -> V {
-        V du = N::visc(ae, SC(su, cE), aw, SC(su, cW), an, SC(su, cN), as, SC(su, cS), aa,
-                       SC(su, c));
-        if (sfx != NOF)
-          du = N::mad(negx ? fcx : N::neg(fcx), N::sub(SC(sfx, cE), SC(sfx, cW)), du);
-        if (sfy != NOF)
-          du = N::mad(negy ? fcy : N::neg(fcy), N::sub(SC(sfy, cN), SC(sfy, cS)), du);
-        if (kfx != NOF) {
-          du = N::mad(nkx ? fx0 : N::neg(fx0), N::sub(SK(kfx, kSE), SK(kfx, kSW)), du);
-          du = N::mad(nkx ? fx1 : N::neg(fx1), N::sub(SK(kfx, kNE), SK(kfx, kNW)), du);
+      V du[8];
+      if constexpr (U) {
+        bool sp = false;
+        march_du<N, T, M3, G, true>(sc, sk, c, kSW, ae, aw, an, as, dtx, dty, dt, ux0, ux1, uy0,
+                                    uy1, ax.e0[gi], ax.e1[gi], ay.e0[gj], ay.e1[gj], du, sp);
+        if (sp) {  // a real branch, as in march_corner
+          double slow[8];
+          march_du_fp64<T, M3, G>(sc, sk, c, kSW, ae, aw, an, as, dtx, dty, dt, ux0, ux1, uy0,
+                                  uy1, slow);
+#pragma unroll
+          for (int v = 0; v < (M3 ? 8 : 6); v++) du[v] = slow[v];
         }
-        if (kfy != NOF) {
-          du = N::mad(nky ? fy0 : N::neg(fy0), N::sub(SK(kfy, kNW), SK(kfy, kSW)), du);
-          du = N::mad(nky ? fy1 : N::neg(fy1), N::sub(SK(kfy, kNE), SK(kfy, kSE)), du);
-        }
-        if constexpr (G) {
-          if (gs >= 0) {  // mlwsrch part 1 and mlwsrcf
-            du = N::mad(N::scale(dt, 0.5f), SC(T::GC + gs, c), du);
-            du = N::mad(dt8, to_cell(T::GK + gs), du);
-          }
-        }
-        return du;
-      };
-      const double ro_new =
-          ro0 + N::out(dvar(CRO, CRX, false, CRY, false, KRX, false, KRY, false));
-      const double bx_new =
-          bx0 + N::out(dvar(CBX, NOF, false, CEZ, false, NOF, false, KEZ, false));
-      const double by_new =
-          by0 + N::out(dvar(CBY, CEZ, true, NOF, false, KEZ, true, NOF, false));
+      } else {
+        bool sp = false;
+        march_du<N, T, M3, G, false>(sc, sk, c, kSW, ae, aw, an, as, dtx, dty, dt, ux0, ux1, uy0,
+                                     uy1, 0.0f, 0.0f, 0.0f, 0.0f, du, sp);
+      }
+      const double ro_new = ro0 + N::out(du[0]), bx_new = bx0 + N::out(du[4]);
+      const double by_new = by0 + N::out(du[5]);
+      const V ee = N::add(SC(CEE, c), du[1]), rx = N::add(SC(CRX, c), du[2]);
+      const V ry = N::add(SC(CRY, c), du[3]);
       double bz_new = 0.0;
-      if constexpr (M3)
-        bz_new = bz0 + N::out(dvar(CBZ, CEY, false, CEX, true, KEY, false, KEX, true));
-      const V ee = N::add(SC(CEE, c), dvar(CEE, CFX, false, CFY, false, KFX, false, KFY, false, 0));
-      const V rx = N::add(SC(CRX, c), dvar(CRX, CXX, false, CXY, false, KXX, false, KXY, false, 1));
-      const V ry = N::add(SC(CRY, c), dvar(CRY, CXY, false, CYY, false, KXY, false, KYY, false, 2));
       V rz = N::zero();
-      if constexpr (M3)
-        rz = N::add(SC(CRZ, c), dvar(CRZ, CXZ, false, CYZ, false, KXZ, false, KYZ, false));
+      if constexpr (M3) {
+        rz = N::add(SC(CRZ, c), du[6]);
+        bz_new = bz0 + N::out(du[7]);
+      }
       // vector potential: mlwsrch part 1 + mlwsrcf with s = -ez, -ezh
       B[Q::AZ * n + g] =
-          az0 - N::out(N::mad(dt8, to_cell(KEZ), N::mul(N::scale(dt, 0.5f), SC(CEZ, c))));
+          az0 - N::out(N::mad(dt8, march_to_cell<N, T>(sk, KEZ, kSW, ux0, ux1, uy0, uy1),
+                              N::mul(N::scale(dt, 0.5f), SC(CEZ, c))));
       // back to primitives (mlw_m3.f:365-374)
       const V ro = N::in(ro_new), bx = N::in(bx_new), by = N::in(by_new);
       const V rinv = N::rcp(ro), vx = N::mul(rx, rinv), vy = N::mul(ry, rinv);
@@ -703,8 +783,8 @@ __device__ __forceinline__ void march_block(const MarchArgs &m, const Axis &ax, 
   }
 }
 
-// The marching step of one grid: block (strip, segment of `seg` rows).
-template <class N, int CH, bool M3, bool G, bool R, int AVF>
+// The marching step of one grid (U: both axes are uniform): block (strip, segment of `seg` rows).
+template <class N, int CH, bool M3, bool G, bool R, int AVF, bool U>
 __global__ void __launch_bounds__(March<CH, M3, G>::NT, 2)
     k_mlw2d_march(MarchArgs m, Axis ax, Axis ay, Phys ph, Ctl *__restrict__ ctl, int seg) {
   extern __shared__ double smem_march[];
@@ -718,7 +798,7 @@ __global__ void __launch_bounds__(March<CH, M3, G>::NT, 2)
     m.bad = &ctl->nonfinite;
   }
   const int jb = 1 + blockIdx.y * seg;
-  march_block<N, CH, M3, G, R, AVF>(m, ax, ay, ph, blockIdx.x, gridDim.x, jb,
+  march_block<N, CH, M3, G, R, AVF, U>(m, ax, ay, ph, blockIdx.x, gridDim.x, jb,
                                     min(m.jx - 2, jb + seg - 1), smem_march);
 }
 
@@ -759,13 +839,13 @@ inline int balance_seg_waves(int strips, int rows, int ch, int slots) {
   return best;
 }
 
-template <class N, int CH, bool M3, bool G, bool R, int AVF = 0>
-cudaError_t launch_march(const MarchArgs &m, const Axis &ax, const Axis &ay, const Phys &ph,
+template <class N, int CH, bool M3, bool G, bool R, int AVF, bool U>
+cudaError_t launch_march_u(const MarchArgs &m, const Axis &ax, const Axis &ay, const Phys &ph,
                          Ctl *ctl, cudaStream_t s, bool waves = false) {
   using T = March<CH, M3, G>;
   static std::mutex mu;
   static int sms_of[64] = {}, slots_of[64] = {};
-  auto kern = k_mlw2d_march<N, CH, M3, G, R, AVF>;
+  auto kern = k_mlw2d_march<N, CH, M3, G, R, AVF, U>;
   int dev = 0, sms = 0, slots = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -795,6 +875,16 @@ cudaError_t launch_march(const MarchArgs &m, const Axis &ax, const Axis &ay, con
   kern<<<grid, T::NT, T::smem_bytes, s>>>(m, ax, ay, ph, ctl, seg);
   count_launch();
   return cudaGetLastError();
+}
+
+template <class N, int CH, bool M3, bool G, bool R, int AVF = 0>
+cudaError_t launch_march(const MarchArgs &m, const Axis &ax, const Axis &ay, const Phys &ph,
+                         Ctl *ctl, cudaStream_t s, bool waves = false) {
+  if constexpr (std::is_same<N, F64N>::value) {
+    if (ax.uniform && ay.uniform)
+      return launch_march_u<N, CH, M3, G, R, AVF, true>(m, ax, ay, ph, ctl, s, waves);
+  }
+  return launch_march_u<N, CH, M3, G, R, AVF, false>(m, ax, ay, ph, ctl, s, waves);
 }
 
 }  // namespace
