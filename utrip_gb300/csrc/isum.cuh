@@ -38,16 +38,23 @@ __device__ __forceinline__ unsigned bits(double x) {
   return ((unsigned)__double2hiint(x) & 0x7fffffffu) | (unsigned)__double2loint(x);
 }
 
-// x 2^(e - expo(x)) as an integer in units of 2^-(52+G) of the power of two of
-// exponent E >= e: |result| < 2^(53+G)
+// |x| 2^(e - expo(x)) as an integer in units of 2^-(52+G) of the power of two of
+// exponent E >= e: below 2^(53+G).  E is not `special`, so it is 0 or the fields are
+// 64 and up, and where e is 0 (zeros; subnormals beside a normal E) the hidden bit
+// set here is shifted out with the rest.
+template <int G> __device__ __forceinline__ unsigned long long mag(double x, unsigned e,
+                                                                   unsigned E) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  unsigned long long m =
+      (unsigned long long)(__funnelshift_l(lo, hi, 11) | 0x80000000u) << 32 | lo << 11;
+  const unsigned top = max(E, 0x04000000u) + ((unsigned)(11 - G) << 20);
+  asm("shr.u64 %0, %0, %1;" : "+l"(m) : "r"((top - e) >> 20));  // shifts beyond 63 give 0
+  return m;
+}
+// the same with x's sign
 template <int G> __device__ __forceinline__ long long at(double x, unsigned e, unsigned E) {
-  const int hi = __double2hiint(x);
-  const unsigned lo = (unsigned)__double2loint(x);
-  const unsigned h = ((unsigned)hi & 0xfffffu) | min(e, 0x100000u);  // 0: no hidden bit
-  unsigned long long m = ((unsigned long long)h << 32 | lo) << G;
-  asm("shr.u64 %0, %0, %1;" : "+l"(m) : "r"((E - e) >> 20));  // shifts beyond 63 give 0
-  const long long s = hi >> 31;
-  return ((long long)m ^ s) - s;
+  const long long s = __double2hiint(x) >> 31;
+  return ((long long)mag<G>(x, e, E) ^ s) - s;
 }
 
 // the double nearest to s in the units of E (ties to even)
@@ -103,6 +110,87 @@ __device__ __forceinline__ double diff6(double a, double b, double c, double d, 
   const long long z = at<7>(g, eg, E) - at<7>(f, ef, E);
   const int k = __float2int_rn(__fadd_rn(scaled(x, e0), scaled(y, e1)));
   return out<7>(x + y + z + (long long)k, E);
+}
+
+// exponent field of 16 x
+__device__ __forceinline__ unsigned expo16(double x) {
+  const unsigned e = expo(x);
+  return e + min(e, 0x400000u);
+}
+
+// Sums over two planes of four cells each: l and u point at the lower left cell of
+// the lower and the upper plane, a row is CX doubles.
+// the sum of the eight, and the differences along x, y and from lower to upper
+enum Form { kSum, kDx, kDy, kDz };
+template <int CX, int F>
+__device__ __forceinline__ double eight(const double *l, const double *u, bool &sp) {
+  const double v[8] = {l[0], l[1], l[CX], l[CX + 1], u[0], u[1], u[CX], u[CX + 1]};
+  unsigned e[8], E = 0u, any = 0u;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    e[i] = expo(v[i]);
+    E = max(E, e[i]);
+  }
+  sp |= special(E);
+  if (E == 0u) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) any |= bits(v[i]);
+    sp |= any != 0u;
+  }
+  long long s = 0;
+  int n = 0;  // of negative terms: -m is ~m + 1
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const bool neg = F == kDx ? !(i & 1) : F == kDy ? !(i & 2) : F == kDz ? i < 4 : false;
+    const int g = neg ? ~(__double2hiint(v[i]) >> 31) : __double2hiint(v[i]) >> 31;
+    s += (long long)mag<7>(v[i], e[i], E) ^ (long long)g;
+    n -= g;
+  }
+  return out<7>(s + n, E);
+}
+
+// The part of a direction of a cell's change that two corner planes and the central
+// difference give, on axes whose weights are one half up to 2^-32 e:
+//   gu   (b - a) (1 + e0) + (d - c) (1 + e1) of the upper corner plane
+//   ret  gl (1 + ez0) + gu (1 + ez1) + 16 (g - f), gl being the lower plane's gu
+__device__ __forceinline__ double diff_planes(double a, double b, double c, double d, double gl,
+                                              double f, double g, float e0, float e1, float ez0,
+                                              float ez1, double &gu, bool &sp) {
+  const unsigned ea = expo(a), eb = expo(b), ec = expo(c), ed = expo(d), el = expo(gl);
+  const unsigned ef = expo16(f), eg = expo16(g);
+  const unsigned E = max(max(max(ea, eb), max(ec, ed)), max(max(ef, eg), el));
+  sp |= special(E);
+  if (E == 0u) sp |= (bits(a) | bits(b) | bits(c) | bits(d) | bits(f) | bits(g) | bits(gl)) != 0u;
+  const long long x = at<6>(b, eb, E) - at<6>(a, ea, E);
+  const long long y = at<6>(d, ed, E) - at<6>(c, ec, E);
+  const long long z = at<6>(g, eg, E) - at<6>(f, ef, E);
+  const long long l = at<6>(gl, el, E);
+  const long long up = x + y + __float2int_rn(__fadd_rn(scaled(x, e0), scaled(y, e1)));
+  gu = out<6>(up, E);
+  return out<6>(l + up + z + __float2int_rn(__fadd_rn(scaled(l, ez0), scaled(up, ez1))), E);
+}
+// The z flux of a face, 16 times twice its value: the four corner values with
+// weights (1 + ex + ey), 16 (f + g), and the viscosity's w; neg: less the former
+// two.  pu is that of this face, the result its difference from the lower one pl.
+__device__ __forceinline__ double face_planes(double a, double b, double c, double d, double f,
+                                              double g, double w, double pl, bool neg, float ex0,
+                                              float ex1, float ey0, float ey1, double &pu,
+                                              bool &sp) {
+  const unsigned ea = expo(a), eb = expo(b), ec = expo(c), ed = expo(d), el = expo(pl);
+  const unsigned ef = expo16(f), eg = expo16(g), ew = expo(w);
+  const unsigned E =
+      max(max(max(ea, eb), max(ec, ed)), max(max(ef, eg), max(el, ew)));
+  sp |= special(E);
+  if (E == 0u)
+    sp |= (bits(a) | bits(b) | bits(c) | bits(d) | bits(f) | bits(g) | bits(pl) | bits(w)) != 0u;
+  const long long A = at<6>(a, ea, E), B = at<6>(b, eb, E), C = at<6>(c, ec, E);
+  const long long D = at<6>(d, ed, E);
+  const float k = __fadd_rn(__fadd_rn(scaled(A + B, ey0), scaled(C + D, ey1)),
+                            __fadd_rn(scaled(A + C, ex0), scaled(B + D, ex1)));
+  long long s = (A + B) + (C + D) + __float2int_rn(k) + (at<6>(f, ef, E) + at<6>(g, eg, E));
+  s = (neg ? -s : s) + at<6>(w, ew, E);
+  pu = out<6>(s, E);
+  return out<6>(s - at<6>(pl, el, E), E);
 }
 
 }  // namespace isum

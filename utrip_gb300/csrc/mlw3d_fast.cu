@@ -7,16 +7,16 @@
 // What bounds the step is the FP64 pipe (two lanes per SM and clock; HBM is at
 // 2 %), so the kernel is laid out for the fewest FP64 warp instructions:
 //  - A block owns a TX x TY column of cells and marches along z.  Per plane:
-//    the cells of plane k+1, the corners of plane k+1/2, the full step of plane
-//    k.  Each phase numbers its own work items (cells of the halo tile, corners,
-//    interior cells) through the threads, so that its warps are full: 16 x 8
-//    tiles take 6, 5 and 4 warps of a block of 6.
-//  - The predictor's sums over the four cells of a plane (the mean of u, the x
-//    and y differences of the fluxes, the sum of the z flux) are kept in
-//    registers for the next corner plane, which is the other side of that cell
-//    plane: 28 sums a corner, formed once.  Fields needed in two of these forms
-//    (the off-diagonal momentum fluxes, E, the momenta) share their partial
-//    sums: 97 additions a corner where eight-cell sums take 203.
+//    the cells of plane k+1 and, by other warps, the new primitives of plane k-1;
+//    the predictor's sums of the corners of plane k+1/2; their fluxes; the full step
+//    of plane k.  Each phase numbers its own work items (cells of the halo tile,
+//    corners, interior cells) through the threads, so that its warps are full.
+//  - The predictor's eight-cell sums and, on equally spaced axes, the corrector's
+//    differences and face sums are integer sums (isum.cuh): no FP64 instruction.
+//    They are chains of some 150 integer instructions, so two threads share a corner
+//    and a cell, with four of the eight variables each: 20 warps a SM where one
+//    thread for all eight leaves room for 10 (256^3: 16.7 against 16.3 ms, at the
+//    same FP64 work for the shared part done twice).
 //  - The corner quantities are kept at eight times their value (the eight-cell
 //    mean is a sum, every flux is linear in the conserved variables at given
 //    velocity), the factor is in constants and weights: no scaling products.
@@ -29,10 +29,13 @@
 //    needs one plane, and nothing of the cell plane k-1 is kept.
 //  - u_new = u + du with every term of du summed first: its terms round at
 //    their own size.
-//  - reciprocals of fd64.cuh; comparisons on the integer pipe.
-// FP64 warp instructions a zone (32 a warp instruction, 16 x 8 tiles): about
-// 550 against 920 of one that forms each cell's sums for itself.  Shared memory
-// 110 KB, 168 registers: two blocks a SM, whose barriers overlap.
+//  - reciprocals of fd64.cuh; comparisons on the integer pipe; signs flipped on
+//    the upper word (the compiler negates a double with an FP64 addition: 256^3
+//    15.9 -> 14.1 ms for the loops over the variables).
+// FP64 warp instructions a zone (32 a warp instruction, 16 x 8 tiles): 308, against
+// 588 with all sums in FP64 (18.2 ms at 256^3) and 920 of one that forms each cell's
+// sums for itself (29.9 ms).  Shared memory 114 KB, 96 registers: two blocks a SM,
+// whose phases overlap.
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -41,6 +44,7 @@
 #include "cans_internal.h"
 #include "cfl3.cuh"
 #include "fd64.cuh"
+#include "isum.cuh"
 
 namespace cans {
 
@@ -48,39 +52,119 @@ namespace {
 
 // cell slots: conserved, fluxes (XY = fx(ry) = fy(rx), ...), E, velocities
 enum {
-  CRO, CEE, CRX, CRY, CRZ, CBX, CBY, CBZ,
+  CRO, CEE, CRX, CBX, CRY, CRZ, CBY, CBZ,
   CFX, CFY, CFZ,                  // energy fluxes
   CXX, CYY, CZZ, CXY, CXZ, CYZ,   // momentum fluxes
   CEX, CEY, CEZ, CVX, CVY, CVZ, NCF
 };
 // corner slots, all eight times their value; the mass fluxes are the momenta
 enum { KRX, KRY, KRZ, KFX, KFY, KFZ, KXX, KYY, KZZ, KXY, KXZ, KYZ, KEX, KEY, KEZ, NKF };
-// what a corner keeps of its lower cell plane: S the sum over the four cells, X
-// and Y the differences along x and y
-enum {
-  S_RO, S_EE, S_RX, X_RX, S_RY, Y_RY, S_RZ, S_BX, S_BY, S_BZ, X_FX, Y_FY, S_FZ, X_XX, Y_YY,
-  S_ZZ, X_XY, Y_XY, X_XZ, S_XZ, Y_YZ, S_YZ, Y_EX, S_EX, X_EY, S_EY, X_EZ, Y_EZ, NPS
-};
-// what an interior column keeps of its lower corner plane: the x and y
-// differences of seven variables (ro, ee, rx, ry, rz, two of B) and the z face
-// fluxes of eight
+// what an interior column keeps of its lower corner plane: per variable the x and y
+// differences (seven each) and the z face flux
 constexpr int NRET = 22;
+
+// The fields of variable v (cell slot v): its x, y, z fluxes at the cells and corners,
+// -1 where it has none; their signs (of E in the induction equation); its retained x
+// and y differences; its gravity source.  In constant memory: the loops over the
+// variables stay rolled, so that their integer sums (some 600 instructions a pass)
+// stay in the instruction cache.  The two halves of the variables have about the
+// same number of sums (15 and 14 of the predictor, 11 and 10 of the corrector).
+struct VarFields {
+  signed char fx, kx, fy, ky, fz, kz, sx, sy, sz, rx, ry, g;
+};
+__constant__ VarFields kVar[8] = {
+    {CRX, KRX, CRY, KRY, CRZ, KRZ, 1, 1, 1, 0, 0, -1},
+    {CFX, KFX, CFY, KFY, CFZ, KFZ, 1, 1, 1, 1, 1, 0},
+    {CXX, KXX, CXY, KXY, CXZ, KXZ, 1, 1, 1, 2, 2, 1},
+    {-1, -1, CEZ, KEZ, CEY, KEY, 0, 1, -1, 0, 3, -1},
+    {CXY, KXY, CYY, KYY, CYZ, KYZ, 1, 1, 1, 3, 4, 2},
+    {CXZ, KXZ, CYZ, KYZ, CZZ, KZZ, 1, 1, 1, 4, 5, 3},
+    {CEZ, KEZ, -1, -1, CEX, KEX, -1, 0, 1, 5, 0, -1},
+    {CEY, KEY, CEX, KEX, -1, -1, 1, -1, 0, 6, 6, -1}};
 
 template <int TX, int TY, bool G> struct T3F {
   static constexpr int CX = TX + 2, CY = TY + 2, NC = CX * CY;
   static constexpr int KX = TX + 1, KY = TY + 1, NK = KX * KY;
   static constexpr int NI = TX * TY, NQX = KX * TY, NQY = TX * KY;
-  static constexpr int NT = (NC + 31) / 32 * 32;
+  static constexpr int W = 32, NKW = (NK + W - 1) / W * W;  // whole warps of corners
+  static constexpr int NT = 2 * NKW;                        // two threads a corner
+  static constexpr int T0 = NT - (NC + W - 1) / W * W;      // the first of the cells' threads
+  static_assert(NI % W == 0 && T0 >= NI && NT >= 2 * NI && NKW >= NQX && NKW >= NQY, "");
   static constexpr int NR = NRET + (G ? 4 : 0);
   static constexpr size_t smem_bytes =
-      sizeof(double) * (2 * (size_t)NCF * NC + (size_t)NKF * NK + NQX + NQY + (size_t)NR * NI +
-                        32 + (G ? 2 * 4 * (size_t)NC + 4 * (size_t)NK : 0));
+      sizeof(double) * (2 * (size_t)NCF * NC + (size_t)NKF * NK + NQX + NQY +
+                        (size_t)(NR + 4) * NI + 34 + (G ? 2 * 4 * (size_t)NC + 4 * (size_t)NK : 0));
 };
+
+// x with its sign flipped where s < 0 (on its upper word: the negation of a double is
+// an FP64 instruction)
+__device__ __forceinline__ double signed_by(double x, int s) {
+  return __hiloint2double(__double2hiint(x) ^ (s & (int)0x80000000), __double2loint(x));
+}
+
+// The predictor of four variables of one corner with FP64 sums, where an integer sum cannot be formed
+// (isum::special): l and h the lower left cell of the corner's two planes, gl and gh
+// that of the gravity sources, ks the corner's slots.
+template <class T, bool G>
+__device__ __noinline__ void predict_fp64(const double *l, const double *h, const double *gl,
+                                          const double *gh, double *ks, int v0, double cxk,
+                                          double cyk, double czk, double dt) {
+  auto sum = [&](const double *p) { return (p[0] + p[1]) + (p[T::CX] + p[T::CX + 1]); };
+  auto dx = [&](const double *p) { return (p[1] - p[0]) + (p[T::CX + 1] - p[T::CX]); };
+  auto dy = [&](const double *p) { return (p[T::CX] - p[0]) + (p[T::CX + 1] - p[1]); };
+#pragma unroll 1
+  for (int v = v0; v < v0 + 4; v++) {
+    const VarFields q = kVar[v];
+    const size_t x = (size_t)q.fx * T::NC, y = (size_t)q.fy * T::NC, z = (size_t)q.fz * T::NC;
+    const size_t o = (size_t)v * T::NC;
+    double r = sum(l + o) + sum(h + o);
+    if (q.fx >= 0) r = fma(signed_by(cxk, q.sx), dx(l + x) + dx(h + x), r);
+    if (q.fy >= 0) r = fma(signed_by(cyk, q.sy), dy(l + y) + dy(h + y), r);
+    if (q.fz >= 0) r = fma(signed_by(czk, q.sz), sum(h + z) - sum(l + z), r);
+    if constexpr (G) {
+      if (q.g >= 0) {
+        const size_t s = (size_t)q.g * T::NC;
+        r = fma(dt, sum(gl + s) + sum(gh + s), r);
+      }
+    }
+    ks[(size_t)v * T::NK] = r;
+  }
+}
+
+// isum::diff_planes and face_planes of one variable in FP64, with the weights
+// themselves: o = tx, ty, tz, gx, gy, pu of the full step.
+template <class T>
+__device__ __noinline__ void cell_fp64(VarFields q, const double *s0, const double *s1,
+                                       const double *kk, double gxl, double gyl, double pl,
+                                       double w, double ux0, double ux1, double uy0, double uy1,
+                                       double uz0, double uz1, double *o) {
+  o[0] = o[1] = o[3] = o[4] = 0.0;
+  o[5] = w;
+  if (q.fx >= 0) {
+    const double *k = kk + (size_t)q.kx * T::NK, *f = s0 + (size_t)q.fx * T::NC;
+    o[3] = 2.0 * (uy0 * (k[1] - k[0]) + uy1 * (k[T::KX + 1] - k[T::KX]));
+    o[0] = 2.0 * (uz0 * gxl + uz1 * o[3]) + 16.0 * (f[1] - f[-1]);
+  }
+  if (q.fy >= 0) {
+    const double *k = kk + (size_t)q.ky * T::NK, *f = s0 + (size_t)q.fy * T::NC;
+    o[4] = 2.0 * (ux0 * (k[T::KX] - k[0]) + ux1 * (k[T::KX + 1] - k[1]));
+    o[1] = 2.0 * (uz0 * gyl + uz1 * o[4]) + 16.0 * (f[T::CX] - f[-T::CX]);
+  }
+  if (q.fz >= 0) {
+    const double *k = kk + (size_t)q.kz * T::NK;
+    const double *f0 = s0 + (size_t)q.fz * T::NC, *f1 = s1 + (size_t)q.fz * T::NC;
+    const double s = 4.0 * (uy0 * (ux0 * k[0] + ux1 * k[1]) +
+                            uy1 * (ux0 * k[T::KX] + ux1 * k[T::KX + 1]));
+    const double p = s + 16.0 * (f0[0] + f1[0]);
+    o[5] = (q.sz < 0 ? -p : p) + w;
+  }
+  o[2] = o[5] - pl;
+}
 
 }  // namespace
 
-template <int TX, int TY, bool G, bool R, int MINB>
-__global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, MINB)
+template <int TX, int TY, bool G, bool R, int MINB, bool U>
+__global__ void __launch_bounds__(T3F<TX, TY, G>::NT, MINB)
     k_mlw3d_fast(const double *__restrict__ A, double *__restrict__ B, int ix, int jx, int kx,
                  Axis ax, Axis ay, Axis az, Phys ph, double dt_arg, Ctl *__restrict__ ctl,
                  Box3 box, int kchunk, const double *__restrict__ grav,
@@ -92,8 +176,10 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, MINB)
   double *sqx = sk + (size_t)NKF * T::NK;             // q / dxm of plane k
   double *sqy = sqx + T::NQX;
   double *sret = sqy + T::NQY;                        // [NR][NI]
-  double *sred = sret + (size_t)T::NR * T::NI;
-  double *sgc = sred + 32;                            // G: [2][4][NC]
+  double *sun = sret + (size_t)T::NR * T::NI;         // [4][NI]: new values 4 .. 7
+  double *sred = sun + 4 * (size_t)T::NI;
+  double *szc = sred + 32;                            // of plane k: viscosity, flux factor
+  double *sgc = szc + 2;                              // G: [2][4][NC]
   double *sgk = sgc + 2 * 4 * (size_t)T::NC;          // G: [4][NK]
 
   if (ctl != nullptr) {
@@ -108,27 +194,35 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, MINB)
   const int kb = 1 + blockIdx.z * kchunk, ke = min(kx - 2, kb + kchunk - 1);
   if (kb > ke) return;
 
-  // the thread's cell of the halo tile
-  const int hx = tid % T::CX, hy = tid / T::CX;
+  // the thread's cell of the halo tile; ghost cells keep their input values (mlw_m.f
+  // updates only 2..n-1) and are copied by the block of their nearest interior cell
+  const int ct = tid - T::T0, hx = ct % T::CX, hy = ct / T::CX;
   const int gi = i0 - 1 + hx, gj = j0 - 1 + hy;
-  const bool cell = tid < T::NC, in_arr = cell && gi < ix && gj < jx;
-  // its corner, and the corner's predictor coefficients 8 dt / (4 dxm)
-  const int cx = tid % T::KX, cy = tid / T::KX;
-  const bool corner = tid < T::NK;
+  const bool cell = ct >= 0 && ct < T::NC, in_arr = cell && gi < ix && gj < jx;
+  const int ci = min(max(gi, 1), ix - 2), cj = min(max(gj, 1), jx - 2);
+  const bool owned = in_arr && ci >= i0 && ci < i0 + TX && cj >= j0 && cj < j0 + TY;
+  const bool xy_ghost = owned && (gi != ci || gj != cj);
+  // its corner (two threads a corner, four variables each), and the corner's
+  // predictor coefficients -8 dt / (4 dxm)
+  const int kt = tid % T::NKW, kv0 = tid < T::NKW ? 0 : 4;
+  const int cx = kt % T::KX, cy = kt / T::KX;
+  const bool corner = kt < T::NK;
   const bool cor_in = corner && i0 - 1 + cx <= ix - 2 && j0 - 1 + cy <= jx - 2;
   const int p00 = cx + cy * T::CX;
-  const double cxk = cor_in ? 2.0 * dt * ax.dim[i0 - 1 + cx] : 0.0;
-  const double cyk = cor_in ? 2.0 * dt * ay.dim[j0 - 1 + cy] : 0.0;
-  // its interior cell
-  const int lx = tid % TX + 1, ly = tid / TX + 1;
+  const double cxk = cor_in ? -2.0 * dt * ax.dim[i0 - 1 + cx] : 0.0;
+  const double cyk = cor_in ? -2.0 * dt * ay.dim[j0 - 1 + cy] : 0.0;
+  // its interior cell (two threads a cell, four variables each)
+  const int it = tid % T::NI, iv0 = tid < T::NI ? 0 : 4;
+  const int lx = it % TX + 1, ly = it / TX + 1;
   const int ii = i0 - 1 + lx, jj = j0 - 1 + ly;
-  const bool interior = tid < T::NI && ii <= ix - 2 && jj <= jx - 2;
+  const bool interior = tid < 2 * T::NI && ii <= ix - 2 && jj <= jx - 2;
   const int c0 = lx + ly * T::CX;
   const int kSW = (lx - 1) + (ly - 1) * T::KX;
-  // its viscosity faces: qav dm dim of an x and a y face
-  const int fxx = tid % T::KX, fxr = tid / T::KX, fyx = tid % TX, fyr = tid / TX;
-  const bool facex = tid < T::NQX && i0 + fxx < ix && j0 + fxr < jx;
-  const bool facey = tid < T::NQY && i0 + fyx < ix && j0 + fyr < jx;
+  // the viscosity faces (qav dm dim of an x and a y face) of the upper threads
+  const int ft = tid - T::NKW;
+  const int fxx = ft % T::KX, fxr = ft / T::KX, fyx = ft % TX, fyr = ft / TX;
+  const bool facex = ft >= 0 && ft < T::NQX && i0 + fxx < ix && j0 + fxr < jx;
+  const bool facey = ft >= 0 && ft < T::NQY && i0 + fyx < ix && j0 + fyr < jx;
   const double qxc = facex ? ph.qav * ax.dm[i0 - 1 + fxx] * ax.dim[i0 - 1 + fxx] : 0.0;
   const double qyc = facey ? ph.qav * ay.dm[j0 - 1 + fyr] * ay.dim[j0 - 1 + fyr] : 0.0;
 
@@ -138,19 +232,30 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, MINB)
   // ---- cells of plane k (mlw_m.f:74-202) -----------------------------------
   auto load_plane = [&](int k) {
     if (!cell) return;
-    double *sl = cslot(k) + tid;
+    double *sl = cslot(k) + ct;
 #define S(f) sl[(size_t)(f) * T::NC]
     if (!in_arr) {
 #pragma unroll 1
       for (int f = 0; f < NCF; f++) S(f) = 0.0;
       if constexpr (G)
-        for (int f = 0; f < 4; f++) gslot(k)[f * T::NC + tid] = 0.0;
+        for (int f = 0; f < 4; f++) gslot(k)[f * T::NC + ct] = 0.0;
       return;
     }
     const size_t g = (size_t)gi + (size_t)gj * ix + (size_t)k * plane;
     const double ro = A[P3::RO * n + g], pr = A[P3::PR * n + g];
     const double vx = A[P3::VX * n + g], vy = A[P3::VY * n + g], vz = A[P3::VZ * n + g];
     const double bx = A[P3::BX * n + g], by = A[P3::BY * n + g], bz = A[P3::BZ * n + g];
+    if (xy_ghost ? k == 0 || k >= kb && k <= ke || k == kx - 1
+                 : owned && (k == 0 || k == kx - 1)) {
+      B[P3::RO * n + g] = ro;
+      B[P3::PR * n + g] = pr;
+      B[P3::VX * n + g] = vx;
+      B[P3::VY * n + g] = vy;
+      B[P3::VZ * n + g] = vz;
+      B[P3::BX * n + g] = bx;
+      B[P3::BY * n + g] = by;
+      B[P3::BZ * n + g] = bz;
+    }
     const double rx = ro * vx, ry = ro * vy, rz = ro * vz;
     const double ek = 0.5 * fma(rx, vx, fma(ry, vy, rz * vz));
     const double bb = fma(bx, bx, fma(by, by, bz * bz));
@@ -179,7 +284,7 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, MINB)
     S(CYZ) = fma(ry, vz, -pby * bz);
     if constexpr (G) {  // mlw_m_g.f:135-136, 154, 172, 190
       const double gx = grav[g], gy = grav[2 * n + g], gz = grav[4 * n + g];
-      double *gs = gslot(k) + tid;
+      double *gs = gslot(k) + ct;
       gs[0] = fma(rx, gx, fma(ry, gy, rz * gz));
       gs[T::NC] = ro * gx;
       gs[2 * T::NC] = ro * gy;
@@ -188,74 +293,46 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, MINB)
 #undef S
   };
 
-  // ---- the plane sums of a corner ------------------------------------------
-  double P[NPS] = {}, PG[G ? 4 : 1] = {};
-  // q(s, x): the new value of sum s; the caller combines it with P[s] and stores
-  auto plane_sums = [&](int k, auto &&put) {
-    const double *sl = cslot(k) + p00;
-#define F4(f) \
-  const double *q = sl + (size_t)(f) * T::NC; \
-  const double a = q[0], b = q[1], c = q[T::CX], d = q[T::CX + 1]
-    auto sum = [&](int f, int s) { F4(f); put(s, (a + b) + (c + d)); };
-    auto dx = [&](int f, int s) { F4(f); put(s, (b - a) + (d - c)); };
-    auto dy = [&](int f, int s) { F4(f); put(s, (c - a) + (d - b)); };
-    auto sum_dx = [&](int f, int s, int x) {
-      F4(f);
-      const double l = a + c, r = b + d;
-      put(s, l + r);
-      put(x, r - l);
-    };
-    auto sum_dy = [&](int f, int s, int y) {
-      F4(f);
-      const double l = a + b, r = c + d;
-      put(s, l + r);
-      put(y, r - l);
-    };
-    auto dx_dy = [&](int f, int x, int y) {
-      F4(f);
-      const double u = d - a, w = b - c;
-      put(x, u + w);
-      put(y, u - w);
-    };
-    sum(CRO, S_RO);
-    sum_dx(CRX, S_RX, X_RX);
-    sum_dy(CRY, S_RY, Y_RY);
-    sum(CRZ, S_RZ);
-    sum(CEE, S_EE);
-    dx(CFX, X_FX);
-    dy(CFY, Y_FY);
-    sum(CFZ, S_FZ);
-    dx(CXX, X_XX);
-    dx_dy(CXY, X_XY, Y_XY);
-    sum_dx(CXZ, S_XZ, X_XZ);
-    dy(CYY, Y_YY);
-    sum_dy(CYZ, S_YZ, Y_YZ);
-    sum(CZZ, S_ZZ);
-    sum(CBX, S_BX);
-    sum(CBY, S_BY);
-    sum(CBZ, S_BZ);
-    sum_dy(CEX, S_EX, Y_EX);
-    sum_dx(CEY, S_EY, X_EY);
-    dx_dy(CEZ, X_EZ, Y_EZ);
-#undef F4
-  };
-  auto grav_sum = [&](int k, int f) {
-    const double *q = gslot(k) + f * T::NC + p00;
-    return (q[0] + q[1]) + (q[T::CX] + q[T::CX + 1]);
+  // ---- eight times the state predicted at the corners of plane k + 1/2
+  // (mlwhalf.f:49-65), into the corner's own slots 0 .. 7; 0 outside the array
+  auto corner_sums = [&](int k) {
+    if (!cor_in) return;
+    double *ks = sk + kt;
+    const double czk = -2.0 * dt * az.dim[k];
+    const double *L = cslot(k) + p00, *H = cslot(k + 1) + p00;
+    bool sp = false;
+#pragma unroll 1
+    for (int v = kv0; v < kv0 + 4; v++) {
+      const VarFields q = kVar[v];
+      auto at = [&](const double *p, int f) { return p + (size_t)f * T::NC; };
+      double r = isum::eight<T::CX, isum::kSum>(at(L, v), at(H, v), sp);
+      if (q.fx >= 0)
+        r = fma(signed_by(cxk, q.sx), isum::eight<T::CX, isum::kDx>(at(L, q.fx), at(H, q.fx), sp),
+                r);
+      if (q.fy >= 0)
+        r = fma(signed_by(cyk, q.sy), isum::eight<T::CX, isum::kDy>(at(L, q.fy), at(H, q.fy), sp),
+                r);
+      if (q.fz >= 0)
+        r = fma(signed_by(czk, q.sz), isum::eight<T::CX, isum::kDz>(at(L, q.fz), at(H, q.fz), sp),
+                r);
+      if constexpr (G) {  // mlwsrch part 2: dt times the mean of the eight sources
+        if (q.g >= 0) {
+          const size_t o = (size_t)q.g * T::NC + p00;
+          r = fma(dt, isum::eight<T::CX, isum::kSum>(gslot(k) + o, gslot(k + 1) + o, sp), r);
+        }
+      }
+      ks[(size_t)v * T::NK] = r;
+    }
+    if (sp)  // a call, so that the FP64 sums are not predicated in
+      predict_fp64<T, G>(L, H, G ? gslot(k) + p00 : nullptr, G ? gslot(k + 1) + p00 : nullptr, ks,
+                         kv0, cxk, cyk, czk, dt);
   };
 
-  // ---- corners of plane k + 1/2 (mlwhalf.f:49-65, mlw_m.f:205-334) -----------
-  auto corner_plane = [&](int k) {
-    if (!corner) return;
-    double *ks = sk + tid;
+  // ---- fluxes of the corners of plane k + 1/2 (mlw_m.f:205-334) --------------
+  auto corner_fluxes = [&](int k) {
+    double *ks = sk + kt;
 #define KS(f) ks[(size_t)(f) * T::NK]
-    if (!cor_in) {
-#pragma unroll 1
-      for (int f = 0; f < NKF; f++) KS(f) = 0.0;
-      if constexpr (G)
-        for (int f = 0; f < 4; f++) sgk[f * T::NK + tid] = 0.0;
-      return;
-    }
+    if (!cor_in) return;
     const size_t gc = (size_t)(i0 - 1 + cx) + (size_t)(j0 - 1 + cy) * ix + (size_t)k * plane;
     double rq[3] = {0.0, 0.0, 0.0}, gq[3] = {0.0, 0.0, 0.0};
     if constexpr (R) {
@@ -268,41 +345,8 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, MINB)
       gq[1] = grav[3 * n + gc];
       gq[2] = grav[5 * n + gc];
     }
-    const double czk = 2.0 * dt * az.dim[k];
-    // D[s]: sums and x, y differences over both planes, z differences (upper
-    // less lower) of the sums that are z fluxes; S_RZ, S_XZ, ... serve both
-    double D[NPS], Zrz, Zxz, Zyz;
-    plane_sums(k + 1, [&](int s, double x) {
-      const bool z = s == S_FZ || s == S_ZZ || s == S_EX || s == S_EY;
-      if (s == S_RZ) Zrz = x - P[s];
-      if (s == S_XZ) Zxz = x - P[s];
-      if (s == S_YZ) Zyz = x - P[s];
-      D[s] = z ? x - P[s] : x + P[s];
-      P[s] = x;
-    });
-    const double ro = fma(-czk, Zrz, fma(-cyk, D[Y_RY], fma(-cxk, D[X_RX], D[S_RO])));
-    double ee = fma(-czk, D[S_FZ], fma(-cyk, D[Y_FY], fma(-cxk, D[X_FX], D[S_EE])));
-    double rx = fma(-czk, Zxz, fma(-cyk, D[Y_XY], fma(-cxk, D[X_XX], D[S_RX])));
-    double ry = fma(-czk, Zyz, fma(-cyk, D[Y_YY], fma(-cxk, D[X_XY], D[S_RY])));
-    double rz = fma(-czk, D[S_ZZ], fma(-cyk, D[Y_YZ], fma(-cxk, D[X_XZ], D[S_RZ])));
-    // B: d(bx) = -(dy Ez - dz Ey), d(by) = -(dz Ex - dx Ez), d(bz) = -(dx Ey - dy Ex)
-    const double bx = fma(czk, D[S_EY], fma(-cyk, D[Y_EZ], D[S_BX]));
-    const double by = fma(-czk, D[S_EX], fma(cxk, D[X_EZ], D[S_BY]));
-    const double bz = fma(cyk, D[Y_EX], fma(-cxk, D[X_EY], D[S_BZ]));
-    if constexpr (G) {  // mlwsrch part 2: dt times the mean of the eight sources
-      double x[4];
-#pragma unroll
-      for (int f = 0; f < 4; f++) {
-        x[f] = grav_sum(k + 1, f);
-        PG[f] += x[f];
-      }
-      ee = fma(dt, PG[0], ee);
-      rx = fma(dt, PG[1], rx);
-      ry = fma(dt, PG[2], ry);
-      rz = fma(dt, PG[3], rz);
-#pragma unroll
-      for (int f = 0; f < 4; f++) PG[f] = x[f];
-    }
+    const double ro = KS(CRO), ee = KS(CEE), rx = KS(CRX), ry = KS(CRY), rz = KS(CRZ);
+    const double bx = KS(CBX), by = KS(CBY), bz = KS(CBZ);
     // primitives and fluxes of the eightfold state: B B terms carry 64
     const double k4 = 0.125 * ph.pi4i, k8 = 0.125 * ph.pi8i;
     const double ri = fd::rcp(ro);
@@ -331,231 +375,198 @@ __global__ void __launch_bounds__(((TX + 2) * (TY + 2) + 31) / 32 * 32, MINB)
     KS(KXZ) = fma(rx, vz, -pbx * bz);
     KS(KYZ) = fma(ry, vz, -pby * bz);
     if constexpr (G) {  // mlw_m_g.f:289-290, 308, 326, 344
-      sgk[tid] = fma(rx, gq[0], fma(ry, gq[1], rz * gq[2]));
-      sgk[T::NK + tid] = ro * gq[0];
-      sgk[2 * T::NK + tid] = ro * gq[1];
-      sgk[3 * T::NK + tid] = ro * gq[2];
+      sgk[kt] = fma(rx, gq[0], fma(ry, gq[1], rz * gq[2]));
+      sgk[T::NK + kt] = ro * gq[0];
+      sgk[2 * T::NK + kt] = ro * gq[1];
+      sgk[3 * T::NK + kt] = ro * gq[2];
     }
 #undef KS
   };
 
   // ---- per-column constants of the full step --------------------------------
-  double uy0 = 0, uy1 = 0, ux0 = 0, ux1 = 0, dtx = 0, dty = 0, w00 = 0, w10 = 0, w01 = 0,
-         w11 = 0, mxy = 0;
+  double uy0 = 0, uy1 = 0, ux0 = 0, ux1 = 0, dtx = 0, dty = 0, cx_ = 0, cy_ = 0, mxy = 0;
+  float ex0 = 0, ex1 = 0, ey0 = 0, ey1 = 0;
   if (interior) {
     ux0 = ax.u0[ii];
     ux1 = ax.u1[ii];
     uy0 = ay.u0[jj];
     uy1 = ay.u1[jj];
+    ex0 = ax.e0[ii];
+    ex1 = ax.e1[ii];
+    ey0 = ay.e0[jj];
+    ey1 = ay.e1[jj];
     dtx = dt * ax.di[ii];
     dty = dt * ay.di[jj];
-    // corner weights of a z face over 4: twice the mean of eightfold values
-    w00 = 0.25 * (ux0 * uy0);
-    w10 = 0.25 * (ux1 * uy0);
-    w01 = 0.25 * (ux0 * uy1);
-    w11 = 0.25 * (ux1 * uy1);
+    cx_ = -0.015625 * dtx;
+    cy_ = -0.015625 * dty;
     mxy = fd::maxp(ax.di[ii] * ax.di[ii], ay.di[jj] * ay.di[jj]);
   }
-  auto ret = [&](int r) -> double & { return sret[(size_t)r * T::NI + tid]; };
-  // corner differences along x (uy0 (SE - SW) + uy1 (NE - NW)) and y, and the
-  // corner average of the z face
-  auto kdx = [&](int f) {
-    const double *q = sk + (size_t)f * T::NK + kSW;
-    return fma(uy1, q[T::KX + 1] - q[T::KX], uy0 * (q[1] - q[0]));
-  };
-  auto kdy = [&](int f) {
-    const double *q = sk + (size_t)f * T::NK + kSW;
-    return fma(ux1, q[T::KX + 1] - q[1], ux0 * (q[T::KX] - q[0]));
-  };
-  auto kz = [&](int f, double s) {  // s + the average
-    const double *q = sk + (size_t)f * T::NK + kSW;
-    return fma(w11, q[T::KX + 1], fma(w01, q[T::KX], fma(w10, q[1], fma(w00, q[0], s))));
-  };
-  auto gkz = [&](int f) {
-    const double *q = sgk + (size_t)f * T::NK + kSW;
-    return fma(w11, q[T::KX + 1], fma(w01, q[T::KX], fma(w10, q[1], w00 * q[0])));
-  };
-  // twice the z flux of variable v through the face between planes k and k+1:
-  // F_k + F_k+1 + 2 (corner average) - 4 qz (u_k+1 - u_k)
-  auto z_face = [&](const double *s0, const double *s1, int v, int sf, int kf, bool neg,
-                    double qz4) {
-    const size_t o = (size_t)v * T::NC + c0;
-    const double du = s1[o] - s0[o];
-    if (sf < 0) return -qz4 * du;
-    const size_t of = (size_t)sf * T::NC + c0;
-    const double s = kz(kf, s0[of] + s1[of]);
-    return fma(-qz4, du, neg ? -s : s);
-  };
-  auto z_visc = [&](const double *s0, const double *s1, int k) {
-    const double q =
-        fd::abs_(s1[(size_t)CVZ * T::NC + c0] - s0[(size_t)CVZ * T::NC + c0]) - CANS_AV_EPS;
-    return 4.0 * (ph.qav * az.dm[k] * az.dim[k]) * fd::pos_part(q);
-  };
+  auto ret = [&](int r) -> double & { return sret[(size_t)r * T::NI + it]; };
 
-  // ---- prologue: the sums of plane kb-1, corners kb-1/2, what they leave ----
-  load_plane(kb - 1);
-  load_plane(kb);
-  __syncthreads();
-  if (cor_in) {
-    plane_sums(kb - 1, [&](int s, double x) { P[s] = x; });
-    if constexpr (G) {
-#pragma unroll
-      for (int f = 0; f < 4; f++) PG[f] = grav_sum(kb - 1, f);
-    }
-  }
-  corner_plane(kb - 1);
-  __syncthreads();
-  // fields of the seven x differences, y differences and the z faces, in the
-  // order of ret()
-  auto each_x = [&](auto &&f) {
-    f(0, CRO, CRX, KRX, false); f(1, CEE, CFX, KFX, false); f(2, CRX, CXX, KXX, false);
-    f(3, CRY, CXY, KXY, false); f(4, CRZ, CXZ, KXZ, false); f(5, CBY, CEZ, KEZ, true);
-    f(6, CBZ, CEY, KEY, false);
-  };
-  if (interior) {
-    const double *s0 = cslot(kb - 1), *s1 = cslot(kb);
-    const double qz4 = z_visc(s0, s1, kb - 1);
-    each_x([&](int r, int, int, int kf, bool) { ret(r) = kdx(kf); });
-    ret(7) = kdy(KRY); ret(8) = kdy(KFY); ret(9) = kdy(KXY); ret(10) = kdy(KYY);
-    ret(11) = kdy(KYZ); ret(12) = kdy(KEZ); ret(13) = kdy(KEX);
-    ret(14) = z_face(s0, s1, CRO, CRZ, KRZ, false, qz4);
-    ret(15) = z_face(s0, s1, CEE, CFZ, KFZ, false, qz4);
-    ret(16) = z_face(s0, s1, CRX, CXZ, KXZ, false, qz4);
-    ret(17) = z_face(s0, s1, CRY, CYZ, KYZ, false, qz4);
-    ret(18) = z_face(s0, s1, CRZ, CZZ, KZZ, false, qz4);
-    ret(19) = z_face(s0, s1, CBX, CEY, KEY, true, qz4);
-    ret(20) = z_face(s0, s1, CBY, CEX, KEX, false, qz4);
-    ret(21) = z_face(s0, s1, CBZ, -1, 0, false, qz4);
-    if constexpr (G) {
-#pragma unroll
-      for (int f = 0; f < 4; f++) ret(NRET + f) = gkz(f);
-    }
-  }
-  __syncthreads();
-
-  double kmax = 0.0;  // largest CFL key of the thread's cells
+  double un[4] = {0.0, 0.0, 0.0, 0.0};  // the new values of the thread's variables
+  double kmax = 0.0;                    // largest CFL key of the thread's cells
   bool bad = false;
 
-  for (int k = kb; k <= ke; k++) {
-    // (a) cell plane k+1 over plane k-1
-    load_plane(k + 1);
+  // ---- the new primitives of plane k and their CFL key -----------------------
+  auto finish = [&](int k) {
+    if (tid >= T::NI || !interior) return;
+    const double ro = un[CRO], ee = un[CEE], rx = un[CRX], bx = un[CBX];
+    const double ry = sun[tid], rz = sun[T::NI + tid], by = sun[2 * T::NI + tid];
+    const double bz = sun[3 * T::NI + tid];
+    const double ri = fd::rcp(ro);
+    const double vx = rx * ri, vy = ry * ri, vz = rz * ri;
+    const double ek = fma(rx, vx, fma(ry, vy, rz * vz));
+    const double bb = fma(bx, bx, fma(by, by, bz * bz));
+    const double pr = ph.gm1 * fma(-ph.pi8i, bb, fma(-0.5, ek, ee));
+    const size_t g = (size_t)ii + (size_t)jj * ix + (size_t)k * plane;
+    B[P3::RO * n + g] = ro;
+    B[P3::PR * n + g] = pr;
+    B[P3::VX * n + g] = vx;
+    B[P3::VY * n + g] = vy;
+    B[P3::VZ * n + g] = vz;
+    B[P3::BX * n + g] = bx;
+    B[P3::BY * n + g] = by;
+    B[P3::BZ * n + g] = bz;
+    if (ctl != nullptr && ii >= box.lo[0] && ii <= box.hi[0] && jj >= box.lo[1] &&
+        jj <= box.hi[1] && k >= box.lo[2] && k <= box.hi[2]) {
+      // the largest (v^2 + cs^2 + ca^2) max(1/dx^2, 1/dy^2, 1/dz^2) gives the
+      // smallest time step (cfl_m.f:52-59, pi in single precision)
+      const double s = fma(ph.pi4i_cfl, bb, fma(ph.gm, pr, ek)) * ri;
+      const double key = s * fd::maxp(mxy, az.di[k] * az.di[k]);
+      if (!fd::is_nan(key)) kmax = fd::max_(key, kmax);
+      bad |= bad_cell(ro, pr, key);
+    }
+  };
+
+  // outside the array the corners are never formed
+  for (int q = tid; q < NKF * T::NK; q += T::NT) sk[q] = 0.0;
+  if constexpr (G)
+    for (int q = tid; q < 4 * T::NK; q += T::NT) sgk[q] = 0.0;
+  for (int q = tid; q < T::NR * T::NI; q += T::NT) sret[q] = 0.0;
+  load_plane(kb - 1);
+  load_plane(kb);
+  // k = kb - 1 only leaves what the columns keep of the corners kb - 1/2
+  for (int k = kb - 1;; k++) {
+    // (a) the primitives of plane k-1 (the first warps); cell plane k+1 over plane
+    // k-1 (the others)
+    if (k > kb) finish(k - 1);
+    if (k > ke) break;
+    if (k >= kb) load_plane(k + 1);
     __syncthreads();
-    // (b) corner plane k+1/2, viscosity faces of plane k
-    corner_plane(k);
-    {
+    // (b) the sums of corner plane k+1/2
+    corner_sums(k);
+    __syncthreads();
+    // (c) their fluxes (the lower half), viscosity faces of plane k (the upper)
+    if (tid < T::NKW) {
+      corner_fluxes(k);
+    } else {
       const double *sl = cslot(k);
-      if (tid < T::NQX) {
-        const double *v = sl + (size_t)CVX * T::NC + fxx + (fxr + 1) * T::CX;
-        sqx[tid] = qxc * fd::pos_part(fd::abs_(v[1] - v[0]) - CANS_AV_EPS);
+      if (ft == 0) {
+        szc[0] = -64.0 * ph.qav * az.dm[k] * az.dim[k];
+        szc[1] = -0.015625 * dt * az.di[k];
       }
-      if (tid < T::NQY) {
+      if (ft < T::NQX) {
+        const double *v = sl + (size_t)CVX * T::NC + fxx + (fxr + 1) * T::CX;
+        sqx[ft] = qxc * fd::pos_part(fd::abs_(v[1] - v[0]) - CANS_AV_EPS);
+      }
+      if (ft < T::NQY) {
         const double *v = sl + (size_t)CVY * T::NC + fyx + 1 + fyr * T::CX;
-        sqy[tid] = qyc * fd::pos_part(fd::abs_(v[T::CX] - v[0]) - CANS_AV_EPS);
+        sqy[ft] = qyc * fd::pos_part(fd::abs_(v[T::CX] - v[0]) - CANS_AV_EPS);
       }
     }
     __syncthreads();
-    // (c) full step of plane k
+    // (d) full step of plane k
     if (interior) {
-      const double *s0 = cslot(k), *s1 = cslot(k + 1);
+      const double *s0 = cslot(k) + c0, *s1 = cslot(k + 1) + c0, *kk = sk + kSW;
       const double ae = dtx * sqx[lx + (ly - 1) * T::KX], aw = dtx * sqx[lx - 1 + (ly - 1) * T::KX];
       const double an = dty * sqy[lx - 1 + ly * TX], as = dty * sqy[lx - 1 + (ly - 1) * TX];
       const double aa = (ae + aw) + (an + as);
-      const double fcx = 0.25 * dtx, fcy = 0.25 * dty;
-      const double uz0 = az.u0[k], uz1 = az.u1[k], dtz = dt * az.di[k];
-      // the corner differences carry 8: hdt / 8 = dt / 16
-      const double hx0 = 0.0625 * dtx * uz0, hx1 = 0.0625 * dtx * uz1;
-      const double hy0 = 0.0625 * dty * uz0, hy1 = 0.0625 * dty * uz1;
-      const double hz = 0.25 * dtz;
-      const double qz4 = z_visc(s0, s1, k);
-      auto visc = [&](int v) {
-        const double *q = s0 + (size_t)v * T::NC + c0;
-        return fma(ae, q[1], fma(aw, q[-1], fma(an, q[T::CX], fma(as, q[-T::CX], -aa * q[0]))));
-      };
-      auto add_x = [&](double du, int r, int sf, int kf, bool neg) {
-        const double *q = s0 + (size_t)sf * T::NC + c0;
-        const double g1 = kdx(kf), g0 = ret(r);
-        ret(r) = g1;
-        const double s = neg ? 1.0 : -1.0;
-        return fma(s * hx1, g1, fma(s * hx0, g0, fma(s * fcx, q[1] - q[-1], du)));
-      };
-      auto add_y = [&](double du, int r, int sf, int kf, bool neg) {
-        const double *q = s0 + (size_t)sf * T::NC + c0;
-        const double g1 = kdy(kf), g0 = ret(r);
-        ret(r) = g1;
-        const double s = neg ? 1.0 : -1.0;
-        return fma(s * hy1, g1, fma(s * hy0, g0, fma(s * fcy, q[T::CX] - q[-T::CX], du)));
-      };
-      auto add_z = [&](double du, int r, int v, int sf, int kf, bool neg) {
-        const double f1 = z_face(s0, s1, v, sf, kf, neg, qz4), f0 = ret(r);
-        ret(r) = f1;
-        return fma(-hz, f1 - f0, du);
-      };
-      auto source = [&](double du, int f) {  // mlwsrch part 1 and mlwsrcf
-        if constexpr (G) {
-          const double g1 = gkz(f), g0 = ret(NRET + f);
-          ret(NRET + f) = g1;
-          du = fma(0.5 * dt, gslot(k)[(size_t)f * T::NC + c0], du);
-          du = fma(0.25 * dt * uz0, g0, du);
-          du = fma(0.25 * dt * uz1, g1, du);
+      // 64 times the z viscosity of the upper face, negative
+      const double qz = szc[0] * fd::pos_part(fd::abs_(s1[(size_t)CVZ * T::NC] -
+                                                       s0[(size_t)CVZ * T::NC]) - CANS_AV_EPS);
+      // the corner sums carry 8 and weights of 1/2 a plane and axis, the z flux 32
+      const double cz_ = szc[1];
+#pragma unroll 1
+      for (int j = 0; j < 4; j++) {
+        const int v = iv0 + j;
+        const VarFields q = kVar[v];
+        const double *u = s0 + (size_t)v * T::NC;
+        const double *fx = s0 + (size_t)q.fx * T::NC, *fy = s0 + (size_t)q.fy * T::NC;
+        const double *kx_ = kk + (size_t)q.kx * T::NK, *ky = kk + (size_t)q.ky * T::NK;
+        const double *kz = kk + (size_t)q.kz * T::NK;
+        const double *f0 = s0 + (size_t)q.fz * T::NC, *f1 = s1 + (size_t)q.fz * T::NC;
+        const double gxl = ret(8 + q.rx), gyl = ret(15 + q.ry), pl = ret(v);
+        const double w = qz * (s1[(size_t)v * T::NC] - u[0]);
+        double gx = 0.0, gy = 0.0, pu = w;           // what the next plane keeps
+        double tx = 0.0, ty = 0.0, tz;               // differences of the directions
+        double du = fma(ae, u[1], fma(aw, u[-1], fma(an, u[T::CX],
+                                                     fma(as, u[-T::CX], -aa * u[0]))));
+        if constexpr (U) {
+          bool sp = false;
+          const float ez0 = az.e0[k], ez1 = az.e1[k];
+          if (q.fx >= 0)
+            tx = isum::diff_planes(kx_[0], kx_[1], kx_[T::KX], kx_[T::KX + 1], gxl, fx[-1], fx[1],
+                                   ey0, ey1, ez0, ez1, gx, sp);
+          if (q.fy >= 0)
+            ty = isum::diff_planes(ky[0], ky[T::KX], ky[1], ky[T::KX + 1], gyl, fy[-T::CX],
+                                   fy[T::CX], ex0, ex1, ez0, ez1, gy, sp);
+          if (q.fz >= 0)
+            tz = isum::face_planes(kz[0], kz[1], kz[T::KX], kz[T::KX + 1], f0[0], f1[0], w, pl,
+                                   q.sz < 0, ex0, ex1, ey0, ey1, pu, sp);
+          else
+            tz = w - pl;
+          if (sp) {  // a call, as in corner_plane
+            double o[6];
+            cell_fp64<T>(q, s0, s1, kk, gxl, gyl, pl, w, ux0, ux1, uy0, uy1, az.u0[k], az.u1[k],
+                         o);
+            tx = o[0];
+            ty = o[1];
+            tz = o[2];
+            gx = o[3];
+            gy = o[4];
+            pu = o[5];
+          }
+        } else {
+          const double uz0 = 2.0 * az.u0[k], uz1 = 2.0 * az.u1[k];
+          if (q.fx >= 0) {
+            gx = fma(2.0 * uy1, kx_[T::KX + 1] - kx_[T::KX], 2.0 * uy0 * (kx_[1] - kx_[0]));
+            tx = fma(16.0, fx[1] - fx[-1], fma(uz1, gx, uz0 * gxl));
+          }
+          if (q.fy >= 0) {
+            gy = fma(2.0 * ux1, ky[T::KX + 1] - ky[1], 2.0 * ux0 * (ky[T::KX] - ky[0]));
+            ty = fma(16.0, fy[T::CX] - fy[-T::CX], fma(uz1, gy, uz0 * gyl));
+          }
+          if (q.fz >= 0) {
+            const double s = fma(2.0 * uy1, fma(2.0 * ux1, kz[T::KX + 1], 2.0 * ux0 * kz[T::KX]),
+                                 2.0 * uy0 * fma(2.0 * ux1, kz[1], 2.0 * ux0 * kz[0]));
+            pu = fma(q.sz < 0 ? -1.0 : 1.0, fma(16.0, f0[0] + f1[0], s), w);
+          }
+          tz = pu - pl;
         }
-        return du;
-      };
-      auto old = [&](int v) { return s0[(size_t)v * T::NC + c0]; };
-      const double ro = old(CRO) + add_z(add_y(add_x(visc(CRO), 0, CRX, KRX, false), 7, CRY, KRY,
-                                               false), 14, CRO, CRZ, KRZ, false);
-      const double rx = old(CRX) + source(add_z(add_y(add_x(visc(CRX), 2, CXX, KXX, false), 9, CXY,
-                                                      KXY, false), 16, CRX, CXZ, KXZ, false), 1);
-      const double ry = old(CRY) + source(add_z(add_y(add_x(visc(CRY), 3, CXY, KXY, false), 10, CYY,
-                                                      KYY, false), 17, CRY, CYZ, KYZ, false), 2);
-      const double rz = old(CRZ) + source(add_z(add_y(add_x(visc(CRZ), 4, CXZ, KXZ, false), 11, CYZ,
-                                                      KYZ, false), 18, CRZ, CZZ, KZZ, false), 3);
-      const double bx = old(CBX) + add_z(add_y(visc(CBX), 12, CEZ, KEZ, false), 19, CBX, CEY, KEY,
-                                         true);
-      const double by = old(CBY) + add_z(add_x(visc(CBY), 5, CEZ, KEZ, true), 20, CBY, CEX, KEX,
-                                         false);
-      const double bz = old(CBZ) + add_z(add_y(add_x(visc(CBZ), 6, CEY, KEY, false), 13, CEX, KEX,
-                                               true), 21, CBZ, -1, 0, false);
-      const double ee = old(CEE) + source(add_z(add_y(add_x(visc(CEE), 1, CFX, KFX, false), 8, CFY,
-                                                      KFY, false), 15, CEE, CFZ, KFZ, false), 0);
-      const double ri = fd::rcp(ro);
-      const double vx = rx * ri, vy = ry * ri, vz = rz * ri;
-      const double ek = fma(rx, vx, fma(ry, vy, rz * vz));
-      const double bb = fma(bx, bx, fma(by, by, bz * bz));
-      const double pr = ph.gm1 * fma(-ph.pi8i, bb, fma(-0.5, ek, ee));
-      const size_t g = (size_t)ii + (size_t)jj * ix + (size_t)k * plane;
-      B[P3::RO * n + g] = ro;
-      B[P3::PR * n + g] = pr;
-      B[P3::VX * n + g] = vx;
-      B[P3::VY * n + g] = vy;
-      B[P3::VZ * n + g] = vz;
-      B[P3::BX * n + g] = bx;
-      B[P3::BY * n + g] = by;
-      B[P3::BZ * n + g] = bz;
-      if (ctl != nullptr && ii >= box.lo[0] && ii <= box.hi[0] && jj >= box.lo[1] &&
-          jj <= box.hi[1] && k >= box.lo[2] && k <= box.hi[2]) {
-        // the largest (v^2 + cs^2 + ca^2) max(1/dx^2, 1/dy^2, 1/dz^2) gives the
-        // smallest time step (cfl_m.f:52-59, pi in single precision)
-        const double s = fma(ph.pi4i_cfl, bb, fma(ph.gm, pr, ek)) * ri;
-        const double key = s * fd::maxp(mxy, az.di[k] * az.di[k]);
-        if (!fd::is_nan(key)) kmax = fd::max_(key, kmax);
-        bad |= bad_cell(ro, pr, key);
-      }
-    }
-    // ghost cells keep their input values (mlw_m.f updates only 2..n-1); each
-    // is copied by the block owning its nearest interior cell, plane by plane,
-    // plus the z ghost planes at the chunk ends
-    if (in_arr) {
-      const int ci = min(max(gi, 1), ix - 2), cj = min(max(gj, 1), jx - 2);
-      if (ci >= i0 && ci < i0 + TX && cj >= j0 && cj < j0 + TY) {
-        const bool xy_ghost = (gi == 0 || gi == ix - 1 || gj == 0 || gj == jx - 1);
-        auto copy = [&](int kk) {
-          const size_t g = (size_t)gi + (size_t)gj * ix + (size_t)kk * plane;
+        if (q.fx >= 0) ret(8 + q.rx) = gx;
+        if (q.fy >= 0) ret(15 + q.ry) = gy;
+        ret(v) = pu;
+        du = fma(signed_by(cx_, q.sx), tx, du);
+        du = fma(signed_by(cy_, q.sy), ty, du);
+        du = fma(cz_, tz, du);
+        if constexpr (G) {  // mlwsrch part 1 and mlwsrcf
+          if (q.g >= 0) {
+            const double *p = sgk + (size_t)q.g * T::NK + kSW;
+            const double g1 = fma(uy1, fma(ux1, p[T::KX + 1], ux0 * p[T::KX]),
+                                  uy0 * fma(ux1, p[1], ux0 * p[0]));
+            const double g0 = ret(NRET + q.g);
+            ret(NRET + q.g) = g1;
+            du = fma(0.5 * dt, gslot(k)[(size_t)q.g * T::NC + c0], du);
+            du = fma(0.0625 * dt, fma(az.u0[k], g0, az.u1[k] * g1), du);
+          }
+        }
+        const double r = u[0] + du;
+        if (iv0) {
+          sun[(size_t)j * T::NI + it] = r;
+        } else {
 #pragma unroll
-          for (int v = 0; v < P3::N; v++) B[v * n + g] = A[v * n + g];
-        };
-        if (xy_ghost) copy(k);
-        if (k == 1) copy(0);
-        if (k == kx - 2) copy(kx - 1);
+          for (int m = 0; m < 4; m++) un[m] = m == j ? r : un[m];
+        }
       }
     }
     __syncthreads();
@@ -571,7 +582,7 @@ namespace {
 
 constexpr int kMaxDevices3F = 64;
 
-template <int TX, int TY, bool G, bool R, int MINB>
+template <int TX, int TY, bool G, bool R, int MINB, bool U>
 cudaError_t launch3f(const double *A, double *B, int ix, int jx, int kx, const Axis &ax,
                      const Axis &ay, const Axis &az, const Phys &ph, double dt, Ctl *ctl,
                      Box3 box, int kmax, cudaStream_t s, const double *grav,
@@ -584,7 +595,7 @@ cudaError_t launch3f(const double *A, double *B, int ix, int jx, int kx, const A
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= kMaxDevices3F) return cudaErrorInvalidDevice;
-  auto kern = k_mlw3d_fast<TX, TY, G, R, MINB>;
+  auto kern = k_mlw3d_fast<TX, TY, G, R, MINB, U>;
   {
     std::lock_guard<std::mutex> lk(mu);
     if (!slots_of[dev]) {
@@ -610,15 +621,15 @@ cudaError_t launch3f(const double *A, double *B, int ix, int jx, int kx, const A
   return cudaGetLastError();
 }
 
-template <bool G, bool R>
+template <bool G, bool R, bool U>
 cudaError_t pick3f(int tile, const double *A, double *B, int ix, int jx, int kx, const Axis &ax,
                    const Axis &ay, const Axis &az, const Phys &ph, double dt, Ctl *ctl, Box3 box,
                    cudaStream_t s, const double *grav, const double *res) {
   if (tile == 2)
-    return launch3f<16, 12, G, R, 1>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box, 64, s, grav,
-                                     res);
-  return launch3f<16, 8, G, R, G ? 1 : 2>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box,
-                                          tile == 1 ? 32 : 64, s, grav, res);
+    return launch3f<16, 12, G, R, 1, U>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box, 64, s, grav,
+                                        res);
+  return launch3f<16, 8, G, R, G ? 1 : 2, U>(A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box,
+                                             tile == 1 ? 32 : 64, s, grav, res);
 }
 }  // namespace
 
@@ -629,11 +640,11 @@ cudaError_t launch_mlw3d_fast(int tile, const double *A, double *B, int ix, int 
                               double dt, Ctl *ctl, Box3 box, cudaStream_t s, const double *grav,
                               const double *res) {
   if (ix < 3 || jx < 3 || kx < 3 || (grav && res)) return cudaErrorInvalidValue;
-  if (grav)
-    return pick3f<true, false>(tile, A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box, s, grav, res);
-  if (res)
-    return pick3f<false, true>(tile, A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box, s, grav, res);
-  return pick3f<false, false>(tile, A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box, s, grav, res);
+  const bool u = ax.uniform && ay.uniform && az.uniform;
+  auto f = grav ? (u ? pick3f<true, false, true> : pick3f<true, false, false>)
+           : res ? (u ? pick3f<false, true, true> : pick3f<false, true, false>)
+                 : (u ? pick3f<false, false, true> : pick3f<false, false, false>);
+  return f(tile, A, B, ix, jx, kx, ax, ay, az, ph, dt, ctl, box, s, grav, res);
 }
 
 }  // namespace cans
