@@ -10,12 +10,20 @@
 // per stage would be launch-bound, so the whole loop runs inside one launch of
 // a cluster of CS blocks.  Each block keeps its segment of the grid (plus one
 // halo cell per side) in shared memory for the whole run; after each step
-// neighbours exchange halo cells through distributed shared memory and the
-// CFL minimum is reduced across the cluster, so no host round trip happens
-// per step.  One cluster barrier per step (the CFL reduction, which also
-// publishes the new cells for the halo exchange) when the boundary program
-// reads only the cells of the blocks that run it; a second one before the
-// boundary fill when a rule is periodic.
+// each block writes its edge cells into its neighbours' halos and its CFL
+// minimum into every block through distributed shared memory, so no host round
+// trip happens per step.  One cluster barrier per step (it publishes both) when
+// the boundary program reads only the cells of the blocks that run it; a second
+// one before the boundary fill when a rule is periodic.
+//
+// What bounds a step is its chain: FP64 instructions of 64 clocks each on a
+// quarter of the SM that has one or two warps, and the latencies between them
+// (the cluster barrier, remote and L2 accesses).  So the profiles are read through
+// the read-only cache (a barrier does not empty it), the loop's constants are read
+// once, minima are integer minima, nothing is read from another block, and the
+// plain step's arithmetic takes the fewest FP64 instructions (f1 below): a step of
+// 1024 cells on 16 blocks 12.9 -> 7.4 us, 64 spicule runs 50 -> 47 us (those are
+// bound by the FP64 pipe: 512 cells a SM).
 //
 // The BG variant is mlw_m_bg (cans1d/hdmlw/mlw_m_bg.f:2-271): the same
 // two-stage step on the cross-section-weighted variables (ro, e, rx, ry r,
@@ -34,6 +42,7 @@
 #include "cans_common.cuh"
 #include "cans_internal.h"
 #include "df64.cuh"
+#include "fd64.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -173,6 +182,112 @@ __device__ __forceinline__ F<E> torque_add(const Run1D &p, F<E> vy, F<E> dt, lon
 //   XS[2][l] = the static x-momentum flux difference and source of the
 //            corner predictor (times dt);
 //   XS[3][l] = those of the cell update, cell and corner terms (times dt/2).
+// Unsigned keys in the order of the doubles, and the smallest key of a warp
+__device__ __forceinline__ unsigned long long min_key(double x) {
+  return (unsigned long long)fd::key(x) ^ 0x8000000000000000ull;
+}
+__device__ __forceinline__ double from_min_key(unsigned long long k) {
+  const long long b = (long long)(k ^ 0x8000000000000000ull);
+  return __longlong_as_double(b ^ (long long)((unsigned long long)(b >> 63) >> 1));
+}
+__device__ __forceinline__ unsigned long long warp_min_key(unsigned long long k) {
+  const unsigned hi = __reduce_min_sync(0xffffffffu, (unsigned)(k >> 32));
+  const unsigned lo =
+      __reduce_min_sync(0xffffffffu, (unsigned)(k >> 32) == hi ? (unsigned)k : 0xffffffffu);
+  return (unsigned long long)hi << 32 | lo;
+}
+
+// ---- the fast policy of the plain step (mlw_m) ------------------------------
+// A warp's FP64 instruction takes its quarter of the SM 64 clocks whatever its
+// lanes do, and a block of the cluster has two to four warps: the step is the sum
+// of its FP64 instructions.  So the corner state and fluxes are kept at twice
+// their value and the viscosity coefficient at four times (constants carry the
+// factors), every term of the update is summed before one product with dt/dx, and
+// reciprocals and roots are fd64.cuh's: 120 FP64 instructions a cell where one
+// operation of the reference after the other takes 270.
+namespace f1 {
+__device__ __forceinline__ void cell(const Run1D &p, const double *pc, int L, int l, int g,
+                                     double *U, double *FX) {
+  const double ro = pc[l], pr = pc[L + l], vx = pc[2 * L + l], vy = pc[3 * L + l],
+               by = pc[4 * L + l], bx = __ldg(p.bx + g);
+  const double rx = ro * vx, ry = ro * vy;
+  const double ek = 0.5 * fma(rx, vx, ry * vy), bb = by * by;
+  const double me = fma(vx, by, -(vy * bx)), pb = p.ph.pi4i * by;  // -ez
+  U[l] = ro;
+  // the field's energy last, as an exact product: update takes the same one away
+  U[L + l] = fma(p.ph.pi8i, bb, fma(pr, p.ph.gm1i, ek));
+  U[2 * L + l] = rx;
+  U[3 * L + l] = ry;
+  U[4 * L + l] = by;
+  FX[l] = rx;
+  FX[L + l] = fma(pb, me, fma(pr, p.ph.ggm1, ek) * vx);
+  FX[2 * L + l] = fma(rx, vx, fma(bb, p.ph.pi8i, pr));
+  FX[3 * L + l] = fma(rx, vy, -(pb * bx));
+  FX[4 * L + l] = me;
+}
+
+// the corner between local cells l and l+1: twice its fluxes, four times the
+// viscosity coefficient over dxm
+__device__ __forceinline__ void corner(const Run1D &p, const double *pc, int L, int l, int g,
+                                       const double *U, const double *FX, double *K, double *Q,
+                                       double m2dt) {
+  const double dxim = __ldg(p.ax.dim + g), c = m2dt * dxim;
+  double un[NV1];
+#pragma unroll
+  for (int v = 0; v < NV1; v++)
+    un[v] = fma(c, FX[v * L + l + 1] - FX[v * L + l], U[v * L + l + 1] + U[v * L + l]);
+  const double bxm2 = 2.0 * __ldg(p.bxm + g), k4 = 0.5 * p.ph.pi4i, k8 = 0.5 * p.ph.pi8i;
+  const double ri = fd::rcp(un[0]);
+  const double vx = un[2] * ri, vy = un[3] * ri, by = un[4];
+  const double ek = 0.5 * fma(un[2], vx, un[3] * vy), bb = by * by;
+  const double pr = p.ph.gm1 * fma(-k8, bb, un[1] - ek);
+  const double me = fma(vx, by, -(vy * bxm2)), pb = k4 * by;
+  K[l] = un[2];
+  K[L + l] = fma(pb, me, fma(pr, p.ph.ggm1, ek) * vx);
+  K[2 * L + l] = fma(un[2], vx, fma(bb, k8, pr));
+  K[3 * L + l] = fma(un[2], vy, -(pb * bxm2));
+  K[4 * L + l] = me;
+  const double a =
+      fd::pos_part(fd::abs_(pc[2 * L + l + 1] - pc[2 * L + l]) - CANS_AV_EPS);
+  Q[l] = 4.0 * p.ph.qav * __ldg(p.ax.dm + g) * a * dxim;
+}
+
+// the new primitives of own cell l
+__device__ __forceinline__ void update(const Run1D &p, double *pn, int L, int l, int g,
+                                       const double *U, const double *FX, const double *K,
+                                       const double *Q, double mdt4) {
+  const double c = mdt4 * __ldg(p.ax.di + g);  // -dt / (4 dx)
+  const double ql = Q[l], qm = Q[l - 1], qs = ql + qm;
+  double u[NV1];
+#pragma unroll
+  for (int v = 0; v < NV1; v++) {
+    const double uc = U[v * L + l];
+    double t = (FX[v * L + l + 1] - FX[v * L + l - 1]) + (K[v * L + l] - K[v * L + l - 1]);
+    t = fma(qs, uc, t);
+    t = fma(-ql, U[v * L + l + 1], t);
+    t = fma(-qm, U[v * L + l - 1], t);
+    u[v] = fma(c, t, uc);
+  }
+  const double ri = fd::rcp(u[0]);
+  const double vx = u[2] * ri, vy = u[3] * ri;
+  const double ek2 = fma(u[2], vx, u[3] * vy);
+  pn[l] = u[0];
+  pn[L + l] = p.ph.gm1 * fma(-p.ph.pi8i, u[4] * u[4], fma(-0.5, ek2, u[1]));
+  pn[2 * L + l] = vx;
+  pn[3 * L + l] = vy;
+  pn[4 * L + l] = u[4];
+}
+
+// safety * dx / (|vx| + c_f) of one cell (cfl_m.f:53-60)
+__device__ __forceinline__ double cfl(const Run1D &p, const double *pc, int L, int l, int g,
+                                      double safety) {
+  const double by = pc[4 * L + l], bx = __ldg(p.bx + g);
+  const double bb = fma(bx, bx, by * by);
+  const double s = fma(p.ph.pi4i, bb, p.ph.gm * pc[L + l]) * fd::rcp(pc[l]);
+  return safety * (__ldg(p.ax.d + g) * fd::rcp(fd::abs_(pc[2 * L + l]) + fd::sqrt_(s)));
+}
+}  // namespace f1
+
 namespace d1 {
 using R = df::DF;
 __device__ __forceinline__ R in(double x) { return num_in<R>(x); }
@@ -209,14 +324,14 @@ __device__ __forceinline__ void cell(const Run1D &p, const double *pc, int L, in
   const size_t nx = (size_t)p.ix;
   const R ro = in(pc[l]), pr = in(pc[L + l]), vx = in(pc[2 * L + l]), vy = in(pc[3 * L + l]),
           by = in(pc[4 * L + l]);
-  const R bx = in(p.bx[g]);
+  const R bx = in(__ldg(p.bx + g));
   const R ek = half(ro) * fma(vy, vy, sq(vx));
   const R rx = ro * vx;
   const R ez = fma(vy, bx, -(vx * by));
   if constexpr (BG) {
     const double *bg = p.bg;
-    const R sc = in(bg[2 * nx + g]), rr = in(bg[6 * nx + g]), gx = in(bg[g]),
-            dsc = in(bg[4 * nx + g]), drr = in(bg[8 * nx + g]), rri = in(RI[2 * L + l]);
+    const R sc = in(__ldg(bg + 2 * nx + g)), rr = in(__ldg(bg + 6 * nx + g)), gx = in(__ldg(bg + g)),
+            dsc = in(__ldg(bg + 4 * nx + g)), drr = in(__ldg(bg + 8 * nx + g)), rri = in(RI[2 * L + l]);
     const R pty = fma(sq(by), c.pi8i, pr);  // pressure without pi8i bx^2
     const R eey = fma(pr, c.gm1i, fma(c.pi8i, sq(by), ek));
     const R ep = fma(pr, c.ggm1, ek);
@@ -260,20 +375,20 @@ __device__ __forceinline__ void corner(const Run1D &p, const double *pc, int L, 
                                        const double *SS, double *K, double *SH, double *Q,
                                        R dt, const Phys1 &c) {
   const size_t nx = (size_t)p.ix;
-  const R dxim = in(p.ax.dim[g]);
+  const R dxim = in(__ldg(p.ax.dim + g));
   R un[NV1];
 #pragma unroll
   for (int v = 0; v < NV1; v++) {
     const R uh = half(ld(&U[v * L + l + 1]) + ld(&U[v * L + l]));
     un[v] = fma(-dt, dxim * (ld(&FX[v * L + l + 1]) - ld(&FX[v * L + l])), uh);
   }
-  const R bxm = in(p.bxm[g]);
+  const R bxm = in(__ldg(p.bxm + g));
   if constexpr (BG) {
     const double *bg = p.bg;
     un[1] = fma(dt, half(ld(&SS[l + 1]) + ld(&SS[l])), un[1]);
     un[2] = fma(dt, half(ld(&SS[L + l + 1]) + ld(&SS[L + l])) + ld(&XS[2 * L + l]), un[2]);
-    const R scm = in(bg[3 * nx + g]), rrm = in(bg[7 * nx + g]), gxm = in(bg[nx + g]),
-            dscm = in(bg[5 * nx + g]), drrm = in(bg[9 * nx + g]);
+    const R scm = in(__ldg(bg + 3 * nx + g)), rrm = in(__ldg(bg + 7 * nx + g)), gxm = in(__ldg(bg + nx + g)),
+            dscm = in(__ldg(bg + 5 * nx + g)), drrm = in(__ldg(bg + 9 * nx + g));
     const R si = in(RI[L + l]), rrmi = in(RI[3 * L + l]), ri = rcp(un[0]);
     const R roh = un[0] * si, eeh = un[1] * si, vxh = un[2] * ri, vyh = un[3] * ri * rrmi,
             byh = un[4] * si * rrm;
@@ -309,7 +424,7 @@ __device__ __forceinline__ void corner(const Run1D &p, const double *pc, int L, 
   // q = qav dxm max(0, |vx(i+1) - vx(i)| - 1.0e-4), the threshold a
   // single-precision literal in the reference, so exactly the float 1.0e-4f
   const R a = fabs(in(pc[2 * L + l + 1]) - in(pc[2 * L + l])) - 1.0e-4f;
-  const R q = a > 0.0f ? c.qav * in(p.ax.dm[g]) * a : R(0.0f);
+  const R q = a > 0.0f ? c.qav * in(__ldg(p.ax.dm + g)) * a : R(0.0f);
   st(&Q[l], q * dxim);
 }
 
@@ -320,7 +435,7 @@ __device__ __forceinline__ void update(const Run1D &p, double *pn, int L, int l,
                                        const double *FX,
                                        const double *SS, const double *K, const double *SH,
                                        const double *Q, R dt, const Phys1 &c) {
-  const R hdt = half(dt), dxi = in(p.ax.di[g]), hdx = half(dxi);
+  const R hdt = half(dt), dxi = in(__ldg(p.ax.di + g)), hdx = half(dxi);
   const R ql = ld(&Q[l]), qm = ld(&Q[l - 1]);
   R u[NV1];
 #pragma unroll
@@ -330,8 +445,8 @@ __device__ __forceinline__ void update(const Run1D &p, double *pn, int L, int l,
     du = fma(-hdt, dxi * (ld(&K[v * L + l]) - ld(&K[v * L + l - 1])), du);
     if (BG && (v == 1 || v == 2))
       du = fma(hdt,
-               fma(in(p.ax.u0[g]), ld(&SH[(v - 1) * L + l - 1]),
-                   in(p.ax.u1[g]) * ld(&SH[(v - 1) * L + l])),
+               fma(in(__ldg(p.ax.u0 + g)), ld(&SH[(v - 1) * L + l - 1]),
+                   in(__ldg(p.ax.u1 + g)) * ld(&SH[(v - 1) * L + l])),
                du);
     const R uc = ld(&U[v * L + l]);
     du = fma(dt, dxi * (ql * (ld(&U[v * L + l + 1]) - uc) - qm * (uc - ld(&U[v * L + l - 1]))),
@@ -370,10 +485,10 @@ __device__ __forceinline__ void update(const Run1D &p, double *pn, int L, int l,
 __device__ __forceinline__ double cfl(const Run1D &p, const double *pc, int L, int l, int g,
                                       double safety, const Phys1 &c) {
   const R ro = in(pc[l]), pr = in(pc[L + l]), vx = in(pc[2 * L + l]), by = in(pc[4 * L + l]);
-  const R bx = in(p.bx[g]);
+  const R bx = in(__ldg(p.bx + g));
   const R s = fma(c.gm, pr, fma(bx, bx, sq(by)) * c.pi4i) * rcp(ro);
   const R den = fabs(vx) + sqrt_(s);
-  return num_out(in(safety) * in(p.ax.d[g]) * rcp(den));
+  return num_out(in(safety) * in(__ldg(p.ax.d + g)) * rcp(den));
 }
 }  // namespace d1
 
@@ -389,13 +504,15 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
   const int r = (int)cluster.block_rank();
   const int tid = threadIdx.x, NT = blockDim.x;
   const int ix = p.ix, L = p.lmax;
-  extern __shared__ double sm[];
+  extern __shared__ __align__(16) double sm[];
   // layout: prim[2][5][L], U[5][L], FX[5][L], K[5][L], Q[L],
   // (BG: SS[2][L] cell sources, SH[2][L] corner sources, RI[4][L] the
   // reciprocals 1/sc, 1/scm, 1/rr, 1/rrm of the own cells; BG and DFP: XS[4][L]
-  // the static-field terms of the double-float stages), slots[2][CS],
-  // bad[2][CS], red[32]
-  double *prim = sm;
+  // the static-field terms of the double-float stages), after slots[2][CS], which
+  // every block of the cluster fills in every block, and red[32]
+  ulonglong2 *slots = (ulonglong2 *)sm;  // key of the block's CFL minimum; 1: a bad cell
+  unsigned long long *red = (unsigned long long *)(slots + 2 * CS);
+  double *prim = (double *)(red + 32);
   double *U = prim + 2 * NV1 * L;
   double *FX = U + NV1 * L;
   double *K = FX + NV1 * L;
@@ -404,9 +521,6 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
   double *SH = SS + (BG ? 2 * L : 0);
   double *RI = SH + (BG ? 2 * L : 0);
   double *XS = RI + (BG ? 4 * L : 0);
-  double *slots = XS + ((BG && DFP) ? 4 * L : 0);
-  double *bslots = slots + 2 * CS;  // per block: 1 if its CFL saw a bad cell
-  double *red = bslots + 2 * CS;
   const double *bg = p.bg;
   const size_t nx = (size_t)ix;
   __shared__ double s_dt, s_t, s_tp, s_pending;
@@ -439,10 +553,10 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
       // the cross-section and radius profiles are constant through the run:
       // the fast policy multiplies by their reciprocals instead of dividing
       // by them every step (1.0 / x, the value the step's own 1.0 / sc gave)
-      RI[0 * L + l] = 1.0 / bg[2 * nx + g];
-      RI[1 * L + l] = 1.0 / bg[3 * nx + g];
-      RI[2 * L + l] = 1.0 / bg[6 * nx + g];
-      RI[3 * L + l] = 1.0 / bg[7 * nx + g];
+      RI[0 * L + l] = 1.0 / __ldg(bg + 2 * nx + g);
+      RI[1 * L + l] = 1.0 / __ldg(bg + 3 * nx + g);
+      RI[2 * L + l] = 1.0 / __ldg(bg + 6 * nx + g);
+      RI[3 * L + l] = 1.0 / __ldg(bg + 7 * nx + g);
     }
     if constexpr (BG && DFP) {
       // formed in FP64: differences of nearly equal terms
@@ -456,15 +570,15 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
       auto shs = [&](int gg) { return c8 * bm2(gg) * bg[5 * nx + gg]; };
       if (l <= nl - 2) {
         num_st(&XS[l], d1::in(es(g + 1) - es(g)));
-        num_st(&XS[L + l], d1::in(0.5 * (es(g + 1) + es(g)) / bg[3 * nx + g] - c8 * bm2(g)));
-        num_st(&XS[2 * L + l], d1::in(-ax.dim[g] * (fxs(g + 1) - fxs(g)) +
+        num_st(&XS[L + l], d1::in(0.5 * (es(g + 1) + es(g)) / __ldg(bg + 3 * nx + g) - c8 * bm2(g)));
+        num_st(&XS[2 * L + l], d1::in(-__ldg(ax.dim + g) * (fxs(g + 1) - fxs(g)) +
                                       0.5 * (sss(g + 1) + sss(g))));
       }
       if (l >= 1 && l <= nl - 2)
         num_st(&XS[3 * L + l],
-               d1::in(-(0.5 * ax.di[g]) * (fxs(g + 1) - fxs(g - 1)) + sss(g) -
-                      ax.di[g] * (kxs(g) - kxs(g - 1)) + ax.u0[g] * shs(g - 1) +
-                      ax.u1[g] * shs(g)));
+               d1::in(-(0.5 * __ldg(ax.di + g)) * (fxs(g + 1) - fxs(g - 1)) + sss(g) -
+                      __ldg(ax.di + g) * (kxs(g) - kxs(g - 1)) + __ldg(ax.u0 + g) * shs(g - 1) +
+                      __ldg(ax.u1 + g) * shs(g)));
     }
   }
   if (tid == 0) {
@@ -477,58 +591,69 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
       s_done = 0; s_merr = 0; s_pause = 0;
     }
   }
+  // the loop's constants: read from the control block here, not by one thread in the
+  // serial part of every step
+  const double c_safety = p.ctl ? p.ctl->safety : 1.0, c_dtmin = p.ctl ? p.ctl->dtmin : 0.0;
+  const double c_tend = p.ctl ? p.ctl->tend : 0.0;
+  const double c_dtout = p.ctl && p.ctl->pause_on_output ? p.ctl->dtout : 0.0;
+  const long long c_nstop = p.ctl ? p.ctl->nstop : 0;
+  const bool c_stop_bad = p.ctl && p.ctl->stop_on_bad;
   int cur = 0;
   __syncthreads();
 
-  // CFL of the own cells (cfl_m.f:53-60) reduced over the cluster into
-  // slots[par] of block 0; returns the minimum after a cluster barrier, and
-  // in any_bad whether a cell of any block had a non-positive density or
-  // pressure or a time step that is not a number (counted in ctl->nonfinite).
+  // CFL of the own cells (cfl_m.f:53-60) reduced over the cluster; valid on thread
+  // 0: the minimum after a cluster barrier, and in any_bad whether a cell of any
+  // block had a non-positive density or pressure or a time step that is not a
+  // number (counted in ctl->nonfinite).  The minimum is one of unsigned keys (the
+  // integer min of a warp is two instructions, five exchanges of doubles are ten
+  // FP64 comparisons), and each block writes it into every block's slots, so that
+  // no block reads another's memory after the barrier.
   auto cluster_cfl = [&](int buf, int par, bool &any_bad) -> double {
-    double dmin = __longlong_as_double(0x7ff0000000000000LL);
+    unsigned long long kmin = min_key(__longlong_as_double(0x7ff0000000000000LL));
     bool bad = false;
-    const FT safety(p.ctl ? p.ctl->safety : 1.0), pi4c(p.ph.pi4i);
+    const FT safety(c_safety), pi4c(p.ph.pi4i);
     for (int l = 1 + tid; l <= nl - 2; l += NT) {
       const int g = lo - 1 + l;
+      double dtq;
       if constexpr (DFP) {
-        const double dtq = d1::cfl(p, &P(buf, 0, 0), L, l, g, safety.v, cdf);
-        if (dtq < dmin || dmin != dmin) dmin = dtq;
-        bad |= bad_cell(P(buf, 0, l), P(buf, 1, l), dtq);
-        continue;
+        dtq = d1::cfl(p, &P(buf, 0, 0), L, l, g, safety.v, cdf);
+      } else if constexpr (!E && !BG) {
+        dtq = f1::cfl(p, &P(buf, 0, 0), L, l, g, safety.v);
+      } else {
+        const FT ro(P(buf, 0, l)), pr(P(buf, 1, l)), vx(P(buf, 2, l)), by(P(buf, 4, l));
+        const FT bx(__ldg(p.bx + g));
+        const FT onero = 1.0 / ro;
+        const FT ca2 = (bx * bx + by * by) * pi4c * onero;
+        const FT cs2 = gm * pr * onero;
+        const FT dtcfl = FT(__ldg(ax.d + g)) / (fabs_(vx) + fsqrt(cs2 + ca2));
+        dtq = (safety * dtcfl).v;
       }
-      const FT ro(P(buf, 0, l)), pr(P(buf, 1, l)), vx(P(buf, 2, l)), by(P(buf, 4, l));
-      const FT bx(p.bx[g]);
-      const FT onero = 1.0 / ro;
-      const FT ca2 = (bx * bx + by * by) * pi4c * onero;
-      const FT cs2 = gm * pr * onero;
-      const FT dtcfl = FT(ax.d[g]) / (fabs_(vx) + fsqrt(cs2 + ca2));
-      const double dtq = (safety * dtcfl).v;
-      if (dtq < dmin || dmin != dmin) dmin = dtq;
-      bad |= bad_cell(ro.v, pr.v, dtq);
+      const unsigned long long k = min_key(dtq);
+      if (!fd::is_nan(dtq) && k < kmin) kmin = k;
+      bad |= bad_cell(P(buf, 0, l), P(buf, 1, l), dtq);
     }
-    dmin = warp_min(dmin);
-    if ((tid & 31) == 0) red[tid >> 5] = dmin;
+    kmin = warp_min_key(kmin);
+    if ((tid & 31) == 0) red[tid >> 5] = kmin;
     const int blk_bad = __syncthreads_or(bad);
-    if (tid == 0) {
-      double x = red[0];
-      for (int w = 1; w < (NT + 31) / 32; w++) x = (red[w] < x || x != x) ? red[w] : x;
-      double *dst = cluster.map_shared_rank(slots, 0);
-      dst[par * CS + r] = x;
-      double *dstb = cluster.map_shared_rank(bslots, 0);
-      dstb[par * CS + r] = blk_bad ? 1.0 : 0.0;
-      if (blk_bad && p.ctl) atomicAdd(&p.ctl->nonfinite, 1);
+    if (tid < 32) {
+      kmin = warp_min_key(tid < (NT + 31) / 32 ? red[tid] : ~0ull);
+      for (int c = tid; c < CS; c += 32)
+        cluster.map_shared_rank(slots, c)[par * CS + r] =
+            make_ulonglong2(kmin, blk_bad ? 1ull : 0ull);
+      if (tid == 0 && blk_bad && p.ctl) atomicAdd(&p.ctl->nonfinite, 1);
     }
     cluster.sync();
-    double *src = cluster.map_shared_rank(slots, 0);
-    double *srcb = cluster.map_shared_rank(bslots, 0);
-    double m = (double)1.e20f;  // the reference's starting minimum
     any_bad = false;
-    for (int k = 0; k < CS; k++) {
-      const double x = src[par * CS + k];
-      if (x < m) m = x;
-      any_bad |= srcb[par * CS + k] != 0.0;
+    if (tid >= 32) return 0.0;
+    kmin = min_key((double)1.e20f);  // the reference's starting minimum
+    bool b = false;
+    for (int c = tid; c < CS; c += 32) {
+      const ulonglong2 x = slots[par * CS + c];
+      kmin = x.x < kmin ? x.x : kmin;
+      b |= x.y != 0;
     }
-    return m;
+    any_bad = __any_sync(0xffffffffu, b);
+    return from_min_key(warp_min_key(kmin));
   };
 
   int par = 0;
@@ -539,7 +664,7 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
     if (tid == 0) {  // first iteration always starts (do-while loop)
       s_ns += 1;
       s_dt = dt0;
-      if (dt0 < p.ctl->dtmin) {
+      if (dt0 < c_dtmin) {
         s_merr = 9001;
         s_done = 1;
       } else {
@@ -564,8 +689,8 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
         const int g = lo - 1 + l;
         const FT ro(P(cur, 0, l)), pr(P(cur, 1, l)), vx(P(cur, 2, l)), vy(P(cur, 3, l)),
             by(P(cur, 4, l));
-        const FT bx(p.bx[g]), gx(bg[g]), sc(bg[2 * nx + g]), dsc(bg[4 * nx + g]),
-            rr(bg[6 * nx + g]), drr(bg[8 * nx + g]);
+        const FT bx(__ldg(p.bx + g)), gx(__ldg(bg + g)), sc(__ldg(bg + 2 * nx + g)), dsc(__ldg(bg + 4 * nx + g)),
+            rr(__ldg(bg + 6 * nx + g)), drr(__ldg(bg + 8 * nx + g));
         const FT vv = vx * vx + vy * vy;
         const FT bb = by * by + bx * bx;
         FT ee, ep;
@@ -599,22 +724,18 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
           FX[4 * L + l] = ((-ez) * sc * rri).v;
         }
       }
+    } else if constexpr (!E) {
+      for (int l = tid; l < nl; l += NT) f1::cell(p, &P(cur, 0, 0), L, l, lo - 1 + l, U, FX);
     } else
     for (int l = tid; l < nl; l += NT) {
       const int g = lo - 1 + l;
       const FT ro(P(cur, 0, l)), pr(P(cur, 1, l)), vx(P(cur, 2, l)), vy(P(cur, 3, l)),
           by(P(cur, 4, l));
-      const FT bx(p.bx[g]);
+      const FT bx(__ldg(p.bx + g));
       const FT vv = vx * vx + vy * vy;
       const FT bb = by * by;
-      FT ee, ep;
-      if constexpr (E) {
-        ee = pr / gm1 + 0.5 * ro * vv + pi8i * bb;
-        ep = pr * gm / gm1 + 0.5 * ro * vv;
-      } else {
-        ee = pr * p.ph.gm1i + 0.5 * ro * vv + pi8i * bb;
-        ep = pr * p.ph.ggm1 + 0.5 * ro * vv;
-      }
+      const FT ee = pr / gm1 + 0.5 * ro * vv + pi8i * bb;
+      const FT ep = pr * gm / gm1 + 0.5 * ro * vv;
       const FT rx = ro * vx;
       const FT ez = -vx * by + vy * bx;
       U[0 * L + l] = ro.v; U[1 * L + l] = ee.v; U[2 * L + l] = rx.v;
@@ -637,7 +758,7 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
       // and sources (:188-234)
       for (int l = tid; l < nl - 1; l += NT) {
         const int g = lo - 1 + l;
-        const FT dxim(ax.dim[g]);
+        const FT dxim(__ldg(ax.dim + g));
         FT un[NV1];
 #pragma unroll
         for (int v = 0; v < NV1; v++) {
@@ -647,8 +768,8 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
         }
         un[1] = un[1] + dt * (0.5 * (FT(SS[0 * L + l + 1]) + FT(SS[0 * L + l])));
         un[2] = un[2] + dt * (0.5 * (FT(SS[1 * L + l + 1]) + FT(SS[1 * L + l])));
-        const FT scm(bg[3 * nx + g]), rrm(bg[7 * nx + g]), gxm(bg[nx + g]),
-            dscm(bg[5 * nx + g]), drrm(bg[9 * nx + g]), bxm(p.bxm[g]);
+        const FT scm(__ldg(bg + 3 * nx + g)), rrm(__ldg(bg + 7 * nx + g)), gxm(__ldg(bg + nx + g)),
+            dscm(__ldg(bg + 5 * nx + g)), drrm(__ldg(bg + 9 * nx + g)), bxm(__ldg(p.bxm + g));
         FT roh, eeh, vxh, vyh, byh;
         if constexpr (E) {
           roh = un[0] / scm;
@@ -689,14 +810,18 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
                            (prh + bb * pi8i) * dscm).v;
           K[4 * L + l] = ((-ezh) * scm * rrmi).v;
         }
-        const FT q = qav * FT(ax.dm[g]) *
+        const FT q = qav * FT(__ldg(ax.dm + g)) *
                      max0(fabs_(FT(P(cur, 2, l + 1)) - FT(P(cur, 2, l))) - CANS_AV_EPS);
         Q[l] = (q * dxim).v;
       }
+    } else if constexpr (!E) {
+      const double m2dt = -2.0 * s_dt;
+      for (int l = tid; l < nl - 1; l += NT)
+        f1::corner(p, &P(cur, 0, 0), L, l, lo - 1 + l, U, FX, K, Q, m2dt);
     } else
     for (int l = tid; l < nl - 1; l += NT) {
       const int g = lo - 1 + l;  // corner between g and g+1
-      const FT dxim(ax.dim[g]);
+      const FT dxim(__ldg(ax.dim + g));
       FT un[NV1];
 #pragma unroll
       for (int v = 0; v < NV1; v++) {
@@ -705,29 +830,20 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
         un[v] = uh - dt * dfdx;
       }
       const FT roh = un[0], eeh = un[1], rxh = un[2], ryh = un[3], byh = un[4];
-      FT vxh, vyh;
-      if constexpr (E) {
-        vxh = rxh / roh;
-        vyh = ryh / roh;
-      } else {
-        const FT rinv(1.0 / roh.v);
-        vxh = rxh * rinv;
-        vyh = ryh * rinv;
-      }
+      const FT vxh = rxh / roh;
+      const FT vyh = ryh / roh;
       const FT vv = vxh * vxh + vyh * vyh;
       const FT bb = byh * byh;
       const FT prh = gm1 * (eeh - 0.5 * roh * vv - pi8i * bb);
-      const FT bxm(p.bxm[g]);
+      const FT bxm(__ldg(p.bxm + g));
       const FT ezh = -vxh * byh + vyh * bxm;
-      FT eph;
-      if constexpr (E) eph = prh * gm / gm1 + 0.5 * roh * vv;
-      else eph = prh * p.ph.ggm1 + 0.5 * roh * vv;
+      const FT eph = prh * gm / gm1 + 0.5 * roh * vv;
       K[0 * L + l] = (roh * vxh).v;
       K[1 * L + l] = (eph * vxh - byh * ezh * pi4i).v;
       K[2 * L + l] = (roh * (vxh * vxh) + prh + byh * byh * pi8i).v;
       K[3 * L + l] = (roh * vxh * vyh - bxm * byh * pi4i).v;
       K[4 * L + l] = (-ezh).v;
-      const FT q = qav * FT(ax.dm[g]) *
+      const FT q = qav * FT(__ldg(ax.dm + g)) *
                    max0(fabs_(FT(P(cur, 2, l + 1)) - FT(P(cur, 2, l))) - CANS_AV_EPS);
       Q[l] = (q * dxim).v;
     }
@@ -745,7 +861,7 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
       // update and conversion (mlw_m_bg.f:251-268) and the torque
       for (int l = 1 + tid; l <= nl - 2; l += NT) {
         const int g = lo - 1 + l;
-        const FT hdt = 0.5 * dt, dxi(ax.di[g]);
+        const FT hdt = 0.5 * dt, dxi(__ldg(ax.di + g));
         const FT hdx = 0.5 * dxi;
         FT u[NV1];
 #pragma unroll
@@ -755,14 +871,14 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
           if (v == 1 || v == 2) du = du + hdt * FT(SS[(v - 1) * L + l]);
           du = du - hdt * (dxi * (FT(K[v * L + l]) - FT(K[v * L + l - 1])));
           if (v == 1 || v == 2)
-            du = du + hdt * (FT(ax.u0[g]) * FT(SH[(v - 1) * L + l - 1]) +
-                             FT(ax.u1[g]) * FT(SH[(v - 1) * L + l]));
+            du = du + hdt * (FT(__ldg(ax.u0 + g)) * FT(SH[(v - 1) * L + l - 1]) +
+                             FT(__ldg(ax.u1 + g)) * FT(SH[(v - 1) * L + l]));
           const FT uc(U[v * L + l]);
           du = du + dt * (dxi * (FT(Q[l]) * (FT(U[v * L + l + 1]) - uc) -
                                  FT(Q[l - 1]) * (uc - FT(U[v * L + l - 1]))));
           u[v] = uc + du;
         }
-        const FT sc(bg[2 * nx + g]), rr(bg[6 * nx + g]), bx(p.bx[g]);
+        const FT sc(__ldg(bg + 2 * nx + g)), rr(__ldg(bg + 6 * nx + g)), bx(__ldg(p.bx + g));
         FT ro, ee, rx, ry, by, vx, vy;
         if constexpr (E) {
           ro = u[0] / sc;
@@ -786,10 +902,14 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
         P(nb, 0, l) = ro.v; P(nb, 1, l) = pr.v; P(nb, 2, l) = vx.v;
         P(nb, 3, l) = vy.v; P(nb, 4, l) = by.v;
       }
+    } else if constexpr (!E) {
+      const double mdt4 = -0.25 * s_dt;
+      for (int l = 1 + tid; l <= nl - 2; l += NT)
+        f1::update(p, &P(nb, 0, 0), L, l, lo - 1 + l, U, FX, K, Q, mdt4);
     } else
     for (int l = 1 + tid; l <= nl - 2; l += NT) {
       const int g = lo - 1 + l;
-      const FT hdt = 0.5 * dt, dxi(ax.di[g]);
+      const FT hdt = 0.5 * dt, dxi(__ldg(ax.di + g));
       const FT hdx = 0.5 * dxi;
       FT u[NV1];
 #pragma unroll
@@ -803,15 +923,8 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
         u[v] = uc + du;
       }
       const FT ro = u[0], ee = u[1], rx = u[2], ry = u[3], by = u[4];
-      FT vx, vy;
-      if constexpr (E) {
-        vx = rx / ro;
-        vy = ry / ro;
-      } else {
-        const FT rinv(1.0 / ro.v);
-        vx = rx * rinv;
-        vy = ry * rinv;
-      }
+      const FT vx = rx / ro;
+      const FT vy = ry / ro;
       const FT pr = gm1 * (ee - 0.5 * ro * (vx * vx + vy * vy) - pi8i * (by * by));
       P(nb, 0, l) = ro.v; P(nb, 1, l) = pr.v; P(nb, 2, l) = vx.v;
       P(nb, 3, l) = vy.v; P(nb, 4, l) = by.v;
@@ -854,13 +967,13 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
         return make_int2(rr, l);
       };
       auto get = [&](int g1) -> double {
+        if (p.bnd_local) return P(nb, v, g1 - lo);
         const int2 o = owner(g1);
         double *base = cluster.map_shared_rank(prim, o.x);
         return base[(size_t)nb * NVS + (size_t)v * L + o.y];
       };
-      auto put = [&](int g1, double x) {
-        const int2 o = owner(g1);
-        P(nb, v, o.y) = x;  // faces only write cells of this block
+      auto put = [&](int g1, double x) {  // faces only write cells of this block
+        P(nb, v, p.bnd_local ? g1 - lo : owner(g1).y) = x;
       };
       if (r == 0)
         bd1_face(p.bc.kind[v][0], 0, p.bc.margin, ix, p.bc.q0[v][0], ax.dm, get, put);
@@ -887,41 +1000,38 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
       if (nev) atomicAdd(&p.ctl->nfloor, (unsigned long long)nev);
       __syncthreads();
     }
-    // ---- CFL of the own cells, reduced over the cluster; its cluster barrier
-    // also publishes every block's final cells for the halo exchange ---------
+    // ---- the edge cells into the neighbours' halos, the CFL of the own cells,
+    // reduced over the cluster; its cluster barrier publishes both ------------
+    if (tid < NV1) {
+      if (r > 0)
+        cluster.map_shared_rank(prim, r - 1)[(size_t)nb * NVS + (size_t)tid * L +
+                                             own_count(r - 1) + 1] = P(nb, tid, 1);
+      if (r < CS - 1)
+        cluster.map_shared_rank(prim, r + 1)[(size_t)nb * NVS + (size_t)tid * L] =
+            P(nb, tid, nl - 2);
+    }
     bool badn;
     const double dtn = cluster_cfl(nb, par, badn);
     par ^= 1;
-    if (tid < NV1) {
-      if (r > 0) {
-        const double *nbp = cluster.map_shared_rank(prim, r - 1);
-        const int ln = own_count(r - 1);  // neighbour's last own cell
-        P(nb, tid, 0) = nbp[(size_t)nb * NVS + (size_t)tid * L + ln];
-      }
-      if (r < CS - 1) {
-        const double *nbp = cluster.map_shared_rank(prim, r + 1);
-        P(nb, tid, nl - 1) = nbp[(size_t)nb * NVS + (size_t)tid * L + 1];
-      }
-    }
     cur = nb;
     if (tid == 0) {
       // end of the loop body (main.f:155-199) and start of the next
       s_nexec += 1;
-      if (p.ctl->pause_on_output && p.ctl->dtout > 0.0) {
-        const long long nt1 = (long long)(s_tp / p.ctl->dtout);
-        const long long nt2 = (long long)(s_t / p.ctl->dtout);
+      if (c_dtout > 0.0) {
+        const long long nt1 = (long long)(s_tp / c_dtout);
+        const long long nt2 = (long long)(s_t / c_dtout);
         if (nt1 < nt2) s_pause = 1;
       }
       s_pending = dtn;  // CFL of the state just written, for a later resume
-      if (!(s_ns < p.ctl->nstop && s_t < p.ctl->tend)) {
+      if (!(s_ns < c_nstop && s_t < c_tend)) {
         s_done = 1;
-      } else if (!s_pause && p.ctl->stop_on_bad && badn) {
+      } else if (!s_pause && c_stop_bad && badn) {
         s_merr = 9100;  // CANS_ERR_NONFINITE: the state just written has a bad cell
         s_done = 1;
       } else if (!s_pause) {
         s_ns += 1;
         s_dt = dtn;
-        if (dtn < p.ctl->dtmin) {
+        if (dtn < c_dtmin) {
           s_merr = 9001;
           s_done = 1;
         } else {
