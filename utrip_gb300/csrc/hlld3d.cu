@@ -30,6 +30,7 @@
 #include "cans_internal.h"
 #include "cfl3.cuh"
 #include "hlld_flux.cuh"
+#include "isum.cuh"
 
 namespace cans {
 
@@ -138,13 +139,6 @@ __device__ __forceinline__ bool near_degenerate(const double *L, const double *R
   return en > 0 && et + 6 <= en && 2 * en - 1019 >= ep;
 }
 
-// minmod of the fast policy (flmt of inp_tvdminmod.f:118 up to the sign of a
-// zero result), on the integer pipe
-__device__ __forceinline__ double minmod(double a, double b) {
-  const long long x = __double_as_longlong(a) ^ __double_as_longlong(b);
-  return x >= 0 ? fd::mul_sign(fd::minp(fd::abs_(a), fd::abs_(b)), a) : 0.0;
-}
-
 template <bool E, int STAGE, bool QF>
 __global__ void __launch_bounds__(kThreads)
     k_hlld_flux(const double *__restrict__ P, double *__restrict__ Fl, Geo g,
@@ -180,9 +174,7 @@ __global__ void __launch_bounds__(kThreads)
           wl[v] = (t0 + T(0.5) * flmt(t0 - T(dm), t1 - t0)).v;
           wr[v] = (t1 - T(0.5) * flmt(T(d2) - t1, t1 - t0)).v;
         } else {
-          const double gc = d1 - d0;
-          wl[v] = fma(0.5, minmod(d0 - dm, gc), d0);
-          wr[v] = fma(-0.5, minmod(d2 - d1, gc), d1);
+          isum::muscl(dm, d0, d1, d2, wl[v], wr[v]);
         }
       }
     }
@@ -258,7 +250,7 @@ __global__ void __launch_bounds__(kThreads)
       if (v == U_BX + a) continue;
       const T f0(__ldg(Fa + v * g.n + c)), fm(__ldg(Fa + v * g.n + c - s));
       if constexpr (E) u[v] = u[v] - dts * ((f0 - fm) / T(pd[ca]));
-      else u[v] = u[v] - w * (f0 - fm);
+      else u[v] = u[v] - w * T(isum::sub_rn(f0.v, fm.v));
     }
   }
   to_primitive<E>(u, K.gm1, mu2, p);

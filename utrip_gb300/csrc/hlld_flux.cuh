@@ -334,7 +334,7 @@ __device__ __forceinline__ void hlld_flux_t(const HlldK &K, const double *L,
 //    the inner root's (g + B^2)^2 - 4 g Bx^2, g = gm p, as the sum of squares
 //    (g - Bx^2)^2 + Bt^2 (2 (g + Bx^2) + Bt^2), which no rounding makes negative;
 //  - reciprocals, roots and comparisons of fd64.cuh.
-// Measured on the 128^3 box with an oblique field (134^3 cells): 6.6 ms a step
+// Measured on the 128^3 box with an oblique field (134^3 cells): 6.6 ms a step (6.3 with isum.cuh)
 // where the reference's branches with both sides formed took 12.3 ms.
 // A star state within zfloor of its singular denominator keeps the side's own
 // state (hlld_flux.f90:281-342), by selects.
@@ -415,7 +415,8 @@ __device__ __forceinline__ void hlld_flux_fast(const HlldK &K, const double *L,
     fby = fma(sp, bys - by, fby);
     fbz = fma(sp, bzs - bz, fbz);
     // between the Alfven waves (with bx = 0 they are the contact)
-    const bool inner = right ? (__double2hiint(sa) >= 0 && sa != 0.0) : __double2hiint(sa) < 0;
+    const int sah = __double2hiint(sa);
+    const bool inner = right ? sah >= 0 && (sah | __double2loint(sa)) != 0 : sah < 0;
     if (inner) {
       const double sdo = right ? dl : dr, mo = right ? ml : mr;
       const double sdmo = (right ? sl : sr) - sm;
@@ -426,7 +427,8 @@ __device__ __forceinline__ void hlld_flux_fast(const HlldK &K, const double *L,
       const double qo = fd::sqrt_(roo);
       const double iv = fd::rcp(rs + qo), qq = rs * qo;
       // sign(bx) with the sides exchanged for the right one
-      const double flip = right ? -bx : bx;
+      const double flip =
+          __hiloint2double(__double2hiint(bx) ^ (right ? (int)0x80000000 : 0), 0);
       const double vyd = iv * (fma(rs, vys, qo * vyo) + fd::mul_sign(byo - bys, flip));
       const double vzd = iv * (fma(rs, vzs, qo * vzo) + fd::mul_sign(bzo - bzs, flip));
       const double byd = iv * fma(rs, byo, fma(qo, bys, qq * fd::mul_sign(vyo - vys, flip)));

@@ -193,5 +193,87 @@ __device__ __forceinline__ double face_planes(double a, double b, double c, doub
   return out<6>(s - at<6>(pl, el, E), E);
 }
 
+// x + y rounded to nearest, the FP64 addition's result to the bit: the smaller operand
+// is aligned to the larger with ten guard bits and what falls off them is kept as
+// one sticky bit.  Some fifty integer instructions.
+__device__ __forceinline__ double add2(double x, double y, bool &sp) {
+  const unsigned hx = (unsigned)__double2hiint(x), lx = (unsigned)__double2loint(x);
+  const unsigned hy = (unsigned)__double2hiint(y), ly = (unsigned)__double2loint(y);
+  const bool sw = ((unsigned long long)(hy & 0x7fffffffu) << 32 | ly) >
+                  ((unsigned long long)(hx & 0x7fffffffu) << 32 | lx);
+  const unsigned hg = sw ? hy : hx, lg = sw ? ly : lx, hs = sw ? hx : hy, ls = sw ? lx : ly;
+  const unsigned E = hg & 0x7ff00000u;
+  sp |= special(E);
+  if (E == 0u) sp |= ((hg & 0x7fffffffu) | lg) != 0u;
+  auto sig = [](unsigned hi, unsigned lo) {  // the hidden bit at 62
+    return (unsigned long long)((__funnelshift_l(lo, hi, 10) & 0x3fffffffu) | 0x40000000u) << 32 |
+           lo << 10;
+  };
+  const unsigned sh = (E - (hs & 0x7ff00000u)) >> 20;
+  const unsigned long long small = sig(hs, ls);
+  unsigned long long t = small, back;
+  asm("shr.u64 %0, %0, %1;" : "+l"(t) : "r"(sh));
+  asm("shl.b64 %0, %1, %2;" : "=l"(back) : "l"(t), "r"(sh));
+  t |= back != small ? 1ull : 0ull;
+  const long long opp = (long long)((int)(hg ^ hs) >> 31);
+  unsigned long long m = sig(hg, lg) + (unsigned long long)(((long long)t ^ opp) - opp);
+  m = E != 0u ? m : 0ull;
+  const int lz = __clzll((long long)m);
+  asm("shl.b64 %0, %0, %1;" : "+l"(m) : "r"(lz));
+  const unsigned lo = (unsigned)m;
+  const unsigned up = ((lo & 0x7ffu) + 0x3ffu + ((lo >> 11) & 1u)) >> 11;
+  const unsigned f = m ? E - ((unsigned)lz << 20) : 0u, sg = m ? hg : hg & hs;
+  const unsigned long long b = (m >> 11) + up;
+  return __hiloint2double((int)(((unsigned)(b >> 32) + f) | (sg & 0x80000000u)), (int)b);
+}
+__device__ __forceinline__ double neg(double x) {  // on the upper word: -x is an FP64 addition
+  return __hiloint2double(__double2hiint(x) ^ (int)0x80000000, __double2loint(x));
+}
+static __device__ __noinline__ double add_fp64(double x, double y) { return x + y; }
+// x - y, the FP64 subtraction's result
+__device__ __forceinline__ double sub_rn(double x, double y) {
+  bool sp = false;
+  const double r = add2(x, neg(y), sp);
+  return sp ? add_fp64(x, neg(y)) : r;
+}
+// x / 2 of a normal number or zero
+__device__ __forceinline__ double half_of(double x, bool &sp) {
+  const unsigned e = expo(x);
+  if (e <= 0x100000u) sp |= bits(x) != 0u;
+  return __hiloint2double(__double2hiint(x) - (int)min(e, 0x100000u), __double2loint(x));
+}
+
+// The minmod face states between cells 0 and 1 of a line of four: d0 + minmod(d0 - dm,
+// d1 - d0) / 2 and d1 - minmod(d2 - d1, d1 - d0) / 2 (up to the sign of a zero
+// minmod), bit for bit what five FP64 instructions give.
+// Measured on the 128^3 boxes: Roe-MUSCL 9.0 -> 8.6 ms a step, HLLD 6.5 -> 6.3; with
+// sub_rn in the updates 8.5 (the sums inside the Roe flux too: 8.9, as their
+// integer temporaries halve the warps in flight).
+__device__ __forceinline__ double minmod(double a, double b) {
+  const long long x = __double_as_longlong(a) ^ __double_as_longlong(b);
+  const unsigned long long p = (unsigned long long)__double_as_longlong(a) & 0x7fffffffffffffffull;
+  const unsigned long long q = (unsigned long long)__double_as_longlong(b) & 0x7fffffffffffffffull;
+  const unsigned long long m = p < q ? p : q;
+  const unsigned long long s = (unsigned long long)__double_as_longlong(a) & 0x8000000000000000ull;
+  return __longlong_as_double(x >= 0 ? (long long)(m | s) : 0ll);
+}
+static __device__ __noinline__ double2 muscl_fp64(double dm, double d0, double d1, double d2) {
+  const double g = d1 - d0;
+  return make_double2(fma(0.5, minmod(d0 - dm, g), d0), fma(-0.5, minmod(d2 - d1, g), d1));
+}
+__device__ __forceinline__ void muscl(double dm, double d0, double d1, double d2, double &wl,
+                                      double &wr) {
+  bool sp = false;
+  const double g = add2(d1, neg(d0), sp);
+  const double l = minmod(add2(d0, neg(dm), sp), g), r = minmod(add2(d2, neg(d1), sp), g);
+  wl = add2(d0, half_of(l, sp), sp);
+  wr = add2(d1, neg(half_of(r, sp)), sp);
+  if (sp) {
+    const double2 w = muscl_fp64(dm, d0, d1, d2);
+    wl = w.x;
+    wr = w.y;
+  }
+}
+
 }  // namespace isum
 }  // namespace cans

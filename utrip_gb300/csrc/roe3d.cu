@@ -37,6 +37,7 @@
 #include "cans_common.cuh"
 #include "cans_internal.h"
 #include "cfl3.cuh"
+#include "isum.cuh"
 #include "roe_flux.cuh"
 
 namespace cans {
@@ -145,13 +146,6 @@ __device__ __forceinline__ void roe_flux(const RoeK &K, const double *L,
   else roe_flux_fast<ND == 3>(K, L, R, f);
 }
 
-// minmod(a, b) of the fast policy: equal to flmt(a, b) of tvdminmod.f:15 up
-// to the sign of a zero result; the sign test runs on the integer pipe.
-__device__ __forceinline__ double minmod(double a, double b) {
-  const long long x = __double_as_longlong(a) ^ __double_as_longlong(b);
-  return x >= 0 ? fd::mul_sign(fd::minp(fd::abs_(a), fd::abs_(b)), a) : 0.0;
-}
-
 // Conserved variables of a primitive state (roe_m.f:42-47).
 template <bool E>
 __device__ __forceinline__ void to_conserved(const RoeK &K, const double *p,
@@ -217,7 +211,7 @@ __device__ __forceinline__ void add_divergence(F<E> *u, const double *__restrict
     if (v == U_BX + a) continue;
     const T fm(__ldg(Fa + v * g.n + c - st)), f0(__ldg(Fa + v * g.n + c));
     if constexpr (E) u[v] = u[v] + T(fac) * ((fm - f0) / T(d));
-    else u[v] = u[v] + w * (fm - f0);
+    else u[v] = u[v] + w * T(isum::sub_rn(fm.v, f0.v));
   }
 }
 
@@ -328,9 +322,7 @@ __global__ void __launch_bounds__(kRoeThreads)
         wl[v] = (d0 + T(0.5) * flmt(d1 - d0, d0 - dm)).v;
         wr[v] = (d1 - T(0.5) * flmt(d1 - d0, d2 - d1)).v;
       } else {
-        const double gl = d0.v - dm.v, gc = d1.v - d0.v, gr = d2.v - d1.v;
-        wl[v] = fma(0.5, minmod(gl, gc), d0.v);
-        wr[v] = fma(-0.5, minmod(gr, gc), d1.v);
+        isum::muscl(dm.v, d0.v, d1.v, d2.v, wl[v], wr[v]);
       }
     }
     to_frame<ND>(a, wl, L);

@@ -245,7 +245,7 @@ __device__ __forceinline__ void roe_flux_ref(const RoeK &K, const double *L,
 //  - the factors sq4r and sign(bx) common to the 2 x 2 systems' numerators and
 //    determinants cancel, the energy's eigenvector sums are those of the density
 //    and momenta (roe_flux_fast_r), and the halves are taken once at the end.
-// Measured on the 128^3 box (134^3 cells): 9.3 ms a step; with CUDA's roots and
+// Measured on the 128^3 box (134^3 cells): 9.3 ms a step (8.5 with the sums of isum.cuh around it); with CUDA's roots and
 // reciprocals and the sums term by term 12.3 ms.
 
 __device__ __forceinline__ double rcp_(double x) { return fd::rcp(x); }
@@ -255,6 +255,8 @@ __device__ __forceinline__ double sqrt_(double x) { return fd::sqrt_(x); }
 __device__ __forceinline__ double maxp_(double a, double b) { return fd::maxp(a, b); }
 __device__ __forceinline__ double pos_(double a) { return fd::pos_part(a); }
 __device__ __forceinline__ double muls_(double a, double s) { return fd::mul_sign(a, s); }
+// on the upper word (fabs is an FP64 instruction where nothing folds it)
+__device__ __forceinline__ double abs_(double a) { return fd::abs_(a); }
 // a >= b for values that are not negative
 __device__ __forceinline__ bool gep_(double a, double b) { return !fd::ltp(a, b); }
 
@@ -276,6 +278,7 @@ __device__ __forceinline__ df::DF pos_(df::DF a) { return a.d.h > 0.0f ? a : df:
 __device__ __forceinline__ df::DF muls_(df::DF a, df::DF s) {
   return signbit(s.d.h) ? -a : a;
 }
+__device__ __forceinline__ df::DF abs_(df::DF a) { return fabs(a); }
 __device__ __forceinline__ bool gep_(df::DF a, df::DF b) { return !df::gt(b.d, a.d); }
 
 // The constants of the fast flux in its number type.
@@ -343,7 +346,7 @@ __device__ __forceinline__ void roe_flux_fast_r(const RoeKR<R> &K, const R *L, c
   const R cfast = cfast2 * rcf;
   const R rrb = rsq_(rhobar);
   const R cs = sqrt_(cs2);
-  const R ca = fabs(bxb) * K.sq4pii * rrb;
+  const R ca = abs_(bxb) * K.sq4pii * rrb;
   const R cslow2 = cs2 * ca2 * (rcf * rcf);
   const R cslow = cs * ca * rcf;
   // singular points
@@ -352,7 +355,7 @@ __device__ __forceinline__ void roe_flux_fast_r(const RoeKR<R> &K, const R *L, c
   const R rbt = rsq_(bt2 + one - sp);
   const R betay = spb ? byb * rbt : K.sqh;
   const R betaz = spb ? bzb * rbt : K.sqh;
-  const bool sp2b = gep_(fma(bt2, pib, fabs(dcs)), K.eps12);
+  const bool sp2b = gep_(fma(bt2, pib, abs_(dcs)), K.eps12);
   const R sp2 = sp2b ? one : zero;
   const R cfca = pos_(cfast2 - ca2);
   const R cfcs = pos_(cfast2 - cslow2);
@@ -371,10 +374,10 @@ __device__ __forceinline__ void roe_flux_fast_r(const RoeKR<R> &K, const R *L, c
   // eigenvalues with the entropy floor
   const R du = ur - ul;
   const R eeps = half * pos_(du);
-  const R elpf = -maxp_(fabs(ub + cfast), eeps), elmf = -maxp_(fabs(ub - cfast), eeps);
-  const R elps = -maxp_(fabs(ub + cslow), eeps), elms = -maxp_(fabs(ub - cslow), eeps);
-  const R elpa = -maxp_(fabs(ub + ca), eeps), elma = -maxp_(fabs(ub - ca), eeps);
-  const R elze = -maxp_(fabs(ub), eeps);
+  const R elpf = -maxp_(abs_(ub + cfast), eeps), elmf = -maxp_(abs_(ub - cfast), eeps);
+  const R elps = -maxp_(abs_(ub + cslow), eeps), elms = -maxp_(abs_(ub - cslow), eeps);
+  const R elpa = -maxp_(abs_(ub + ca), eeps), elma = -maxp_(abs_(ub - ca), eeps);
+  const R elze = -maxp_(abs_(ub), eeps);
   // wave amplitudes.  With s = sign(bx), sq4r = sqrt(4 pi / rhobar),
   // sqr4 = 1 / sq4r: p11 = P11 sq4r, p12 = P12 sq4r, q21 = -s A, q22 = s B, so
   // the common factors cancel between the numerators and the determinants

@@ -133,3 +133,49 @@ extern "C" int cans_probe_isum(const double *x, double *y, int *f, int n) {
   cudaFree(d);
   return e == cudaSuccess ? 0 : 2;
 }
+
+namespace {
+// z = x + y by isum::add2; f = 1 where it must be formed in FP64
+__global__ void k_add2(const double *x, const double *y, double *z, int *f, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  bool sp = false;
+  z[i] = cans::isum::add2(x[i], y[i], sp);
+  f[i] = sp ? 1 : 0;
+}
+// the face states of cells x[4i .. 4i+3]: y[2i], y[2i+1]
+__global__ void k_muscl(const double *x, double *y, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n)
+    cans::isum::muscl(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3], y[2 * i], y[2 * i + 1]);
+}
+}  // namespace
+
+// Host arrays of n values each.  Synchronous; 0 on success.
+extern "C" int cans_probe_add2(const double *x, const double *y, double *z, int *f, int n) {
+  if (n < 1 || !x || !y || !z || !f) return 1;
+  double *d = nullptr;
+  const size_t b = sizeof(double) * (size_t)n;
+  if (cudaMalloc(&d, 4 * b) != cudaSuccess) return 2;
+  int *df = reinterpret_cast<int *>(d + 3 * (size_t)n);
+  cudaMemcpy(d, x, b, cudaMemcpyHostToDevice);
+  cudaMemcpy(d + n, y, b, cudaMemcpyHostToDevice);
+  k_add2<<<(n + 255) / 256, 256>>>(d, d + n, d + 2 * (size_t)n, df, n);
+  cudaMemcpy(z, d + 2 * (size_t)n, b, cudaMemcpyDeviceToHost);
+  const cudaError_t e = cudaMemcpy(f, df, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e == cudaSuccess ? 0 : 2;
+}
+
+// Host arrays of 4 n and 2 n values.  Synchronous; 0 on success.
+extern "C" int cans_probe_muscl(const double *x, double *y, int n) {
+  if (n < 1 || !x || !y) return 1;
+  double *d = nullptr;
+  const size_t b = sizeof(double) * (size_t)n;
+  if (cudaMalloc(&d, 6 * b) != cudaSuccess) return 2;
+  cudaMemcpy(d, x, 4 * b, cudaMemcpyHostToDevice);
+  k_muscl<<<(n + 255) / 256, 256>>>(d, d + 4 * (size_t)n, n);
+  const cudaError_t e = cudaMemcpy(y, d + 4 * (size_t)n, 2 * b, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e == cudaSuccess ? 0 : 2;
+}
