@@ -126,117 +126,71 @@ __device__ __forceinline__ void prim_forward(const R *u, const PhysR<R> &ph, R *
   p[P_BZ] = u[C_BZ];
 }
 
-// Transpose of (1): given the adjoints aU, aX, aY of U, FX, FY at the point
-// p, add (d(U,FX,FY)/dP)^T (aU, aX, aY) to ap.
-template <class R>
-__device__ __forceinline__ void cell_reverse(const R *p, const PhysR<R> &ph, const R *aU,
-                                             const R *aX, const R *aY, R *ap) {
+// Transpose of (1): given the adjoints of U, FX, FY at the point p, read from aU, aX,
+// aY with stride kT (HASU: of U too), return ap = (d(U,FX,FY)/dP)^T of them.  The sums
+// over the terms are factored: the derivatives of the mass and momentum fluxes share
+// sx = d(FX)/d(rho vx), sy and q = d(..)/d(rho v^2 / 2), 70 products where one term
+// after the other takes 150.
+template <class R, bool HASU>
+__device__ __forceinline__ void cell_reverse(const R *p, const PhysR<R> &ph, const double *aU,
+                                             const double *aX, const double *aY, R *ap) {
   const R ro = p[P_RO], pr = p[P_PR], vx = p[P_VX], vy = p[P_VY], vz = p[P_VZ];
   const R bx = p[P_BX], by = p[P_BY], bz = p[P_BZ];
-  const R vv = vx * vx + vy * vy + vz * vz;
-  const R ex = -vy * bz + vz * by, ey = -vz * bx + vx * bz, ez = -vx * by + vy * bx;
-  const R ep = pr * ph.ggm1 + 0.5f * ro * vv;
-  const R p4 = ph.pi4i, p8 = ph.pi8i;
-  R aro(0.0f), apr(0.0f), avx(0.0f), avy(0.0f), avz(0.0f), abx(0.0f), aby(0.0f),
-      abz(0.0f);
-  R aep(0.0f), aex(0.0f), aey(0.0f), aez(0.0f), avv(0.0f), abb(0.0f);
-  // U
-  aro += aU[C_RO];
-  apr += aU[C_EE] * ph.gm1i;
-  aro += aU[C_EE] * 0.5f * vv;
-  avv += aU[C_EE] * 0.5f * ro;
-  abb += aU[C_EE] * p8;
-  aro += aU[C_RX] * vx + aU[C_RY] * vy + aU[C_RZ] * vz;
-  avx += aU[C_RX] * ro;
-  avy += aU[C_RY] * ro;
-  avz += aU[C_RZ] * ro;
-  abx += aU[C_BX];
-  aby += aU[C_BY];
-  abz += aU[C_BZ];
-  // FX
-  aro += aX[C_RO] * vx;
-  avx += aX[C_RO] * ro;
-  aep += aX[C_EE] * vx;
-  avx += aX[C_EE] * ep;
-  abz += aX[C_EE] * p4 * ey;
-  aey += aX[C_EE] * p4 * bz;
-  aby -= aX[C_EE] * p4 * ez;
-  aez -= aX[C_EE] * p4 * by;
-  aro += aX[C_RX] * vx * vx;
-  avx += aX[C_RX] * 2.0f * ro * vx;
-  apr += aX[C_RX];
-  aby += aX[C_RX] * p8 * 2.0f * by;
-  abz += aX[C_RX] * p8 * 2.0f * bz;
-  abx -= aX[C_RX] * p8 * 2.0f * bx;
-  aro += aX[C_RY] * vy * vx;
-  avy += aX[C_RY] * ro * vx;
-  avx += aX[C_RY] * ro * vy;
-  aby -= aX[C_RY] * p4 * bx;
-  abx -= aX[C_RY] * p4 * by;
-  aro += aX[C_RZ] * vz * vx;
-  avz += aX[C_RZ] * ro * vx;
-  avx += aX[C_RZ] * ro * vz;
-  abz -= aX[C_RZ] * p4 * bx;
-  abx -= aX[C_RZ] * p4 * bz;
-  aez -= aX[C_BY];
-  aey += aX[C_BZ];
-  // FY
-  aro += aY[C_RO] * vy;
-  avy += aY[C_RO] * ro;
-  aep += aY[C_EE] * vy;
-  avy += aY[C_EE] * ep;
-  abx += aY[C_EE] * p4 * ez;
-  aez += aY[C_EE] * p4 * bx;
-  abz -= aY[C_EE] * p4 * ex;
-  aex -= aY[C_EE] * p4 * bz;
-  aro += aY[C_RX] * vx * vy;
-  avx += aY[C_RX] * ro * vy;
-  avy += aY[C_RX] * ro * vx;
-  abx -= aY[C_RX] * p4 * by;
-  aby -= aY[C_RX] * p4 * bx;
-  aro += aY[C_RY] * vy * vy;
-  avy += aY[C_RY] * 2.0f * ro * vy;
-  apr += aY[C_RY];
-  abx += aY[C_RY] * p8 * 2.0f * bx;
-  abz += aY[C_RY] * p8 * 2.0f * bz;
-  aby -= aY[C_RY] * p8 * 2.0f * by;
-  aro += aY[C_RZ] * vz * vy;
-  avz += aY[C_RZ] * ro * vy;
-  avy += aY[C_RZ] * ro * vz;
-  abz -= aY[C_RZ] * p4 * by;
-  aby -= aY[C_RZ] * p4 * bz;
-  aez += aY[C_BX];
-  aex -= aY[C_BZ];
-  // ep, E, |v|^2, |B|^2
-  apr += aep * ph.ggm1;
-  aro += aep * 0.5f * vv;
-  avv += aep * 0.5f * ro;
-  avy -= aex * bz;
-  abz -= aex * vy;
-  avz += aex * by;
-  aby += aex * vz;
-  avz -= aey * bx;
-  abx -= aey * vz;
-  avx += aey * bz;
-  abz += aey * vx;
-  avx -= aez * by;
-  aby -= aez * vx;
-  avy += aez * bx;
-  abx += aez * vy;
-  avx += 2.0f * vx * avv;
-  avy += 2.0f * vy * avv;
-  avz += 2.0f * vz * avv;
-  abx += 2.0f * bx * abb;
-  aby += 2.0f * by * abb;
-  abz += 2.0f * bz * abb;
-  ap[P_RO] += aro;
-  ap[P_PR] += apr;
-  ap[P_VX] += avx;
-  ap[P_VY] += avy;
-  ap[P_VZ] += avz;
-  ap[P_BX] += abx;
-  ap[P_BY] += aby;
-  ap[P_BZ] += abz;
+  auto X = [&](int v) { return num_ld<R>(aX + v * kT); };
+  auto Y = [&](int v) { return num_ld<R>(aY + v * kT); };
+  auto U = [&](int v) { return num_ld<R>(aU + v * kT); };
+  const R vv = fma(vx, vx, fma(vy, vy, vz * vz));
+  const R ex = fma(vz, by, -(vy * bz)), ey = fma(vx, bz, -(vz * bx)), ez = fma(vy, bx, -(vx * by));
+  const R ep = fma(pr, ph.ggm1, 0.5f * ro * vv);
+  const R xe = X(C_EE), ye = Y(C_EE), tx = xe * ph.pi4i, ty = ye * ph.pi4i;
+  const R xx = X(C_RX), xy = X(C_RY), xz = X(C_RZ), yx = Y(C_RX), yy = Y(C_RY), yz = Y(C_RZ);
+  // adjoints of ep and E, and of rho v^2 / 2
+  const R aep = fma(xe, vx, ye * vy);
+  const R aex = -(fma(ty, bz, Y(C_BZ))), aey = fma(tx, bz, X(C_BZ));
+  const R aez = fma(ty, bx, Y(C_BX)) - fma(tx, by, X(C_BY));
+  R q = aep, db = yy - xx, mx, my, mz;
+  if constexpr (HASU) q = q + U(C_EE);
+  const R sx = fma(xx, vx, fma(xy, vy, fma(xz, vz, X(C_RO))));
+  const R sy = fma(yx, vx, fma(yy, vy, fma(yz, vz, Y(C_RO))));
+  mx = fma(xx, vx, fma(yx, vy, fma(vx, q, sx)));
+  my = fma(xy, vx, fma(yy, vy, fma(vy, q, sy)));
+  mz = fma(xz, vx, fma(yz, vy, vz * q));
+  R aro = fma(vx, sx, fma(vy, sy, 0.5f * vv * q));
+  R apr = fma(aep, ph.ggm1, xx + yy);
+  const R p82 = 2.0f * ph.pi8i;
+  // of pi8i times the squares of bx, by, bz
+  R qx = db, qy = -db, qz = xx + yy;
+  R abx, aby, abz;
+  if constexpr (HASU) {
+    const R ue = U(C_EE), ux = U(C_RX), uy = U(C_RY), uz = U(C_RZ);
+    mx = mx + ux;
+    my = my + uy;
+    mz = mz + uz;
+    aro = aro + fma(ux, vx, fma(uy, vy, fma(uz, vz, U(C_RO))));
+    apr = fma(ue, ph.gm1i, apr);
+    qx = qx + ue;
+    qy = qy + ue;
+    qz = qz + ue;
+    abx = fma(p82 * bx, qx, U(C_BX));
+    aby = fma(p82 * by, qy, U(C_BY));
+    abz = fma(p82 * bz, qz, U(C_BZ));
+  } else {
+    abx = p82 * bx * qx;
+    aby = p82 * by * qy;
+    abz = p82 * bz * qz;
+  }
+  const R xyx = xy + yx;
+  abx = fma(-ph.pi4i, fma(xyx, by, xz * bz), abx);
+  aby = fma(-ph.pi4i, fma(xyx, bx, yz * bz), aby);
+  abz = fma(-ph.pi4i, fma(xz, bx, yz * by), abz);
+  ap[P_RO] = aro;
+  ap[P_PR] = apr;
+  ap[P_VX] = fma(ro, mx, fma(xe, ep, fma(aey, bz, -(aez * by))));
+  ap[P_VY] = fma(ro, my, fma(ye, ep, fma(aez, bx, -(aex * bz))));
+  ap[P_VZ] = fma(ro, mz, fma(aex, by, -(aey * bx)));
+  ap[P_BX] = fma(ty, ez, fma(aez, vy, fma(-aey, vz, abx)));
+  ap[P_BY] = fma(-tx, ez, fma(aex, vz, fma(-aez, vx, aby)));
+  ap[P_BZ] = fma(tx, ey, fma(-ty, ex, fma(aey, vx, fma(-aex, vy, abz))));
 }
 
 // Transpose of prim_forward at the point whose primitives are p: given ap,
@@ -309,6 +263,8 @@ __global__ void __launch_bounds__(kT, kMinBlocks)
                   double dt_) {
   const size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (c >= g.n) return;
+  __shared__ double sm[2 * 8 * kT];
+  double *sX = sm + threadIdx.x, *sY = sX + 8 * kT;
   const PhysR<R> ph = phys_r<R>(ph_);
   const R dt = num_in<R>(dt_);
   const int p = (int)(c % g.ix), q = (int)(c / g.ix);
@@ -317,46 +273,53 @@ __global__ void __launch_bounds__(kT, kMinBlocks)
   for (int v = 0; v < 8; v++) out[v] = R(0.0f);
   if (p <= g.ix - 2 && q <= g.jx - 2) {
     const size_t c00 = c, c10 = c + 1, c01 = c + g.ix, c11 = c + g.ix + 1;
+    // The eight variables in rolled loops, their results in shared memory: unrolled,
+    // the kernels outgrow the instruction cache (gather, 256^2: half of the stalled
+    // cycles; 47.8 -> 31.8 us with the shorter cell_reverse, corners 24.4 -> 20.3).
     // forward corner state (mlwhalf.f part 2)
-    const R hdxim = 0.5f * num_in<R>(ax.dim[p]), hdyim = 0.5f * num_in<R>(ay.dim[q]);
-    R uh[8];
-#pragma unroll
+    const R cx = -(0.5f * dt * num_in<R>(ax.dim[p])), cy = -(0.5f * dt * num_in<R>(ay.dim[q]));
+#pragma unroll 1
     for (int v = 0; v < 8; v++) {
       const double *U = CU + v * g.n, *FX = CU + (8 + v) * g.n, *FY = CU + (16 + v) * g.n;
-      const R avg = 0.25f * (num_ld<R>(U + c10) + num_ld<R>(U + c00) + num_ld<R>(U + c11) +
-                             num_ld<R>(U + c01));
-      const R dfdx = hdxim * (num_ld<R>(FX + c10) - num_ld<R>(FX + c00) +
-                              num_ld<R>(FX + c11) - num_ld<R>(FX + c01));
-      const R dfdy = hdyim * (num_ld<R>(FY + c01) - num_ld<R>(FY + c00) +
-                              num_ld<R>(FY + c11) - num_ld<R>(FY + c10));
-      uh[v] = avg - dt * dfdx - dt * dfdy;
+      const R s = (num_ld<R>(U + c10) + num_ld<R>(U + c00)) +
+                  (num_ld<R>(U + c11) + num_ld<R>(U + c01));
+      const R dx = (num_ld<R>(FX + c10) - num_ld<R>(FX + c00)) +
+                   (num_ld<R>(FX + c11) - num_ld<R>(FX + c01));
+      const R dy = (num_ld<R>(FY + c01) - num_ld<R>(FY + c00)) +
+                   (num_ld<R>(FY + c11) - num_ld<R>(FY + c10));
+      num_st(sX + v * kT, fma(cy, dy, fma(cx, dx, 0.25f * s)));
     }
     R ph8[8];
-    prim_forward(uh, ph, ph8);
+    {
+      R uh[8];
+#pragma unroll
+      for (int v = 0; v < 8; v++) uh[v] = num_ld<R>(sX + v * kT);
+      prim_forward(uh, ph, ph8);
+    }
     // adjoint of GX, GY at this corner: the cells (p,q), (p+1,q), (p,q+1),
-    // (p+1,q+1) that read it in mlwfull (0-based cell indices)
+    // (p+1,q+1) that read it in mlwfull (0-based cell indices); 0 for those the step
+    // does not update
+    const R zero(0.0f);
     const bool i00 = interior(g, p, q), i10 = interior(g, p + 1, q),
                i01 = interior(g, p, q + 1), i11 = interior(g, p + 1, q + 1);
     const R hx0 = 0.5f * dt * num_in<R>(ax.di[p]), hx1 = 0.5f * dt * num_in<R>(ax.di[p + 1]);
     const R hy0 = 0.5f * dt * num_in<R>(ay.di[q]), hy1 = 0.5f * dt * num_in<R>(ay.di[q + 1]);
     const R uy1q = num_in<R>(ay.u1[q]), uy0q1 = num_in<R>(ay.u0[q + 1]);
     const R ux1p = num_in<R>(ax.u1[p]), ux0p1 = num_in<R>(ax.u0[p + 1]);
-    R aX[8], aY[8];
-#pragma unroll
-    for (int v = 0; v < 8; v++) {
+    const R x00 = i00 ? -(hx0 * uy1q) : zero, x10 = i10 ? hx1 * uy1q : zero;
+    const R x01 = i01 ? -(hx0 * uy0q1) : zero, x11 = i11 ? hx1 * uy0q1 : zero;
+    const R y00 = i00 ? -(hy0 * ux1p) : zero, y10 = i10 ? -(hy0 * ux0p1) : zero;
+    const R y01 = i01 ? hy1 * ux1p : zero, y11 = i11 ? hy1 * ux0p1 : zero;
+#pragma unroll 1
+    for (int v = 0; v < 8; v++) {  // A1 is 0 outside the interior
       const double *a = A1 + v * g.n;
-      const R l00 = i00 ? num_ld<R>(a + c00) : R(0.0f), l10 = i10 ? num_ld<R>(a + c10) : R(0.0f);
-      const R l01 = i01 ? num_ld<R>(a + c01) : R(0.0f), l11 = i11 ? num_ld<R>(a + c11) : R(0.0f);
-      aX[v] = -hx0 * uy1q * l00 + hx1 * uy1q * l10 - hx0 * uy0q1 * l01 + hx1 * uy0q1 * l11;
-      aY[v] = -hy0 * ux1p * l00 - hy0 * ux0p1 * l10 + hy1 * ux1p * l01 + hy1 * ux0p1 * l11;
+      const R l00 = num_ld<R>(a + c00), l10 = num_ld<R>(a + c10);
+      const R l01 = num_ld<R>(a + c01), l11 = num_ld<R>(a + c11);
+      num_st(sX + v * kT, fma(x00, l00, fma(x10, l10, fma(x01, l01, x11 * l11))));
+      num_st(sY + v * kT, fma(y00, l00, fma(y10, l10, fma(y01, l01, y11 * l11))));
     }
-    R aP[8], zero8[8];
-#pragma unroll
-    for (int v = 0; v < 8; v++) {
-      aP[v] = R(0.0f);
-      zero8[v] = R(0.0f);
-    }
-    cell_reverse(ph8, ph, zero8, aX, aY, aP);
+    R aP[8];
+    cell_reverse<R, false>(ph8, ph, nullptr, sX, sY, aP);
     prim_reverse(ph8, ph, aP, out);
   }
 #pragma unroll
@@ -372,6 +335,8 @@ __global__ void __launch_bounds__(kT, kMinBlocks)
                  Axis ax, Axis ay, Phys ph_, double dt_) {
   const size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (c >= g.n) return;
+  __shared__ double sm[3 * 8 * kT];
+  double *sU = sm + threadIdx.x, *sX = sU + 8 * kT, *sY = sX + 8 * kT;
   const PhysR<R> ph = phys_r<R>(ph_);
   const R dt = num_in<R>(dt_);
   const int i = (int)(c % g.ix), j = (int)(c / g.ix);
@@ -458,9 +423,8 @@ __global__ void __launch_bounds__(kT, kMinBlocks)
   const R wym_b = (in_c && j >= 1) ? dt * dim_ym * di_y : zero;
   const R wyp_a = in_c ? dt * dim_y * di_y : zero;
   const R wyp_b = in_yp ? dt * dim_y * di_yp : zero;
-  R aU[8], aX[8], aY[8];
   R aqxm = zero, aqxp = zero, aqym = zero, aqyp = zero;
-#pragma unroll
+#pragma unroll 1
   for (int v = 0; v < 8; v++) {
     const double *a = A1 + v * n, *h = A2 + v * n;
     const R l0 = in_c ? num_ld<R>(a + c) : zero;
@@ -471,23 +435,25 @@ __global__ void __launch_bounds__(kT, kMinBlocks)
     const R ylo = hmm + hpm, yhi = hmp + hpp;  // corners below / above
     // U' = U + du on the interior; 0.25 of each surrounding corner
     R au = fma(R(0.25f), ylo + yhi, l0);
-    if (av) au += cxm * lxm + cxp * lxp + cym * lym + cyp * lyp - c0 * l0;
-    aU[v] = au;
-    aX[v] = hxp * lxp - hxm * lxm + pxp * (hpm + hpp) - pxm * (hmm + hmp);
-    aY[v] = hyp * lyp - hym * lym + pyp * yhi - pym * ylo;
+    if (av) au = fma(cxm, lxm, fma(cxp, lxp, fma(cym, lym, fma(cyp, lyp, fma(-c0, l0, au)))));
+    num_st(sU + v * kT, au);
+    num_st(sX + v * kT, fma(hxp, lxp, fma(-hxm, lxm, fma(pxp, hpm + hpp, -(pxm * (hmm + hmp))))));
+    num_st(sY + v * kT, fma(hyp, lyp, fma(-hym, lym, fma(pyp, yhi, -(pym * ylo)))));
     if (av) {
       const double *U = CU + v * n;
       const R u0 = num_ld<R>(U + c);
-      if (aqxm_on) aqxm += (u0 - num_ld<R>(U + c - sx)) * (wxm_a * lxm - wxm_b * l0);
-      if (aqxp_on) aqxp += (num_ld<R>(U + c + sx) - u0) * (wxp_a * l0 - wxp_b * lxp);
-      if (aqym_on) aqym += (u0 - num_ld<R>(U + c - sy)) * (wym_a * lym - wym_b * l0);
-      if (aqyp_on) aqyp += (num_ld<R>(U + c + sy) - u0) * (wyp_a * l0 - wyp_b * lyp);
+      if (aqxm_on)
+        aqxm = fma(u0 - num_ld<R>(U + c - sx), fma(wxm_a, lxm, -(wxm_b * l0)), aqxm);
+      if (aqxp_on)
+        aqxp = fma(num_ld<R>(U + c + sx) - u0, fma(wxp_a, l0, -(wxp_b * lxp)), aqxp);
+      if (aqym_on)
+        aqym = fma(u0 - num_ld<R>(U + c - sy), fma(wym_a, lym, -(wym_b * l0)), aqym);
+      if (aqyp_on)
+        aqyp = fma(num_ld<R>(U + c + sy) - u0, fma(wyp_a, l0, -(wyp_b * lyp)), aqyp);
     }
   }
   R ap[8];
-#pragma unroll
-  for (int v = 0; v < 8; v++) ap[v] = zero;
-  cell_reverse(p, ph, aU, aX, aY, ap);
+  cell_reverse<R, true>(p, ph, sU, sX, sY, ap);
   // q(face) = qav dxm max(0, |v(+) - v(-)| - eps): the cell is (+) of the
   // lower face and (-) of the upper face
   ap[P_VX] += aqxm * gxm - aqxp * gxp;

@@ -822,6 +822,26 @@ inline int balance_seg(int strips, int rows, int ch, int sms) {
   }
   return best;
 }
+// The same for the FP64 step, two of whose blocks fit an SM.  A block alone leaves
+// the pipes to its own latencies, a second one beside it fills them: the cost is that
+// of pairs and of the odd block, in units of a fifth of a microsecond, fitted to the
+// kernel at 64^2 .. 512^2 (a block of 3, 4, 7, 14, 32 rows alone on its SM 26, 27,
+// 36, 56, 113 us; two of 7, 27 rows 49, 146 us).
+inline int balance_seg_pairs(int strips, int rows, int ch, int sms) {
+  int best = rows;
+  long long best_cost = -1;
+  for (int seg = 1; seg <= rows; seg++) {
+    const long long blocks = (long long)strips * ((rows + seg - 1) / seg);
+    const long long per_sm = (blocks + sms - 1) / sms, chunks = (seg + ch - 1) / ch;
+    const long long cost =
+        per_sm / 2 * (80 + 40 * chunks + 18 * seg) + per_sm % 2 * (75 + 25 * chunks + 11 * seg);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best = seg;
+    }
+  }
+  return best;
+}
 // The same with whole chunks per block, balanced by waves of resident
 // blocks (slots = SMs x resident blocks per SM): for a step that is bound by
 // latency more than by one pipe, fewer and longer blocks can win.
@@ -870,7 +890,8 @@ cudaError_t launch_march_u(const MarchArgs &m, const Axis &ax, const Axis &ay, c
   }
   const int strips = (m.ix - 2 + T::TX - 1) / T::TX, rows = m.jx - 2;
   const int seg = waves ? balance_seg_waves(strips, rows, CH, slots)
-                        : balance_seg(strips, rows, CH, sms);
+                  : std::is_same<N, F64N>::value ? balance_seg_pairs(strips, rows, CH, sms)
+                                                 : balance_seg(strips, rows, CH, sms);
   const dim3 grid(strips, (rows + seg - 1) / seg);
   kern<<<grid, T::NT, T::smem_bytes, s>>>(m, ax, ay, ph, ctl, seg);
   count_launch();
