@@ -106,6 +106,37 @@ __device__ __forceinline__ D rcp(D y) {
   return fast_two_sum(r, __fmul_rn(r, e));
 }
 
+// Sums of several values: exact two-sums of the heads in a tree, the tails and the
+// errors added up beside them, one normalisation.  The error terms are those of a
+// chain of add, of order u^2 of the largest operand each.
+__device__ __forceinline__ float fadd3(float a, float b, float c) {
+  return __fadd_rn(__fadd_rn(a, b), c);
+}
+// a + b + c + d, not normalised
+__device__ __forceinline__ D raw4(D a, D b, D c, D d) {
+  const D p = two_sum(a.h, b.h), q = two_sum(c.h, d.h), s = two_sum(p.h, q.h);
+  return {s.h, __fadd_rn(__fadd_rn(__fadd_rn(a.l, b.l), __fadd_rn(c.l, d.l)),
+                         fadd3(p.l, q.l, s.l))};
+}
+__device__ __forceinline__ D norm2(D a, D b) {  // a + b of such sums
+  const D s = two_sum(a.h, b.h);
+  return fast_two_sum(s.h, fadd3(a.l, b.l, s.l));
+}
+__device__ __forceinline__ D add4(D a, D b, D c, D d) {
+  const D s = raw4(a, b, c, d);
+  return fast_two_sum(s.h, s.l);
+}
+// (b - a) (1 + e0) + (d - c) (1 + e1) + 4 (g - f) for small e0, e1 (2^-36)
+__device__ __forceinline__ D diff6(D a, D b, D c, D d, D f, D g, float e0, float e1) {
+  const D p = two_sum(b.h, -a.h), q = two_sum(d.h, -c.h);
+  const D r = two_sum(__fmul_rn(4.0f, g.h), __fmul_rn(-4.0f, f.h));
+  const D s = two_sum(p.h, q.h), t = two_sum(s.h, r.h);
+  const float k = __fmaf_rn(p.h, e0, __fmul_rn(q.h, e1));
+  const float l = __fmaf_rn(4.0f, __fsub_rn(g.l, f.l),
+                            __fadd_rn(__fsub_rn(b.l, a.l), __fsub_rn(d.l, c.l)));
+  return fast_two_sum(t.h, __fadd_rn(__fadd_rn(l, fadd3(p.l, q.l, k)), fadd3(r.l, s.l, t.l)));
+}
+
 // sign tests of a normalised value: its head carries the sign (or is 0 with
 // a zero tail)
 __device__ __forceinline__ bool pos(D x) { return x.h > 0.0f; }

@@ -16,9 +16,10 @@
 // 34 CH threads (whole warps): one per cell of the new rows, per corner, and per
 // updated cell (32 CH of them).
 //
-// The FP64 step is bound by the FP64 pipe (85 to 88 % busy, HBM at 2 %): a warp
-// instruction of it takes 64 issue slots, of which the step uses 9 %.  So the
-// algebra is arranged for the fewest FP64 instructions:
+// The FP64 step is bound by the FP64 pipe (71 % busy at 512^2, 88 % at most; HBM at
+// 3 %) and by the latency of the integer sums that relieve it: an FP64 warp
+// instruction takes 64 issue slots, of which the step uses 30 %.  So the algebra is
+// arranged for the fewest FP64 instructions, 219 a cell:
 //   - the momentum flux is symmetric (fx(ry) = fy(rx)), the total pressure formed
 //     once, the corner mass fluxes are the half-step momenta;
 //   - the corner values are kept at four times their value (the mean of u is a
@@ -27,10 +28,16 @@
 //   - a field needed as a sum and a difference, or as both differences, shares
 //     its partial sums;
 //   - viscosity as one linear combination of five values;
+//   - the predictor's cell sums and, on equally spaced axes, the corner and central
+//     differences of a direction are integer sums (isum.cuh);
 //   - what depends on the column alone is formed once per block;
 //   - reciprocals of fd64.cuh; comparisons on the integer pipe.
 // u_new = u + du, the terms of du summed first; ro and B, which are state
 // variables, are added to in FP64 in both policies.
+//
+// The double-float step takes the same sums with one normalisation each (df64.cuh) and
+// its eight variables in a rolled loop.  Measured at 512^2, a step: FP64 217 (a tile
+// that recomputes its halo) -> 145 us, double-float 98 -> 88 us.
 //
 // AVF records (1) or holds (2) the viscosity's branch of every face: see
 // mlw2d_tile.cuh.
@@ -95,6 +102,11 @@ struct DFN {
                                            V u) {
     return mad(as, sub(us, u), mad(an, sub(un, u), mad(aw, sub(uw, u), mul(ae, sub(ue, u)))));
   }
+  static __device__ __forceinline__ V add4(V a, V b, V c, V d) { return df::add4(a, b, c, d); }
+  static __device__ __forceinline__ V diff6(V a, V b, V c, V d, V f, V g, float e0, float e1,
+                                            bool &) {
+    return df::diff6(a, b, c, d, f, g, __fmul_rn(e0, 0x1p-32f), __fmul_rn(e1, 0x1p-32f));
+  }
   static __device__ __forceinline__ V rcp(V a) { return df::rcp(a); }
   static __device__ __forceinline__ V addf(V a, float b) { return df::addf(a, b); }
   static __device__ __forceinline__ V absd(V a) { return df::absd(a); }
@@ -119,6 +131,11 @@ struct F64N {
   static __device__ __forceinline__ V visc(V ae, V ue, V aw, V uw, V an, V un, V as, V us, V aa,
                                            V u) {
     return fma(as, us, fma(an, un, fma(aw, uw, fma(ae, ue, aa * u))));
+  }
+  static __device__ __forceinline__ V add4(V a, V b, V c, V d) { return (a + b) + (c + d); }
+  static __device__ __forceinline__ V diff6(V a, V b, V c, V d, V f, V g, float e0, float e1,
+                                            bool &sp) {
+    return isum::diff6(a, b, c, d, f, g, e0, e1, sp);
   }
   static __device__ __forceinline__ V rcp(V a) { return fd::rcp(a); }
   static __device__ __forceinline__ V addf(V a, float b) { return a + (double)b; }
@@ -265,17 +282,17 @@ template <class N, class T> struct Cells4 {
   __device__ __forceinline__ V sum(int f) {
     V a, b, c, d;
     load(f, a, b, c, d);
-    return N::add(N::add(b, a), N::add(c, d));
+    return N::add4(b, a, c, d);
   }
   __device__ __forceinline__ V dx(int f) {
     V a, b, c, d;
     load(f, a, b, c, d);
-    return N::add(N::sub(b, a), N::sub(c, d));
+    return N::add4(b, N::neg(a), c, N::neg(d));
   }
   __device__ __forceinline__ V dy(int f) {
     V a, b, c, d;
     load(f, a, b, c, d);
-    return N::add(N::sub(d, a), N::sub(c, b));
+    return N::add4(d, N::neg(a), c, N::neg(b));
   }
   __device__ __forceinline__ void sum_dx(int f, V &s, V &x) {
     V a, b, c, d;
@@ -472,13 +489,25 @@ __device__ __forceinline__ typename N::V march_to_cell(const typename N::V *sk, 
   return N::mad(uy1, t, N::mul(uy0, s));
 }
 
+// The fields of march_du's variables, in the order of du: conserved slot, x flux at the
+// cells and corners and whether it enters negated, y flux, gravity source.
+struct VarFields2 {
+  signed char su, fx, nx, kfx, fy, ny, kfy, gs;
+};
+__constant__ VarFields2 kVar2[8] = {
+    {CRO, CRX, 0, KRX, CRY, 0, KRY, -1}, {CEE, CFX, 0, KFX, CFY, 0, KFY, 0},
+    {CRX, CXX, 0, KXX, CXY, 0, KXY, 1},  {CRY, CXY, 0, KXY, CYY, 0, KYY, 2},
+    {CBX, NOF, 0, NOF, CEZ, 0, KEZ, -1}, {CBY, CEZ, 1, KEZ, NOF, 0, NOF, -1},
+    {CRZ, CXZ, 0, KXZ, CYZ, 0, KYZ, -1}, {CBZ, CEY, 0, KEY, CEX, 1, KEX, -1}};
+
 // The changes of the conserved variables of cell c (ro, ee, rx, ry, bx, by, rz,
 // bz): viscosity, central differences, corrector, gravity sources.  ae .. as are dt
 // q / (dx dxm) of the four faces, dtx = dt / dx, dty = dt / dy.
 //
 // U: the weights u0, u1 are one half up to ex0 .. ey1 (Axis::e0, e1), and the two
 // corner differences and the central difference of a direction are one integer
-// sum (isum::diff6): one FP64 instruction a direction where six are needed.
+// sum (isum::diff6): one FP64 instruction a direction where six are needed; in
+// double-float one sum (df::diff6) and one product.
 // sp is set where such a sum must be formed in FP64.
 template <class N, class T, bool M3, bool G, bool U>
 __device__ __forceinline__ void march_du(const typename N::V *sc, const typename N::V *sk, int c,
@@ -505,13 +534,13 @@ __device__ __forceinline__ void march_du(const typename N::V *sc, const typename
     if constexpr (U) {
       // fx0 (SE - SW) + fx1 (NE - NW) + fcx (E - W) = dtx/16 diff6
       if (fx != NOF) {
-        const double q = isum::diff6(SK(kfx, kSW), SK(kfx, kSE), SK(kfx, kNW), SK(kfx, kNE),
-                                     SC(fx, cW), SC(fx, cE), ey0, ey1, sp);
+        const V q = N::diff6(SK(kfx, kSW), SK(kfx, kSE), SK(kfx, kNW), SK(kfx, kNE),
+                             SC(fx, cW), SC(fx, cE), ey0, ey1, sp);
         d = N::mad(nx ? dtx16 : N::neg(dtx16), q, d);
       }
       if (fy != NOF) {
-        const double q = isum::diff6(SK(kfy, kSW), SK(kfy, kNW), SK(kfy, kSE), SK(kfy, kNE),
-                                     SC(fy, cS), SC(fy, cN), ex0, ex1, sp);
+        const V q = N::diff6(SK(kfy, kSW), SK(kfy, kNW), SK(kfy, kSE), SK(kfy, kNE),
+                             SC(fy, cS), SC(fy, cN), ex0, ex1, sp);
         d = N::mad(ny ? dty16 : N::neg(dty16), q, d);
       }
     } else {
@@ -535,14 +564,27 @@ __device__ __forceinline__ void march_du(const typename N::V *sc, const typename
     }
     return d;
   };
-  du[0] = var(CRO, CRX, false, KRX, CRY, false, KRY);
-  du[4] = var(CBX, NOF, false, NOF, CEZ, false, KEZ);
-  du[5] = var(CBY, CEZ, true, KEZ, NOF, false, NOF);
-  if constexpr (M3) du[7] = var(CBZ, CEY, false, KEY, CEX, true, KEX);
-  du[1] = var(CEE, CFX, false, KFX, CFY, false, KFY, 0);
-  du[2] = var(CRX, CXX, false, KXX, CXY, false, KXY, 1);
-  du[3] = var(CRY, CXY, false, KXY, CYY, false, KYY, 2);
-  if constexpr (M3) du[6] = var(CRZ, CXZ, false, KXZ, CYZ, false, KYZ);
+  if constexpr (std::is_same<N, DFN>::value) {
+    // rolled: unrolled, the step outgrows the instruction cache (a sixth of the stalled
+    // cycles at 512^2); FP64's sums are fewer instructions
+#pragma unroll 1
+    for (int v = 0; v < (M3 ? 8 : 6); v++) {
+      const VarFields2 q = kVar2[v];
+      const V d = var(q.su, q.fx, q.nx, q.kfx, q.fy, q.ny, q.kfy, G ? q.gs : -1);
+#pragma unroll
+      for (int k = 0; k < (M3 ? 8 : 6); k++)
+        if (k == v) du[k] = d;
+    }
+  } else {
+    du[0] = var(CRO, CRX, false, KRX, CRY, false, KRY);
+    du[4] = var(CBX, NOF, false, NOF, CEZ, false, KEZ);
+    du[5] = var(CBY, CEZ, true, KEZ, NOF, false, NOF);
+    if constexpr (M3) du[7] = var(CBZ, CEY, false, KEY, CEX, true, KEX);
+    du[1] = var(CEE, CFX, false, KFX, CFY, false, KFY, 0);
+    du[2] = var(CRX, CXX, false, KXX, CXY, false, KXY, 1);
+    du[3] = var(CRY, CXY, false, KXY, CYY, false, KYY, 2);
+    if constexpr (M3) du[6] = var(CRZ, CXZ, false, KXZ, CYZ, false, KYZ);
+  }
 #undef SC
 #undef SK
 }
@@ -689,12 +731,14 @@ __device__ __forceinline__ void march_block(const MarchArgs &m, const Axis &ax, 
         bool sp = false;
         march_du<N, T, M3, G, true>(sc, sk, c, kSW, ae, aw, an, as, dtx, dty, dt, ux0, ux1, uy0,
                                     uy1, ax.e0[gi], ax.e1[gi], ay.e0[gj], ay.e1[gj], du, sp);
-        if (sp) {  // a real branch, as in march_corner
-          double slow[8];
-          march_du_fp64<T, M3, G>(sc, sk, c, kSW, ae, aw, an, as, dtx, dty, dt, ux0, ux1, uy0,
-                                  uy1, slow);
+        if constexpr (std::is_same<N, F64N>::value) {
+          if (sp) {  // a real branch, as in march_corner
+            double slow[8];
+            march_du_fp64<T, M3, G>(sc, sk, c, kSW, ae, aw, an, as, dtx, dty, dt, ux0, ux1, uy0,
+                                    uy1, slow);
 #pragma unroll
-          for (int v = 0; v < (M3 ? 8 : 6); v++) du[v] = slow[v];
+            for (int v = 0; v < (M3 ? 8 : 6); v++) du[v] = slow[v];
+          }
         }
       } else {
         bool sp = false;
@@ -802,32 +846,15 @@ __global__ void __launch_bounds__(March<CH, M3, G>::NT, 2)
                                     min(m.jx - 2, jb + seg - 1), smem_march);
 }
 
-// Rows per block of the marching kernel.  The step is bound by the
-// arithmetic pipes, so a launch takes as long as its busiest SM: the blocks
-// an SM gets (all blocks spread evenly over the SMs) times the rows a block
-// computes -- its segment, the two-row prologue and one row's worth of
-// barriers per chunk.  A segment need not be a whole number of chunks (its
-// last chunk may be short, as at the end of the grid).
+// Rows per block of the marching kernel, two of whose blocks fit an SM: a launch
+// takes as long as its busiest SM.  A block alone leaves the pipes to its own
+// latencies, a second one beside it fills them: the cost is that of pairs and of the
+// odd block, in units of a fifth of a microsecond, fitted to the FP64 step at 64^2 ..
+// 512^2 (a block of 3, 4, 7, 14, 32 rows alone on its SM 26, 27, 36, 56, 113 us; two
+// of 7, 27 rows 49, 146 us).  A segment need not be a whole number of chunks (its
+// last chunk may be short, as at the end of the grid).  Against the blocks an SM gets
+// times their rows: 192^2 48.9 -> 35.0, 256^2 56 -> 49, 384^2 113 -> 98 us a step.
 inline int balance_seg(int strips, int rows, int ch, int sms) {
-  int best = rows;
-  long long best_cost = -1;
-  for (int seg = ch > 1 ? ch / 2 : 1; seg <= rows; seg++) {
-    const long long blocks = (long long)strips * ((rows + seg - 1) / seg);
-    const long long per_sm = (blocks + sms - 1) / sms;
-    const long long cost = per_sm * (seg + 2 + (seg + ch - 1) / ch);
-    if (best_cost < 0 || cost < best_cost) {
-      best_cost = cost;
-      best = seg;
-    }
-  }
-  return best;
-}
-// The same for the FP64 step, two of whose blocks fit an SM.  A block alone leaves
-// the pipes to its own latencies, a second one beside it fills them: the cost is that
-// of pairs and of the odd block, in units of a fifth of a microsecond, fitted to the
-// kernel at 64^2 .. 512^2 (a block of 3, 4, 7, 14, 32 rows alone on its SM 26, 27,
-// 36, 56, 113 us; two of 7, 27 rows 49, 146 us).
-inline int balance_seg_pairs(int strips, int rows, int ch, int sms) {
   int best = rows;
   long long best_cost = -1;
   for (int seg = 1; seg <= rows; seg++) {
@@ -890,8 +917,7 @@ cudaError_t launch_march_u(const MarchArgs &m, const Axis &ax, const Axis &ay, c
   }
   const int strips = (m.ix - 2 + T::TX - 1) / T::TX, rows = m.jx - 2;
   const int seg = waves ? balance_seg_waves(strips, rows, CH, slots)
-                  : std::is_same<N, F64N>::value ? balance_seg_pairs(strips, rows, CH, sms)
-                                                 : balance_seg(strips, rows, CH, sms);
+                        : balance_seg(strips, rows, CH, sms);
   const dim3 grid(strips, (rows + seg - 1) / seg);
   kern<<<grid, T::NT, T::smem_bytes, s>>>(m, ax, ay, ph, ctl, seg);
   count_launch();
@@ -901,10 +927,8 @@ cudaError_t launch_march_u(const MarchArgs &m, const Axis &ax, const Axis &ay, c
 template <class N, int CH, bool M3, bool G, bool R, int AVF = 0>
 cudaError_t launch_march(const MarchArgs &m, const Axis &ax, const Axis &ay, const Phys &ph,
                          Ctl *ctl, cudaStream_t s, bool waves = false) {
-  if constexpr (std::is_same<N, F64N>::value) {
-    if (ax.uniform && ay.uniform)
-      return launch_march_u<N, CH, M3, G, R, AVF, true>(m, ax, ay, ph, ctl, s, waves);
-  }
+  if (ax.uniform && ay.uniform)
+    return launch_march_u<N, CH, M3, G, R, AVF, true>(m, ax, ay, ph, ctl, s, waves);
   return launch_march_u<N, CH, M3, G, R, AVF, false>(m, ax, ay, ph, ctl, s, waves);
 }
 

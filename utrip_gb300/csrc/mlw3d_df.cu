@@ -59,20 +59,6 @@ __device__ __forceinline__ Flux3 fluxes3(D rx, D ry, D rz, D vx, D vy, D vz, D b
   return o;
 }
 
-__device__ __forceinline__ float fadd3(float a, float b, float c) {
-  return __fadd_rn(__fadd_rn(a, b), c);
-}
-// a + b + c + d and a + b + c, not normalised
-__device__ __forceinline__ D raw4(D a, D b, D c, D d) {
-  const D p = df::two_sum(a.h, b.h), q = df::two_sum(c.h, d.h), s = df::two_sum(p.h, q.h);
-  return {s.h, __fadd_rn(__fadd_rn(__fadd_rn(a.l, b.l), __fadd_rn(c.l, d.l)),
-                         fadd3(p.l, q.l, s.l))};
-}
-__device__ __forceinline__ D norm2(D a, D b) {  // a + b
-  const D s = df::two_sum(a.h, b.h);
-  return df::fast_two_sum(s.h, fadd3(a.l, b.l, s.l));
-}
-
 // sums and differences of the eight cells of a corner (l, u: lower left cells of its
 // planes), as isum::eight
 enum Form { kSum, kDx, kDy, kDz };
@@ -82,9 +68,9 @@ template <int CX, int F> __device__ __forceinline__ D eight(const D *l, const D 
 #pragma unroll
     for (int i = 0; i < 4; i++)
       if (F == kDx ? !(i & 1) : F == kDy ? !(i & 2) : neg) v[i] = df::neg(v[i]);
-    return raw4(v[0], v[1], v[2], v[3]);
+    return df::raw4(v[0], v[1], v[2], v[3]);
   };
-  return norm2(plane(l, F == kDz), plane(u, false));
+  return df::norm2(plane(l, F == kDz), plane(u, false));
 }
 
 // weights of a corner difference or average on one axis: 2 u0, 2 u1, which are
@@ -102,7 +88,7 @@ template <> struct Weights<true> {
     const float k = __fmaf_rn(p.h, e0, __fmul_rn(q.h, e1));
     return df::fast_two_sum(
         s.h, __fadd_rn(__fadd_rn(__fsub_rn(b.l, a.l), __fsub_rn(d.l, c.l)),
-                       __fadd_rn(fadd3(p.l, q.l, s.l), k)));
+                       __fadd_rn(df::fadd3(p.l, q.l, s.l), k)));
   }
   // w0 l + w1 u + 16 (g - f)
   __device__ __forceinline__ D planes(D l, D u, D f, D g) const {
@@ -111,7 +97,7 @@ template <> struct Weights<true> {
     const D s = df::two_sum(x.h, y.h);
     const float k = __fmaf_rn(l.h, e0, __fmul_rn(u.h, e1));
     const float t = __fmaf_rn(16.0f, __fsub_rn(g.l, f.l), __fadd_rn(l.l, u.l));
-    return df::fast_two_sum(s.h, __fadd_rn(t, __fadd_rn(fadd3(x.l, y.l, s.l), k)));
+    return df::fast_two_sum(s.h, __fadd_rn(t, __fadd_rn(df::fadd3(x.l, y.l, s.l), k)));
   }
 };
 template <> struct Weights<false> {
@@ -130,11 +116,11 @@ template <> struct Weights<false> {
 // the corner average of a z face, 32 times its value, + 16 (f + g)
 __device__ __forceinline__ D face(const Weights<true> &x, const Weights<true> &y, D a, D b, D c,
                                   D d, D f, D g) {
-  const D p = raw4(a, b, c, d);
+  const D p = df::raw4(a, b, c, d);
   const float k = __fadd_rn(__fmaf_rn(__fadd_rn(a.h, b.h), y.e0, __fmul_rn(__fadd_rn(c.h, d.h), y.e1)),
                             __fmaf_rn(__fadd_rn(a.h, c.h), x.e0, __fmul_rn(__fadd_rn(b.h, d.h), x.e1)));
   const D q = df::two_sum(__fmul_rn(16.0f, f.h), __fmul_rn(16.0f, g.h));
-  return norm2({p.h, __fadd_rn(p.l, k)}, {q.h, __fmaf_rn(16.0f, __fadd_rn(f.l, g.l), q.l)});
+  return df::norm2({p.h, __fadd_rn(p.l, k)}, {q.h, __fmaf_rn(16.0f, __fadd_rn(f.l, g.l), q.l)});
 }
 __device__ __forceinline__ D face(const Weights<false> &x, const Weights<false> &y, D a, D b, D c,
                                   D d, D f, D g) {
