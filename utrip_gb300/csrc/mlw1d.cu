@@ -21,8 +21,9 @@
 // (the cluster barrier, remote and L2 accesses).  So the profiles are read through
 // the read-only cache (a barrier does not empty it), the loop's constants are read
 // once, minima are integer minima, nothing is read from another block, and the
-// plain step's arithmetic takes the fewest FP64 instructions (f1 below): a step of
-// 1024 cells on 16 blocks 12.9 -> 7.4 us, 64 spicule runs 50 -> 47 us (those are
+// plain step's arithmetic takes the fewest FP64 instructions (f1 below) and is shared
+// out to idle warps where a block has some: a step of 1024 cells on 16 blocks 12.9 ->
+// 6.9 us, 64 spicule runs 50 -> 47 us (those are
 // bound by the FP64 pipe: 512 cells a SM).
 //
 // The BG variant is mlw_m_bg (cans1d/hdmlw/mlw_m_bg.f:2-271): the same
@@ -204,7 +205,9 @@ __device__ __forceinline__ unsigned long long warp_min_key(unsigned long long k)
 // their value and the viscosity coefficient at four times (constants carry the
 // factors), every term of the update is summed before one product with dt/dx, and
 // reciprocals and roots are fd64.cuh's: 120 FP64 instructions a cell where one
-// operation of the reference after the other takes 270.
+// operation of the reference after the other takes 270 (12.9 -> 7.5 us a step of 1024
+// cells on 16 blocks).  Their chain is shortened by the warps such a block leaves idle:
+// the viscosity faces beside the corners, two threads a cell in the update (6.9 us).
 namespace f1 {
 __device__ __forceinline__ void cell(const Run1D &p, const double *pc, int L, int l, int g,
                                      double *U, double *FX) {
@@ -226,12 +229,18 @@ __device__ __forceinline__ void cell(const Run1D &p, const double *pc, int L, in
   FX[4 * L + l] = me;
 }
 
-// the corner between local cells l and l+1: twice its fluxes, four times the
-// viscosity coefficient over dxm
-__device__ __forceinline__ void corner(const Run1D &p, const double *pc, int L, int l, int g,
-                                       const double *U, const double *FX, double *K, double *Q,
-                                       double m2dt) {
-  const double dxim = __ldg(p.ax.dim + g), c = m2dt * dxim;
+// four times the viscosity coefficient over dxm of the corner between l and l+1
+__device__ __forceinline__ void visc(const Run1D &p, const double *pc, int L, int l, int g,
+                                     double *Q) {
+  const double a =
+      fd::pos_part(fd::abs_(pc[2 * L + l + 1] - pc[2 * L + l]) - CANS_AV_EPS);
+  Q[l] = 4.0 * p.ph.qav * __ldg(p.ax.dm + g) * a * __ldg(p.ax.dim + g);
+}
+
+// the corner between local cells l and l+1: twice its fluxes
+__device__ __forceinline__ void corner(const Run1D &p, int L, int l, int g, const double *U,
+                                       const double *FX, double *K, double m2dt) {
+  const double c = m2dt * __ldg(p.ax.dim + g);
   double un[NV1];
 #pragma unroll
   for (int v = 0; v < NV1; v++)
@@ -247,35 +256,46 @@ __device__ __forceinline__ void corner(const Run1D &p, const double *pc, int L, 
   K[2 * L + l] = fma(un[2], vx, fma(bb, k8, pr));
   K[3 * L + l] = fma(un[2], vy, -(pb * bxm2));
   K[4 * L + l] = me;
-  const double a =
-      fd::pos_part(fd::abs_(pc[2 * L + l + 1] - pc[2 * L + l]) - CANS_AV_EPS);
-  Q[l] = 4.0 * p.ph.qav * __ldg(p.ax.dm + g) * a * dxim;
 }
 
-// the new primitives of own cell l
-__device__ __forceinline__ void update(const Run1D &p, double *pn, int L, int l, int g,
-                                       const double *U, const double *FX, const double *K,
-                                       const double *Q, double mdt4) {
-  const double c = mdt4 * __ldg(p.ax.di + g);  // -dt / (4 dx)
-  const double ql = Q[l], qm = Q[l - 1], qs = ql + qm;
-  double u[NV1];
-#pragma unroll
-  for (int v = 0; v < NV1; v++) {
-    const double uc = U[v * L + l];
-    double t = (FX[v * L + l + 1] - FX[v * L + l - 1]) + (K[v * L + l] - K[v * L + l - 1]);
-    t = fma(qs, uc, t);
-    t = fma(-ql, U[v * L + l + 1], t);
-    t = fma(-qm, U[v * L + l - 1], t);
-    u[v] = fma(c, t, uc);
-  }
-  const double ri = fd::rcp(u[0]);
-  const double vx = u[2] * ri, vy = u[3] * ri;
-  const double ek2 = fma(u[2], vx, u[3] * vy);
-  pn[l] = u[0];
-  pn[L + l] = p.ph.gm1 * fma(-p.ph.pi8i, u[4] * u[4], fma(-0.5, ek2, u[1]));
+// the new conserved variable v of own cell l; c = -dt / (4 dx)
+__device__ __forceinline__ double advance(int L, int l, const double *U, const double *FX,
+                                          const double *K, double c, double ql, double qm,
+                                          double qs, int v) {
+  const double uc = U[v * L + l];
+  double t = (FX[v * L + l + 1] - FX[v * L + l - 1]) + (K[v * L + l] - K[v * L + l - 1]);
+  t = fma(qs, uc, t);
+  t = fma(-ql, U[v * L + l + 1], t);
+  t = fma(-qm, U[v * L + l - 1], t);
+  return fma(c, t, uc);
+}
+// The new primitives of own cell l in two parts, of one thread or of two: the density
+// and velocities (the result is twice the kinetic energy), and the field with the
+// pressure's slot holding ee - by^2/8pi, which pressure() completes.
+__device__ __forceinline__ double update_v(const Run1D &p, double *pn, int L, int l, int g,
+                                           const double *U, const double *FX, const double *K,
+                                           const double *Q, double mdt4) {
+  const double c = mdt4 * __ldg(p.ax.di + g), ql = Q[l], qm = Q[l - 1], qs = ql + qm;
+  const double ro = advance(L, l, U, FX, K, c, ql, qm, qs, 0);
+  const double rx = advance(L, l, U, FX, K, c, ql, qm, qs, 2);
+  const double ry = advance(L, l, U, FX, K, c, ql, qm, qs, 3);
+  const double ri = fd::rcp(ro), vx = rx * ri, vy = ry * ri;
+  pn[l] = ro;
   pn[2 * L + l] = vx;
   pn[3 * L + l] = vy;
-  pn[4 * L + l] = u[4];
+  return fma(rx, vx, ry * vy);
+}
+__device__ __forceinline__ void update_b(const Run1D &p, double *pn, int L, int l, int g,
+                                         const double *U, const double *FX, const double *K,
+                                         const double *Q, double mdt4) {
+  const double c = mdt4 * __ldg(p.ax.di + g), ql = Q[l], qm = Q[l - 1], qs = ql + qm;
+  const double ee = advance(L, l, U, FX, K, c, ql, qm, qs, 1);
+  const double by = advance(L, l, U, FX, K, c, ql, qm, qs, 4);
+  pn[4 * L + l] = by;
+  pn[L + l] = fma(-p.ph.pi8i, by * by, ee);
+}
+__device__ __forceinline__ void pressure(const Run1D &p, double *pn, int L, int l, double ek2) {
+  pn[L + l] = p.ph.gm1 * fma(-0.5, ek2, pn[L + l]);
 }
 
 // safety * dx / (|vx| + c_f) of one cell (cfl_m.f:53-60)
@@ -816,8 +836,13 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
       }
     } else if constexpr (!E) {
       const double m2dt = -2.0 * s_dt;
-      for (int l = tid; l < nl - 1; l += NT)
-        f1::corner(p, &P(cur, 0, 0), L, l, lo - 1 + l, U, FX, K, Q, m2dt);
+      // warps beyond the corners' take the viscosity faces: a chain beside the other
+      const int wc = NT > (nl + 30) / 32 * 32 ? (nl + 30) / 32 * 32 : 0;
+      if (tid >= wc)
+        for (int l = tid - wc; l < nl - 1; l += NT - wc)
+          f1::visc(p, &P(cur, 0, 0), L, l, lo - 1 + l, Q);
+      if (tid < wc || wc == 0)
+        for (int l = tid; l < nl - 1; l += NT) f1::corner(p, L, l, lo - 1 + l, U, FX, K, m2dt);
     } else
     for (int l = tid; l < nl - 1; l += NT) {
       const int g = lo - 1 + l;  // corner between g and g+1
@@ -904,8 +929,24 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
       }
     } else if constexpr (!E) {
       const double mdt4 = -0.25 * s_dt;
-      for (int l = 1 + tid; l <= nl - 2; l += NT)
-        f1::update(p, &P(nb, 0, 0), L, l, lo - 1 + l, U, FX, K, Q, mdt4);
+      double *pn = &P(nb, 0, 0);
+      const int wu = (nl + 29) / 32 * 32;  // whole warps of own cells
+      if (NT >= 2 * wu) {  // two threads a cell, in warps of their own
+        const int l = 1 + (tid < wu ? tid : tid - wu), g = lo - 1 + l;
+        double ek2 = 0.0;
+        if (tid < wu) {
+          if (l <= nl - 2) ek2 = f1::update_v(p, pn, L, l, g, U, FX, K, Q, mdt4);
+        } else if (tid < 2 * wu && l <= nl - 2) {
+          f1::update_b(p, pn, L, l, g, U, FX, K, Q, mdt4);
+        }
+        __syncthreads();
+        if (tid < wu && l <= nl - 2) f1::pressure(p, pn, L, l, ek2);
+      } else {
+        for (int l = 1 + tid; l <= nl - 2; l += NT) {
+          f1::update_b(p, pn, L, l, lo - 1 + l, U, FX, K, Q, mdt4);
+          f1::pressure(p, pn, L, l, f1::update_v(p, pn, L, l, lo - 1 + l, U, FX, K, Q, mdt4));
+        }
+      }
     } else
     for (int l = 1 + tid; l <= nl - 2; l += NT) {
       const int g = lo - 1 + l;
@@ -1213,6 +1254,9 @@ cudaError_t launch_mlw1d(bool exact, double *S, const double *bx,
   // one thread per cell of the block's segment (whole warps, 256 at most):
   // threads without a cell would only wait at the barriers of every stage
   int nt = ((p.lmax + 31) / 32) * 32;
+  // the plain fast step: two threads a cell in its update, where that stays within 256
+  const int nt2 = 2 * ((p.lmax - 2 + 31) / 32) * 32;
+  if (!exact && !bgv && !dfp && nt2 <= 256) nt = nt2 > nt ? nt2 : nt;
   nt = nt < 32 ? 32 : (nt > 256 ? 256 : nt);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(CS, 1, 1);
