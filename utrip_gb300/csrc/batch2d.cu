@@ -116,13 +116,13 @@ __global__ void __launch_bounds__(March<kBatchCH, M3, false>::NT, 2)
 // run's k_bcframe2d does them, and the reset of the work queue for the next
 // step.  One launch for what were three; the frame CFL of a run, on one SM
 // before, spreads over the blocks of its row of the grid.
-template <bool E, bool M3>
+template <bool E, bool M3, bool MIX>
 __global__ void __launch_bounds__(32 * Prim<M3>::N)
     k_bcframe_batch(const BatchGrid *__restrict__ grids, const BcTable *__restrict__ tables,
                     unsigned int *queue) {
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *queue = 0u;
   const BatchGrid &G = grids[blockIdx.y];
-  bcframe2d<E, M3>(G.ix, G.jx, G.ax, G.ay, G.ph, tables[blockIdx.y], G.ctl, blockIdx.x,
+  bcframe2d<E, M3, MIX>(G.ix, G.jx, G.ax, G.ay, G.ph, tables[blockIdx.y], G.ctl, blockIdx.x,
                    gridDim.x);
 }
 
@@ -245,6 +245,7 @@ struct cans_batch {
   std::vector<BatchGrid> hgrids;
   BatchGrid *d_grids = nullptr;
   BcTable *d_bc = nullptr;
+  bool mixed = false;  // a run's program is one of bc_mixed
   unsigned int *d_queue = nullptr;
   int nitems = 0, frame_blocks = 1;
   int uniform = 1;  // every run's axes are (Axis::uniform)
@@ -286,7 +287,12 @@ int sync_tables(cans_batch *b) {
   b->nitems = item;
   b->frame_blocks = std::min((frame + 31) / 32, 152 * 4);
   std::vector<BcTable> bcs(b->ngrids);
-  for (int r = 0; r < b->ngrids; r++) bcs[r] = b->g[r].bc;
+  b->mixed = false;
+  for (int r = 0; r < b->ngrids; r++) {
+    bcs[r] = b->g[r].bc;
+    bcs[r].mixed = bc_mixed(bcs[r]) ? 1 : 0;
+    b->mixed |= bcs[r].mixed != 0;
+  }
   BK(cudaMemcpyAsync(b->d_grids, b->hgrids.data(), sizeof(BatchGrid) * b->ngrids,
                      cudaMemcpyHostToDevice, b->s));
   BK(cudaMemcpyAsync(b->d_bc, bcs.data(), sizeof(BcTable) * b->ngrids,
@@ -316,13 +322,16 @@ int enqueue_batch_iteration(cans_batch *b) {
   const bool m3 = b->solver == CANS_SOLVER_MLW_M3_2D;
   const dim3 grid(b->frame_blocks, b->ngrids);
   const int nt = 32 * b->nvar;
-  if (b->exact) {
-    if (m3) k_bcframe_batch<true, true><<<grid, nt, 0, b->s>>>(b->d_grids, b->d_bc, b->d_queue);
-    else k_bcframe_batch<true, false><<<grid, nt, 0, b->s>>>(b->d_grids, b->d_bc, b->d_queue);
-  } else {
-    if (m3) k_bcframe_batch<false, true><<<grid, nt, 0, b->s>>>(b->d_grids, b->d_bc, b->d_queue);
-    else k_bcframe_batch<false, false><<<grid, nt, 0, b->s>>>(b->d_grids, b->d_bc, b->d_queue);
-  }
+  const bool x = b->mixed;
+  auto k = m3 ? (b->exact ? (x ? k_bcframe_batch<true, true, true>
+                               : k_bcframe_batch<true, true, false>)
+                          : (x ? k_bcframe_batch<false, true, true>
+                               : k_bcframe_batch<false, true, false>))
+              : (b->exact ? (x ? k_bcframe_batch<true, false, true>
+                               : k_bcframe_batch<true, false, false>)
+                          : (x ? k_bcframe_batch<false, false, true>
+                               : k_bcframe_batch<false, false, false>));
+  k<<<grid, nt, 0, b->s>>>(b->d_grids, b->d_bc, b->d_queue);
   count_launch();
   BK(cudaGetLastError());
   return CANS_OK;

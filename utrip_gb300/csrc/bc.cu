@@ -12,6 +12,7 @@
 #include "cans_common.cuh"
 #include "cans_internal.h"
 #include "bc_line.cuh"
+#include "bcframe2d.cuh"
 
 namespace cans {
 
@@ -55,9 +56,48 @@ static cudaError_t bc_axis(int nvar, double *S, int n0, int n1, int n2,
   return cudaGetLastError();
 }
 
+// The x rules of every row and then the y rules of every column in one launch: a
+// thread computes the value that both leave at one frame cell of one variable
+// (bc_xy_value, as k_bcframe2d does), reading only cells no rule changes.  Two
+// launches a line a thread take 9.4 us at 256^2, this one 5.
+__global__ void k_bc2d(int nvar, double *S, int ix, int jx, BcTable bc, const double *dxm,
+                       const double *dym, const Ctl *ctl) {
+  if (ctl != nullptr) {
+    if (ctl->done | ctl->pause) return;
+    S = ctl->buf[ctl->cur ^ 1];
+  }
+  const int m = bc.margin, w = m + 1;
+  const size_t n = (size_t)ix * jx;
+  const long long cells = frame_cells(ix, jx, w, 0), total = cells * nvar;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
+       t += (long long)gridDim.x * blockDim.x) {
+    const int v = (int)(t / cells);
+    int i, j;
+    frame_cell(t % cells, ix, jx, w, 0, i, j);
+    const int kxl = bc.kind[v][0], kxh = bc.kind[v][1];
+    const int kyl = bc.kind[v][2], kyh = bc.kind[v][3];
+    const bool cy = bd_changes(kyl, kyh, m, jx, j + 1);
+    if (!cy && !bd_changes(kxl, kxh, m, ix, i + 1)) continue;
+    double *sv = S + (size_t)v * n;
+    sv[(size_t)i + (size_t)j * ix] =
+        bc_xy_value(sv, ix, jx, m, kxl, kxh, kyl, kyh, bc.q0[v][0], bc.q0[v][1], bc.q0[v][2],
+                    bc.q0[v][3], dxm, dym, i + 1, j + 1, cy);
+  }
+}
+
 cudaError_t launch_bc2d(int nvar, double *S, int ix, int jx, const Axis &ax,
                         const Axis &ay, const BcTable &bc, const Ctl *ctl,
                         cudaStream_t s) {
+  // below that, and in a mixed program, a rule may read a cell that the opposite
+  // face's rule changes
+  if (ix >= 2 * bc.margin + 3 && jx >= 2 * bc.margin + 3 && !bc_mixed(bc)) {
+    const long long total = frame_cells(ix, jx, bc.margin + 1, 0) * nvar;
+    int blocks = (int)((total + 127) / 128);
+    if (blocks > 152 * 8) blocks = 152 * 8;
+    k_bc2d<<<blocks, 128, 0, s>>>(nvar, S, ix, jx, bc, ax.dm, ay.dm, ctl);
+    count_launch();
+    return cudaGetLastError();
+  }
   cudaError_t e = bc_axis(nvar, S, ix, jx, 1, 0, bc, ax.dm, ctl, s);
   if (e != cudaSuccess) return e;
   return bc_axis(nvar, S, ix, jx, 1, 1, bc, ay.dm, ctl, s);

@@ -100,7 +100,8 @@ static __device__ __noinline__ double bc_xy_value(const double *sv, int ix, int 
 // reduces the CFL over the frame as k_frame2d does, from the values in
 // registers, and the last block ends the iteration.
 // `block` of `nblocks` blocks of 32 Prim<M3>::N threads.
-template <bool E, bool M3>
+// MIX: the program may be one of bc_mixed.
+template <bool E, bool M3, bool MIX>
 __device__ __forceinline__ void bcframe2d(int ix, int jx, const Axis &ax, const Axis &ay,
                                           const Phys &ph, const BcTable &bc, Ctl *ctl, int block,
                                           int nblocks) {
@@ -115,6 +116,24 @@ __device__ __forceinline__ void bcframe2d(int ix, int jx, const Axis &ax, const 
   const int m = bc.margin, w = m + 1;
   const long long total = frame_cells(ix, jx, w, 0);
   const int c = threadIdx.x & 31, v = threadIdx.x >> 5;
+  // a program of bc_mixed: one block, rule by rule
+  const bool mixed = MIX && bc.mixed != 0;
+  if (mixed) {
+    if (block != 0) return;
+    nblocks = 1;
+    for (int axis = 0; axis < 2; axis++) {
+      const int len = axis ? jx : ix, lines = axis ? ix : jx;
+      for (int t = threadIdx.x; t < lines * P::N; t += blockDim.x) {
+        const int u = t / lines, line = t % lines;
+        double *l = S + (size_t)u * n + (size_t)line * (axis ? 1 : ix);
+        for (int f = 0; f < 2; f++)
+          if (bc.kind[u][2 * axis + f] >= 0)
+            bd_line(bc.kind[u][2 * axis + f], f, m, m, l, len, axis ? (size_t)ix : 1,
+                    bc.q0[u][2 * axis + f], axis ? ay.dm : ax.dm);
+      }
+      __syncthreads();
+    }
+  }
   double dmin = __longlong_as_double(0x7ff0000000000000LL);
   bool bad = false;
   for (long long f0 = block * 32LL; f0 < total; f0 += nblocks * 32LL) {
@@ -127,10 +146,11 @@ __device__ __forceinline__ void bcframe2d(int ix, int jx, const Axis &ax, const 
       const int kyl = bc.kind[v][2], kyh = bc.kind[v][3];
       const bool cx = bd_changes(kxl, kxh, m, ix, i + 1);
       const bool cy = bd_changes(kyl, kyh, m, jx, j + 1);
-      const double val = bc_xy_value(sv, ix, jx, m, kxl, kxh, kyl, kyh, bc.q0[v][0],
-                                     bc.q0[v][1], bc.q0[v][2], bc.q0[v][3], ax.dm, ay.dm,
-                                     i + 1, j + 1, cy);
-      if (cx || cy) S[(size_t)v * n + (size_t)i + (size_t)j * ix] = val;
+      const double val =
+          mixed ? sv[(size_t)i + (size_t)j * ix]
+                : bc_xy_value(sv, ix, jx, m, kxl, kxh, kyl, kyh, bc.q0[v][0], bc.q0[v][1],
+                              bc.q0[v][2], bc.q0[v][3], ax.dm, ay.dm, i + 1, j + 1, cy);
+      if (!mixed && (cx || cy)) S[(size_t)v * n + (size_t)i + (size_t)j * ix] = val;
       q[v][c] = val;
     }
     __syncthreads();

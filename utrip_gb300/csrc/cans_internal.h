@@ -63,10 +63,21 @@ struct BcTable {
   int margin;
   int kind[kMaxVar][6];
   double q0[kMaxVar][6];
+  int mixed;  // 2-D: bc_mixed, set by the launchers that apply both axes at once
 };
 
 enum BdKind { BD_NONE = -1, BD_PER = 0, BD_SPP = 1, BD_SPN = 2, BD_SMP = 3,
               BD_SMN = 4, BD_FRE = 5, BD_CNS = 6, BD_FRD = 7 };
+
+// Does a 2-D program have a variable whose lower face is periodic while its upper face
+// zeroes its boundary cell (bdsmn)?  The lower rule then reads the cell that the
+// upper one changes, so the threads of a one-pass fill would race.
+inline bool bc_mixed(const BcTable &bc) {
+  for (int v = 0; v < kMaxVar; v++)
+    for (int f = 0; f < 4; f += 2)
+      if (bc.kind[v][f] == BD_PER && bc.kind[v][f + 1] == BD_SMN) return true;
+  return false;
+}
 
 // Region whose CFL the step kernel reduces (0-based inclusive box).  Cells
 // outside it are reduced after the boundary fill by the frame kernel.

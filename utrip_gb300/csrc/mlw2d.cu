@@ -233,10 +233,10 @@ __global__ void k_frame2d(const double *__restrict__ S, int ix, int jx,
   }
 }
 
-template <bool E, bool M3>
+template <bool E, bool M3, bool MIX>
 __global__ void __launch_bounds__(32 * Prim<M3>::N)
     k_bcframe2d(int ix, int jx, Axis ax, Axis ay, Phys ph, BcTable bc, Ctl *ctl) {
-  bcframe2d<E, M3>(ix, jx, ax, ay, ph, bc, ctl, blockIdx.x, gridDim.x);
+  bcframe2d<E, M3, MIX>(ix, jx, ax, ay, ph, bc, ctl, blockIdx.x, gridDim.x);
 }
 
 cudaError_t launch_bcframe2d(int solver, bool exact, int nvar, int ix, int jx, const Axis &ax,
@@ -250,13 +250,17 @@ cudaError_t launch_bcframe2d(int solver, bool exact, int nvar, int ix, int jx, c
   if (blocks < 1) blocks = 1;
   if (blocks > 152 * 4) blocks = 152 * 4;
   const int nt = 32 * nvar;
-  if (solver == 1) {
-    if (exact) k_bcframe2d<true, true><<<blocks, nt, 0, s>>>(ix, jx, ax, ay, ph, bc, ctl);
-    else k_bcframe2d<false, true><<<blocks, nt, 0, s>>>(ix, jx, ax, ay, ph, bc, ctl);
-  } else {
-    if (exact) k_bcframe2d<true, false><<<blocks, nt, 0, s>>>(ix, jx, ax, ay, ph, bc, ctl);
-    else k_bcframe2d<false, false><<<blocks, nt, 0, s>>>(ix, jx, ax, ay, ph, bc, ctl);
-  }
+  BcTable t = bc;
+  t.mixed = bc_mixed(bc) ? 1 : 0;
+  auto k = solver == 1 ? (exact ? (t.mixed ? k_bcframe2d<true, true, true>
+                                           : k_bcframe2d<true, true, false>)
+                                : (t.mixed ? k_bcframe2d<false, true, true>
+                                           : k_bcframe2d<false, true, false>))
+                       : (exact ? (t.mixed ? k_bcframe2d<true, false, true>
+                                           : k_bcframe2d<true, false, false>)
+                                : (t.mixed ? k_bcframe2d<false, false, true>
+                                           : k_bcframe2d<false, false, false>));
+  k<<<blocks, nt, 0, s>>>(ix, jx, ax, ay, ph, t, ctl);
   count_launch();
   return cudaGetLastError();
 }
