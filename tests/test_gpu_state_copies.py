@@ -56,3 +56,28 @@ def test_restarted_run_steps_as_a_fresh_one(gpu, which):
     assert got[1][1] == got[2][1] and got[0][1] < got[1][1]
     for a, b in zip(got[1][0], got[2][0]):
         assert np.array_equal(a, b)
+
+
+def test_a_started_run_has_taken_its_arrays(gpu):
+    """The page-locked arrays may be filled again once start has returned, also with
+    work of an earlier loop in front of the push."""
+    s = setups.random_state_1d(1026, seed=9)
+    src = [pinned(a) for a in s["state"]]
+    run = drivers.make_run(s)
+    for _ in range(3):
+        for p, a in zip(src, s["state"]):
+            p[...] = a
+        run.push(src)
+        run.start(nstop=10 ** 9, safety=s["safety"], dtmin=s["dtmin"])
+        for p in src:
+            p[...] = -1.0
+        run.advance(2000)
+    assert run.query().merr == 0 and np.all(run.pull()[0] > 0.0)
+    run.push(src)
+    for p, a in zip(src, s["state"]):
+        p[...] = a
+    run.push(src)
+    out = run.pull()
+    run.close()
+    for a, b in zip(out, s["state"]):
+        assert np.array_equal(a, b)

@@ -1447,6 +1447,7 @@ struct cans_run {
   double *buf[2] = {nullptr, nullptr};
   Ctl *ctl = nullptr;          // device control block
   Ctl host_ctl{};              // last copy read back
+  bool push_pending = false;   // no wait since the last push
   cudaStream_t s = nullptr;
   bool own_stream = false;
   int tile = 0;
@@ -1672,6 +1673,7 @@ int read_ctl(cans_run *h) {
   CK(cudaMemcpyAsync(&h->host_ctl, h->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost,
                      h->s));
   CK(cudaStreamSynchronize(h->s));
+  h->push_pending = false;
   return CANS_OK;
 }
 
@@ -1707,8 +1709,8 @@ double *mapped_array(double *p, size_t n) {
 // The nvar arrays of n doubles between host and device, on stream s.  A small state
 // in page-locked arrays goes in one launch that reads or writes them in place: a
 // copy costs some 4 us of the host each, whatever its size (64 runs of five arrays of
-// 1026, a run: push 34 -> 16 us, start 21 -> 7, pull 41 -> 28, with the wait left out
-// above); beyond 1 MB the copy engine's rate counts.
+// 1026, a run: push 34 -> 16 us, start 21 -> 10, pull 41 -> 28, with the wait left
+// out above); beyond 1 MB the copy engine's rate counts.
 constexpr int kMaxVars = 16;
 struct HostArrays {
   double *p[kMaxVars];
@@ -1962,6 +1964,7 @@ extern "C" int cans_run_push(cans_run *h, double *const *host) {
   int cur;
   const int rc = current_buffer(h, &cur);
   if (rc) return rc;
+  h->push_pending = true;
   return host_state<true>(host, h->buf[cur], h->nvar, h->n, h->s);
 }
 
@@ -1993,6 +1996,11 @@ extern "C" int cans_run_start(cans_run *h, double t0, double tend,
   int cur;
   const int rc = current_buffer(h, &cur);
   if (rc) return rc;
+  // a started run has taken its host arrays: a program may fill them again
+  if (h->push_pending) {
+    CK(cudaStreamSynchronize(h->s));
+    h->push_pending = false;
+  }
   Ctl c = h->host_ctl;  // of which buf, cur and (replaced by the first CFL) dt stay
   c.t = t0;
   c.tp = t0;
