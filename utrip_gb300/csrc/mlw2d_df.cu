@@ -11,7 +11,7 @@
 
 namespace cans {
 
-// Chunks of 8 or 6 rows, segments balanced by the blocks an SM gets or by waves of
+// Chunks of 8 or 6 rows, segments balanced by pairs of blocks an SM or by waves of
 // resident blocks (balance_seg, balance_seg_waves): every configuration gives
 // the same bits.
 int mlw2d_df_tile_count() { return 7; }

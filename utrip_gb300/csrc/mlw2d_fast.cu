@@ -24,7 +24,7 @@ cudaError_t pick_terms(int tile, const MarchArgs &m, const Axis &ax, const Axis 
 
 }  // namespace
 
-// Even tiles balance the segments by the blocks an SM gets, odd ones by waves of
+// Even tiles balance the segments by pairs of blocks an SM, odd ones by waves of
 // resident blocks; the results are the same bits.
 cudaError_t launch_mlw2d_fast(int solver, int tile, const double *A, double *B, int ix, int jx,
                               const Axis &ax, const Axis &ay, const Phys &ph,
