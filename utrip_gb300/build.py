@@ -73,7 +73,7 @@ def build(verbose: bool = False, extra: list[str] | None = None) -> Path:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
         os.replace(tmp, lib)
     probe = LIBDIR / PROBELIB
-    deps = [PROBE, CSRC / "fd64.cuh", CSRC / "isum.cuh"]
+    deps = [PROBE, *CSRC.glob("*.cuh"), *CSRC.glob("*.h")]
     if not probe.exists() or any(probe.stat().st_mtime < d.stat().st_mtime for d in deps):
         cmd = [nvcc(), ARCH, "-O3", "-std=c++17", "-Xcompiler", "-fPIC", f"-I{CSRC}", "-shared",
                str(PROBE), "-o", str(probe)]

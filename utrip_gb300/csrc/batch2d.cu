@@ -245,7 +245,7 @@ struct cans_batch {
   std::vector<BatchGrid> hgrids;
   BatchGrid *d_grids = nullptr;
   BcTable *d_bc = nullptr;
-  bool mixed = false;  // a run's program is one of bc_mixed
+  bool mixed = false;  // a run's program cannot be applied in one pass (bc_one_pass)
   unsigned int *d_queue = nullptr;
   int nitems = 0, frame_blocks = 1;
   int uniform = 1;  // every run's axes are (Axis::uniform)
@@ -290,7 +290,7 @@ int sync_tables(cans_batch *b) {
   b->mixed = false;
   for (int r = 0; r < b->ngrids; r++) {
     bcs[r] = b->g[r].bc;
-    bcs[r].mixed = bc_mixed(bcs[r]) ? 1 : 0;
+    bcs[r].mixed = bc_one_pass(bcs[r], b->g[r].ix, b->g[r].jx) ? 0 : 1;
     b->mixed |= bcs[r].mixed != 0;
   }
   BK(cudaMemcpyAsync(b->d_grids, b->hgrids.data(), sizeof(BatchGrid) * b->ngrids,

@@ -88,9 +88,9 @@ __global__ void k_bc2d(int nvar, double *S, int ix, int jx, BcTable bc, const do
 cudaError_t launch_bc2d(int nvar, double *S, int ix, int jx, const Axis &ax,
                         const Axis &ay, const BcTable &bc, const Ctl *ctl,
                         cudaStream_t s) {
-  // below that, and in a mixed program, a rule may read a cell that the opposite
-  // face's rule changes
-  if (ix >= 2 * bc.margin + 3 && jx >= 2 * bc.margin + 3 && !bc_mixed(bc)) {
+  // two frames and a cell between them on each axis, and no rule that reads what the
+  // opposite face's rule changes
+  if (ix >= 2 * bc.margin + 3 && jx >= 2 * bc.margin + 3 && bc_one_pass(bc, ix, jx)) {
     const long long total = frame_cells(ix, jx, bc.margin + 1, 0) * nvar;
     int blocks = (int)((total + 127) / 128);
     if (blocks > 152 * 8) blocks = 152 * 8;

@@ -100,7 +100,7 @@ static __device__ __noinline__ double bc_xy_value(const double *sv, int ix, int 
 // reduces the CFL over the frame as k_frame2d does, from the values in
 // registers, and the last block ends the iteration.
 // `block` of `nblocks` blocks of 32 Prim<M3>::N threads.
-// MIX: the program may be one of bc_mixed.
+// MIX: the program may be one that bc_one_pass refuses; it is then filled rule by rule.
 template <bool E, bool M3, bool MIX>
 __device__ __forceinline__ void bcframe2d(int ix, int jx, const Axis &ax, const Axis &ay,
                                           const Phys &ph, const BcTable &bc, Ctl *ctl, int block,
@@ -116,7 +116,7 @@ __device__ __forceinline__ void bcframe2d(int ix, int jx, const Axis &ax, const 
   const int m = bc.margin, w = m + 1;
   const long long total = frame_cells(ix, jx, w, 0);
   const int c = threadIdx.x & 31, v = threadIdx.x >> 5;
-  // a program of bc_mixed: one block, rule by rule
+  // where a rule reads what another changes (!bc_one_pass): one block, rule by rule
   const bool mixed = MIX && bc.mixed != 0;
   if (mixed) {
     if (block != 0) return;

@@ -63,20 +63,37 @@ struct BcTable {
   int margin;
   int kind[kMaxVar][6];
   double q0[kMaxVar][6];
-  int mixed;  // 2-D: bc_mixed, set by the launchers that apply both axes at once
+  int mixed;  // 2-D: !bc_one_pass, set by the launchers that apply both axes at once
 };
 
 enum BdKind { BD_NONE = -1, BD_PER = 0, BD_SPP = 1, BD_SPN = 2, BD_SMP = 3,
               BD_SMN = 4, BD_FRE = 5, BD_CNS = 6, BD_FRD = 7 };
 
-// Does a 2-D program have a variable whose lower face is periodic while its upper face
-// zeroes its boundary cell (bdsmn)?  The lower rule then reads the cell that the
-// upper one changes, so the threads of a one-pass fill would race.
-inline bool bc_mixed(const BcTable &bc) {
+// May a 2-D program be applied in one pass over the frame, each thread computing the
+// value that all rules leave at its cell?  It reads the sources of the lower rules
+// (an upper rule's are read through them), and none of those may be a cell that the
+// upper rule of the axis changes, or the threads race.  The last cell (1-based) a lower
+// rule reads and the first one an upper rule changes, margin m, extent n:
+//   bdper n-m;  bdspp, bdspn 2m;  bdsmp, bdsmn 2m+1;  bdfre m+1;  bdfrd m+2
+//   bdsmn n-m, which it zeroes;  the others n-m+1
+// They meet for bdper against bdsmn at every extent, else only below 3m+2 cells.  Below
+// 3m cells bdper also reads what it writes itself.
+inline bool bc_one_pass(const BcTable &bc, int ix, int jx) {
+  const int m = bc.margin;
   for (int v = 0; v < kMaxVar; v++)
-    for (int f = 0; f < 4; f += 2)
-      if (bc.kind[v][f] == BD_PER && bc.kind[v][f + 1] == BD_SMN) return true;
-  return false;
+    for (int axis = 0; axis < 2; axis++) {
+      const int n = axis ? jx : ix, lo = bc.kind[v][2 * axis], hi = bc.kind[v][2 * axis + 1];
+      if ((lo == BD_PER || hi == BD_PER) && n < 3 * m) return false;
+      if (lo < 0 || hi < 0) continue;
+      const int reads = lo == BD_PER                       ? n - m
+                        : lo == BD_SPP || lo == BD_SPN     ? 2 * m
+                        : lo == BD_SMP || lo == BD_SMN     ? 2 * m + 1
+                        : lo == BD_FRE                     ? m + 1
+                        : lo == BD_FRD                     ? m + 2
+                                                           : 0;
+      if (reads >= (hi == BD_SMN ? n - m : n - m + 1)) return false;
+    }
+  return true;
 }
 
 // Region whose CFL the step kernel reduces (0-based inclusive box).  Cells

@@ -251,7 +251,7 @@ cudaError_t launch_bcframe2d(int solver, bool exact, int nvar, int ix, int jx, c
   if (blocks > 152 * 4) blocks = 152 * 4;
   const int nt = 32 * nvar;
   BcTable t = bc;
-  t.mixed = bc_mixed(bc) ? 1 : 0;
+  t.mixed = bc_one_pass(bc, ix, jx) ? 0 : 1;
   auto k = solver == 1 ? (exact ? (t.mixed ? k_bcframe2d<true, true, true>
                                            : k_bcframe2d<true, true, false>)
                                 : (t.mixed ? k_bcframe2d<false, true, true>

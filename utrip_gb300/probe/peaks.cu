@@ -2,9 +2,11 @@
 // and FP32 fused-multiply-add throughput.  Built into its own library,
 // libcansprobe.so, beside libcansgpu.so: it is measurement tooling for
 // bench.py, not part of the C ABI of the solver.  It also evaluates the FP64
-// functions of fd64.cuh and the sums of isum.cuh on arrays, for their tests.
+// functions of fd64.cuh and the sums of isum.cuh on arrays, and host rules of the
+// launchers, for their tests.
 #include <cuda_runtime.h>
 
+#include "cans_internal.h"
 #include "fd64.cuh"
 #include "isum.cuh"
 
@@ -178,4 +180,15 @@ extern "C" int cans_probe_muscl(const double *x, double *y, int n) {
   const cudaError_t e = cudaMemcpy(y, d + 4 * (size_t)n, 2 * b, cudaMemcpyDeviceToHost);
   cudaFree(d);
   return e == cudaSuccess ? 0 : 2;
+}
+
+// May the rules kind[0..3] (x lower and upper face, y lower and upper) of a variable be
+// applied in one pass (bc_one_pass)?  Host only.
+extern "C" int cans_probe_bc_one_pass(int margin, int ix, int jx, const int *kind) {
+  cans::BcTable bc{};
+  bc.margin = margin;
+  for (auto &row : bc.kind)
+    for (int f = 0; f < 6; f++) row[f] = cans::BD_NONE;
+  for (int f = 0; f < 4; f++) bc.kind[cans::kMaxVar - 1][f] = kind[f];
+  return cans::bc_one_pass(bc, ix, jx) ? 1 : 0;
 }
