@@ -619,7 +619,9 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
   const long long c_nstop = p.ctl ? p.ctl->nstop : 0;
   const bool c_stop_bad = p.ctl && p.ctl->stop_on_bad;
   int cur = 0;
-  __syncthreads();
+  // every block of the cluster has started and loaded its cells: only now may another
+  // one write its halos and slots (once a launch)
+  cluster.sync();
 
   // CFL of the own cells (cfl_m.f:53-60) reduced over the cluster; valid on thread
   // 0: the minimum after a cluster barrier, and in any_bad whether a cell of any
