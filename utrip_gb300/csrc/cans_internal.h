@@ -69,29 +69,40 @@ struct BcTable {
 enum BdKind { BD_NONE = -1, BD_PER = 0, BD_SPP = 1, BD_SPN = 2, BD_SMP = 3,
               BD_SMN = 4, BD_FRE = 5, BD_CNS = 6, BD_FRD = 7 };
 
+// Of the rule `kind` on the lower face of a line of n cells with margin m: the last
+// cell (1-based) that it reads and the last one that it changes, 0 where there is none.
+// On the upper face both count from the other end.
+inline int bc_reads(int kind, int m, int n) {
+  switch (kind) {
+    case BD_PER: return n - m;
+    case BD_SPP: case BD_SPN: return 2 * m;
+    case BD_SMP: case BD_SMN: return 2 * m + 1;
+    case BD_FRE: return m + 1;
+    case BD_FRD: return m + 2;
+    default: return 0;
+  }
+}
+inline int bc_changes(int kind, int m) { return kind < 0 ? 0 : kind == BD_SMN ? m + 1 : m; }
+
+// Does a face's rule read a cell that the other face's rule changes, so that the upper
+// one has to wait for the lower one?  Periodic rules meet bdsmn at every extent, the
+// others only below 3m+2 cells.
+inline bool bc_faces_meet(int lo, int hi, int m, int n) {
+  return bc_reads(lo, m, n) + bc_changes(hi, m) > n || bc_reads(hi, m, n) + bc_changes(lo, m) > n;
+}
+
 // May a 2-D program be applied in one pass over the frame, each thread computing the
 // value that all rules leave at its cell?  It reads the sources of the lower rules
 // (an upper rule's are read through them), and none of those may be a cell that the
-// upper rule of the axis changes, or the threads race.  The last cell (1-based) a lower
-// rule reads and the first one an upper rule changes, margin m, extent n:
-//   bdper n-m;  bdspp, bdspn 2m;  bdsmp, bdsmn 2m+1;  bdfre m+1;  bdfrd m+2
-//   bdsmn n-m, which it zeroes;  the others n-m+1
-// They meet for bdper against bdsmn at every extent, else only below 3m+2 cells.  Below
-// 3m cells bdper also reads what it writes itself.
+// upper rule of the axis changes, or the threads race: bdper against bdsmn, and pairs
+// below 3m+2 cells.  Below 3m cells bdper also reads what it writes itself.
 inline bool bc_one_pass(const BcTable &bc, int ix, int jx) {
   const int m = bc.margin;
   for (int v = 0; v < kMaxVar; v++)
     for (int axis = 0; axis < 2; axis++) {
       const int n = axis ? jx : ix, lo = bc.kind[v][2 * axis], hi = bc.kind[v][2 * axis + 1];
       if ((lo == BD_PER || hi == BD_PER) && n < 3 * m) return false;
-      if (lo < 0 || hi < 0) continue;
-      const int reads = lo == BD_PER                       ? n - m
-                        : lo == BD_SPP || lo == BD_SPN     ? 2 * m
-                        : lo == BD_SMP || lo == BD_SMN     ? 2 * m + 1
-                        : lo == BD_FRE                     ? m + 1
-                        : lo == BD_FRD                     ? m + 2
-                                                           : 0;
-      if (reads >= (hi == BD_SMN ? n - m : n - m + 1)) return false;
+      if (hi >= 0 && bc_reads(lo, m, n) + bc_changes(hi, m) > n) return false;
     }
   return true;
 }

@@ -13,15 +13,17 @@
 // each block writes its edge cells into its neighbours' halos and its CFL
 // minimum into every block through distributed shared memory, so no host round
 // trip happens per step.  One cluster barrier per step (it publishes both) when
-// the boundary program reads only the cells of the blocks that run it; a second
-// one before the boundary fill when a rule is periodic.
+// the boundary program reads only the cells of the blocks that run it.  Where a rule
+// is periodic or reaches past its block, a second one stands before the fill, a
+// third between the faces if one reads what the other changes, and a fourth before
+// chkdav, which floors cells that another block's rule may be reading.
 //
 // What bounds a step is its chain: FP64 instructions of 64 clocks each on a
 // quarter of the SM that has one or two warps, and the latencies between them
 // (the cluster barrier, remote and L2 accesses).  So the profiles are read through
 // the read-only cache (a barrier does not empty it), the loop's constants are read
-// once, minima are integer minima, nothing is read from another block, and the
-// plain step's arithmetic takes the fewest FP64 instructions (f1 below) and is shared
+// once, minima are integer minima, halos and minima are written into the blocks that
+// need them (only such boundary rules read another block's cells), and the plain step's arithmetic takes the fewest FP64 instructions (f1 below) and is shared
 // out to idle warps where a block has some: a step of 1024 cells on 16 blocks 12.9 ->
 // 6.9 us, 64 spicule runs 50 -> 47 us (those are
 // bound by the FP64 pipe: 512 cells a SM).
@@ -32,8 +34,8 @@
 // mlwsrch.f / mlwsrcf.f, and bx included in the energy.  The spicule loop
 // (cans1d/md_spicule/hdmlw/main.f:160-219) adds two options that any 1-D
 // loop may use: the torque source of trqalfven.f after the step, and the
-// chkdav floor of ro and pr after the boundary fill (one extra cluster
-// barrier), with the events counted in the control block.
+// chkdav floor of ro and pr after the boundary fill, with the events counted in the
+// control block.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -64,6 +66,7 @@ struct Run1D {
   double floor;          // chkdav floor of ro and pr (used when chk)
   int chk;
   int bnd_local;         // 1: no boundary rule reads another block's cells
+  int bnd_order;         // 1: the upper face's rules wait for the lower face's blocks
   Axis ax;
   Phys ph;
   BcTable bc;
@@ -995,9 +998,9 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
     // then it must wait for the whole cluster.
     if (p.bnd_local) __syncthreads();
     else cluster.sync();
-    // ---- boundary program (bnd.f:9-19): lower face by block 0, upper face
+    // ---- boundary program (bnd.f:9-19): lower face by block 0, then the upper face
     // by the last block; cells of other blocks are read through DSMEM -------
-    if (tid < NV1 && (r == 0 || r == CS - 1)) {
+    auto face = [&](int mbnd) {
       const int v = tid;
       auto owner = [&](int g1) {  // 1-based global cell -> (rank, local)
         const int g = g1 - 1;
@@ -1018,12 +1021,13 @@ __device__ __forceinline__ void mlw1d_body(const Run1D &p) {
       auto put = [&](int g1, double x) {  // faces only write cells of this block
         P(nb, v, p.bnd_local ? g1 - lo : owner(g1).y) = x;
       };
-      if (r == 0)
-        bd1_face(p.bc.kind[v][0], 0, p.bc.margin, ix, p.bc.q0[v][0], ax.dm, get, put);
-      if (r == CS - 1)
-        bd1_face(p.bc.kind[v][1], 1, p.bc.margin, ix, p.bc.q0[v][1], ax.dm, get, put);
-    }
-    __syncthreads();
+      bd1_face(p.bc.kind[v][mbnd], mbnd, p.bc.margin, ix, p.bc.q0[v][mbnd], ax.dm, get, put);
+    };
+    if (tid < NV1 && r == 0) face(0);
+    if (p.bnd_order) cluster.sync();
+    if (tid < NV1 && r == CS - 1) face(1);
+    if (p.chk && !p.bnd_local) cluster.sync();  // the rules' remote reads are done
+    else __syncthreads();
     // ---- chkdav of ro, then pr (chkdav.f:68-76), every cell incl. ghosts ----
     if (p.chk) {
       unsigned int nev = 0;
@@ -1214,9 +1218,11 @@ bool fill_run1d(Run1D &p, double *S, const double *bx, const double *bxm, const 
   // a face rule reads at most 2*margin cells in from its end of the line
   // (bdsmp*: cell b+margin); block 0 and the last block own at least q cells
   p.bnd_local = 2 * bc.margin <= p.q ? 1 : 0;
-  for (int v = 0; v < NV1; v++)
+  for (int v = 0; v < NV1; v++) {
     for (int f = 0; f < 2; f++)
       if (bc.kind[v][f] == BD_PER) p.bnd_local = 0;
+    if (CS > 1 && bc_faces_meet(bc.kind[v][0], bc.kind[v][1], bc.margin, ix)) p.bnd_order = 1;
+  }
   return true;
 }
 }  // namespace

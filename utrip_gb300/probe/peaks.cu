@@ -192,3 +192,9 @@ extern "C" int cans_probe_bc_one_pass(int margin, int ix, int jx, const int *kin
   for (int f = 0; f < 4; f++) bc.kind[cans::kMaxVar - 1][f] = kind[f];
   return cans::bc_one_pass(bc, ix, jx) ? 1 : 0;
 }
+
+// Does one of the rules lo and hi of a line's faces read what the other changes
+// (bc_faces_meet)?  Host only.
+extern "C" int cans_probe_bc_faces_meet(int margin, int n, int lo, int hi) {
+  return cans::bc_faces_meet(lo, hi, margin, n) ? 1 : 0;
+}
