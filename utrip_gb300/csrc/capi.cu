@@ -7,6 +7,7 @@
 // and replays it as a CUDA graph; the drop-in entry points serve a Fortran
 // driver that still calls cfl_m3 / mlw_m3 / bd* once per step.
 #include <cuda_runtime.h>
+#include <unistd.h>
 
 #include <atomic>
 #include <cmath>
@@ -21,6 +22,7 @@
 
 #include "cans_gpu.h"
 #include "cans_internal.h"
+#include "host_range.h"
 
 namespace cans {
 
@@ -1694,16 +1696,15 @@ int current_buffer(cans_run *h, int *cur) {
 
 // Device address of a page-locked host array of n doubles, or nullptr.
 double *mapped_array(double *p, size_t n) {
-  cudaPointerAttributes a, b;
-  if (((uintptr_t)p & 7) || cudaPointerGetAttributes(&a, p) != cudaSuccess ||
-      cudaPointerGetAttributes(&b, p + n - 1) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer ||
-      (double *)b.devicePointer != (double *)a.devicePointer + (n - 1))
-    return nullptr;
-  return (double *)a.devicePointer;
+  static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+  return mapped_range(p, n, page, [](void *q) -> void * {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
+  });
 }
 
 // The nvar arrays of n doubles between host and device, on stream s.  A small state

@@ -8,6 +8,7 @@
 
 #include "cans_internal.h"
 #include "fd64.cuh"
+#include "host_range.h"
 #include "isum.cuh"
 
 namespace {
@@ -197,4 +198,20 @@ extern "C" int cans_probe_bc_one_pass(int margin, int ix, int jx, const int *kin
 // (bc_faces_meet)?  Host only.
 extern "C" int cans_probe_bc_faces_meet(int margin, int n, int lo, int hi) {
   return cans::bc_faces_meet(lo, hi, margin, n) ? 1 : 0;
+}
+
+// Would the array of n doubles at address p pass as page-locked (mapped_range) with the
+// nseg registrations [lo, hi) at seg[2i], seg[2i+1] of whole pages, the device address
+// being that of the host plus shift[i]?  No memory is touched.
+extern "C" int cans_probe_mapped_range(unsigned long long p, unsigned long long n,
+                                       unsigned long long page, const unsigned long long *seg,
+                                       const unsigned long long *shift, int nseg) {
+  return cans::mapped_range((double *)(uintptr_t)p, n, page,
+                            [=](void *q) -> void * {
+                              const uintptr_t a = (uintptr_t)q;
+                              for (int i = 0; i < nseg; i++)
+                                if (a >= seg[2 * i] && a < seg[2 * i + 1])
+                                  return (void *)(a + shift[i]);
+                              return nullptr;
+                            }) != nullptr;
 }
