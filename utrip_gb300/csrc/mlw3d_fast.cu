@@ -446,11 +446,14 @@ __global__ void __launch_bounds__(T3F<TX, TY, G>::NT, MINB)
         const int v = iv0 + j;
         const VarFields q = kVar[v];
         const double *u = s0 + (size_t)v * T::NC;
-        const double *fx = s0 + (size_t)q.fx * T::NC, *fy = s0 + (size_t)q.fy * T::NC;
-        const double *kx_ = kk + (size_t)q.kx * T::NK, *ky = kk + (size_t)q.ky * T::NK;
-        const double *kz = kk + (size_t)q.kz * T::NK;
-        const double *f0 = s0 + (size_t)q.fz * T::NC, *f1 = s1 + (size_t)q.fz * T::NC;
-        const double gxl = ret(8 + q.rx), gyl = ret(15 + q.ry), pl = ret(v);
+        // of field 0, unread, where the variable has no flux in the direction
+        const int qx = max(q.fx, 0), qy = max(q.fy, 0), qz_ = max(q.fz, 0);
+        const double *fx = s0 + qx * T::NC, *fy = s0 + qy * T::NC;
+        const double *kx_ = kk + max(q.kx, 0) * T::NK, *ky = kk + max(q.ky, 0) * T::NK;
+        const double *kz = kk + max(q.kz, 0) * T::NK;
+        const double *f0 = s0 + qz_ * T::NC, *f1 = s1 + qz_ * T::NC;
+        const double gxl = q.fx >= 0 ? ret(8 + q.rx) : 0.0, gyl = q.fy >= 0 ? ret(15 + q.ry) : 0.0;
+        const double pl = ret(v);
         const double w = qz * (s1[(size_t)v * T::NC] - u[0]);
         double gx = 0.0, gy = 0.0, pu = w;           // what the next plane keeps
         double tx = 0.0, ty = 0.0, tz;               // differences of the directions

@@ -21,7 +21,8 @@ constexpr int NRET = 22;
 
 // The fields of variable v (cell slot v): its x, y, z fluxes at the cells and corners,
 // -1 where it has none; their signs (of E in the induction equation); its retained x
-// and y differences; its gravity source.  In constant memory: the loops over the
+// and y differences (a word of the column each, of one thread; -1 with the flux); its
+// gravity source.  In constant memory: the loops over the
 // variables stay rolled, so that their integer sums (some 600 instructions a pass)
 // stay in the instruction cache.  The two halves of the variables have about the
 // same number of sums (15 and 14 of the predictor, 11 and 10 of the corrector).
@@ -32,10 +33,10 @@ __constant__ VarFields kVar[8] = {
     {CRX, KRX, CRY, KRY, CRZ, KRZ, 1, 1, 1, 0, 0, -1},
     {CFX, KFX, CFY, KFY, CFZ, KFZ, 1, 1, 1, 1, 1, 0},
     {CXX, KXX, CXY, KXY, CXZ, KXZ, 1, 1, 1, 2, 2, 1},
-    {-1, -1, CEZ, KEZ, CEY, KEY, 0, 1, -1, 0, 3, -1},
+    {-1, -1, CEZ, KEZ, CEY, KEY, 0, 1, -1, -1, 3, -1},
     {CXY, KXY, CYY, KYY, CYZ, KYZ, 1, 1, 1, 3, 4, 2},
     {CXZ, KXZ, CYZ, KYZ, CZZ, KZZ, 1, 1, 1, 4, 5, 3},
-    {CEZ, KEZ, -1, -1, CEX, KEX, -1, 0, 1, 5, 0, -1},
+    {CEZ, KEZ, -1, -1, CEX, KEX, -1, 0, 1, 5, -1, -1},
     {CEY, KEY, CEX, KEX, -1, -1, 1, -1, 0, 6, 6, -1}};
 
 template <int TX, int TY, bool G> struct T3F {
