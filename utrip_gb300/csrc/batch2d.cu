@@ -4,7 +4,8 @@
 // layer of cans2d/md_mhdkh/hdmlw/model.f) for many grid sizes and plasma
 // betas.  Run one at a time, a small grid fills a fraction of the 152 SMs and
 // every step pays the launch latency of its kernels.  Here one loop iteration
-// of every run is two launches in total:
+// of every run is two launches in total (three where equally spaced and stretched
+// meshes are in one batch):
 //   1. a persistent step kernel: one block per resident slot; each block pulls
 //      (run, tile) work items from a device work queue and applies the single
 //      run's block (mlw2d_march.cuh; exact policy: mlw2d_tile.cuh) with the
@@ -41,6 +42,11 @@ struct BatchGrid {
   int ntx, nty;   // tiles of the current configuration
   int tile0;      // first work item of this run
 };
+
+// The step's launches, each with a work queue of its own: the runs whose axes are all
+// equally spaced and the others (exact policy: one launch for all).  A run is stepped by
+// the instance of its own mesh whatever it shares the batch with.
+constexpr int kQueues = 2;
 
 // The next work item of a persistent block, or -1: the run it belongs to in *run,
 // its tile in *tile.
@@ -120,7 +126,7 @@ template <bool E, bool M3, bool MIX>
 __global__ void __launch_bounds__(32 * Prim<M3>::N)
     k_bcframe_batch(const BatchGrid *__restrict__ grids, const BcTable *__restrict__ tables,
                     unsigned int *queue) {
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *queue = 0u;
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < kQueues) queue[threadIdx.x] = 0u;
   const BatchGrid &G = grids[blockIdx.y];
   bcframe2d<E, M3, MIX>(G.ix, G.jx, G.ax, G.ay, G.ph, tables[blockIdx.y], G.ctl, blockIdx.x,
                    gridDim.x);
@@ -242,13 +248,13 @@ struct cans_batch {
     int stop_on_bad = 0;
   };
   std::vector<Grid> g;
-  std::vector<BatchGrid> hgrids;
+  std::vector<BatchGrid> hgrids;  // the runs of each of the step's launches in turn
   BatchGrid *d_grids = nullptr;
   BcTable *d_bc = nullptr;
   bool mixed = false;  // a run's program cannot be applied in one pass (bc_one_pass)
   unsigned int *d_queue = nullptr;
-  int nitems = 0, frame_blocks = 1;
-  int uniform = 1;  // every run's axes are (Axis::uniform)
+  int nruns[kQueues] = {}, nitems[kQueues] = {};  // of each of the step's launches
+  int frame_blocks = 1;
   cudaGraphExec_t graph = nullptr;
   int graph_iters = 0, graph_nodes = 0;
 };
@@ -265,11 +271,22 @@ void drop_graph(cans_batch *b) {
 // run descriptions and boundary tables.
 int sync_tables(cans_batch *b) {
   const BatchConfig c = b->exact ? kConfigs[b->config] : kFastConfigs[b->config];
-  int item = 0, frame = 0;
-  b->hgrids.resize(b->ngrids);
-  for (int r = 0; r < b->ngrids; r++) {
-    auto &G = b->g[r];
-    BatchGrid &H = b->hgrids[r];
+  int frame = 0;
+  b->hgrids.clear();
+  std::vector<int> order;  // runs by launch
+  for (int q = 0; q < kQueues; q++) {
+    b->nruns[q] = b->nitems[q] = 0;
+    for (int r = 0; r < b->ngrids; r++)
+      if ((b->exact || (b->g[r].ax.uniform && b->g[r].ay.uniform) ? 0 : 1) == q) {
+        order.push_back(r);
+        b->nruns[q]++;
+      }
+  }
+  for (int k = 0; k < b->ngrids; k++) {
+    auto &G = b->g[order[k]];
+    int &item = b->nitems[k < b->nruns[0] ? 0 : 1];
+    b->hgrids.emplace_back();
+    BatchGrid &H = b->hgrids.back();
     H.ctl = G.ctl;
     H.ax = G.ax;
     H.ay = G.ay;
@@ -284,14 +301,14 @@ int sync_tables(cans_batch *b) {
     item += H.ntx * H.nty;
     frame = std::max(frame, (int)frame_cells(G.ix, G.jx, w, 0));
   }
-  b->nitems = item;
   b->frame_blocks = std::min((frame + 31) / 32, 152 * 4);
   std::vector<BcTable> bcs(b->ngrids);
   b->mixed = false;
-  for (int r = 0; r < b->ngrids; r++) {
-    bcs[r] = b->g[r].bc;
-    bcs[r].mixed = bc_one_pass(bcs[r], b->g[r].ix, b->g[r].jx) ? 0 : 1;
-    b->mixed |= bcs[r].mixed != 0;
+  for (int k = 0; k < b->ngrids; k++) {
+    auto &G = b->g[order[k]];
+    bcs[k] = G.bc;
+    bcs[k].mixed = bc_one_pass(G.bc, G.ix, G.jx) ? 0 : 1;
+    b->mixed |= bcs[k].mixed != 0;
   }
   BK(cudaMemcpyAsync(b->d_grids, b->hgrids.data(), sizeof(BatchGrid) * b->ngrids,
                      cudaMemcpyHostToDevice, b->s));
@@ -304,15 +321,17 @@ int sync_tables(cans_batch *b) {
 
 int step_launch(cans_batch *b, int cfg) {
   const bool m3 = b->solver == CANS_SOLVER_MLW_M3_2D;
-  cudaError_t e;
-  if (b->exact)
-    e = m3 ? launch_batch<true>(cfg, b->d_grids, b->ngrids, b->nitems, b->d_queue, b->s)
-           : launch_batch<false>(cfg, b->d_grids, b->ngrids, b->nitems, b->d_queue, b->s);
-  else
-    e = (m3 ? b->uniform ? launch_batch_fast<true, true> : launch_batch_fast<true, false>
-            : b->uniform ? launch_batch_fast<false, true> : launch_batch_fast<false, false>)(
-        cfg, b->d_grids, b->ngrids, b->nitems, b->d_queue, b->s);
-  BK(e);
+  for (int q = 0; q < kQueues; q++) {
+    if (b->nruns[q] == 0) continue;
+    const BatchGrid *grids = b->d_grids + (q ? b->nruns[0] : 0);
+    if (b->exact)
+      BK((m3 ? launch_batch<true> : launch_batch<false>)(cfg, grids, b->nruns[q], b->nitems[q],
+                                                         b->d_queue + q, b->s));
+    else
+      BK((m3 ? q ? launch_batch_fast<true, false> : launch_batch_fast<true, true>
+             : q ? launch_batch_fast<false, false> : launch_batch_fast<false, true>)(
+          cfg, grids, b->nruns[q], b->nitems[q], b->d_queue + q, b->s));
+  }
   return CANS_OK;
 }
 
@@ -425,7 +444,6 @@ extern "C" int cans_batch_create(cans_batch **out, int ngrids,
     place_axis(G.ay, G.metrics + nmx, d.jx);
     G.ax.uniform = build_axis_host(d.ix, d.dx, d.dxm, h.data());
     G.ay.uniform = build_axis_host(d.jx, d.dy, d.dym, h.data() + nmx);
-    if (!G.ax.uniform || !G.ay.uniform) b->uniform = 0;
     e = cudaMemcpyAsync(G.metrics, h.data(), sizeof(double) * nm, cudaMemcpyHostToDevice, b->s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->s);
     if (e != cudaSuccess) return bail(bfail(e, "cudaMemcpy(metrics)"));
@@ -441,8 +459,8 @@ extern "C" int cans_batch_create(cans_batch **out, int ngrids,
   }
   e = cudaMalloc(&b->d_grids, sizeof(BatchGrid) * ngrids);
   if (e == cudaSuccess) e = cudaMalloc(&b->d_bc, sizeof(BcTable) * ngrids);
-  if (e == cudaSuccess) e = cudaMalloc(&b->d_queue, sizeof(unsigned int));
-  if (e == cudaSuccess) e = cudaMemsetAsync(b->d_queue, 0, sizeof(unsigned int), b->s);
+  if (e == cudaSuccess) e = cudaMalloc(&b->d_queue, kQueues * sizeof(unsigned int));
+  if (e == cudaSuccess) e = cudaMemsetAsync(b->d_queue, 0, kQueues * sizeof(unsigned int), b->s);
   if (e != cudaSuccess) return bail(bfail(e, "cudaMalloc(batch tables)"));
   int rc = sync_tables(b);
   if (rc) return bail(rc);
@@ -520,7 +538,7 @@ extern "C" int cans_batch_start(cans_batch *b, double t0, double tend, long long
   k_prepare_batch<<<(b->ngrids + 127) / 128, 128, 0, b->s>>>(b->d_grids, b->ngrids);
   count_launch();
   BK(cudaGetLastError());
-  BK(cudaMemsetAsync(b->d_queue, 0, sizeof(unsigned int), b->s));
+  BK(cudaMemsetAsync(b->d_queue, 0, kQueues * sizeof(unsigned int), b->s));
   BK(cudaStreamSynchronize(b->s));
   return CANS_OK;
 }
@@ -611,13 +629,13 @@ extern "C" int cans_batch_autotune(cans_batch *b, int trial_steps, int *config) 
     b->config = c;
     int rc = sync_tables(b);
     if (rc) return rc;
-    BK(cudaMemsetAsync(b->d_queue, 0, sizeof(unsigned int), b->s));
+    BK(cudaMemsetAsync(b->d_queue, 0, kQueues * sizeof(unsigned int), b->s));
     if ((rc = step_launch(b, c))) return rc;  // warm-up
-    BK(cudaMemsetAsync(b->d_queue, 0, sizeof(unsigned int), b->s));
+    BK(cudaMemsetAsync(b->d_queue, 0, kQueues * sizeof(unsigned int), b->s));
     BK(cudaEventRecord(e0, b->s));
     for (int k = 0; k < trial_steps; k++) {
       if ((rc = step_launch(b, c))) return rc;
-      BK(cudaMemsetAsync(b->d_queue, 0, sizeof(unsigned int), b->s));
+      BK(cudaMemsetAsync(b->d_queue, 0, kQueues * sizeof(unsigned int), b->s));
     }
     BK(cudaEventRecord(e1, b->s));
     BK(cudaEventSynchronize(e1));
