@@ -47,6 +47,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "balance2d.h"
 #include "cans_common.cuh"
 #include "cans_internal.h"
 #include "df64.cuh"
@@ -844,46 +845,6 @@ __global__ void __launch_bounds__(March<CH, M3, G>::NT, 2)
   const int jb = 1 + blockIdx.y * seg;
   march_block<N, CH, M3, G, R, AVF, U>(m, ax, ay, ph, blockIdx.x, gridDim.x, jb,
                                     min(m.jx - 2, jb + seg - 1), smem_march);
-}
-
-// Rows per block of the marching kernel, two of whose blocks fit an SM: a launch
-// takes as long as its busiest SM.  A block alone leaves the pipes to its own
-// latencies, a second one beside it fills them: the cost is that of pairs and of the
-// odd block, in units of a fifth of a microsecond, fitted to the FP64 step at 64^2 ..
-// 512^2 (a block of 3, 4, 7, 14, 32 rows alone on its SM 26, 27, 36, 56, 113 us; two
-// of 7, 27 rows 49, 146 us).  A segment need not be a whole number of chunks (its
-// last chunk may be short, as at the end of the grid).  Against the blocks an SM gets
-// times their rows: 192^2 48.9 -> 35.0, 256^2 56 -> 49, 384^2 113 -> 98 us a step.
-inline int balance_seg(int strips, int rows, int ch, int sms) {
-  int best = rows;
-  long long best_cost = -1;
-  for (int seg = 1; seg <= rows; seg++) {
-    const long long blocks = (long long)strips * ((rows + seg - 1) / seg);
-    const long long per_sm = (blocks + sms - 1) / sms, chunks = (seg + ch - 1) / ch;
-    const long long cost =
-        per_sm / 2 * (80 + 40 * chunks + 18 * seg) + per_sm % 2 * (75 + 25 * chunks + 11 * seg);
-    if (best_cost < 0 || cost < best_cost) {
-      best_cost = cost;
-      best = seg;
-    }
-  }
-  return best;
-}
-// The same with whole chunks per block, balanced by waves of resident
-// blocks (slots = SMs x resident blocks per SM): for a step that is bound by
-// latency more than by one pipe, fewer and longer blocks can win.
-inline int balance_seg_waves(int strips, int rows, int ch, int slots) {
-  int best = ch, best_cost = -1;
-  for (int seg = ch; seg <= rows + ch - 1; seg += ch) {
-    const int blocks = strips * ((rows + seg - 1) / seg);
-    const int waves = (blocks + slots - 1) / slots;
-    const int cost = waves * (seg + 2);
-    if (best_cost < 0 || cost < best_cost) {
-      best_cost = cost;
-      best = seg;
-    }
-  }
-  return best;
 }
 
 template <class N, int CH, bool M3, bool G, bool R, int AVF, bool U>

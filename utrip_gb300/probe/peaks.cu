@@ -6,6 +6,7 @@
 // launchers, for their tests.
 #include <cuda_runtime.h>
 
+#include "balance2d.h"
 #include "cans_internal.h"
 #include "fd64.cuh"
 #include "host_range.h"
@@ -214,4 +215,9 @@ extern "C" int cans_probe_mapped_range(unsigned long long p, unsigned long long 
                                   return (void *)(a + shift[i]);
                               return nullptr;
                             }) != nullptr;
+}
+
+// Rows of a segment as the marching steps choose them (balance_seg).  Host only.
+extern "C" int cans_probe_balance_seg(int strips, int rows, int ch, int sms) {
+  return cans::balance_seg(strips, rows, ch, sms);
 }
