@@ -20,6 +20,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -155,20 +156,33 @@ static const BatchConfig kFastConfigs[] = {
 constexpr int kNumConfigs = sizeof(kConfigs) / sizeof(kConfigs[0]);
 static_assert(sizeof(kFastConfigs) == sizeof(kConfigs), "one index serves both policies");
 
-// Persistent blocks: as many as the device holds at once.
+// Blocks of a persistent kernel that a device holds at once: asked, and the kernel's
+// shared memory set, once per device under a lock (batches of several host threads and
+// devices share a kernel).
+struct Resident {
+  std::mutex mu;
+  int of[64] = {};
+};
 template <class Kern, class... Args>
-static cudaError_t launch_persistent(Kern kern, int &resident, int nt, size_t smem, int nitems,
+static cudaError_t launch_persistent(Kern kern, Resident &r, int nt, size_t smem, int nitems,
                                      cudaStream_t s, Args... args) {
-  if (resident == 0) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-    int per_sm = 0, dev = 0, sms = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nt, smem);
-    if (e != cudaSuccess) return e;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    resident = (per_sm > 0 ? per_sm : 1) * sms;
+  int dev = 0, resident = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  {
+    std::lock_guard<std::mutex> lk(r.mu);
+    if (!r.of[dev]) {
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+      int per_sm = 0, sms = 0;
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nt, smem);
+      if (e != cudaSuccess) return e;
+      e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      if (e != cudaSuccess) return e;
+      r.of[dev] = (per_sm > 0 ? per_sm : 1) * sms;
+    }
+    resident = r.of[dev];
   }
   const int blocks = resident < nitems ? resident : nitems;
   kern<<<blocks > 0 ? blocks : 1, nt, smem, s>>>(args...);
@@ -180,7 +194,7 @@ template <bool M3, int TX, int TY, int RPT>
 static cudaError_t launch_batch_cfg(const BatchGrid *grids, int ngrids, int nitems,
                                     unsigned int *queue, cudaStream_t s) {
   using T = Tile<TX, TY, M3, RPT>;
-  static int resident = 0;  // per template instance
+  static Resident resident;  // per template instance
   return launch_persistent(k_mlw2d_batch<M3, TX, TY, RPT>, resident, T::NT, T::smem_bytes, nitems,
                            s, grids, ngrids, nitems, queue);
 }
@@ -201,7 +215,7 @@ template <bool M3, bool U>
 static cudaError_t launch_batch_fast(int cfg, const BatchGrid *grids, int ngrids, int nitems,
                                      unsigned int *queue, cudaStream_t s) {
   using T = March<kBatchCH, M3, false>;
-  static int resident = 0;  // per template instance
+  static Resident resident;  // per template instance
   return launch_persistent(k_mlw2d_batch_fast<M3, U>, resident, T::NT, T::smem_bytes, nitems, s,
                            grids, ngrids, nitems, kFastConfigs[cfg].ty, queue);
 }
