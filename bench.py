@@ -12,7 +12,7 @@ one step, as it does in a production run of this size.
 `--impl reference` times the CPU restatement of the reference Fortran (the
 oracle, with every host thread) on the same workload.  Under torchrun every
 rank runs an independent replica ("replicas only": the mLW path has no
-exchange on one GPU per run); rank 0 prints one JSON line.
+exchange on one GPU per run); rank 0 prints one JSON line, behind a line `details {...}` with its long parts.
 """
 from __future__ import annotations
 
@@ -1344,6 +1344,20 @@ def cpu_baseline(n, seconds_target=15.0):
                          "sample": f"{steps1} loop iterations in {el1:.1f} s"}}
 
 
+# what the result line leaves to the details line in front of it: some 30 KB, more than
+# the end of a captured output holds, which would cut the headline off
+DETAILS = ("df64_policy", "parity_vs_oracle", "workloads")
+
+
+def emit(line):
+    """Print the result: a line `details {...}` with the long parts, then the one JSON
+    line with everything else."""
+    details = {k: line[k] for k in DETAILS if k in line}
+    if details:
+        print("details " + json.dumps(details), flush=True)
+    print(json.dumps({k: v for k, v in line.items() if k not in DETAILS}), flush=True)
+
+
 def run_reference(args, ws, rank):
     if rank != 0:
         return
@@ -1580,7 +1594,7 @@ def run_ours(args, ws, rank, local):
         line["workloads"] = extras
     if not args.no_cpu_baseline:
         line["cpu_baseline"] = cpu_baseline(n)
-    print(json.dumps(line), flush=True)
+    emit(line)
 
 
 def main():
