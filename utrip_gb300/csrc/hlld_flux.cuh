@@ -338,7 +338,6 @@ __device__ __forceinline__ void hlld_flux_t(const HlldK &K, const double *L,
 // where the reference's branches with both sides formed took 12.3 ms.
 // A star state within zfloor of its singular denominator keeps the side's own
 // state (hlld_flux.f90:281-342), by selects.
-constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;
 __device__ __forceinline__ void hlld_flux_fast(const HlldK &K, const double *L,
                                                const double *R, double bx, double *f) {
   const double bb = bx * bx;
@@ -352,10 +351,13 @@ __device__ __forceinline__ void hlld_flux_fast(const HlldK &K, const double *L,
   const double c2r = (kr + fd::sqrt_(fma(btr, kr + hr, er * er))) * fd::rcp(R[0]);
   // max(cfl, cfr), min(vl, vr) and max(vl, vr) as Fortran's on NaNs: the right one unless
   // the left one compares.  Unsigned, a negative square or a NaN is beyond infinity.
-  const unsigned long long ul = (unsigned long long)__double_as_longlong(c2l);
-  const unsigned long long ur = (unsigned long long)__double_as_longlong(c2r);
-  const double cf = fd::sqrt_(0.5 * (ul <= kInfBits && ul > ur ? c2l : c2r));
-  const bool lt = fd::lt(L[2], R[2]), num = !(fd::is_nan(L[2]) || fd::is_nan(R[2]));
+  // (On the upper words: an operation gives quiet NaNs, above 0x7ff00000.)
+  auto up = [](double x) { return (unsigned)__double2hiint(x); };
+  const bool cl = up(c2l) <= 0x7ff00000u && (unsigned long long)__double_as_longlong(c2l) >
+                                                (unsigned long long)__double_as_longlong(c2r);
+  const double cf = fd::sqrt_(0.5 * (cl ? c2l : c2r));
+  const bool num = max(up(L[2]) & 0x7fffffffu, up(R[2]) & 0x7fffffffu) <= 0x7ff00000u;
+  const bool lt = fd::lt(L[2], R[2]);
   const double sl = (lt && num ? L[2] : R[2]) - cf, sr = (lt || !num ? R[2] : L[2]) + cf;
   // contact speed
   const double dl = sl - L[2], dr = sr - R[2];
@@ -364,9 +366,8 @@ __device__ __forceinline__ void hlld_flux_fast(const HlldK &K, const double *L,
   const double sm = (fma(mr, R[2], -ml * L[2]) + (ptl - ptr)) * fd::rcp(mr - ml);
   // the side of the face and whether it is supersonic
   // (neither for a NaN, which the star states then carry into every component)
-  const unsigned hsl = (unsigned)__double2hiint(sl), hsr = (unsigned)__double2hiint(sr);
-  const bool supl = hsl <= 0x7ff00000u;
-  const bool supr = !supl && (hsr - 0x80000000u <= 0x7ff00000u || sr == 0.0);
+  const bool supl = up(sl) <= 0x7ff00000u;
+  const bool supr = !supl && (up(sr) - 0x80000000u <= 0x7ff00000u || sr == 0.0);
   const bool right = !supl && (supr || __double2hiint(sm) < 0);
   const double ro = right ? R[0] : L[0], pr = right ? R[1] : L[1];
   const double vx = right ? R[2] : L[2], vy = right ? R[3] : L[3], vz = right ? R[4] : L[4];
