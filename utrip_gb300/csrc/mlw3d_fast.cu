@@ -446,12 +446,15 @@ __global__ void __launch_bounds__(T3F<TX, TY, G>::NT, MINB)
         const int v = iv0 + j;
         const VarFields q = kVar[v];
         const double *u = s0 + (size_t)v * T::NC;
-        // of field 0, unread, where the variable has no flux in the direction
-        const int qx = max(q.fx, 0), qy = max(q.fy, 0), qz_ = max(q.fz, 0);
-        const double *fx = s0 + qx * T::NC, *fy = s0 + qy * T::NC;
-        const double *kx_ = kk + max(q.kx, 0) * T::NK, *ky = kk + max(q.ky, 0) * T::NK;
-        const double *kz = kk + max(q.kz, 0) * T::NK;
-        const double *f0 = s0 + qz_ * T::NC, *f1 = s1 + qz_ * T::NC;
+        // the variable's fluxes at cell offset d and at the corners; called only where it
+        // has one in the direction
+        auto fx = [&](int d) { return s0[q.fx * T::NC + d]; };
+        auto fy = [&](int d) { return s0[q.fy * T::NC + d]; };
+        auto kx_ = [&](int d) { return kk[q.kx * T::NK + d]; };
+        auto ky = [&](int d) { return kk[q.ky * T::NK + d]; };
+        auto kz = [&](int d) { return kk[q.kz * T::NK + d]; };
+        auto f0 = [&]() { return s0[q.fz * T::NC]; };
+        auto f1 = [&]() { return s1[q.fz * T::NC]; };
         const double gxl = q.fx >= 0 ? ret(8 + q.rx) : 0.0, gyl = q.fy >= 0 ? ret(15 + q.ry) : 0.0;
         const double pl = ret(v);
         const double w = qz * (s1[(size_t)v * T::NC] - u[0]);
@@ -463,13 +466,13 @@ __global__ void __launch_bounds__(T3F<TX, TY, G>::NT, MINB)
           bool sp = false;
           const float ez0 = az.e0[k], ez1 = az.e1[k];
           if (q.fx >= 0)
-            tx = isum::diff_planes(kx_[0], kx_[1], kx_[T::KX], kx_[T::KX + 1], gxl, fx[-1], fx[1],
+            tx = isum::diff_planes(kx_(0), kx_(1), kx_(T::KX), kx_(T::KX + 1), gxl, fx(-1), fx(1),
                                    ey0, ey1, ez0, ez1, gx, sp);
           if (q.fy >= 0)
-            ty = isum::diff_planes(ky[0], ky[T::KX], ky[1], ky[T::KX + 1], gyl, fy[-T::CX],
-                                   fy[T::CX], ex0, ex1, ez0, ez1, gy, sp);
+            ty = isum::diff_planes(ky(0), ky(T::KX), ky(1), ky(T::KX + 1), gyl, fy(-T::CX),
+                                   fy(T::CX), ex0, ex1, ez0, ez1, gy, sp);
           if (q.fz >= 0)
-            tz = isum::face_planes(kz[0], kz[1], kz[T::KX], kz[T::KX + 1], f0[0], f1[0], w, pl,
+            tz = isum::face_planes(kz(0), kz(1), kz(T::KX), kz(T::KX + 1), f0(), f1(), w, pl,
                                    q.sz < 0, ex0, ex1, ey0, ey1, pu, sp);
           else
             tz = w - pl;
@@ -487,17 +490,17 @@ __global__ void __launch_bounds__(T3F<TX, TY, G>::NT, MINB)
         } else {
           const double uz0 = 2.0 * az.u0[k], uz1 = 2.0 * az.u1[k];
           if (q.fx >= 0) {
-            gx = fma(2.0 * uy1, kx_[T::KX + 1] - kx_[T::KX], 2.0 * uy0 * (kx_[1] - kx_[0]));
-            tx = fma(16.0, fx[1] - fx[-1], fma(uz1, gx, uz0 * gxl));
+            gx = fma(2.0 * uy1, kx_(T::KX + 1) - kx_(T::KX), 2.0 * uy0 * (kx_(1) - kx_(0)));
+            tx = fma(16.0, fx(1) - fx(-1), fma(uz1, gx, uz0 * gxl));
           }
           if (q.fy >= 0) {
-            gy = fma(2.0 * ux1, ky[T::KX + 1] - ky[1], 2.0 * ux0 * (ky[T::KX] - ky[0]));
-            ty = fma(16.0, fy[T::CX] - fy[-T::CX], fma(uz1, gy, uz0 * gyl));
+            gy = fma(2.0 * ux1, ky(T::KX + 1) - ky(1), 2.0 * ux0 * (ky(T::KX) - ky(0)));
+            ty = fma(16.0, fy(T::CX) - fy(-T::CX), fma(uz1, gy, uz0 * gyl));
           }
           if (q.fz >= 0) {
-            const double s = fma(2.0 * uy1, fma(2.0 * ux1, kz[T::KX + 1], 2.0 * ux0 * kz[T::KX]),
-                                 2.0 * uy0 * fma(2.0 * ux1, kz[1], 2.0 * ux0 * kz[0]));
-            pu = fma(q.sz < 0 ? -1.0 : 1.0, fma(16.0, f0[0] + f1[0], s), w);
+            const double s = fma(2.0 * uy1, fma(2.0 * ux1, kz(T::KX + 1), 2.0 * ux0 * kz(T::KX)),
+                                 2.0 * uy0 * fma(2.0 * ux1, kz(1), 2.0 * ux0 * kz(0)));
+            pu = fma(q.sz < 0 ? -1.0 : 1.0, fma(16.0, f0() + f1(), s), w);
           }
           tz = pu - pl;
         }
