@@ -70,8 +70,8 @@ def parse():
     p.add_argument("--profile-case", default=None,
                    choices=["mlw3d", "roe3d", "hlld3d", "adjoint2d", "batch", "roe2d",
                             "gravity2d", "resistive2d", "gravity3d", "resistive3d",
-                            "spicule", "spicule_group", "single", "mlw2d", "mlw2d_df",
-                            "mlw3d_df"],
+                            "spicule", "spicule_group", "tube", "single", "mlw2d",
+                            "mlw2d_df", "mlw3d_df"],
                    help="run one small fixed case of a secondary path (for ncu) and exit")
     return p.parse_args()
 
@@ -93,8 +93,8 @@ def profile_case(case, n, tile=-1, df64=False):
         st = run.query()
         run.close()
         out = {"case": case, "n": n, "steps": int(st.nexec), "merr": int(st.merr)}
-    elif case == "spicule":
-        s = setups.spicule_1d(n)
+    elif case in ("spicule", "tube"):
+        s = setups.spicule_1d(n) if case == "spicule" else setups.shock_tube_1d(n)
         run = drivers.make_run(s, df64=df64)
         run.push(s["state"])
         run.start(nstop=200, tend=s["tend"], safety=s["safety"], dtmin=s["dtmin"])

@@ -1710,8 +1710,8 @@ double *mapped_array(double *p, size_t n) {
 // The nvar arrays of n doubles between host and device, on stream s.  A small state
 // in page-locked arrays goes in one launch that reads or writes them in place: a
 // copy costs some 4 us of the host each, whatever its size (64 runs of five arrays of
-// 1026, a run: push 34 -> 16 us, start 21 -> 10, pull 41 -> 28, with the wait left
-// out above); beyond 1 MB the copy engine's rate counts.
+// 1026, a run, with the control block left unread: push 34 -> 16 us, start 21 -> 15, of
+// which it waits for the push, pull 41 -> 25); beyond 1 MB the copy engine's rate counts.
 constexpr int kMaxVars = 16;
 struct HostArrays {
   double *p[kMaxVars];

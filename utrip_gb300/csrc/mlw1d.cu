@@ -23,10 +23,11 @@
 // (the cluster barrier, remote and L2 accesses).  So the profiles are read through
 // the read-only cache (a barrier does not empty it), the loop's constants are read
 // once, minima are integer minima, halos and minima are written into the blocks that
-// need them (only such boundary rules read another block's cells), and the plain step's arithmetic takes the fewest FP64 instructions (f1 below) and is shared
-// out to idle warps where a block has some: a step of 1024 cells on 16 blocks 12.9 ->
-// 6.9 us, 64 spicule runs 50 -> 47 us (those are
-// bound by the FP64 pipe: 512 cells a SM).
+// need them (only the rules above read another block's cells), and the plain step's
+// arithmetic takes the fewest FP64 instructions (f1 below) and is shared out to idle
+// warps where a block has some: a step of 1024 cells on 16 blocks 12.9 -> 6.9 us, 64
+// spicule runs 51 -> 45 us in launches of 100 steps (those are bound by the FP64 pipe:
+// 512 cells a SM).
 //
 // The BG variant is mlw_m_bg (cans1d/hdmlw/mlw_m_bg.f:2-271): the same
 // two-stage step on the cross-section-weighted variables (ro, e, rx, ry r,
